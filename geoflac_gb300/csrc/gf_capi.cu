@@ -152,8 +152,6 @@ void fill_params(DevParams &P, const gf_params &p) {
         double den_el = 3.0 * lambda + 2.0 * p.rm[k];
         if (std::fabs(den_el) < 1e-30) den_el = den_el < 0.0 ? -1e-30 : 1e-30;
         P.sh_lam_den[k] = lambda / den_el;
-        P.sh_r2mu_y[k] = 1.0 / (2.0 * p.rm[k]);
-        P.sh_r2mu_yl[k] = std::fma(-P.sh_r2mu_y[k], 2.0 * p.rm[k], 1.0) * P.sh_r2mu_y[k];
     }
     P.f_fmagma_max = (float)p.fmagma_max;
     P.topo_kappa = p.topo_kappa;

@@ -228,52 +228,92 @@ __device__ __forceinline__ long long gf_rcp_sig(unsigned mhi, unsigned lo) {
     const long long Dp = -(long long)(M * (unsigned long long)(2 * t + 1));
     return t + (Dp > 0 ? 1 : (Dp + (long long)(2 * M) < 0 ? -1 : 0));
 }
-__device__ __forceinline__ double gf_rcp(double b) {
+// -x on the integer pipe
+__device__ __forceinline__ double gf_neg(double x) {
     unsigned lo, hi;
-    gf_dsplit(b, lo, hi);
-    const unsigned E = (hi >> 20) & 0x7ffu;
-    if (E - 573u > 900u) return gf_rcp_rare(b);
-    const unsigned sign = hi & 0x80000000u, mhi = hi & 0xfffffu;
-    if ((mhi | lo) == 0u) return gf_djoin(0u, sign | ((2046u - E) << 20));
-    const unsigned long long bits = ((unsigned long long)(2044u - E) << 52) + (unsigned long long)gf_rcp_sig(mhi, lo);
-    return gf_djoin((unsigned)bits, (unsigned)(bits >> 32) | sign);
+    gf_dsplit(x, lo, hi);
+    return gf_djoin(lo, hi ^ 0x80000000u);
 }
 
 // RN(a/b) without the FP64 pipe, for a zero or inside gf_dmid and b inside
 // gf_dmid (others take the IEEE division out of line).  With significands
 // Ma, Mb, the quotient's significand is RN(Q), Q = Ma 2^k / Mb in
-// [2^52, 2^53) (k = 52 if Ma >= Mb, else 53): q = floor(Ma t / 2^(105-k))
-// from t = RN(2^105 / Mb) lies within 2 of Q; the exact residual
-// Ma 2^k - Mb q (below 2^55 in magnitude, so its low 64 bits are exact)
-// brings q to floor(Q) with at most two steps each way, and 2 (residual) >
-// Mb rounds it up (no ties: a quotient of two 53-bit significands is never
-// halfway between two 53-bit values).  Restated on words and checked
+// [2^52, 2^53) (k = 52 if Ma >= Mb, else 53): Ma t / 2^(105-k) from t =
+// RN(2^105 / Mb) lies within Ma / 2^(106-k) < 1 of Q, so q, its value
+// rounded to an integer, lies within 3/2 of Q and RN(Q) is q - 1, q or q + 1;
+// twice the exact residual Ma 2^k - Mb q (below 2^55, so its low 64 bits
+// are exact) against +-Mb decides (no ties: a quotient of two 53-bit
+// significands is never halfway between two 53-bit values).  Restated on words and checked
 // against IEEE division by tests/test_int_reciprocal.py.
 __device__ __noinline__ double gf_ddiv_rare(double a, double b) { return a / b; }
-__device__ __forceinline__ double gf_ddiv(double a, double b) {
+// The denominator's part of gf_ddiv, for quotients that share it: its
+// significand, t = RN(2^105 / Mb) and whether b lies inside gf_dmid.
+struct GfIntRecip {
+    double b;
+    unsigned long long t;
+};
+__device__ __forceinline__ GfIntRecip gf_int_recip(double b) {
+    unsigned lb, hb;
+    gf_dsplit(b, lb, hb);
+    return GfIntRecip{b, (unsigned long long)gf_rcp_sig(hb & 0xfffffu, lb)};
+}
+__device__ __forceinline__ double gf_ddiv_by(double a, const GfIntRecip &r) {
     unsigned la, ha, lb, hb;
     gf_dsplit(a, la, ha);
-    gf_dsplit(b, lb, hb);
+    gf_dsplit(r.b, lb, hb);
     const unsigned Ea = (ha >> 20) & 0x7ffu, Eb = (hb >> 20) & 0x7ffu;
     const bool za = ((ha << 1) | la) == 0u;
-    if (!((Ea - 573u <= 900u || za) && Eb - 573u <= 900u)) return gf_ddiv_rare(a, b);
+    if (!((Ea - 573u <= 900u || za) && Eb - 573u <= 900u)) return gf_ddiv_rare(a, r.b);
     const unsigned sign = (ha ^ hb) & 0x80000000u;
     if (za) return gf_djoin(0u, sign);
     const unsigned long long Ma = ((unsigned long long)((ha & 0xfffffu) | 0x100000u) << 32) | la;
     const unsigned long long Mb = ((unsigned long long)((hb & 0xfffffu) | 0x100000u) << 32) | lb;
-    const unsigned long long t = (unsigned long long)gf_rcp_sig(hb & 0xfffffu, lb);
+    const unsigned long long t = r.t;
     const int k = Ma >= Mb ? 52 : 53;
-    unsigned long long q = (__umul64hi(Ma, t) << (k - 41)) | ((Ma * t) >> (105 - k));
-    long long res = (long long)((Ma << k) - Mb * q);
-    if (res < 0) { --q; res += (long long)Mb; }
-    if (res < 0) { --q; res += (long long)Mb; }
-    if (res >= (long long)Mb) { ++q; res -= (long long)Mb; }
-    if (res >= (long long)Mb) { ++q; res -= (long long)Mb; }
-    q += 2 * res > (long long)Mb ? 1u : 0u;
+    unsigned long long q = (__umul64hi(Ma, t) << (k - 41)) + ((((Ma * t) >> (104 - k)) + 1) >> 1);
+    const long long res = 2 * (long long)((Ma << k) - Mb * q);
+    q += res > (long long)Mb ? 1 : (res < -(long long)Mb ? -1 : 0);
     const unsigned long long bits = ((unsigned long long)(1074 - k + (int)Ea - (int)Eb) << 52) + q;
     return gf_djoin((unsigned)bits, (unsigned)(bits >> 32) | sign);
 }
+__device__ __forceinline__ double gf_ddiv(double a, double b) { return gf_ddiv_by(a, gf_int_recip(b)); }
+// RN(1/b) from the same part
+__device__ __forceinline__ double gf_rcp_by(const GfIntRecip &r) {
+    unsigned lo, hi;
+    gf_dsplit(r.b, lo, hi);
+    const unsigned E = (hi >> 20) & 0x7ffu;
+    if (E - 573u > 900u) return gf_rcp_rare(r.b);
+    const unsigned sign = hi & 0x80000000u;
+    if (((hi & 0xfffffu) | lo) == 0u) return gf_djoin(0u, sign | ((2046u - E) << 20));
+    const unsigned long long bits = ((unsigned long long)(2044u - E) << 52) + r.t;
+    return gf_djoin((unsigned)bits, (unsigned)(bits >> 32) | sign);
+}
+__device__ __forceinline__ double gf_rcp(double b) { return gf_rcp_by(gf_int_recip(b)); }
 __device__ __forceinline__ float gf_ddiv(float a, float b) { return a / b; }
+
+// gf_mul for kernels with many products (the rheology): a zero operand takes
+// the FP64 multiply out of line as well, which leaves one range test for
+// both operands and no select on the result (38 -> 30 instructions)
+__device__ __forceinline__ double gf_mulq(double a, double b) {
+    unsigned la, ha, lb, hb;
+    gf_dsplit(a, la, ha);
+    gf_dsplit(b, lb, hb);
+    if (max(ha * 2u - (573u << 21), hb * 2u - (573u << 21)) >= (901u << 21)) return gf_mul_rare(a, b);
+    const unsigned mh = (ha & 0xfffffu) | 0x100000u, nh = (hb & 0xfffffu) | 0x100000u;
+    const unsigned long long p0 = (unsigned long long)la * lb;
+    unsigned long long t = (unsigned long long)la * nh + (p0 >> 32);
+    t += (unsigned long long)mh * lb;
+    const unsigned long long u = (unsigned long long)mh * nh + (t >> 32);
+    const unsigned w2 = (unsigned)(u >> 32), w1 = (unsigned)u, w0 = (unsigned)t, wm = (unsigned)p0;
+    const unsigned top = w2 >> 9, sh = 12u - top;
+    const unsigned mhi = __funnelshift_l(w1, w2, sh), mlo = __funnelshift_l(w0, w1, sh);
+    const unsigned rem = w0 << sh, x = min(wm, 1u) | (mlo & 1u);
+    const unsigned up = (rem + x) > 0x80000000u ? 1u : 0u;
+    const unsigned S = (ha & 0xfff00000u) + (hb & 0xfff00000u) - (1024u << 20) + (top << 20);
+    const unsigned long long r = ((unsigned long long)(mhi + S) << 32 | mlo) + up;
+    return gf_djoin((unsigned)r, (unsigned)(r >> 32));
+}
+__device__ __forceinline__ float gf_mulq(float a, float b) { return a * b; }
 
 // x * 2^K (K = -2 .. 2, the constant factors 0.25 .. 4 of the step): the
 // exponent field moves by K while x and the result are normal doubles, a
@@ -357,52 +397,6 @@ __device__ __forceinline__ bool gf_ratio_below_cut(double r) {
     const unsigned long long cut = (unsigned long long)__double_as_longlong(0.01);
     if ((b & 0x7fffffffffffffffull) > 0x7ff0000000000000ull) return false;
     return (b >> 63) ? true : b < cut;
-}
-
-// Division by a shared denominator with the bits of IEEE division.  For a
-// denominator b: y = RN(1/b) (one IEEE division) and yl = RN(RN(1 - b y) y),
-// so that y + yl is 1/b to 2^-105 relative (1 - b y is exact in an FMA).
-// Each quotient a / b then costs one multiply and three FMAs:
-//   q = RN(a y + RN(a yl))   within 0.5 ulp + 2^-104 |a/b|: faithful,
-//   r = a - b q              exact in an FMA because q is faithful,
-//   RN(q + r y)              = RN(a/b) by Markstein's theorem (a faithful
-//                            quotient and the correctly rounded reciprocal;
-//                            P. Markstein, IBM J. Res. Dev. 34 (1990) 111-119).
-// Operands outside gf_dmid take an IEEE division; a zero numerator gives
-// a * y, the signed zero of IEEE division.  Restated in exact arithmetic and
-// checked against IEEE division (random and near-midpoint quotients) by
-// tests/test_division.py.
-struct GfRecip {
-    double b, y, yl;
-    bool ok;
-};
-__device__ __forceinline__ GfRecip gf_recip_y(double b, double y) { // y = 1.0 / b
-    GfRecip r;
-    r.b = b;
-    r.y = y;
-    r.yl = fma(-y, b, 1.0) * y;
-    r.ok = gf_dmid(b);
-    return r;
-}
-// a pair computed ahead (y = RN(1/b) exactly; yl need only be near (1 - b y) y)
-__device__ __forceinline__ GfRecip gf_recip_pre(double b, double y, double yl) {
-    GfRecip r;
-    r.b = b;
-    r.y = y;
-    r.yl = yl;
-    r.ok = gf_dmid(b);
-    return r;
-}
-// (out of line, so that the common path issues none of its FP64 instructions)
-__device__ __noinline__ double gf_div_rare(double a, double b, double y, bool ok) {
-    return (ok && gf_dzero(a)) ? a * y : a / b;
-}
-// IMUL: the product a * yl on the integer pipes (gf_mul), for kernels small
-// enough that its thirty instructions cost less than the FP64 slot
-template <bool IMUL = false> __device__ __forceinline__ double gf_div(double a, const GfRecip &r) {
-    if (!(r.ok && gf_dmid(a))) return gf_div_rare(a, r.b, r.y, r.ok);
-    const double q = fma(a, r.y, IMUL ? gf_mul(a, r.yl) : a * r.yl);
-    return fma(fma(-q, r.b, a), r.y, q);
 }
 
 // x = hi + lo with hi = float(x): the hi/lo split of the mixed path
@@ -781,10 +775,10 @@ __device__ __forceinline__ void maxwell(R bulkm, const MaxwellConsts<R> &m, R &s
         s33d = s33 - s0;
     }
     const R rmu2 = gf_scale<1>(rmu);
-    s11d = (s11d * vic1 + rmu2 * de11d) * vic2;
-    s22d = (s22d * vic1 + rmu2 * de22d) * vic2;
-    s12 = (s12 * vic1 + rmu2 * de12) * vic2;
-    s0 = s0 + bulkm * dv;
+    s11d = gf_mulq(gf_mulq(s11d, vic1) + gf_mulq(rmu2, de11d), vic2);
+    s22d = gf_mulq(gf_mulq(s22d, vic1) + gf_mulq(rmu2, de22d), vic2);
+    s12 = gf_mulq(gf_mulq(s12, vic1) + gf_mulq(rmu2, de12), vic2);
+    s0 = s0 + gf_mulq(bulkm, dv);
     s11 = s11d + s0;
     s22 = s22d + s0;
     if constexpr (sizeof(R) == sizeof(double)) {
@@ -872,10 +866,10 @@ __device__ __forceinline__ void plastic(const PlasticConsts<R> &c, R rmu, R &dep
     R e1 = c.e1, e2 = c.e2, anphi = c.anphi, anpsi = c.anpsi, ten_max = c.ten_max;
     // (de33 is +0 in plane strain: gf_add_z / gf_mul_z take it on the
     // integer pipes)
-    R s11i = s11 + gf_add_z(de22, de33) * e2 + de11 * e1;
-    R s22i = s22 + gf_add_z(de11, de33) * e2 + de22 * e1;
-    R s12i = s12 + gf_scale<1>(de12) * rmu;
-    R s33i = gf_add_z(s33 + (de11 + de22) * e2, gf_mul_z(de33, e1));
+    R s11i = s11 + gf_mulq(gf_add_z(de22, de33), e2) + gf_mulq(de11, e1);
+    R s22i = s22 + gf_mulq(gf_add_z(de11, de33), e2) + gf_mulq(de22, e1);
+    R s12i = s12 + gf_mulq(gf_scale<1>(de12), rmu);
+    R s33i = gf_add_z(s33 + gf_mulq(de11 + de22, e2), gf_mul_z(de33, e1));
     if constexpr (sizeof(R) == sizeof(double)) {
         if (plastic_keeps_trial(c, s11i, s22i, s12i)) {
             s11 = s11i; s22 = s22i; s33 = s33i; s12 = s12i;
@@ -1103,6 +1097,19 @@ __device__ __forceinline__ void pre_plast(const DevParams &P, const DevArrays &A
 // the table holds the values the element path computes, from the same
 // functions on the same inputs; other elements (mixed phases, strain
 // inside the softening interval, melt weakening) take the element path.
+template <class R> __device__ __forceinline__ int plastic_branch(const DevParams &P, int iph, R pls) {
+    R pl1, pl2;
+    if constexpr (sizeof(R) == sizeof(float)) {
+        pl1 = P.f_pl1[iph]; pl2 = P.f_pl2[iph];
+        if (pls < pl1) return 0;
+        if (pls < pl2) return __float_as_uint(pls) == __float_as_uint(pl1) ? 1 : -1;
+    } else {
+        pl1 = P.plstrain1[iph]; pl2 = P.plstrain2[iph];
+        if (pls < pl1) return 0;
+        if (pls < pl2) return __double_as_longlong(pls) == __double_as_longlong(pl1) ? 1 : -1;
+    }
+    return 2;
+}
 template <class R>
 __device__ __forceinline__ int plastic_table_state(const DevParams &P, const DevArrays &A, const GfDims &d, GF_IDX e,
                                                    int iph, R pls) {
@@ -1115,17 +1122,7 @@ __device__ __forceinline__ int plastic_table_state(const DevParams &P, const Dev
             return -1;
         }
     }
-    R pl1, pl2;
-    if constexpr (sizeof(R) == sizeof(float)) {
-        pl1 = P.f_pl1[iph]; pl2 = P.f_pl2[iph];
-        if (pls < pl1) return 0;
-        if (pls < pl2) return __float_as_uint(pls) == __float_as_uint(pl1) ? 1 : -1;
-    } else {
-        pl1 = P.plstrain1[iph]; pl2 = P.plstrain2[iph];
-        if (pls < pl1) return 0;
-        if (pls < pl2) return __double_as_longlong(pls) == __double_as_longlong(pl1) ? 1 : -1;
-    }
-    return 2;
+    return plastic_branch(P, iph, pls);
 }
 
 } // namespace gfk

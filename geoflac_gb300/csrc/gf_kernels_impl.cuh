@@ -3,15 +3,6 @@
 
 #include "gf_kernels.cuh"
 
-// resident CTAs per SM the register allocation of k_rheol is sized for:
-// 2 for FP64 (128 registers; its spills cost less than the latency that 16
-// warps per SM hide: 0.703 -> 0.678 ms against 255 registers and 8 warps),
-// 3 for the mixed path (80 registers; its few spills cost less than the
-// occupancy they buy)
-#ifndef GF_RHEOL_MINB
-#define GF_RHEOL_MINB (sizeof(R) == sizeof(float) ? 3 : 2)
-#endif
-
 // internal linkage: each precision's translation unit has its own copy
 namespace {
 namespace gfk {
@@ -25,7 +16,7 @@ __device__ __forceinline__ void node_ji(const GfDims &d, GF_IDX n, int &j, int &
     j = (int)(n - (GF_IDX)i * d.nz);
 }
 
-inline unsigned grid_for(GF_IDX n) { return (unsigned)((n + GF_THREADS - 1) / GF_THREADS); }
+inline unsigned grid_for(GF_IDX n, int threads = GF_THREADS) { return (unsigned)((n + threads - 1) / threads); }
 
 // ======================================================================
 // Mixed path: the element's share of the node forces of fl_node.f90.  For
@@ -65,7 +56,8 @@ __device__ __forceinline__ void elem_corner_forces(const float dx[3][4], const f
 }
 
 // ======================================================================
-// fl_rheol (fl_rheol.f90:4-389): one thread per element.
+// fl_rheol (fl_rheol.f90:4-389) in the mixed path: one thread per element
+// (the FP64 path: k_rheol_tri).
 template <class R> __device__ __forceinline__ void b_k_rheol(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d, int update_visc, int nloop, GF_IDX e) {
     if (e >= d.E) return;
     const DevParams &P = *Pp;
@@ -77,12 +69,12 @@ template <class R> __device__ __forceinline__ void b_k_rheol(const DevParams *__
     R *st = (R *)A.stress0;
     const R *area = (const R *)A.area;
 
-    GF_IDX n1 = gf_node(d, j, i), n3 = gf_node(d, j, i + 1);
+    GF_IDX n1 = gf_node(d, j, i);
     R vx[4], vy[4];
     R ar[4];
     for (int k = 0; k < 4; ++k) ar[k] = area[gf_ek(d, e, k)];
     R dx[3][4], dz[3][4], sr[3][4];
-    if constexpr (sizeof(R) == sizeof(float)) {
+    {
         // FP32 from the hi/lo splits: coordinates and velocities relative to
         // the quad's node 1 (each triangle's shape derivatives sum to zero,
         // so a common velocity offset drops out of the strain rates)
@@ -90,13 +82,6 @@ template <class R> __device__ __forceinline__ void b_k_rheol(const DevParams *__
         load_vel_rel(A, d, j, i, vx, vy);
         load_quad_rel(A, d, j, i, qf);
         shape_derivs_f(qf, ar, dx, dz);
-    } else {
-        const double *vel = A.vel;
-        vx[0] = R(vel[n1]); vx[1] = R(vel[n1 + 1]); vx[2] = R(vel[n3]); vx[3] = R(vel[n3 + 1]);
-        vy[0] = R(vel[d.N + n1]); vy[1] = R(vel[d.N + n1 + 1]); vy[2] = R(vel[d.N + n3]); vy[3] = R(vel[d.N + n3 + 1]);
-        Quad q;
-        load_quad(A.cord, d, j, i, q);
-        shape_derivs<R>(q, ar, dx, dz);
     }
     // node triplets of triangles A,B,C,D: (1,2,3), (3,2,4), (1,2,4), (1,4,3)
     const int tn[4][3] = {{0, 1, 2}, {2, 1, 3}, {0, 1, 3}, {0, 3, 2}};
@@ -146,22 +131,14 @@ template <class R> __device__ __forceinline__ void b_k_rheol(const DevParams *__
 
     int iph = A.iphase[e] - 1;
     int irh = P.irheol[iph];
-    R bulkm, rmu;
-    if constexpr (sizeof(R) == sizeof(float)) {
-        bulkm = P.f_bulkm[iph];
-        rmu = P.f_rm[iph];
-    } else {
-        bulkm = R(P.bulkm[iph]);
-        rmu = R(P.rm[iph]);
-    }
+    const R bulkm = P.f_bulkm[iph], rmu = P.f_rm[iph];
     R stherm = R(0.0);
     if (P.istress_therm > 0)
         stherm = R(-P.alfa[iph] * P.bulkm[iph] * (A.temp[n1] - A.temp0[n1]));
     R *aps = (R *)A.aps;
     R aps_e = aps[e];
     // mixed path: stored normal stresses are deviations from -pref
-    R pref = R(0);
-    if constexpr (sizeof(R) == sizeof(float)) pref = A.pr_hi[e]; // == float(p_ref)
+    const R pref = A.pr_hi[e]; // == float(p_ref)
     R hardn = 0;
     PlasticConsts<R> pc;
     if (irh == 6 || irh >= 11) {
@@ -176,8 +153,7 @@ template <class R> __device__ __forceinline__ void b_k_rheol(const DevParams *__
         } else {
             R coh = 0, phi = 0, psi = 0;
             pre_plast<R>(P, A, d, e, aps_e, coh, phi, psi, hardn);
-            pc = plastic_consts<R>(bulkm, rmu, coh, phi, psi,
-                                   sizeof(R) == sizeof(float) ? R(P.f_ten_off) : R(P.ten_off));
+            pc = plastic_consts<R>(bulkm, rmu, coh, phi, psi, P.f_ten_off);
         }
     }
     R *visn = (R *)A.visn;
@@ -221,10 +197,8 @@ template <class R> __device__ __forceinline__ void b_k_rheol(const DevParams *__
                         m);
             plas_mod = plas_mod || m;
             maxwell<R>(bulkm, mc, sv[0][k], sv[1][k], sv[3][k], sv[2][k], de11, de22, de33, de12, dv, P.ndim);
-            if (sizeof(R) == sizeof(float)) {
-                sumD = sumD + (de11 - de22);
-                sumD12 = sumD12 + de12;
-            }
+            sumD = sumD + (de11 - de22);
+            sumD12 = sumD12 + de12;
         }
     }
     if (!ok) set_status(C, 22, (int)e);
@@ -238,7 +212,7 @@ template <class R> __device__ __forceinline__ void b_k_rheol(const DevParams *__
         b = sv[2][0] + sv[2][1] + sv[2][2] + sv[2][3];
         R sII_visc = a * a + gf_scale<2>(b * b);
         use_visc = !(sII_plas < sII_visc);
-        if (sizeof(R) == sizeof(float) && !plas_mod) {
+        if (!plas_mod) {
             R pa = sp[0][0] + sp[0][1] + sp[0][2] + sp[0][3] - sp[1][0] - sp[1][1] - sp[1][2] - sp[1][3];
             R pb = sp[2][0] + sp[2][1] + sp[2][2] + sp[2][3];
             R S = s0v[0][0] + s0v[0][1] + s0v[0][2] + s0v[0][3] - s0v[1][0] - s0v[1][1] - s0v[1][2] - s0v[1][3];
@@ -251,30 +225,14 @@ template <class R> __device__ __forceinline__ void b_k_rheol(const DevParams *__
     for (int k = 0; k < 4; ++k)
 #pragma unroll
         for (int c = 0; c < 4; ++c) sn[c][k] = use_visc ? sv[c][k] : sp[c][k];
-    // FP64: the reciprocals 1/ar of the stress mixing and the node-force
-    // factors 0.25/ar, one IEEE division per triangle
-    R rar[4];
-    if constexpr (sizeof(R) == sizeof(double)) {
-        if (P.mix_stress == 1 || A.n_frc) {
-#pragma unroll
-            for (int t = 0; t < 4; ++t) rar[t] = gf_rcp(ar[t]); // RN(1/ar) off the FP64 pipe
-        }
-    }
     if (P.mix_stress == 1) {
 #pragma unroll
         for (int h = 0; h < 4; h += 2) {
             R ra = ar[h], rb = ar[h + 1];
             R s0a = gf_scale<-1>(sn[0][h] + sn[1][h]);
             R s0b = gf_scale<-1>(sn[0][h + 1] + sn[1][h + 1]);
-            R s0;
-            if constexpr (sizeof(R) == sizeof(double)) {
-                const GfRecip qa = gf_recip_y(ra, rar[h]), qb = gf_recip_y(rb, rar[h + 1]);
-                R quad_area = qa.y + qb.y;
-                s0 = gf_ddiv(gf_div(s0a, qb) + gf_div(s0b, qa), quad_area);
-            } else {
-                R quad_area = R(1.0) / ra + R(1.0) / rb;
-                s0 = (s0a / rb + s0b / ra) / quad_area;
-            }
+            R quad_area = R(1.0) / ra + R(1.0) / rb;
+            R s0 = (s0a / rb + s0b / ra) / quad_area;
             sn[0][h] = sn[0][h] - s0a + s0;
             sn[1][h] = sn[1][h] - s0a + s0;
             sn[0][h + 1] = sn[0][h + 1] - s0b + s0;
@@ -291,33 +249,7 @@ template <class R> __device__ __forceinline__ void b_k_rheol(const DevParams *__
     for (int k = 0; k < 4; ++k)
 #pragma unroll
         for (int c = 0; c < 4; ++c) st[gf_s(d, e, c, k)] = sn[c][k];
-    if constexpr (sizeof(R) == sizeof(double)) {
-        // fl_node's force terms of this element (fl_node.f90:50-254), each
-        // the expression the node gather evaluates, from the stresses just
-        // stored: the node kernel then sums them in the reference's order
-        // instead of recomputing four elements' shape derivatives and twelve
-        // divisions per node (the mesh does not move before fl_node)
-        if (A.n_frc) {
-            const int kk[4][3] = {{1, 2, 3}, {0, 1, 2}, {0, 1, 3}, {0, 2, 3}};
-            const int mm[4][3] = {{2, 2, 1}, {1, 1, 1}, {2, 0, 2}, {0, 0, 0}};
-            double *nf = A.n_frc;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int qd = 3 - c;
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const int t = kk[qd][k], m = mm[qd][k];
-                    // 0.25 * RN(1/ar) == RN(0.25/ar) while both are normal
-                    R factor = gf_dmid(ar[t]) ? gf_scale<-2>(rar[t]) : R(0.25) / ar[t];
-                    R fx = factor * (sn[0][t] * dx[m][t] + sn[2][t] * dz[m][t]);
-                    R fy = factor * (sn[2][t] * dx[m][t] + sn[1][t] * dz[m][t]);
-                    nf[(GF_IDX)(6 * c + 2 * k) * d.E + e] = fx;
-                    nf[(GF_IDX)(6 * c + 2 * k + 1) * d.E + e] = fy;
-                }
-            }
-        }
-    }
-    if constexpr (sizeof(R) == sizeof(float)) {
+    {
         // the node gather's corner forces of the new stresses (the mesh does
         // not move before fl_node); shape derivatives taken again rather than
         // kept live through the stress update
@@ -331,85 +263,47 @@ template <class R> __device__ __forceinline__ void b_k_rheol(const DevParams *__
         R quad_area = ar[0] + ar[1] + ar[2] + ar[3];
         aps_e = aps_e + gf_ddiv(depl[0] * ar[0] + depl[1] * ar[1] + depl[2] * ar[2] + depl[3] * ar[3], quad_area);
         if (aps_e < R(0.0)) aps_e = R(0.0);
-        if constexpr (sizeof(R) == sizeof(float)) {
-            if (P.f_tau_heal != 0.0f) aps_e = aps_e / (1.0f + dt / P.f_tau_heal);
-        } else {
-            if (P.tau_heal != 0.0) aps_e = aps_e / (R(1.0) + dt / R(P.tau_heal));
-        }
+        if (P.f_tau_heal != 0.0f) aps_e = aps_e / (1.0f + dt / P.f_tau_heal);
         aps[e] = aps_e;
     }
     // accumulates the element-averaged start-of-step stress (s11/s22/s12 are
     // reassigned before this point in fl_rheol.f90:181-183)
     R *strain = (R *)A.strain;
-    if (sizeof(R) == sizeof(float)) { // total stress, not the stored deviation
-        s11 = s11 - pref;
-        s22 = s22 - pref;
-    }
+    s11 = s11 - pref; // total stress, not the stored deviation
+    s22 = s22 - pref;
     strain[gf_ek(d, e, 0)] = strain[gf_ek(d, e, 0)] + s11 * dt;
     strain[gf_ek(d, e, 1)] = strain[gf_ek(d, e, 1)] + s22 * dt;
     strain[gf_ek(d, e, 2)] = strain[gf_ek(d, e, 2)] + s12 * dt;
     if (P.ishearh == 1) {
         R qsum = R(0.0);
-        if constexpr (sizeof(R) == sizeof(float)) {
-            R lambda = bulkm - R(2.0 / 3.0) * rmu, mu = rmu;
-            R den_el = R(3.0) * lambda + R(2.0) * mu;
-            if (m_abs(den_el) < R(1e-30)) den_el = den_el < R(0) ? R(-1e-30) : R(1e-30);
-            // the same elastic-strain differences with one reciprocal and the
-            // stress changes taken first
-            const float lamr = lambda / den_el, inv2mu = 1.0f / (2.0f * mu);
+        R lambda = bulkm - R(2.0 / 3.0) * rmu, mu = rmu;
+        R den_el = R(3.0) * lambda + R(2.0) * mu;
+        if (m_abs(den_el) < R(1e-30)) den_el = den_el < R(0) ? R(-1e-30) : R(1e-30);
+        // the same elastic-strain differences with one reciprocal and the
+        // stress changes taken first
+        const float lamr = lambda / den_el, inv2mu = 1.0f / (2.0f * mu);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                float f11 = sn[0][k], f22 = sn[1][k], f12 = sn[2][k], f33 = sn[3][k];
-                float dtr = ((f11 - s0v[0][k]) + (f22 - s0v[1][k])) + (f33 - s0v[3][k]);
-                float d11 = sr[0][k] * dt - ((f11 - s0v[0][k]) - lamr * dtr) * inv2mu;
-                float d22 = sr[1][k] * dt - ((f22 - s0v[1][k]) - lamr * dtr) * inv2mu;
-                float d12 = sr[2][k] * dt - (f12 - s0v[2][k]) * inv2mu;
-                float d33 = -(((f33 - s0v[3][k]) - lamr * dtr) * inv2mu);
-                float a11 = 0.5f * (s0v[0][k] + f11), a22 = 0.5f * (s0v[1][k] + f22),
-                      a12 = 0.5f * (s0v[2][k] + f12), a33 = 0.5f * (s0v[3][k] + f33);
-                float qk = a11 * d11 + a22 * d22 + 2.0f * a12 * d12 + a33 * d33;
-                qk -= pref * (d11 + d22 + d33); // isotropic reference part
-                qsum = qsum + 0.25f * qk;
-            }
-        } else {
-            // the 32 quotients by 2 mu (fl_rheol.f90:352-362) share one
-            // reciprocal; gf_div gives each the bits of the division.  The
-            // phase's lambda / den_el and reciprocal pair of 2 mu are the
-            // same expressions evaluated once per phase at set-up.
-            const GfRecip r2mu = gf_recip_pre(R(2.0) * rmu, P.sh_r2mu_y[iph], P.sh_r2mu_yl[iph]);
-            auto by2mu = [&](R a) { return gf_div(a, r2mu); };
-            const R lam_den = P.sh_lam_den[iph];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                R f11 = sn[0][k], f22 = sn[1][k], f12 = sn[2][k], f33 = sn[3][k];
-                R tr0 = s0v[0][k] + s0v[1][k] + s0v[3][k];
-                R lt0 = lam_den * tr0;
-                R e11a = by2mu(s0v[0][k] - lt0);
-                R e22a = by2mu(s0v[1][k] - lt0);
-                R e33a = by2mu(s0v[3][k] - lt0);
-                R e12a = by2mu(s0v[2][k]);
-                R tr1 = f11 + f22 + f33;
-                R lt1 = lam_den * tr1;
-                R e11b = by2mu(f11 - lt1);
-                R e22b = by2mu(f22 - lt1);
-                R e33b = by2mu(f33 - lt1);
-                R e12b = by2mu(f12);
-                R d11 = sr[0][k] * dt - (e11b - e11a);
-                R d22 = sr[1][k] * dt - (e22b - e22a);
-                R d12 = sr[2][k] * dt - (e12b - e12a);
-                R d33 = gf_zero_minus(e33b - e33a);
-                R a11 = gf_scale<-1>(s0v[0][k] + f11), a22 = gf_scale<-1>(s0v[1][k] + f22),
-                  a12 = gf_scale<-1>(s0v[2][k] + f12), a33 = gf_scale<-1>(s0v[3][k] + f33);
-                R qk = a11 * d11 + a22 * d22 + gf_scale<1>(a12) * d12 + a33 * d33;
-                qsum = qsum + gf_scale<-2>(qk);
-            }
+        for (int k = 0; k < 4; ++k) {
+            float f11 = sn[0][k], f22 = sn[1][k], f12 = sn[2][k], f33 = sn[3][k];
+            float dtr = ((f11 - s0v[0][k]) + (f22 - s0v[1][k])) + (f33 - s0v[3][k]);
+            float d11 = sr[0][k] * dt - ((f11 - s0v[0][k]) - lamr * dtr) * inv2mu;
+            float d22 = sr[1][k] * dt - ((f22 - s0v[1][k]) - lamr * dtr) * inv2mu;
+            float d12 = sr[2][k] * dt - (f12 - s0v[2][k]) * inv2mu;
+            float d33 = -(((f33 - s0v[3][k]) - lamr * dtr) * inv2mu);
+            float a11 = 0.5f * (s0v[0][k] + f11), a22 = 0.5f * (s0v[1][k] + f22),
+                  a12 = 0.5f * (s0v[2][k] + f12), a33 = 0.5f * (s0v[3][k] + f33);
+            float qk = a11 * d11 + a22 * d22 + 2.0f * a12 * d12 + a33 * d33;
+            qk -= pref * (d11 + d22 + d33); // isotropic reference part
+            qsum = qsum + 0.25f * qk;
         }
         shr = shr + qsum;
     }
     sshrheat[e] = shr;
     (void)nloop;
 }
-template <class R> __global__ void __launch_bounds__(GF_THREADS, GF_RHEOL_MINB) k_rheol(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d, int update_visc, int nloop) {
+// mixed path: 3 CTAs per SM (80 registers; its few spills cost less than the
+// occupancy they buy)
+template <class R> __global__ void __launch_bounds__(GF_THREADS, 3) k_rheol(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d, int update_visc, int nloop) {
     gf_pdl_entry();
     b_k_rheol<R>(Pp, C, A, d, update_visc, nloop, (GF_IDX)blockIdx.x * blockDim.x + threadIdx.x);
 }
@@ -747,63 +641,35 @@ __global__ void __launch_bounds__(GF_THREADS) k_move_cord(DevClock *__restrict__
     b_k_move_cord(C, A, d, (GF_IDX)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
+// mixed path, one element per thread (the FP64 path: k_move_tri)
 template <class R> __device__ __forceinline__ void b_k_move_elem(DevClock *__restrict__ C, DevArrays A, GfDims d, int advance_time, GF_IDX e) {
     if (e >= d.E) return;
     int j, i;
     elem_ji(d, e, j, i);
     const double dtd = C->dt;
     if (advance_time && e == 0) C->time = C->time + dtd; // par.f90:86, after every reader of time
-    const bool fp32_path = sizeof(R) == sizeof(float);
-    Quad q;
     QuadF qf;
-    double xv[4], yv[4];
     float rvx[4], rvy[4];
-    if (fp32_path) {
-        load_quad_rel(A, d, j, i, qf);
-        load_vel_rel(A, d, j, i, rvx, rvy);
-    } else {
-        load_quad(A.cord, d, j, i, q);
-        GF_IDX n1 = gf_node(d, j, i), n3 = gf_node(d, j, i + 1);
-        const double *vel = A.vel;
-        xv[0] = vel[n1]; xv[1] = vel[n1 + 1]; xv[2] = vel[n3]; xv[3] = vel[n3 + 1];
-        yv[0] = vel[d.N + n1]; yv[1] = vel[d.N + n1 + 1]; yv[2] = vel[d.N + n3]; yv[3] = vel[d.N + n3 + 1];
-    }
+    load_quad_rel(A, d, j, i, qf);
+    load_vel_rel(A, d, j, i, rvx, rvy);
     R *area = (R *)A.area;
     R *dvol = (R *)A.dvol;
     R *st = (R *)A.stress0;
     R *strain = (R *)A.strain;
     const int nd1[4] = {0, 2, 0, 0}, nd2[4] = {1, 1, 1, 3}, nd3[4] = {2, 3, 3, 2};
     bool neg = false;
-    const bool fp32 = sizeof(R) == sizeof(float);
     // the surface nodes also moved by diff_topo's dtopo (zero without it)
     float tz[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    if (fp32 && j == 0) {
+    if (j == 0) {
         tz[0] = gf_d2f(A.dtopo[i]);
         tz[2] = gf_d2f(A.dtopo[i + 1]);
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         int a = nd1[k], b = nd2[k], c = nd3[k];
-        const double *xc = q.x, *yc = q.y;
         R ar_old = area[gf_ek(d, e, k)];
         R dw12, ar_new;
-        if (!fp32) {
-            // fl_move.f90:70-90 with the reference's operations
-            // (products on the integer pipes: gf_mul, the bits of the FP64
-            // multiply, which this FP64-bound kernel has few enough of)
-            double det = ((gf_mul(xc[b], yc[c]) - gf_mul(yc[b], xc[c])) - (gf_mul(xc[a], yc[c]) - gf_mul(yc[a], xc[c]))) +
-                         (gf_mul(xc[a], yc[b]) - gf_mul(yc[a], xc[b]));
-            dvol[gf_ek(d, e, k)] = R(gf_mul(det, (double)ar_old) - 1.0);
-            const double rdet = gf_rcp(det); // RN(1/det) off the FP64 pipe
-            ar_new = R(rdet);
-            // the rotation's quotient by det (gf_ddiv: the bits of the division)
-            double dw = gf_mul(gf_ddiv(gf_scale<-1>(gf_mul(xv[a], xc[c] - xc[b]) + gf_mul(xv[b], xc[a] - xc[c]) +
-                                                    gf_mul(xv[c], xc[b] - xc[a]) + gf_mul(yv[a], yc[c] - yc[b]) +
-                                                    gf_mul(yv[b], yc[a] - yc[c]) + gf_mul(yv[c], yc[b] - yc[a])),
-                                       det),
-                               dtd);
-            dw12 = R(dw);
-        } else {
+        {
             // FP32 from edge vectors of the relative coordinates: det = B x C
             // with B = b - a, C = c - a.  dvol = det_new*area_old - 1 is taken
             // as (det_new - det_old)*area_old with the change of det expanded
@@ -827,14 +693,14 @@ template <class R> __device__ __forceinline__ void b_k_move_elem(DevClock *__res
         area[gf_ek(d, e, k)] = ar_new;
         neg |= !(ar_new > R(0));
         R s11 = st[gf_s(d, e, 0, k)], s22 = st[gf_s(d, e, 1, k)], s12 = st[gf_s(d, e, 2, k)];
-        st[gf_s(d, e, 0, k)] = s11 + gf_mul(gf_scale<1>(s12), dw12);
-        st[gf_s(d, e, 1, k)] = s22 - gf_mul(gf_scale<1>(s12), dw12);
-        st[gf_s(d, e, 2, k)] = s12 + gf_mul(dw12, s22 - s11);
+        st[gf_s(d, e, 0, k)] = s11 + 2.0f * s12 * dw12;
+        st[gf_s(d, e, 1, k)] = s22 - 2.0f * s12 * dw12;
+        st[gf_s(d, e, 2, k)] = s12 + dw12 * (s22 - s11);
         if (k == 0) {
             R e11 = strain[gf_ek(d, e, 0)], e22 = strain[gf_ek(d, e, 1)], e12 = strain[gf_ek(d, e, 2)];
-            strain[gf_ek(d, e, 0)] = e11 + gf_mul(gf_scale<1>(e12), dw12);
-            strain[gf_ek(d, e, 1)] = e22 - gf_mul(gf_scale<1>(e12), dw12);
-            strain[gf_ek(d, e, 2)] = e12 + gf_mul(dw12, e22 - e11);
+            strain[gf_ek(d, e, 0)] = e11 + 2.0f * e12 * dw12;
+            strain[gf_ek(d, e, 1)] = e22 - 2.0f * e12 * dw12;
+            strain[gf_ek(d, e, 2)] = e12 + dw12 * (e22 - e11);
         }
     }
     if (neg) set_status(C, 40, (int)e);
@@ -1906,14 +1772,18 @@ template <class R> __global__ void k_convert_back(const R *__restrict__ src, dou
 } // namespace gfk
 } // namespace
 
+#ifdef GF_FP64_UNIT
+#include "gf_tri64.cuh"
+#endif
+
 // ---------------------------------------------------------------- launchers
 // Launch with programmatic stream serialization (the kernel starts with
 // gf_pdl_entry); `n` items, GF_THREADS per CTA.
 template <class... KArgs, class... Args>
-inline void gf_launch_pdl(void (*kern)(KArgs...), unsigned grid, cudaStream_t s, Args... args) {
+inline void gf_launch_pdl(void (*kern)(KArgs...), unsigned grid, unsigned threads, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3(grid);
-    lc.blockDim = dim3(GF_THREADS);
+    lc.blockDim = dim3(threads);
     lc.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1922,10 +1792,11 @@ inline void gf_launch_pdl(void (*kern)(KArgs...), unsigned grid, cudaStream_t s,
     lc.numAttrs = 1;
     cudaLaunchKernelEx(&lc, kern, (KArgs)args...);
 }
-#define GF_LAUNCH(kern, n, ...)                                                                                        \
+#define GF_LAUNCH(kern, n, ...) GF_LAUNCH_T(kern, n, GF_THREADS, __VA_ARGS__)
+#define GF_LAUNCH_T(kern, n, thr, ...)                                                                                      \
     do {                                                                                                               \
         if ((n) > 0) {                                                                                                 \
-            gf_launch_pdl(kern, gfk::grid_for(n), g.s, __VA_ARGS__);                                                   \
+            gf_launch_pdl(kern, gfk::grid_for(n, thr), thr, g.s, __VA_ARGS__);                                                  \
             ++*g.launches;                                                                                             \
         }                                                                                                              \
     } while (0)
@@ -2022,7 +1893,12 @@ template <class R> void GfKernels<R>::therm(const GfLaunch &g, int sweeps, int k
 
 template <class R> void GfKernels<R>::rheol(const GfLaunch &g, int update_visc, int avg_mode) {
     using namespace gfk;
+#ifdef GF_FP64_UNIT
+    if (update_visc) GF_LAUNCH(k_rheol_visc, g.d.E, g.P, g.A, g.d);
+    GF_LAUNCH_T(k_rheol_tri, 4 * g.d.E, GF_TRI_T, g.P, g.C, g.A, g.d);
+#else
     GF_LAUNCH(k_rheol<R>, g.d.E, g.P, g.C, g.A, g.d, update_visc, 0);
+#endif
     if (avg_mode > 0) {
         GF_LAUNCH(k_rheol_avg<R>, g.d.E, g.C, g.A, g.d, avg_mode == 2 ? 1 : 0);
         if (avg_mode == 2) {
@@ -2074,7 +1950,11 @@ template <class R> void GfKernels<R>::move_cord(const GfLaunch &g) {
 }
 template <class R> void GfKernels<R>::move_elem(const GfLaunch &g) {
     using namespace gfk;
+#ifdef GF_FP64_UNIT
+    GF_LAUNCH(k_move_tri, 4 * g.d.E, g.C, g.A, g.d, g.advance_time);
+#else
     GF_LAUNCH(k_move_elem<R>, g.d.E, g.C, g.A, g.d, g.advance_time);
+#endif
 }
 template <class R> void GfKernels<R>::move(const GfLaunch &g) {
     move_cord(g);
