@@ -33,6 +33,7 @@ UNITS = [
     ("gf_io.cu", ["-fmad=false"]),
     ("gf_batch.cu", ["-fmad=true", "-prec-div=false", "-prec-sqrt=false"]),
     ("fno_gemm.cu", ["-fmad=true"]),
+    ("fno_layer.cu", ["-fmad=true"]),
     ("fno_ops.cu", ["-fmad=true"]),
     ("host_inp.cpp", None),
     ("host_setup.cpp", None),

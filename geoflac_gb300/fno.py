@@ -1,7 +1,8 @@
 """Fourier neural operator that predicts an ensemble member's state several
 hundred steps ahead, trained and run by the library's own kernels
-(include/geoflac_fno.h): every matrix product is the tcgen05 BF16 GEMM with
-FP32 accumulation, every other operation one of the FNO kernels.  PyTorch
+(include/geoflac_fno.h): every matrix product runs on tcgen05 (BF16 operands,
+FP32 accumulation), in the fused forward kernels where the configuration fits
+them (same bits) and as separate GEMMs otherwise.  PyTorch
 only allocates the device buffers and provides the stream.
 
 Architecture (per pixel of an H x W grid, channels last):
@@ -55,6 +56,12 @@ def _lib():
         "gf_fno_pack_target": [vp, vp, vp, vp, ll, vp],
         "gf_fno_unpack": [vp, vp, vp, vp, ll, vp],
         "gf_fno_gather_rows": [vp, vp, vp, i, ll, vp],
+        "gf_fno_layer_ok": [i, i, i, i, i, i, i, i],
+        "gf_fno_row": [vp, i, vp, vp, vp, vp, i, vp, vp, vp, vp, i, i, i, vp],
+        "gf_fno_fwd_h": [vp, vp, vp, i, i, i, i, vp],
+        "gf_fno_modes": [vp, vp, vp, i, i, vp],
+        "gf_fno_inv_h": [vp, vp, vp, i, i, i, i, vp],
+        "gf_fno_proj": [vp, vp, vp, vp, vp, vp, vp, vp, i, i, vp],
     }
     for n, a in sig.items():
         fn = getattr(lib, n)
@@ -171,6 +178,8 @@ class Fno:
             self.mat[k] = torch.from_numpy(np.ascontiguousarray(a)).to(dev).to(bf)
             self.mat[k + "T"] = torch.from_numpy(np.ascontiguousarray(a.T)).to(dev).to(bf)
         self.saved = None
+        # the fused forward kernels take this configuration (same bits)
+        self.fused = bool(self.lib.gf_fno_layer_ok(cfg.H, cfg.W, cfg.C, cfg.m2, cfg.Q, cfg.cin, cfg.P, cfg.cout))
 
     # ---------------------------------------------------------------- kernels
     @property
@@ -271,6 +280,57 @@ class Fno:
             return s_cl, (U, RmT)
         return s_cl, None
 
+    def row(self, v, kin, Z, w, bias, act, z, vout, Xw, rows):
+        _ck(self.lib.gf_fno_row(_p(v), kin, _p(Z), _p(self.mat["IW"]), _p(w), _p(bias), act, _p(self.mat["FW"]),
+                                _p(z), _p(vout), _p(Xw), rows, self.cfg.W, 2 * self.cfg.m2, self.s), "row")
+
+    def forward_fused(self, x, wb, train: bool):
+        """forward() by the fused kernels"""
+        torch, cfg = self.torch, self.cfg
+        B, H, Cc, m2, Q = x.shape[0], cfg.H, cfg.C, cfg.m2, cfg.Q
+        M, rows, bf = B * H * cfg.W, B * H, torch.bfloat16
+
+        def new(*shape, dtype=bf):
+            return torch.empty(shape, dtype=dtype, device="cuda")
+
+        v, Xw = new(M, Cc), new(rows, 2 * m2, Cc)
+        self.row(x, cfg.cin, None, wb["lift_w"], self.p["lift_b"], 0, None, v, Xw, rows)
+        saved = {"x": x, "v": [], "z": [], "spec": [], "wb": wb}
+        vn, V, Z = new(M, Cc), new(cfg.modes, B, 2 * Cc), new(rows, 2 * m2, Cc)
+        U = new(cfg.modes, B, 2 * Cc)
+        for l in range(cfg.layers):
+            last = l == cfg.layers - 1
+            zl = new(M, Cc, dtype=torch.float32) if train else None
+            _ck(self.lib.gf_fno_fwd_h(_p(Xw), _p(self.mat["FH"]), _p(U), B, H, m2, Q, self.s), "fwd_h")
+            _ck(self.lib.gf_fno_modes(_p(U), _p(self.p[f"R{l}"]), _p(V), B, cfg.modes, self.s), "modes")
+            _ck(self.lib.gf_fno_inv_h(_p(V), _p(self.mat["IH"]), _p(Z), B, H, m2, Q, self.s), "inv_h")
+            self.row(v, Cc, Z, wb[f"w{l}"], self.p[f"b{l}"], 0 if last else 1, zl, vn, None if last else Xw, rows)
+            if train:
+                saved["v"].append(v)
+                saved["z"].append(zl)
+                saved["spec"].append((U, self.modes_t(l)))
+                v, vn, U = vn, new(M, Cc), new(cfg.modes, B, 2 * Cc)
+            else:
+                v, vn = vn, v
+        zp = new(M, cfg.P, dtype=torch.float32) if train else None
+        hh = new(M, cfg.P) if train else None
+        out = new(M, cfg.cout, dtype=torch.float32)
+        _ck(self.lib.gf_fno_proj(_p(v), _p(wb["p1_w"]), _p(self.p["p1_b"]), _p(wb["p2_w"]), _p(self.p["p2_b"]),
+                                 _p(zp), _p(hh), _p(out), rows, cfg.W, self.s), "proj")
+        if train:
+            saved.update(vL=v, zp=zp, h=hh)
+            self.saved = saved
+        return out.view(B, H, cfg.W, cfg.cout)
+
+    def modes_t(self, l):
+        """the transposed real blocks of layer l's mode weights (BF16)"""
+        n2 = 2 * self.cfg.C
+        Rm = self.torch.empty((self.cfg.modes, n2, n2), dtype=self.torch.bfloat16, device="cuda")
+        RmT = self.torch.empty_like(Rm)
+        _ck(self.lib.gf_fno_expand_modes(_p(self.p[f"R{l}"]), _p(Rm), _p(RmT), self.cfg.modes, self.cfg.C, self.s),
+            "expand")
+        return RmT
+
     def forward(self, x, train: bool = False):
         """x: BF16 [B, H, W, cin] -> FP32 [B, H, W, cout]"""
         torch, cfg = self.torch, self.cfg
@@ -279,6 +339,8 @@ class Fno:
         bf = torch.bfloat16
         wb = {k: self.bf16(self.p[k]) for k in self.p if not k.startswith("R") and not k.endswith("_b")
               and not (k.startswith("b") and k[1:].isdigit())}
+        if self.fused:
+            return self.forward_fused(x, wb, train)
         # inference keeps only the BF16 activations (no FP32 copies of the
         # pre-activations, which only the backward pass reads)
         z = torch.empty((M, cfg.C), dtype=torch.float32, device="cuda") if train else None

@@ -88,6 +88,32 @@ int gf_fno_mse_weighted(const float *pred, const float *target, void *dpred, int
 /* out = x + y (y may be NULL), FP32 and/or BF16 outputs. */
 int gf_fno_add(const float *x, const float *y, float *out, void *out_bf16, long long n, void *stream);
 
+/* ---- the forward pass in fused kernels (64 channels) ----
+ * gf_fno_layer_ok: 1 if the shapes fit them (C = 64, W = 128, 256 or 384,
+ * H = 64 or 128, 2 m2 and Q multiples of 16 up to 64, cin a multiple of 16 up
+ * to 64, P = 128, cout = 16).  Their results equal the products above, bit for
+ * bit.  BF16 unless said otherwise; K2 = 2 m2; DFT matrices as in
+ * geoflac_gb300/fno.py.
+ * gf_fno_row: rows of W points, z = v Wl^T + bias + IW Z (v [rows W][kin], Wl
+ * [64][kin], bias FP32; Z [rows][K2][64] with rows (k2, re|im), NULL: no such
+ * term); z (FP32, may be NULL) and vout [rows W][64] = GELU(z) (act = 1) or z
+ * are written, and Xw [rows][K2][64] = FW vout (rows: real, then imaginary
+ * parts; NULL: not computed).
+ * gf_fno_fwd_h: Xw [B][H][K2][64] -> U[(k2, q)][b][(c, re|im)].
+ * gf_fno_modes: V[mode][b][re|im][o] from U and the FP32 weights
+ * R[mode][i][o][re, im].
+ * gf_fno_inv_h: V -> Z [B][H][(k2, re|im)][64].
+ * gf_fno_proj: out (FP32 [rows W][16]) = GELU(v P1^T + b1) P2^T + b2; zp (FP32)
+ * and h [rows W][128], if not NULL, receive the pre-activations and GELU(zp). */
+int gf_fno_layer_ok(int H, int W, int C, int m2, int Q, int cin, int P, int cout);
+int gf_fno_row(const void *v, int kin, const void *Z, const void *IW, const void *Wl, const float *bias, int act,
+               const void *FW, float *z, void *vout, void *Xw, int rows, int W, int K2, void *stream);
+int gf_fno_fwd_h(const void *Xw, const void *FH, void *U, int B, int H, int m2, int Q, void *stream);
+int gf_fno_modes(const void *U, const float *R, void *V, int B, int modes, void *stream);
+int gf_fno_inv_h(const void *V, const void *IH, void *Z, int B, int H, int m2, int Q, void *stream);
+int gf_fno_proj(const void *v, const void *P1, const float *b1, const void *P2, const float *b2, float *zp, void *h,
+                float *out, int rows, int W, void *stream);
+
 #ifdef __cplusplus
 }
 #endif
