@@ -34,6 +34,7 @@ UNITS = [
     ("gf_batch.cu", ["-fmad=true", "-prec-div=false", "-prec-sqrt=false"]),
     ("fno_gemm.cu", ["-fmad=true"]),
     ("fno_layer.cu", ["-fmad=true"]),
+    ("fno_back.cu", ["-fmad=true"]),
     ("fno_ops.cu", ["-fmad=true"]),
     ("host_inp.cpp", None),
     ("host_setup.cpp", None),

@@ -251,6 +251,7 @@ template <int BN> int launch(const CUtensorMap &ta, const CUtensorMap &tb, int b
 } // namespace
 
 int gf_fno_layer_error(); // fno_layer.cu
+int gf_fno_back_error();  // fno_back.cu
 
 extern "C" {
 
@@ -291,8 +292,8 @@ int gf_gemm_bf16_ex(const void *A, const void *B, void *C, int batch, int M, int
 }
 
 int gf_gemm_error(void) {
-    const int a = take_tc_error(), b = gf_fno_layer_error();
-    return a != GF_FNO_OK ? a : b;
+    const int a = take_tc_error(), b = gf_fno_layer_error(), c = gf_fno_back_error();
+    return a != GF_FNO_OK ? a : b != GF_FNO_OK ? b : c;
 }
 
 } // extern "C"

@@ -33,117 +33,6 @@
 
 namespace {
 
-constexpr int CH = 64; // channels: one 128-byte swizzled row of BF16
-
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int c0, int c1, uint64_t *bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-                 " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
-                 "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(smem_u32(bar))
-                 : "memory");
-}
-__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3,
-                                            uint64_t *bar) {
-    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-                 " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_u32(dst)),
-                 "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
-                 : "memory");
-}
-__device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, int c4,
-                                            uint64_t *bar) {
-    asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-                 " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(smem_u32(dst)),
-                 "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(smem_u32(bar))
-                 : "memory");
-}
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, int c0, int c1, const void *src) {
-    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
-                     reinterpret_cast<uint64_t>(map)),
-                 "r"(c0), "r"(c1), "r"(smem_u32(src))
-                 : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-// shared-memory writes of this thread become visible to TMA and MMA reads
-__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// shared-memory descriptor of an MN-major operand in 128-byte swizzled rows:
-// row k holds 64 MN values, 8-row groups 1024 bytes apart, further groups of
-// 64 MN values lbo bytes apart
-__device__ __forceinline__ uint64_t sdesc_mn(uint32_t addr, uint32_t lbo) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr >> 4) & 0x3FFF);
-    d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
-    d |= (uint64_t)(1024 >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;
-    return d;
-}
-constexpr uint64_t MN_STEP = 16 * 128 / 16; // 16 rows of K, in 16-byte units
-constexpr uint64_t K_STEP = 2;              // 16 BF16 along a K-major row
-// BF16 x BF16 -> FP32, M = 128; ta / tb: operand A / B is MN-major
-__device__ __forceinline__ constexpr uint32_t idesc_of(int N, int ta, int tb) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)ta << 15) | ((uint32_t)tb << 16) |
-           ((uint32_t)(N >> 3) << 17) | (8u << 24);
-}
-
-template <int N> __device__ __forceinline__ void tmem_ld(uint32_t taddr, float *v);
-template <> __device__ __forceinline__ void tmem_ld<16>(uint32_t taddr, float *v) {
-    uint32_t r[16];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                   "=r"(r[15])
-                 : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-template <> __device__ __forceinline__ void tmem_ld<32>(uint32_t taddr, float *v) {
-    tmem_ld32(taddr, *reinterpret_cast<float(*)[32]>(v));
-}
-
-__device__ __forceinline__ uint4 pack8(const float *v) {
-    uint4 w;
-    __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&w);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) h[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
-    return w;
-}
-__device__ __forceinline__ void st_global8(float *p, const float *v) { // one 32-byte sector (p 32-byte aligned)
-    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
-                 "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
-                 : "memory");
-}
-// 16-byte chunk j of row r in a tile of 128-byte swizzled rows
-__device__ __forceinline__ uint4 *swz(uint8_t *tile, int r, int j) {
-    return reinterpret_cast<uint4 *>(tile + r * 128 + ((j ^ (r & 7)) << 4));
-}
-
-__device__ __forceinline__ uint32_t tmem_alloc(uint32_t *slot, uint32_t cols, int warp) {
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)),
-                     "r"(cols));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
-    fence_before();
-    __syncthreads();
-    fence_after();
-    return *slot;
-}
-__device__ __forceinline__ void tmem_free(uint32_t tmem, uint32_t cols, int warp) {
-    fence_before();
-    __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols));
-}
-__device__ __forceinline__ uint8_t *align1k(uint8_t *p) {
-    return reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(p) + 1023) & ~static_cast<uintptr_t>(1023));
-}
-
 // ---------------------------------------------------------------- rows
 struct RowArgs {
     int rows, K2, kin, act;
@@ -740,39 +629,6 @@ __global__ void __launch_bounds__(128) k_modes(const __grid_constant__ CUtensorM
 }
 
 // ---------------------------------------------------------------- host
-// BF16 tensor map: dims and box innermost first, strides in elements from the
-// second dimension on, 128-byte swizzle, zero fill
-bool map_of(CUtensorMap *m, const void *p, int rank, const long long *dims, const long long *strides, const int *box) {
-    PFN_cuTensorMapEncodeTiled_v12000 enc = encoder();
-    if (!enc) return false;
-    cuuint64_t d[5], s[4];
-    cuuint32_t b[5], e[5] = {1, 1, 1, 1, 1};
-    for (int k = 0; k < rank; ++k) {
-        d[k] = (cuuint64_t)dims[k];
-        b[k] = (cuuint32_t)box[k];
-        if (k) s[k - 1] = (cuuint64_t)strides[k - 1] * 2;
-    }
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void *>(p), d, s, b, e,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-bool map2(CUtensorMap *m, const void *p, long long inner, long long rows, int box_rows) {
-    const long long d[2] = {inner, rows}, s[1] = {inner};
-    const int b[2] = {64, box_rows};
-    return map_of(m, p, 2, d, s, b);
-}
-bool unaligned(const void *p, int a = 16) { return reinterpret_cast<uintptr_t>(p) & (a - 1); }
-int sm_count() {
-    int dev = 0, n = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    return n > 0 ? n : 1;
-}
-template <class K> bool allow_smem(K kern, uint32_t bytes) {
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
-}
-int launched() { return cudaGetLastError() == cudaSuccess ? GF_FNO_OK : GF_FNO_ERR_CUDA; }
-
 template <int NT> int run_row(const CUtensorMap *m, const RowArgs &a, cudaStream_t s) {
     const uint32_t smem = RowSmem<NT>::total(a.K2);
     if (!allow_smem(k_row<NT>, smem)) return GF_FNO_ERR_CUDA;

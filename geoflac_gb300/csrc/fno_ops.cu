@@ -163,11 +163,11 @@ __global__ void k_modes_grad(const float *__restrict__ dRm, float *__restrict__ 
 }
 
 // out[c] (+)= sum over rows of X[r][c]; one block per column group
-__global__ void k_colsum(const float *__restrict__ X, float *__restrict__ out, long long rows, int cols, int accum) {
+template <class T> __global__ void k_colsum(const T *__restrict__ X, float *__restrict__ out, long long rows, int cols, int accum) {
     __shared__ float red[TB];
     const int c = blockIdx.x;
     float s = 0.0f;
-    for (long long r = threadIdx.x; r < rows; r += blockDim.x) s += X[r * cols + c];
+    for (long long r = threadIdx.x; r < rows; r += blockDim.x) s += (float)X[r * cols + c];
     red[threadIdx.x] = s;
     __syncthreads();
     for (int w = TB / 2; w > 0; w >>= 1) {
@@ -180,14 +180,14 @@ __global__ void k_colsum(const float *__restrict__ X, float *__restrict__ out, l
 // column sums, stage 1: block b sums rows [b*rpb, (b+1)*rpb) of a row-major
 // matrix whose column count divides the block size (coalesced reads; each
 // thread stays on one column), partial[b][c]
-__global__ void k_colsum_part(const float *__restrict__ X, float *__restrict__ part, long long rows, int cols,
+template <class T> __global__ void k_colsum_part(const T *__restrict__ X, float *__restrict__ part, long long rows, int cols,
                               long long rpb) {
     __shared__ float red[TB];
     const long long r0 = (long long)blockIdx.x * rpb, r1 = min(rows, r0 + rpb);
     const int per = TB / cols; // rows per pass
     const int c = threadIdx.x % cols, rr = threadIdx.x / cols;
     float s = 0.0f;
-    for (long long r = r0 + rr; r < r1; r += per) s += X[r * cols + c];
+    for (long long r = r0 + rr; r < r1; r += per) s += (float)X[r * cols + c];
     red[threadIdx.x] = s;
     __syncthreads();
     if (threadIdx.x < cols) {
@@ -201,6 +201,7 @@ __global__ void k_sum_batches(const float *__restrict__ src, float *__restrict__
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float s = 0.0f;
+#pragma unroll 16 // sixteen loads in flight; the sum's order is b = 0, 1, ...
     for (int b = 0; b < nb; ++b) s += src[(long long)b * n + i];
     dst[i] = (accum ? dst[i] : 0.0f) + s;
 }
@@ -217,27 +218,71 @@ __global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float
     p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
 }
 
+// x as a double by integer operations: the conversion instruction takes a
+// slot of the FP64 pipe (one warp instruction per 64 cycles)
+__device__ __forceinline__ double f2d(float x) {
+    const unsigned u = __float_as_uint(x), e = (u >> 23) & 0xffu;
+    if (e - 1u >= 254u) return (double)x; // zero, subnormal, infinity, NaN
+    return __hiloint2double((int)((u & 0x80000000u) | ((e + 896u) << 20) | ((u & 0x7fffffu) >> 3)), (int)(u << 29));
+}
 // mean-squared error over n values; loss accumulated in FP64, gradient
-// scale * 2 (pred - target) / n written as BF16 for the backward GEMMs
+// scale * 2 (pred - target) / n written as BF16 for the backward GEMMs.
+// Bound by the FP64 pipe: a weight of 1 costs no FP64 multiply and a thread
+// keeps its sum over four values of every pass, so one value costs a
+// multiply and an addition (50 M values: 1303 us with a tree sum per 256
+// values and converted operands, now 202).
+template <bool VEC>
 __global__ void k_mse(const float *__restrict__ pred, const float *__restrict__ target, void *__restrict__ dpred,
                       int dt, double *__restrict__ loss, long long n, float scale, const float *__restrict__ w,
                       long long w_period, int w_len) {
-    __shared__ double red[TB];
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ double red[TB / 32];
+    constexpr int PER = VEC ? 4 : 1;
+    const long long stride = (long long)gridDim.x * blockDim.x * PER;
     double e = 0.0;
-    if (i < n) {
-        float d = pred[i] - target[i];
-        float wi = w ? w[(i / w_period) % w_len] : 1.0f;
-        e = (double)wi * d * d;
-        if (dpred) stv(dpred, i, dt, scale * 2.0f * wi * d / (float)n);
+    for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * PER; i < n; i += stride) {
+        float p[PER], t[PER], g[PER], wi[PER];
+        if constexpr (VEC) {
+            const float4 a = *reinterpret_cast<const float4 *>(pred + i), b = *reinterpret_cast<const float4 *>(target + i);
+            p[0] = a.x; p[1] = a.y; p[2] = a.z; p[3] = a.w;
+            t[0] = b.x; t[1] = b.y; t[2] = b.z; t[3] = b.w;
+            wi[0] = wi[1] = wi[2] = wi[3] = 1.0f;
+            if (w) {
+                const float4 c = *reinterpret_cast<const float4 *>(w + (unsigned long long)i % (unsigned)w_len);
+                wi[0] = c.x; wi[1] = c.y; wi[2] = c.z; wi[3] = c.w;
+            }
+        } else {
+            p[0] = pred[i];
+            t[0] = target[i];
+            wi[0] = w ? w[(i / w_period) % w_len] : 1.0f;
+        }
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const float d = p[k] - t[k];
+            const double dd = f2d(d);
+            if (wi[k] == 1.0f) e += dd * dd;
+            else e += f2d(wi[k]) * dd * dd;
+            g[k] = scale * 2.0f * wi[k] * d / (float)n;
+        }
+        if (dpred) {
+            if constexpr (VEC) {
+                if (dt) {
+                    __nv_bfloat162 h[2] = {__floats2bfloat162_rn(g[0], g[1]), __floats2bfloat162_rn(g[2], g[3])};
+                    *reinterpret_cast<uint2 *>(reinterpret_cast<__nv_bfloat16 *>(dpred) + i) = *reinterpret_cast<uint2 *>(h);
+                } else {
+                    *reinterpret_cast<float4 *>(reinterpret_cast<float *>(dpred) + i) = make_float4(g[0], g[1], g[2], g[3]);
+                }
+            } else {
+                stv(dpred, i, dt, g[0]);
+            }
+        }
     }
-    red[threadIdx.x] = e;
+    for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = e;
     __syncthreads();
-    for (int w = TB / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-        __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < TB / 32; ++k) e += red[k];
+        atomicAdd(loss, e / (double)n);
     }
-    if (threadIdx.x == 0) atomicAdd(loss, red[0] / (double)n);
 }
 
 // a = x + y (FP32) written as FP32 and/or BF16
@@ -251,19 +296,39 @@ __global__ void k_add(const float *__restrict__ x, const float *__restrict__ y, 
 }
 
 // surrogate input: 9 normalised fields, 4 normalised member parameters,
-// 2 grid coordinates in [-1, 1], one zero channel (16, BF16)
-__global__ void k_pack_input(const float *__restrict__ raw, const float *__restrict__ prm,
-                             const float *__restrict__ stats, __nv_bfloat16 *__restrict__ out, int n, int H, int W) {
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)n * H * W) return;
-    const int gx = (int)(t % W), gy = (int)((t / W) % H), m = (int)(t / ((long long)W * H));
-    const float *r = raw + t * 9;
-    __nv_bfloat16 *o = out + t * 16;
-    for (int c = 0; c < 9; ++c) o[c] = __float2bfloat16_rn((r[c] - stats[c]) / stats[9 + c]);
-    for (int c = 0; c < 4; ++c) o[9 + c] = __float2bfloat16_rn((prm[m * 4 + c] - stats[18 + c]) / stats[22 + c]);
-    o[13] = __float2bfloat16_rn(2.0f * (gx + 0.5f) / W - 1.0f);
-    o[14] = __float2bfloat16_rn(2.0f * (gy + 0.5f) / H - 1.0f);
-    o[15] = __float2bfloat16_rn(0.0f);
+// 2 grid coordinates in [-1, 1], one zero channel (16, BF16).  A CTA takes
+// TB points of one member (`nb` CTAs each): their 36-byte records are staged in
+// shared memory, the member's parameters are normalised once, and a point's
+// 32 bytes leave in two stores (one thread a point with 2-byte stores and 13
+// divisions: 246 us for 64 members, now 43 us).
+__global__ void __launch_bounds__(TB) k_pack_input(const float *__restrict__ raw, const float *__restrict__ prm,
+                                                   const float *__restrict__ stats, __nv_bfloat16 *__restrict__ out,
+                                                   int H, int W, unsigned nb) {
+    __shared__ float rec[TB * 9], st[26], par[4];
+    const int m = blockIdx.x / nb, t = threadIdx.x;
+    const long long np = (long long)H * W, p0 = (long long)(blockIdx.x - m * nb) * TB, base = m * np + p0;
+    const int cnt = (int)min((long long)TB, np - p0);
+    for (int k = t; k < cnt * 9; k += TB) rec[k] = raw[base * 9 + k];
+    if (t < 18) st[t] = stats[t];
+    if (t < 4) par[t] = (prm[m * 4 + t] - stats[18 + t]) / stats[22 + t];
+    __syncthreads();
+    if (t >= cnt) return;
+    const int gx = (int)((p0 + t) % W), gy = (int)((p0 + t) / W);
+    float v[16];
+#pragma unroll
+    for (int c = 0; c < 9; ++c) v[c] = (rec[t * 9 + c] - st[c]) / st[9 + c];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) v[9 + c] = par[c];
+    v[13] = 2.0f * (gx + 0.5f) / W - 1.0f;
+    v[14] = 2.0f * (gy + 0.5f) / H - 1.0f;
+    v[15] = 0.0f;
+    uint4 o[2];
+    __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(o);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) h[c] = __floats2bfloat162_rn(v[2 * c], v[2 * c + 1]);
+    uint4 *dst = reinterpret_cast<uint4 *>(out + (base + t) * 16);
+    dst[0] = o[0];
+    dst[1] = o[1];
 }
 
 // training target: normalised increments (y - x - mean_d) / std_d in 9 of 16 channels
@@ -275,12 +340,19 @@ __global__ void k_pack_target(const float *__restrict__ y, const float *__restri
         out[t * 16 + c] = c < 9 ? (y[t * 9 + c] - x[t * 9 + c] - sd[c]) / sd[9 + c] : 0.0f;
 }
 
-// prediction back to fields: y = x + mean_d + std_d * pred
-__global__ void k_unpack(const float *__restrict__ pred, const float *__restrict__ x, const float *__restrict__ sd,
-                         float *__restrict__ y, long long pts) {
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= pts) return;
-    for (int c = 0; c < 9; ++c) y[t * 9 + c] = x[t * 9 + c] + sd[c] + sd[9 + c] * pred[t * 16 + c];
+// prediction back to fields: y = x + mean_d + std_d * pred, thread per value
+// of the 9-channel records (coalesced; their predictions lie in 64-byte rows)
+__global__ void __launch_bounds__(TB) k_unpack(const float *__restrict__ pred, const float *__restrict__ x,
+                                               const float *__restrict__ sd, float *__restrict__ y, long long pts) {
+    const long long p0 = (long long)blockIdx.x * TB;
+    const int n = 9 * (int)min((long long)TB, pts - p0);
+#pragma unroll
+    for (int r = 0; r < 9; ++r) {
+        const int k = threadIdx.x + r * TB;
+        if (k >= n) return;
+        const int q = k / 9, c = k - 9 * q;
+        y[p0 * 9 + k] = x[p0 * 9 + k] + sd[c] + sd[9 + c] * pred[(p0 + q) * 16 + c];
+    }
 }
 
 // dst[r] = src[idx[r]] for rows of `row_words` 32-bit words
@@ -293,17 +365,42 @@ __global__ void k_gather_rows(const uint32_t *__restrict__ src, uint32_t *__rest
     (void)nrows;
 }
 
+#define FNO_RET(s) return cudaGetLastError() == cudaSuccess ? GF_FNO_OK : GF_FNO_ERR_CUDA
+
+template <class T>
+int run_colsum(const T *X, float *out, long long rows, int cols, int accum, void *stream) {
+    if (!X || !out || rows < 1 || cols < 1) return GF_FNO_ERR_ARG;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (cols <= TB && TB % cols == 0 && rows >= 4096) {
+        // two stages through a fixed scratch of 1024 partial rows
+        static float *part = nullptr;
+        static int part_cols = 0;
+        const int nb = 1024;
+        if (!part || part_cols < cols) {
+            if (part) cudaFree(part);
+            part = nullptr;
+            if (cudaMalloc(&part, sizeof(float) * nb * TB) != cudaSuccess) return GF_FNO_ERR_CUDA;
+            part_cols = TB;
+        }
+        long long rpb = (rows + nb - 1) / nb;
+        k_colsum_part<<<nb, TB, 0, st>>>(X, part, rows, cols, rpb);
+        k_sum_batches<<<nblk(cols), TB, 0, st>>>(part, out, nb, cols, accum);
+    } else {
+        k_colsum<<<(unsigned)cols, TB, 0, st>>>(X, out, rows, cols, accum);
+    }
+    FNO_RET(stream);
+}
+
 } // namespace
 
-#define FNO_RET(s) return cudaGetLastError() == cudaSuccess ? GF_FNO_OK : GF_FNO_ERR_CUDA
 
 extern "C" {
 
 int gf_fno_pack_input(const float *raw, const float *params, const float *stats, void *out, int n, int H, int W,
                       void *stream) {
     if (!raw || !params || !stats || !out || n < 1 || H < 1 || W < 1) return GF_FNO_ERR_ARG;
-    long long pts = (long long)n * H * W;
-    k_pack_input<<<nblk(pts), TB, 0, (cudaStream_t)stream>>>(raw, params, stats, (__nv_bfloat16 *)out, n, H, W);
+    const unsigned nb = nblk((long long)H * W);
+    k_pack_input<<<nb * (unsigned)n, TB, 0, (cudaStream_t)stream>>>(raw, params, stats, (__nv_bfloat16 *)out, H, W, nb);
     FNO_RET(stream);
 }
 
@@ -390,26 +487,10 @@ int gf_fno_modes_grad(const float *dRm, float *dR, int modes, int C, void *strea
 }
 
 int gf_fno_colsum(const float *X, float *out, long long rows, int cols, int accum, void *stream) {
-    if (!X || !out || rows < 1 || cols < 1) return GF_FNO_ERR_ARG;
-    cudaStream_t st = (cudaStream_t)stream;
-    if (cols <= TB && TB % cols == 0 && rows >= 4096) {
-        // two stages through a fixed scratch of 1024 partial rows
-        static float *part = nullptr;
-        static int part_cols = 0;
-        const int nb = 1024;
-        if (!part || part_cols < cols) {
-            if (part) cudaFree(part);
-            part = nullptr;
-            if (cudaMalloc(&part, sizeof(float) * nb * TB) != cudaSuccess) return GF_FNO_ERR_CUDA;
-            part_cols = TB;
-        }
-        long long rpb = (rows + nb - 1) / nb;
-        k_colsum_part<<<nb, TB, 0, st>>>(X, part, rows, cols, rpb);
-        k_sum_batches<<<nblk(cols), TB, 0, st>>>(part, out, nb, cols, accum);
-    } else {
-        k_colsum<<<(unsigned)cols, TB, 0, st>>>(X, out, rows, cols, accum);
-    }
-    FNO_RET(stream);
+    return run_colsum(X, out, rows, cols, accum, stream);
+}
+int gf_fno_colsum_bf16(const void *X, float *out, long long rows, int cols, int accum, void *stream) {
+    return run_colsum((const __nv_bfloat16 *)X, out, rows, cols, accum, stream);
 }
 
 int gf_fno_sum_batches(const float *src, float *dst, int nb, long long n, int accum, void *stream) {
@@ -426,19 +507,30 @@ int gf_fno_adam(float *p, const float *g, float *m, float *v, long long n, float
     FNO_RET(stream);
 }
 
+static int run_mse(const float *pred, const float *target, void *dpred, int dpred_bf16, double *loss, long long n,
+                   float scale, const float *w, long long w_period, int w_len, void *stream) {
+    const uintptr_t al = (uintptr_t)pred | (uintptr_t)target | (uintptr_t)w | ((uintptr_t)dpred << (dpred_bf16 ? 1 : 0));
+    const bool vec = n % 4 == 0 && (al & 15) == 0 && (!w || (w_period == 1 && w_len % 4 == 0));
+    const long long per = (long long)TB * (vec ? 4 : 1);
+    const long long blocks = (n + per - 1) / per;
+    const unsigned grid = (unsigned)(blocks < 2432 ? blocks : 2432); // 16 CTAs on each of 152 SMs
+    if (vec)
+        k_mse<true><<<grid, TB, 0, (cudaStream_t)stream>>>(pred, target, dpred, dpred_bf16, loss, n, scale, w, w_period, w_len);
+    else
+        k_mse<false><<<grid, TB, 0, (cudaStream_t)stream>>>(pred, target, dpred, dpred_bf16, loss, n, scale, w, w_period, w_len);
+    FNO_RET(stream);
+}
+
 int gf_fno_mse(const float *pred, const float *target, void *dpred, int dpred_bf16, double *loss, long long n,
                float scale, void *stream) {
     if (!pred || !target || !loss || n < 1) return GF_FNO_ERR_ARG;
-    k_mse<<<nblk(n), TB, 0, (cudaStream_t)stream>>>(pred, target, dpred, dpred_bf16, loss, n, scale, nullptr, 1, 1);
-    FNO_RET(stream);
+    return run_mse(pred, target, dpred, dpred_bf16, loss, n, scale, nullptr, 1, 1, stream);
 }
 
 int gf_fno_mse_weighted(const float *pred, const float *target, void *dpred, int dpred_bf16, double *loss,
                         long long n, float scale, const float *w, long long w_period, int w_len, void *stream) {
     if (!pred || !target || !loss || !w || n < 1 || w_period < 1 || w_len < 1) return GF_FNO_ERR_ARG;
-    k_mse<<<nblk(n), TB, 0, (cudaStream_t)stream>>>(pred, target, dpred, dpred_bf16, loss, n, scale, w, w_period,
-                                                   w_len);
-    FNO_RET(stream);
+    return run_mse(pred, target, dpred, dpred_bf16, loss, n, scale, w, w_period, w_len, stream);
 }
 
 int gf_fno_add(const float *x, const float *y, float *out, void *out_bf16, long long n, void *stream) {

@@ -62,6 +62,13 @@ def _lib():
         "gf_fno_modes": [vp, vp, vp, i, i, vp],
         "gf_fno_inv_h": [vp, vp, vp, i, i, i, i, vp],
         "gf_fno_proj": [vp, vp, vp, vp, vp, vp, vp, vp, i, i, vp],
+        "gf_fno_colsum_bf16": [vp, vp, ll, i, i, vp],
+        "gf_fno_proj_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, vp],
+        "gf_fno_row_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, vp],
+        "gf_fno_inv_h_bwd": [vp, vp, vp, i, i, i, i, vp],
+        "gf_fno_modes_bwd": [vp, vp, vp, vp, vp, i, i, vp],
+        "gf_fno_fwd_h_bwd": [vp, vp, vp, i, i, i, i, vp],
+        "gf_fno_wgrad": [vp, i, vp, i, i, vp, ll, i, vp],
     }
     for n, a in sig.items():
         fn = getattr(lib, n)
@@ -227,14 +234,18 @@ class Fno:
     def colsum(self, X, out, rows, cols):
         _ck(self.lib.gf_fno_colsum(_p(X), _p(out), rows, cols, 0, self.s), "colsum")
 
+    @staticmethod
+    def wgrad_chunks(M):
+        """how many chunks the M rows of a weight gradient are summed in"""
+        for cand in (512, 384, 256, 128, 64, 32, 16, 8, 4, 2):
+            if M % cand == 0 and (M // cand) % 8 == 0 and M // cand >= 1024:
+                return cand
+        return 1
+
     def wgrad(self, dz_rows, x_rows, M, n_out, n_in, out):
         """out[n_out, n_in] = dz^T x over M rows, split over K chunks"""
         torch = self.torch
-        S = 1
-        for cand in (512, 384, 256, 128, 64, 32, 16, 8, 4, 2, 1):
-            if (M % cand == 0 and (M // cand) % 8 == 0 and M // cand >= 1024) or cand == 1:
-                S = cand
-                break
+        S = self.wgrad_chunks(M)
         Kc = M // S
         # each chunk of Kc rows transposed on its own: dzT[s] = dz[s*Kc:(s+1)*Kc]^T
         dzT = torch.empty((S, n_out, Kc), dtype=torch.bfloat16, device="cuda")
@@ -308,7 +319,7 @@ class Fno:
             if train:
                 saved["v"].append(v)
                 saved["z"].append(zl)
-                saved["spec"].append((U, self.modes_t(l)))
+                saved["spec"].append((U, None))
                 v, vn, U = vn, new(M, Cc), new(cfg.modes, B, 2 * Cc)
             else:
                 v, vn = vn, v
@@ -376,6 +387,7 @@ class Fno:
         H, W, Cc, m2, Q = cfg.H, cfg.W, cfg.C, cfg.m2, cfg.Q
         bf = torch.bfloat16
         U, RmT = sp
+        RmT = self.modes_t(l) if RmT is None else RmT
         ds = torch.empty((B, H, Cc, W), dtype=bf, device="cuda")
         self.tr(ds_cl, ds, B * H, W, Cc)
         dZt = torch.empty((B, H, Cc, 2 * m2), dtype=bf, device="cuda")
@@ -409,6 +421,50 @@ class Fno:
         self.tr(dvt, dv, B * H, Cc, W)
         return dv
 
+    def wgrad_fused(self, A, na, Bm, nb, M, out, transposed=0):
+        """out = A^T Bm (transposed: its transpose) over M rows, in the chunks of wgrad()"""
+        S = self.wgrad_chunks(M)
+        part = self.torch.empty((S, na * nb), dtype=self.torch.float32, device="cuda")
+        _ck(self.lib.gf_fno_wgrad(_p(A), na, _p(Bm), nb, transposed, _p(part), M, S, self.s), "wgrad")
+        _ck(self.lib.gf_fno_sum_batches(_p(part), _p(out), S, na * nb, 0, self.s), "sum_batches")
+
+    def backward_fused(self, dout):
+        """backward() by the fused kernels"""
+        torch, cfg, sv = self.torch, self.cfg, self.saved
+        B, H, W, Cc, m2, Q = dout.shape[0], cfg.H, cfg.W, cfg.C, cfg.m2, cfg.Q
+        rows, M, K2, wb, lib, s = B * H, B * H * W, 2 * m2, sv["wb"], self.lib, self.s
+
+        def new(*shape, dtype=torch.bfloat16):
+            return torch.empty(shape, dtype=dtype, device="cuda")
+
+        IWT = self.mat["IWT"]
+        df1, df = new(M, cfg.P, dtype=torch.float32), new(M, Cc, dtype=torch.float32)
+        dzp, dz, dn, dZ, dXw = new(M, cfg.P), new(M, Cc), new(M, Cc), new(rows, K2, Cc), new(rows, K2, Cc)
+        dV, dU = new(cfg.modes, B, 2 * Cc), new(cfg.modes, B, 2 * Cc)
+        d2 = dout.reshape(M, cfg.cout)
+        self.wgrad_fused(sv["h"], cfg.P, d2, cfg.cout, M, self.g["p2_w"], 1)
+        _ck(lib.gf_fno_colsum_bf16(_p(d2), _p(self.g["p2_b"]), M, cfg.cout, 0, s), "colsum")
+        _ck(lib.gf_fno_proj_bwd(_p(d2), _p(sv["zp"]), _p(wb["p1_w"]), _p(wb["p2_w"]), _p(IWT), _p(dzp), _p(df1),
+                                _p(dz), _p(df), _p(dZ), rows, W, K2, s), "proj_bwd")
+        self.colsum(df1, self.g["p1_b"], M, cfg.P)
+        self.wgrad_fused(dzp, cfg.P, sv["vL"], Cc, M, self.g["p1_w"])
+        for l in reversed(range(cfg.layers)):
+            # dz: gradient of layer l's pre-activations, dZ: its transform along W
+            self.colsum(df, self.g[f"b{l}"], M, Cc)
+            self.wgrad_fused(dz, Cc, sv["v"][l], Cc, M, self.g[f"w{l}"])
+            _ck(lib.gf_fno_inv_h_bwd(_p(dZ), _p(self.mat["IHT"]), _p(dV), B, H, m2, Q, s), "inv_h_bwd")
+            _ck(lib.gf_fno_modes_bwd(_p(dV), _p(sv["spec"][l][0]), _p(self.p[f"R{l}"]), _p(dU), _p(self.g[f"R{l}"]),
+                                     B, cfg.modes, s), "modes_bwd")
+            _ck(lib.gf_fno_fwd_h_bwd(_p(dU), _p(self.mat["FHT"]), _p(dXw), B, H, m2, Q, s), "fwd_h_bwd")
+            z = sv["z"][l - 1] if l else None
+            _ck(lib.gf_fno_row_bwd(_p(dz), _p(dXw), _p(self.mat["FW"]), _p(wb[f"w{l}"]), _p(z), _p(IWT), _p(dn), _p(df),
+                                   _p(dZ) if l else None, rows, W, K2, s), "row_bwd")
+            dz, dn = dn, dz
+        self.colsum(df, self.g["lift_b"], M, Cc)
+        self.wgrad_fused(dz, Cc, sv["x"].reshape(M, cfg.cin), cfg.cin, M, self.g["lift_w"])
+        self.saved = None
+        return self.g
+
     def backward(self, dout):
         """dout: gradient of the loss w.r.t. the output, BF16 [B, H, W, cout]"""
         torch, cfg = self.torch, self.cfg
@@ -416,6 +472,9 @@ class Fno:
         B = dout.shape[0]
         M = B * cfg.H * cfg.W
         bf = torch.bfloat16
+        # batches of eight and whole 128-row tiles per chunk of the weight gradients
+        if self.fused and B % 8 == 0 and (M // self.wgrad_chunks(M)) % 128 == 0:
+            return self.backward_fused(dout)
         wb = sv["wb"]
         d2 = dout.reshape(M, cfg.cout)
         self.wgrad(d2, sv["h"], M, cfg.cout, cfg.P, self.g["p2_w"])

@@ -60,6 +60,7 @@ int gf_fno_expand_modes(const float *R, void *Rm, void *RmT, int modes, int C, v
 int gf_fno_modes_grad(const float *dRm, float *dR, int modes, int C, void *stream);
 /* out[c] (+)= sum_r X[r][c]; dst[i] (+)= sum_b src[b][i]. */
 int gf_fno_colsum(const float *X, float *out, long long rows, int cols, int accum, void *stream);
+int gf_fno_colsum_bf16(const void *X, float *out, long long rows, int cols, int accum, void *stream);
 int gf_fno_sum_batches(const float *src, float *dst, int nb, long long n, int accum, void *stream);
 /* Adam (bias-corrected, decoupled from the loss scale), step counts from 1. */
 int gf_fno_adam(float *p, const float *g, float *m, float *v, long long n, float lr, float b1, float b2, float eps,
@@ -113,6 +114,29 @@ int gf_fno_modes(const void *U, const float *R, void *V, int B, int modes, void 
 int gf_fno_inv_h(const void *V, const void *IH, void *Z, int B, int H, int m2, int Q, void *stream);
 int gf_fno_proj(const void *v, const void *P1, const float *b1, const void *P2, const float *b2, float *zp, void *h,
                 float *out, int rows, int W, void *stream);
+
+/* ---- the backward pass in fused kernels, under the same shapes ----
+ * Gradients BF16, and (df1, df) FP32 for the bias gradients (gf_fno_colsum).
+ * gf_fno_proj_bwd: dzp [rows W][128] = (dout P2) GELU'(zp), dzo [rows W][64] =
+ * dzp P1, dZ [rows][K2][64] = IWT dzo.
+ * gf_fno_row_bwd: dzo = (dz Wl + FW^T dXw) GELU'(z) (z NULL: no factor), dZ =
+ * IWT dzo (NULL: not computed).
+ * gf_fno_inv_h_bwd: dZ -> dV[(k2, q)][b][(c, re|im)].
+ * gf_fno_modes_bwd: dU[mode][b][re|im][c] and dR (FP32) from dV and U.
+ * gf_fno_fwd_h_bwd: dU -> dXw [B][H][K2][64].
+ * gf_fno_wgrad: part[s][j][n] = sum over the s-th of `chunks` equal chunks
+ * (multiples of 128 points) of A[m][j] B[m][n], A [M][na = 64 or 128], B
+ * [M][nb]; transposed (nb = 16): part[s][n][j]. */
+int gf_fno_proj_bwd(const void *dout, const float *zp, const void *P1, const void *P2, const void *IWT, void *dzp,
+                    float *df1, void *dzo, float *df, void *dZ, int rows, int W, int K2, void *stream);
+int gf_fno_row_bwd(const void *dz, const void *dXw, const void *FW, const void *Wl, const float *z, const void *IWT,
+                   void *dzo, float *df, void *dZ, int rows, int W, int K2, void *stream);
+int gf_fno_inv_h_bwd(const void *dZ, const void *IHT, void *dV, int B, int H, int m2, int Q, void *stream);
+int gf_fno_modes_bwd(const void *dV, const void *U, const float *R, void *dU, float *dR, int B, int modes,
+                     void *stream);
+int gf_fno_fwd_h_bwd(const void *dU, const void *FHT, void *dXw, int B, int H, int m2, int Q, void *stream);
+int gf_fno_wgrad(const void *A, int na, const void *B, int nb, int transposed, float *part, long long M, int chunks,
+                 void *stream);
 
 #ifdef __cplusplus
 }
