@@ -15,6 +15,7 @@
 #include "../../include/geoflac_gb300.h"
 #include "gf_ctx.h"
 #include "gf_internal.h"
+#include "gf_math.h"
 #include "gf_member.h"
 
 namespace {
@@ -23,6 +24,7 @@ struct GraphEntry {
     unsigned sig;
     cudaGraphExec_t exec;
     long long nlaunch;
+    int nmarkers; // that change_phase's launch covers (steps with it)
 };
 
 } // namespace
@@ -145,6 +147,8 @@ void fill_params(DevParams &P, const gf_params &p) {
         // the device's per-element expressions, evaluated once per phase
         // (same IEEE operations; host code is built without contraction)
         P.bulkm[k] = p.rl[k] + 2.0 * p.rm[k] / 3.0;
+        P.v_pw[k] = 1.0 / p.pln[k] - 1.0;
+        P.v_pa[k] = gfm::pow(0.75 * p.acoef[k], -1.0 / p.pln[k]);
         P.hsoft[k] = (p.plstrain2[k] != p.plstrain1[k])
                          ? (p.cohesion2[k] - p.cohesion1[k]) / (p.plstrain2[k] - p.plstrain1[k])
                          : 0.0;
@@ -591,12 +595,20 @@ void advance_host(gf_ctx *c, unsigned sig) {
 }
 
 int run_graph(gf_ctx *c, unsigned sig) {
-    for (auto &g : c->graphs)
-        if (g.sig == sig) {
-            GF_CK(cudaGraphLaunch(g.exec, c->s));
-            c->launches += g.nlaunch;
-            return GF_OK;
+    for (size_t k = 0; k < c->graphs.size(); ++k) {
+        GraphEntry &g = c->graphs[k];
+        if (g.sig != sig) continue;
+        // of a captured step only change_phase's launch depends on anything
+        // that changes: it covers the markers there were
+        if ((sig & 2u) && g.nmarkers != c->nmarkers) {
+            cudaGraphExecDestroy(g.exec);
+            c->graphs.erase(c->graphs.begin() + k);
+            break;
         }
+        GF_CK(cudaGraphLaunch(g.exec, c->s));
+        c->launches += g.nlaunch;
+        return GF_OK;
+    }
     cudaGraph_t graph;
     long long before = c->launches;
     GF_CK(cudaStreamBeginCapture(c->s, cudaStreamCaptureModeThreadLocal));
@@ -608,7 +620,7 @@ int run_graph(gf_ctx *c, unsigned sig) {
     if (e != cudaSuccess) return cuda_err(e, "cudaGraphInstantiate");
     long long n = c->launches - before;
     c->launches = before;
-    c->graphs.push_back(GraphEntry{sig, exec, n});
+    c->graphs.push_back(GraphEntry{sig, exec, n, c->nmarkers});
     GF_CK(cudaGraphLaunch(exec, c->s));
     c->launches += n;
     return GF_OK;
@@ -959,7 +971,6 @@ int gf_marker2elem(gf_ctx *c) {
         enqueue_marker2elem<double>(c, g, a);
     GF_CK(cudaMemcpyAsync(&c->nmarkers, c->A.nmarkers, sizeof(int), cudaMemcpyDeviceToHost, c->s));
     GF_CK(cudaStreamSynchronize(c->s));
-    drop_graphs(c); // change_phase's launch covers nmarkers markers
     return take_status(c);
 }
 
@@ -1089,10 +1100,7 @@ static int sync_markers_after_resurface(gf_ctx *c) {
     int nm = c->nmarkers;
     GF_CK(cudaMemcpyAsync(&nm, c->A.nmarkers, sizeof(int), cudaMemcpyDeviceToHost, c->s));
     GF_CK(cudaStreamSynchronize(c->s));
-    if (nm != c->nmarkers) {
-        c->nmarkers = nm;
-        drop_graphs(c);
-    }
+    c->nmarkers = nm; // (run_graph captures change_phase anew)
     return GF_OK;
 }
 
@@ -1183,7 +1191,6 @@ int gf_remesh(gf_ctx *c) {
     GF_CK(cudaMemsetAsync(c->A.dhacc_correction, 0, sizeof(double) * c->p.nx, c->s));
     GF_CK(cudaMemcpyAsync(&c->nmarkers, c->A.nmarkers, sizeof(int), cudaMemcpyDeviceToHost, c->s));
     GF_CK(cudaStreamSynchronize(c->s));
-    drop_graphs(c);
     c->need_remeshing = 0;
     return take_status(c);
 }

@@ -37,6 +37,8 @@ struct DevParams {
     float f_alfa[GF_MAXPH], f_beta[GF_MAXPH], f_fmagma_max, f_rho_magma;
     double diffu[GF_MAXPH]; // conduct / den / cp (dt_mass.f90:130)
     double bulkm[GF_MAXPH]; // rl + 2 rm / 3 (fl_rheol.f90:192)
+    // Eff_visc's per-phase factors (matprops.f90:186-189): 1/n - 1 and (3/4 A)^(-1/n)
+    double v_pw[GF_MAXPH], v_pa[GF_MAXPH];
     double hsoft[GF_MAXPH]; // (cohesion2 - cohesion1) / (plstrain2 - plstrain1) (rh_plastic.f90:264)
     // shear heating's per-phase factor (fl_rheol.f90:344-361): lambda / den_el
     double sh_lam_den[GF_MAXPH];

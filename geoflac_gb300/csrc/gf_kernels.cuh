@@ -520,12 +520,14 @@ __device__ double eff_visc(const DevParams &P, const DevArrays &A, const GfDims 
     double srat = (double)((const R *)A.e2sr)[e];
     if (srat == 0) srat = P.vbc / P.rxbo;
     ev = 0.0;
+    // the logarithm of gfm::pow(srat, .), shared by the phases
+    const double lsr = srat > 0.0 ? gfm::log(srat) : 0.0;
     for (int k = 0; k < P.nphase; ++k) {
         double ratio = A.phase_ratio[gf_pr(d, e, k)];
         if (ratio < 0.01) continue;
-        double pw = 1.0 / P.pln[k] - 1.0;
-        double pw1 = -1.0 / P.pln[k];
-        double vis = 0.25 * gfm::pow(srat, pw) * gfm::pow(0.75 * P.acoef[k], pw1) *
+        const double pw = P.v_pw[k];
+        const double sp = srat > 0.0 && srat != 1.0 && pw != 0.0 ? gfm::exp(pw * lsr) : gfm::pow(srat, pw);
+        double vis = 0.25 * sp * P.v_pa[k] *
                      gfm::exp((P.eactiv[k] + P.vactiv[k] * pres) / (P.pln[k] * r * (tmpr + 273.0))) * 1e6;
         if (vis < P.v_min) vis = P.v_min;
         if (vis > P.v_max) vis = P.v_max;
