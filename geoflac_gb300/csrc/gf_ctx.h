@@ -62,7 +62,9 @@ struct DevClock {
     int status_aux; // element/node index of the first error
     int therm_sweeps_used;  // sweeps of the last fl_therm (converged at the last)
     int therm_unconverged;  // fl_therm calls that hit the sweep cap
-    int therm_flags[GF_THERM_KMAX]; // sweep k changed some value
+    // FP64 thermal sweeps: CTAs that finished sweep k (low half) and, of them,
+    // those that changed some value (high half)
+    int therm_flags[GF_THERM_KMAX];
 };
 
 // Device arrays of a context.  In GF_MODE_MIXED the element fields listed
@@ -90,7 +92,7 @@ struct DevArrays {
     // scratch
     double *t_delta0, *t_delta1; // thermal sweep iterates (node)
     double *t_coef;              // thermal per-element coefficients (18 per element)
-    uint8_t *t_chg;              // FP64 thermal sweeps: node changed in sweep k (2 x N, by parity)
+    uint8_t *t_chg;              // FP64 thermal sweeps: one bit per node, changed in sweep k (by parity)
     double *t_pred;              // FP64 thermal sweeps: each node's last increment (the next start)
     double *p_ref; // mixed: per-element reference pressure; stored normal stresses are total + p_ref
     double *e_dens;                                   // per-element density (rmasses)
@@ -142,7 +144,6 @@ struct GfLaunch {
     int idt_scale;   // host copy of the mass-scaling mode (selects launches)
     int advance_time; // fold par.f90's time += dt into the step's last kernel
     double arc_rate;  // arc extrusion rate 1 - ratio_mantle_mzone - ratio_crust_mzone (diff_topo)
-    unsigned *therm_bar; // grid barrier of the FP64 thermal sweeps (arrivals, generation, error flag)
     int node_terms;      // FP64 fl_node: A.n_frc holds the terms of the current stresses and mesh
 };
 

@@ -711,75 +711,13 @@ template <class R> __global__ void __launch_bounds__(GF_THREADS) k_move_elem(Dev
 }
 
 // ======================================================================
-// fl_therm (fl_therm.f90:393-598).
-//
-// The reference updates temp in place, i outer and j inner: node (j,i) reads
-// new values at its upstream neighbours (j-1,i), (j,i-1), (j+1,i-1) and old
-// values at itself and downstream.  Its result is the unique fixed point of
-//   Tnew(n) = f_n(Tnew(upstream), Told(rest))
-// with f_n the reference's floating-point expression.  The system is lower
-// triangular, so iterating Jacobi-style sweeps of f_n from Told reaches that
-// fixed point exactly (bit for bit) after finitely many sweeps; each sweep
-// contracts the distance by ~kappa*dt/h^2, so a handful of sweeps suffice.
-// A sweep that changes no value proves convergence; later sweeps exit at once.
-//
-// k_therm_prep computes, per element, everything of the triangles A and B that
-// does not depend on temperature (fl_therm.f90:424-567): the shape-derivative
-// products K_ab, real_area13 = (1/area)/6, 0.5*diff/area and
-// src*real_area13, each with the reference's operations.
-
-#define GF_TC 18 // doubles per element: KA[6], KB[6], raA, raB, preA, preB, srA, srB
+// fl_therm (fl_therm.f90:393-598): the FP64 path in gf_therm64.cuh, the mixed
+// path's two sweeps below.
+#define GF_TC 18 // coefficients per element: KA[6], KB[6], raA, raB, preA, preB, srA, srB
 // K index of (a,b), a,b in 0..2 (symmetric)
 __device__ __forceinline__ int kidx(int a, int b) {
     int lo = a < b ? a : b, hi = a < b ? b : a;
     return lo == 0 ? hi : (lo == 1 ? 2 + hi : 5);
-}
-
-template <class R> __device__ __forceinline__ void b_k_therm_prep(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d, double *__restrict__ tc, GF_IDX e) {
-    if (e == 0)
-        for (int k = 0; k < GF_THERM_KMAX; ++k) C->therm_flags[k] = 0; // before any sweep runs
-    if (e >= d.E) return;
-    const DevParams &P = *Pp;
-    int j, i;
-    elem_ji(d, e, j, i);
-    int iph = A.iphase[e] - 1;
-    double cp_eff = P.cp[iph];
-    double dissip = (P.ishearh == 1 && P.itherm != 2) ? (double)((const R *)A.shrheat)[e] : 0.0;
-    // conduct / den / cp of the phase: the same two IEEE divisions as the
-    // reference's cond_eff / dens / cp_eff, taken once per phase at set-up
-    double diff = P.diffu[iph];
-    // the source's quotients by den and cp (gf_ddiv: the bits of the IEEE
-    // divisions, off the FP64 pipe)
-    double src = gf_ddiv(A.source[e] + gf_ddiv(dissip, P.den[iph]), cp_eff);
-    Quad q;
-    load_quad(A.cord, d, j, i, q);
-    const R *area = (const R *)A.area;
-    const GF_IDX E = d.E;
-    // triangle A: local vertices (q1,q2,q3); triangle B: (q3,q2,q4)
-    const int tv[2][3] = {{0, 1, 2}, {2, 1, 3}};
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-        double a = (double)area[gf_ek(d, e, t)];
-        double y1 = q.y[tv[t][0]], y2 = q.y[tv[t][1]], y3 = q.y[tv[t][2]];
-        double x1 = q.x[tv[t][0]], x2 = q.x[tv[t][1]], x3 = q.x[tv[t][2]];
-        // (products on the integer pipes: gf_mul, the bits of the FP64
-        // multiply, which this FP64-bound kernel has few enough of)
-        double dd[3] = {gf_mul(y2 - y3, a), gf_mul(y3 - y1, a), gf_mul(y1 - y2, a)};
-        double zz[3] = {gf_mul(x3 - x2, a), gf_mul(x1 - x3, a), gf_mul(x2 - x1, a)};
-#pragma unroll
-        for (int m = 0; m < 3; ++m)
-#pragma unroll
-            for (int n = m; n < 3; ++n) tc[(t * 6 + kidx(m, n)) * E + e] = gf_mul(dd[m], dd[n]) + gf_mul(zz[m], zz[n]);
-        double inv_area = gf_rcp(a); // RN(1/a) off the FP64 pipe
-        double ra = gf_ddiv(inv_area, 6.0);
-        tc[(12 + t) * E + e] = ra;
-        tc[(14 + t) * E + e] = gf_mul(gf_scale<-1>(diff), inv_area);
-        tc[(16 + t) * E + e] = gf_mul(src, ra);
-    }
-}
-template <class R> __global__ void __launch_bounds__(GF_THREADS) k_therm_prep(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d, double *__restrict__ tc) {
-    gf_pdl_entry();
-    b_k_therm_prep<R>(Pp, C, A, d, tc, (GF_IDX)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // Temperature after the boundary conditions of fl_therm.f90:573-598 (top
@@ -801,73 +739,6 @@ __device__ __forceinline__ double therm_bc_value(const DevParams &P, const DevAr
         }
     }
     return src(gf_node(d, j, ii));
-}
-
-// One node of sweep k.  Tup holds the current iterate; the start (the
-// iterate before sweep 0) is Told + the previous step's increment
-// (A.t_pred), a guess: the fixed point does not depend on it, only how many
-// nodes the sweeps recompute before they reach it (on the 1000x300 model
-// sweep 2 recomputes 16 % of the nodes instead of 82 %).  Self and
-// downstream values always come from Told (A.temp).  Returns whether the
-// node's value changed.  The iterates and the change flags are written by
-// other CTAs of the same (persistent) launch, so their loads bypass L1
-// (__ldcg).
-__device__ __forceinline__ bool therm_sweep_node(DevArrays A, GfDims d, double dt, const double *__restrict__ tc,
-                                                 const double *Tup, double *Tout, int k, GF_IDX n) {
-    int j, i;
-    node_ji(d, n, j, i);
-    // A node's sweep-k value depends on sweep k-1 only through its upstream
-    // neighbours (j-1,i), (j,i-1), (j+1,i-1); if none of them changed in
-    // sweep k-1 its value is the one it had (the same inputs give the same
-    // result), and the FP64 evaluation is skipped.
-    if (k > 0) {
-        const uint8_t *prev = A.t_chg + (GF_IDX)((k - 1) & 1) * d.N;
-        bool recompute = (j != 0 && __ldcg(prev + gf_node(d, j - 1, i))) ||
-                         (i != 0 && __ldcg(prev + gf_node(d, j, i - 1))) ||
-                         (i != 0 && j != d.nz - 1 && __ldcg(prev + gf_node(d, j + 1, i - 1)));
-        if (!recompute) {
-            Tout[n] = __ldcg(Tup + n);
-            return false;
-        }
-    }
-    const int nx = d.nx, nz = d.nz;
-    const GF_IDX E = d.E;
-    const double *T = A.temp;
-    double rhs = 0.0, area_n = 0.0;
-    auto Nd = [&](int jj, int ii) { return gf_node(d, jj, ii); };
-    const double *pred = A.t_pred;
-    auto start = [&](GF_IDX m) { return T[m] + pred[m]; };
-    auto U = [&](int jj, int ii) { return k == 0 ? start(Nd(jj, ii)) : __ldcg(Tup + Nd(jj, ii)); };
-    // triangle t of element e; vs = local index of the updated node; the
-    // three (local vertex, temperature) terms in the reference's order
-    // (products on the integer pipes: gf_mul, the bits of the FP64 multiply;
-    // the first sweeps are bound by the FP64 pipe)
-    auto tri = [&](GF_IDX e, int t, int vs, int v0, double T0, int v1, double T1, int v2, double T2) {
-        double ra = tc[(12 + t) * E + e];
-        area_n = area_n + ra;
-        const double *K = tc + (GF_IDX)t * 6 * E + e;
-        rhs = rhs + tc[(16 + t) * E + e] -
-              gf_mul(tc[(14 + t) * E + e], gf_mul(T0, K[kidx(v0, vs) * E]) + gf_mul(T1, K[kidx(v1, vs) * E]) +
-                                               gf_mul(T2, K[kidx(v2, vs) * E]));
-    };
-    double Ts = T[n];
-    if (j != 0 && i != 0) // element (j-1,i-1), triangle B: vertices (j-1,i), (j,i-1), node
-        tri(gf_elem(d, j - 1, i - 1), 1, 2, 0, U(j - 1, i), 1, U(j, i - 1), 2, Ts);
-    if (j != 0 && i != nx - 1) { // element (j-1,i), triangles A and B
-        GF_IDX e = gf_elem(d, j - 1, i);
-        tri(e, 0, 1, 0, U(j - 1, i), 1, Ts, 2, T[Nd(j - 1, i + 1)]);
-        tri(e, 1, 1, 0, T[Nd(j - 1, i + 1)], 1, Ts, 2, T[Nd(j, i + 1)]);
-    }
-    if (j != nz - 1 && i != 0) { // element (j,i-1), triangles A and B
-        GF_IDX e = gf_elem(d, j, i - 1);
-        tri(e, 0, 2, 0, U(j, i - 1), 1, U(j + 1, i - 1), 2, Ts);
-        tri(e, 1, 0, 0, Ts, 1, U(j + 1, i - 1), 2, T[Nd(j + 1, i)]);
-    }
-    if (j != nz - 1 && i != nx - 1) // element (j,i), triangle A
-        tri(gf_elem(d, j, i), 0, 0, 0, Ts, 1, T[Nd(j + 1, i)], 2, T[Nd(j, i + 1)]);
-    double tn = Ts + gf_ddiv(gf_mul(rhs, dt), area_n);
-    Tout[n] = tn;
-    return !gf_deq(tn, k == 0 ? start(n) : __ldcg(Tup + n));
 }
 
 // Bounded grid barrier of a co-resident (cooperative) launch: generation
@@ -901,55 +772,6 @@ __device__ bool gf_grid_barrier(unsigned *bar, GF_IDX limit) {
     }
     __syncthreads();
     return !bad;
-}
-
-// The FP64 thermal update after k_therm_prep, in one co-resident launch:
-// sweeps until one changes nothing (at most kmax; grid barrier between
-// sweeps, every CTA reads the same flag after it), then the boundary
-// conditions and temp0 = temp (fl_therm.f90:53, 577-598) from the last
-// sweep's buffer.  Node n is always handled by the same thread.
-__global__ void __launch_bounds__(GF_THREADS) k_therm_sweeps(const DevParams *__restrict__ Pp, DevClock *__restrict__ C,
-                                                            DevArrays A, GfDims d, const double *__restrict__ tc,
-                                                            double *b0, double *b1, int kmax, int keep_temp0,
-                                                            unsigned *bar) {
-    const GF_IDX stride = (GF_IDX)gridDim.x * blockDim.x; // a multiple of 32
-    const GF_IDX gt = (GF_IDX)blockIdx.x * blockDim.x + threadIdx.x;
-    const GF_IDX npad = (d.N + 31) / 32 * 32; // equal trip counts within a warp (the vote)
-    const double dt = C->dt;
-    int kc = kmax; // the first sweep that changed nothing
-    for (int k = 0; k < kmax; ++k) {
-        const double *up = k == 0 ? A.temp : ((k - 1) & 1 ? b1 : b0);
-        double *out = (k & 1) ? b1 : b0;
-        bool any = false;
-        for (GF_IDX n = gt; n < npad; n += stride) {
-            bool changed = n < d.N && therm_sweep_node(A, d, dt, tc, up, out, k, n);
-            if (n < d.N) A.t_chg[(GF_IDX)(k & 1) * d.N + n] = changed ? 1 : 0;
-            any = any || changed;
-        }
-        if (__any_sync(0xffffffffu, any) && (threadIdx.x & 31) == 0) C->therm_flags[k] = 1;
-        if (!gf_grid_barrier(bar, 1LL << 24)) {
-            if (gt == 0) set_status(C, GF_ERR_TIMEOUT, k);
-            return;
-        }
-        if (*(volatile int *)&C->therm_flags[k] == 0) {
-            kc = k;
-            break;
-        }
-    }
-    if (gt == 0) {
-        C->therm_sweeps_used = kc + 1;
-        if (kc == kmax) C->therm_unconverged += 1;
-    }
-    const double *src = ((kc < kmax ? kc : kmax - 1) & 1) ? b1 : b0;
-    for (GF_IDX n = gt; n < d.N; n += stride) {
-        int j, i;
-        node_ji(d, n, j, i);
-        double t = therm_bc_value(*Pp, A, d, [src](GF_IDX m) { return __ldcg(src + m); }, j, i);
-        const double told = A.temp[n];
-        if (!keep_temp0) A.temp0[n] = told;
-        A.temp[n] = t;
-        A.t_pred[n] = t - told; // the next step's start: its Told + this increment
-    }
 }
 
 // ---- mixed precision: FP32 coefficients, two sweeps.
@@ -1792,6 +1614,9 @@ inline void gf_launch_pdl(void (*kern)(KArgs...), unsigned grid, unsigned thread
     lc.numAttrs = 1;
     cudaLaunchKernelEx(&lc, kern, (KArgs)args...);
 }
+#ifdef GF_FP64_UNIT
+#include "gf_therm64.cuh"
+#endif
 #define GF_LAUNCH(kern, n, ...) GF_LAUNCH_T(kern, n, GF_THREADS, __VA_ARGS__)
 #define GF_LAUNCH_T(kern, n, thr, ...)                                                                                      \
     do {                                                                                                               \
@@ -1859,36 +1684,9 @@ template <class R> void GfKernels<R>::therm(const GfLaunch &g, int sweeps, int k
         therm_sweeps(g);
         return;
     }
-    int kmax = sweeps > 0 ? (sweeps < GF_THERM_KMAX ? sweeps : GF_THERM_KMAX) : GF_THERM_KMAX;
-    GF_LAUNCH(k_therm_prep<R>, g.d.E, g.P, g.C, g.A, g.d, g.A.t_coef);
-    // the sweeps and the boundary pass: one co-resident launch
-    static int occ[64] = {0}, sms[64] = {0};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    dev = dev & 63;
-    if (occ[dev] == 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[dev], k_therm_sweeps, GF_THREADS, 0);
-        cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
-        if (occ[dev] <= 0) occ[dev] = 1;
-    }
-    const GF_IDX need = (g.d.N + GF_THREADS - 1) / GF_THREADS;
-    const GF_IDX cap = (GF_IDX)occ[dev] * sms[dev];
-    // arrivals and the error flag start at zero in every launch (the
-    // generation counter only has to change)
-    cudaMemsetAsync(g.therm_bar, 0, sizeof(unsigned), g.s);
-    cudaMemsetAsync(g.therm_bar + 2, 0, sizeof(unsigned), g.s);
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3((unsigned)(need < cap ? need : cap));
-    lc.blockDim = dim3(GF_THREADS);
-    lc.stream = g.s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    lc.attrs = attr;
-    lc.numAttrs = 1;
-    cudaLaunchKernelEx(&lc, k_therm_sweeps, g.P, g.C, g.A, g.d, (const double *)g.A.t_coef, g.A.t_delta0,
-                       g.A.t_delta1, kmax, keep_temp0, g.therm_bar);
-    ++*g.launches;
+#ifdef GF_FP64_UNIT
+    therm_launch(g, sweeps > 0 ? (sweeps < GF_THERM_KMAX ? sweeps : GF_THERM_KMAX) : GF_THERM_KMAX, keep_temp0);
+#endif
 }
 
 template <class R> void GfKernels<R>::rheol(const GfLaunch &g, int update_visc, int avg_mode) {
