@@ -151,10 +151,11 @@ struct GfLaunch {
 template <class R> struct GfKernels {
     // keep_temp0: temp0 was taken before the magma sub-model changed temp
     static void therm(const GfLaunch &g, int sweeps, int keep_temp0 = 0);
-    // mixed: the coefficient pass and the two sweeps + boundary pass of
-    // therm, for steps that run the sweeps beside fl_rheol / fl_node
-    static void therm_prep(const GfLaunch &g);
-    static void therm_sweeps(const GfLaunch &g);
+    // mixed: therm, rheol (no viscosity update) and node of a step where these
+    // read nothing therm writes; `move`: and fl_move, where it is the
+    // coordinate update and move_elem alone and no boundary condition of
+    // therm reads coordinates
+    static void step_forces(const GfLaunch &g, int avg_mode, int move);
     static void rheol(const GfLaunch &g, int update_visc, int avg_mode);
     static void node(const GfLaunch &g);
     // mixed: the corner forces of the current stresses (fl_rheol writes them

@@ -887,6 +887,57 @@ __global__ void __launch_bounds__(GF_THREADS) k_therm_apply32(const DevParams *_
     b_k_therm_apply32(Pp, A, d, tnew, (GF_IDX)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
+// ---- mixed precision: the ordinary step in four phases.
+// On steps where fl_rheol and fl_node read nothing that the thermal update
+// writes (no viscosity update, no change_phase, no thermal stress, no Winkler
+// foundation, whose pressure reads the new temperatures) the thermal update
+// shares launches with the mechanics:
+//   a: fl_rheol             beside the sweep coefficients (from the shear
+//                             heating before fl_rheol's averaging rewrites it)
+//   b: fl_node              beside sweep 0 and fl_rheol's averaging
+//   c: the coordinates      beside sweep 1 (the sweeps read no coordinates)
+//   d: fl_move's elements   beside the temperatures' boundary conditions
+// so a step is four dependent launches.  Blocks of one launch take one part
+// each (grid y), the longer part first: in one thread after another the
+// parts' memory latencies add up (no load moves above the stores of the part
+// before), which costs more than the launches saved.
+__global__ void __launch_bounds__(GF_THREADS, 3) k_step_a(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d) {
+    gf_pdl_entry();
+    const GF_IDX e = (GF_IDX)blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.y == 0)
+        b_k_rheol<float>(Pp, C, A, d, 0, 0, e);
+    else
+        b_k_therm_prep32(Pp, A, d, (float *)A.t_coef, e);
+}
+__global__ void __launch_bounds__(GF_THREADS) k_step_b(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d, int avg_mode) {
+    gf_pdl_entry();
+    const GF_IDX n = (GF_IDX)blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.y == 0)
+        b_k_node<float>(Pp, C, A, d, n);
+    else if (blockIdx.y == 1)
+        b_k_therm_sweep32(Pp, C, A, d, (const float *)A.t_coef, (float *)A.t_delta0, A.t_delta1, 0, n);
+    else
+        b_k_rheol_avg<float>(C, A, d, avg_mode == 2 ? 1 : 0, n);
+}
+__global__ void __launch_bounds__(GF_THREADS) k_step_c(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d, int avg_mode) {
+    gf_pdl_entry();
+    const GF_IDX n = (GF_IDX)blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.y == 0) {
+        b_k_therm_sweep32(Pp, C, A, d, (const float *)A.t_coef, (float *)A.t_delta0, A.t_delta1, 1, n);
+        if (avg_mode == 2 && n == 0) b_k_rheol_clock(C, 1);
+    } else if (n < d.N) {
+        b_k_move_cord(C, A, d, (GF_IDX)(blockIdx.y - 1) * d.N + n);
+    }
+}
+__global__ void __launch_bounds__(GF_THREADS) k_step_d(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d, int advance_time) {
+    gf_pdl_entry();
+    const GF_IDX n = (GF_IDX)blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.y == 0)
+        b_k_move_elem<float>(C, A, d, advance_time, n);
+    else
+        b_k_therm_apply32(Pp, A, d, A.t_delta1, n);
+}
+
 // ======================================================================
 // rmasses (rmasses.f90:4-63): per-element density, then a node gather in
 // the reference's colour order with each element's triangles in order.
@@ -1602,9 +1653,9 @@ template <class R> __global__ void k_convert_back(const R *__restrict__ src, dou
 // Launch with programmatic stream serialization (the kernel starts with
 // gf_pdl_entry); `n` items, GF_THREADS per CTA.
 template <class... KArgs, class... Args>
-inline void gf_launch_pdl(void (*kern)(KArgs...), unsigned grid, unsigned threads, cudaStream_t s, Args... args) {
+inline void gf_launch_pdl(void (*kern)(KArgs...), dim3 grid, unsigned threads, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(grid);
+    lc.gridDim = grid;
     lc.blockDim = dim3(threads);
     lc.stream = s;
     cudaLaunchAttribute at[1];
@@ -1662,26 +1713,31 @@ template <class R> void GfKernels<R>::plastic_table(const GfLaunch &g) {
     }
 }
 
-template <class R> void GfKernels<R>::therm_prep(const GfLaunch &g) {
-    using namespace gfk;
-    if (sizeof(R) == sizeof(float)) GF_LAUNCH(k_therm_prep32, g.d.E, g.P, g.A, g.d, (float *)g.A.t_coef);
-}
-
-template <class R> void GfKernels<R>::therm_sweeps(const GfLaunch &g) {
+template <class R> void GfKernels<R>::step_forces(const GfLaunch &g, int avg_mode, int move) {
     using namespace gfk;
     if (sizeof(R) != sizeof(float)) return;
-    const float *tc = (const float *)g.A.t_coef;
-    float *d0 = (float *)g.A.t_delta0;
-    GF_LAUNCH(k_therm_sweep32, g.d.N, g.P, g.C, g.A, g.d, tc, d0, g.A.t_delta1, 0);
-    GF_LAUNCH(k_therm_sweep32, g.d.N, g.P, g.C, g.A, g.d, tc, d0, g.A.t_delta1, 1);
-    GF_LAUNCH(k_therm_apply32, g.d.N, g.P, g.A, g.d, g.A.t_delta1);
+    auto launch = [&](auto kern, unsigned parts, auto... args) {
+        gf_launch_pdl(kern, dim3(grid_for(g.d.N), parts), GF_THREADS, g.s, args...);
+        ++*g.launches;
+    };
+    launch(k_step_a, 2u, g.P, g.C, g.A, g.d);
+    launch(k_step_b, avg_mode > 0 ? 3u : 2u, g.P, g.C, g.A, g.d, avg_mode);
+    launch(k_step_c, move ? 3u : 1u, g.P, g.C, g.A, g.d, avg_mode);
+    if (move)
+        launch(k_step_d, 2u, g.P, g.C, g.A, g.d, g.advance_time);
+    else
+        GF_LAUNCH(k_therm_apply32, g.d.N, g.P, g.A, g.d, g.A.t_delta1);
 }
 
 template <class R> void GfKernels<R>::therm(const GfLaunch &g, int sweeps, int keep_temp0) {
     using namespace gfk;
     if (sizeof(R) == sizeof(float)) {
-        therm_prep(g);
-        therm_sweeps(g);
+        const float *tc = (const float *)g.A.t_coef;
+        float *d0 = (float *)g.A.t_delta0;
+        GF_LAUNCH(k_therm_prep32, g.d.E, g.P, g.A, g.d, (float *)g.A.t_coef);
+        GF_LAUNCH(k_therm_sweep32, g.d.N, g.P, g.C, g.A, g.d, tc, d0, g.A.t_delta1, 0);
+        GF_LAUNCH(k_therm_sweep32, g.d.N, g.P, g.C, g.A, g.d, tc, d0, g.A.t_delta1, 1);
+        GF_LAUNCH(k_therm_apply32, g.d.N, g.P, g.A, g.d, g.A.t_delta1);
         return;
     }
 #ifdef GF_FP64_UNIT
