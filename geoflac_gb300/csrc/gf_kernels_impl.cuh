@@ -1665,6 +1665,26 @@ inline void gf_launch_pdl(void (*kern)(KArgs...), dim3 grid, unsigned threads, c
     lc.numAttrs = 1;
     cudaLaunchKernelEx(&lc, kern, (KArgs)args...);
 }
+// Threads per CTA for n items.  FP64 kernels: fewer than `most`, down to 64,
+// while that leaves SMs without a CTA, since warps that share an SM queue for
+// its FP64 pipe (ten steps of 60x20 elements 1.055 -> 1.020 ms, 241x61 1.265
+// -> 1.220; 32 threads measured the same).  The mixed kernels lose on it
+// (60x20: 0.393 -> 0.416 at 32 threads): theirs is a chain of instructions
+// that warps of one SM fetch once for all.
+inline unsigned gf_threads_for(long long n, unsigned most) {
+#ifdef GF_FP64_UNIT
+    static const int sms = [] {
+        int dev = 0, v = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+        return v;
+    }();
+    while (most > 64 && n <= (long long)(most / 2) * sms) most /= 2;
+#else
+    (void)n;
+#endif
+    return most;
+}
 #ifdef GF_FP64_UNIT
 #include "gf_therm64.cuh"
 #endif
@@ -1672,7 +1692,8 @@ inline void gf_launch_pdl(void (*kern)(KArgs...), dim3 grid, unsigned threads, c
 #define GF_LAUNCH_T(kern, n, thr, ...)                                                                                      \
     do {                                                                                                               \
         if ((n) > 0) {                                                                                                 \
-            gf_launch_pdl(kern, gfk::grid_for(n, thr), thr, g.s, __VA_ARGS__);                                                  \
+            const unsigned _t = gf_threads_for(n, thr);                                                                \
+            gf_launch_pdl(kern, gfk::grid_for(n, _t), _t, g.s, __VA_ARGS__);                                           \
             ++*g.launches;                                                                                             \
         }                                                                                                              \
     } while (0)

@@ -365,7 +365,8 @@ __global__ void __launch_bounds__(GF_THREADS, 4)
 // fl_therm after an optional temp0 = temp of the caller (keep_temp0)
 inline void therm_launch(const GfLaunch &g, int kmax, int keep_temp0) {
     using namespace gfk;
-    gf_launch_pdl(k_therm_prep, grid_for(2 * g.d.E), GF_THREADS, g.s, g.P, g.C, g.A, g.d, g.A.t_coef);
+    const unsigned t = gf_threads_for(2 * g.d.E, GF_THREADS);
+    gf_launch_pdl(k_therm_prep, grid_for(2 * g.d.E, t), t, g.s, g.P, g.C, g.A, g.d, g.A.t_coef);
     ++*g.launches;
     // resident CTAs of the two kernels, once per device
     static int cap_reg[64] = {0}, cap_gen[64] = {0};
