@@ -1,5 +1,5 @@
-"""Ensembles: many independent models advanced by one persistent kernel per
-step (gf_batch_* in include/geoflac_gb300.h)."""
+"""Ensembles: many independent models advanced together, one launch per phase
+of the step (gf_batch_* in include/geoflac_gb300.h)."""
 from __future__ import annotations
 
 import ctypes as C
@@ -44,8 +44,8 @@ class Batch:
         check(self.lib.gf_batch_set_config(self.handle, C.byref(c)), "gf_batch_set_config")
 
     def tune(self, trial_steps: int = 2) -> dict:
-        """Autotune the CTA shape, tile depth and residency (the trial steps
-        advance the members)."""
+        """Autotune the CTA shape and tile depth (the trial steps advance the
+        members)."""
         c = GfBatchConfig()
         ms = C.c_double()
         check(self.lib.gf_batch_tune(self.handle, int(trial_steps), C.byref(c), C.byref(ms)), "gf_batch_tune")

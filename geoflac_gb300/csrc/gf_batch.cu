@@ -1,27 +1,27 @@
 // Ensemble driver: hundreds of independent models of uneven size advanced
-// by one persistent kernel per step.
+// together, one launch per phase of the step.
 //
 // Each member is an ordinary mixed-precision context; a packed member table
 // (device pointers, dimensions, constants) and per-kind tile tables (element,
-// node, 2x node, marker and max(element, node) items) describe the ensemble.
-// A tile is `threads * items_per_thread` consecutive items of ONE member, so
-// a warp never mixes members and the per-member reductions stay warp-local.
-// Every phase of the step (fl_therm, change_phase, fl_rheol, fl_node,
-// fl_move, rmasses, dt_mass) walks all tiles of all members, each CTA a
-// contiguous run of tiles, and the phases are separated by a grid barrier:
-// the ensemble shares the step's phase order, not its dt or its size.  The
-// per-item work is the same device code as the single-model kernels; a
-// member's result does not depend on the other members, the tile depth or
-// the residency (FP32 contraction may differ from the separately compiled
-// single-model kernels at rounding level).
+// node, marker and max(element, node) items) describe the ensemble.  A tile
+// is `threads * items` consecutive items of ONE member, so a warp never mixes
+// members and the per-member reductions stay warp-local.  Every phase of the
+// step (fl_therm, change_phase, fl_rheol, fl_node, fl_move, rmasses, dt_mass)
+// is one launch with a CTA per tile of all members: the ensemble shares the
+// step's phase order, not its dt or its size.  The per-item work is the same
+// device code as the single-model kernels; a member's result does not depend
+// on the other members or the tile depth (FP32 contraction may differ from
+// the separately compiled single-model kernels at rounding level).
 //
-// The grid is co-resident (cooperative launch), sized from the occupancy of
-// the chosen CTA shape; the barrier gives up after a bounded wait and raises
-// an error flag instead of hanging.
+// The launches are chained by programmatic dependent launch (a CTA stages its
+// member's record while the phase before it drains) and replayed from CUDA
+// graphs.  One co-resident kernel that walks all phases between grid barriers
+// was slower at both ends of the range: its registers are those of fl_rheol
+// in every phase (8 warps an SM), and a barrier costs about what a dependent
+// launch does (ten steps and a sample of 64 members of 80x25 to 400x120
+// elements 7.24 against 6.83 ms, of 8 members of 80x25 to 120x36 1.01 against
+// 0.54).  The tile depth: see build_tables.
 
-// Items written in one phase are read in the next within the same kernel:
-// no pointer here may be treated as read-only for the kernel's lifetime.
-#define __restrict__
 // 32-bit indices, as in the mixed instantiation (members are mixed contexts)
 #define GF_IDX int
 #include "gf_kernels_impl.cuh"
@@ -34,7 +34,7 @@
 
 namespace {
 
-enum { K_E = 0, K_N, K_N2, K_M, K_EN, K_KINDS };
+enum { K_E = 0, K_N, K_M, K_EN, K_KINDS };
 
 struct BatchMember {
     const DevParams *P;
@@ -46,223 +46,98 @@ struct BatchMember {
     long long e0;    // elements of the members before this one
 };
 
-struct BatchSync {
-    unsigned count, gen;
-    int err, pad;
-};
-
 struct BatchArgs {
     const BatchMember *members;
     int nmembers;
     const int2 *tile[K_KINDS]; // (member, first item) per tile
     int ntile[K_KINDS];
-    BatchSync *sync;
-    unsigned sig;
-    int ipt;   // items per thread
-    int merge; // every member allows the thermal sweeps beside fl_rheol / fl_node
+    int ipt;  // items per thread
+    int opt;  // the phase's own option (viscosity update, averaging mode, time advance, sweep)
 };
 
-// Bounded grid barrier (gf_grid_barrier: arrivals, generation counter,
-// error flag -- BatchSync has that layout).  Returns false if any CTA gave
-// up waiting; the kernel then returns at once.
-__device__ bool grid_sync(BatchSync *s) { return gfk::gf_grid_barrier(reinterpret_cast<unsigned *>(s), 1LL << 24); }
-
-// Check of the bounded barrier: CTA `absent` of a two-CTA co-resident launch
-// never arrives; the other waits at most `limit` polls and leaves with the
-// error flag set (absent = -1: both arrive and pass).
-__global__ void k_barrier_probe(unsigned *bar, int absent, long long limit, int *passed) {
-    if ((int)blockIdx.x == absent) return;
-    bool ok = gfk::gf_grid_barrier(bar, limit);
-    if (threadIdx.x == 0) passed[blockIdx.x] = ok ? 1 : 0;
+// One phase: CTA (t, part) works on tile t of the phase's kind.  The parts of
+// a phase (grid y, the longest first) are independent of each other and share
+// its launch.  The member's record is constant while steps run, so it is
+// staged before the wait for the phase before.  128 registers at most at the
+// 512 threads a batch may be configured for.
+template <class Ph> __global__ void __launch_bounds__(512) k_phase(BatchArgs a) {
+    __shared__ BatchMember m;
+    const int2 tl = a.tile[Ph::kind][blockIdx.x];
+    const int *src = reinterpret_cast<const int *>(a.members + tl.x);
+    int *dst = reinterpret_cast<int *>(&m);
+    for (int w = threadIdx.x; w < (int)(sizeof(BatchMember) / sizeof(int)); w += blockDim.x) dst[w] = src[w];
+    gfk::gf_pdl_entry();
+    __syncthreads();
+    for (int r = 0; r < a.ipt; ++r) Ph::item(m, (int)blockIdx.y, a.opt, tl.y + r * (int)blockDim.x + (int)threadIdx.x);
 }
-
-// All tiles of one item kind, a contiguous run per CTA; the member record is
-// staged in shared memory whenever the run crosses into the next member.
-template <class F> __device__ void for_tiles(const BatchArgs &a, int kind, BatchMember &sm, int &cur, F &&f) {
-    const int nt = a.ntile[kind];
-    const int per = (nt + gridDim.x - 1) / gridDim.x;
-    const int t0 = blockIdx.x * per, t1 = min(nt, t0 + per);
-    for (int t = t0; t < t1; ++t) {
-        const int2 tl = a.tile[kind][t];
-        if (tl.x != cur) {
-            __syncthreads();
-            const int *src = reinterpret_cast<const int *>(a.members + tl.x);
-            int *dst = reinterpret_cast<int *>(&sm);
-            for (int w = threadIdx.x; w < (int)(sizeof(BatchMember) / sizeof(int)); w += blockDim.x) dst[w] = src[w];
-            __syncthreads();
-            cur = tl.x;
-        }
-        for (int r = 0; r < a.ipt; ++r) f(sm, (long long)tl.y + (long long)r * blockDim.x + threadIdx.x);
-    }
-}
-
 // Per-member scalar work, one thread per member.
-template <class F> __device__ void for_members(const BatchArgs &a, F &&f) {
-    for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < a.nmembers; m += gridDim.x * blockDim.x) f(a.members[m]);
+template <class Ph> __global__ void __launch_bounds__(128) k_phase_members(BatchArgs a) {
+    gfk::gf_pdl_entry();
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < a.nmembers) Ph::member(a.members[k]);
 }
 
-// rmasses, dt_mass and par.f90's time advance after fl_move (shared by both
-// schedules of k_batch_step)
-template <class R> __device__ __forceinline__ void mech_tail(const BatchArgs &a, BatchMember &sm, int &cur, unsigned sig) {
-    using namespace gfk;
-#define GF_SYNC()                                                                                                      \
-    do {                                                                                                               \
-        if (!grid_sync(a.sync)) return;                                                                                \
-    } while (0)
-    const int dtm = (sig & 32u) ? 1 : 0;
-    if (sig & 16u) { // rmasses
-        for_tiles(a, K_E, sm, cur, [&](const BatchMember &m, long long i) {
-            b_k_elem_dens<R>(m.P, m.C, m.A, m.d, i);
-        });
-        GF_SYNC();
-        for_members(a, [&](const BatchMember &m) { b_k_frac_fix<R>(m.P, m.C, m.A, m.d); });
-        GF_SYNC();
-        for_tiles(a, K_N, sm, cur, [&](const BatchMember &m, long long i) {
-            b_k_node_gather_tri<R>((const R *)m.A.e_tri, m.A.rmass, m.d, i);
-        });
-        GF_SYNC();
+#define GF_PHASE(name, k) struct name { static constexpr int kind = k; \
+    static __device__ __forceinline__ void item(const BatchMember &m, int part, int opt, GF_IDX i)
+using namespace gfk;
+// the joint launches of an ordinary step (k_step_a to k_step_d)
+GF_PHASE(PhStepA, K_E) {
+    if (part == 0) b_k_rheol<float>(m.P, m.C, m.A, m.d, 0, 0, i);
+    else b_k_therm_prep32(m.P, m.A, m.d, (float *)m.A.t_coef, i);
+} };
+GF_PHASE(PhStepB, K_N) {
+    if (part == 0) b_k_node<float>(m.P, m.C, m.A, m.d, i);
+    else if (part == 1)
+        b_k_therm_sweep32(m.P, m.C, m.A, m.d, (const float *)m.A.t_coef, (float *)m.A.t_delta0, m.A.t_delta1, 0, i);
+    else b_k_rheol_avg<float>(m.C, m.A, m.d, opt == 2 ? 1 : 0, i);
+} };
+GF_PHASE(PhStepC, K_N) {
+    if (part == 0) {
+        b_k_therm_sweep32(m.P, m.C, m.A, m.d, (const float *)m.A.t_coef, (float *)m.A.t_delta0, m.A.t_delta1, 1, i);
+        if (opt == 2 && i == 0) b_k_rheol_clock(m.C, 1);
+    } else if (m.movegrid && i < m.d.N) {
+        b_k_move_cord(m.C, m.A, m.d, (GF_IDX)((part - 1) * m.d.N) + i);
     }
-    if (dtm) { // dt_mass
-        for_members(a, [&](const BatchMember &m) { b_k_dt_reset(m.C); });
-        GF_SYNC();
-        for_tiles(a, K_EN, sm, cur, [&](const BatchMember &m, long long i) {
-            b_k_dt_reduce<R>(m.P, m.C, m.A, m.d, i);
-        });
-        GF_SYNC();
-        for_members(a, [&](const BatchMember &m) { b_k_dt_scalars(m.P, m.C); });
-        GF_SYNC();
-        for_tiles(a, K_E, sm, cur, [&](const BatchMember &m, long long i) {
-            if (m.idt_scale != 0) b_k_elem_am3<R>(m.P, m.C, m.A, m.d, i);
-        });
-        GF_SYNC();
-        for_tiles(a, K_N, sm, cur, [&](const BatchMember &m, long long i) {
-            if (m.idt_scale != 0)
-                b_k_node_gather_tri<R>((const R *)m.A.e_tri, m.A.amass, m.d, i);
-            else if (i < m.d.N)
-                m.A.amass[i] = m.A.rmass[i];
-        });
-        GF_SYNC();
-    }
-    // par.f90:86: time advanced inside fl_move on steps without dt_mass
-    for_members(a, [&](const BatchMember &m) {
-        if (!m.movegrid || dtm) m.C->time = m.C->time + m.C->dt;
-    });
-#undef GF_SYNC
-}
-
-// One FLAC step (flac.f90:5-91, mixed precision) of every member.
-// MINB: resident CTAs per SM the register allocation is sized for (the whole
-// step is one kernel, so its register count is that of its heaviest phase;
-// a cap trades spills in fl_rheol for occupancy in every phase)
-template <int THREADS, int MINB> __global__ void __launch_bounds__(THREADS, MINB) k_batch_step(BatchArgs a) {
-    using namespace gfk;
-    typedef float R;
-    __shared__ BatchMember sm;
-    int cur = -1;
-    const unsigned sig = a.sig;
-#define GF_SYNC()                                                                                                      \
-    do {                                                                                                               \
-        if (!grid_sync(a.sync)) return;                                                                                \
-    } while (0)
-    // fl_therm
-    for_tiles(a, K_E, sm, cur, [&](const BatchMember &m, long long i) {
-        b_k_therm_prep32(m.P, m.A, m.d, (float *)m.A.t_coef, i);
-    });
-    GF_SYNC();
-    // Steps whose fl_rheol / fl_node read nothing the thermal update writes
-    // (no viscosity update, no change_phase; every member without thermal
-    // stress, Winkler foundation or flux bottom condition): the sweeps share
-    // phases with fl_rheol, fl_node and the coordinate update, which saves
-    // three grid barriers and lets CTAs go on to the next kind of tile.
-    if (a.merge && (sig & 1u) && !(sig & 2u) && !(sig & 4u)) {
-        const int avg = (sig & (8u << 8)) ? 2 : ((sig & (4u << 8)) ? 1 : 0);
-        const int dtm = (sig & 32u) ? 1 : 0;
-        for_tiles(a, K_N, sm, cur, [&](const BatchMember &m, long long i) {
-            b_k_therm_sweep32(m.P, m.C, m.A, m.d, (const float *)m.A.t_coef, (float *)m.A.t_delta0, m.A.t_delta1,
-                              0, i);
-        });
-        for_tiles(a, K_E, sm, cur, [&](const BatchMember &m, long long i) { b_k_rheol<R>(m.P, m.C, m.A, m.d, 0, 0, i); });
-        GF_SYNC();
-        for_tiles(a, K_N, sm, cur, [&](const BatchMember &m, long long i) {
-            b_k_therm_sweep32(m.P, m.C, m.A, m.d, (const float *)m.A.t_coef, (float *)m.A.t_delta0, m.A.t_delta1,
-                              1, i);
-        });
-        if (avg > 0)
-            for_tiles(a, K_E, sm, cur, [&](const BatchMember &m, long long i) {
-                b_k_rheol_avg<R>(m.C, m.A, m.d, avg == 2 ? 1 : 0, i);
-            });
-        for_tiles(a, K_N, sm, cur, [&](const BatchMember &m, long long i) { b_k_node<R>(m.P, m.C, m.A, m.d, i); });
-        GF_SYNC();
-        for_tiles(a, K_N, sm, cur, [&](const BatchMember &m, long long i) {
-            b_k_therm_apply32(m.P, m.A, m.d, m.A.t_delta1, i);
-        });
-        if (avg == 2) for_members(a, [&](const BatchMember &m) { b_k_rheol_clock(m.C, 1); });
-        for_tiles(a, K_N2, sm, cur, [&](const BatchMember &m, long long i) {
-            if (m.movegrid) b_k_move_cord(m.C, m.A, m.d, i);
-        });
-        GF_SYNC();
-        for_tiles(a, K_E, sm, cur, [&](const BatchMember &m, long long i) {
-            if (m.movegrid) b_k_move_elem<R>(m.C, m.A, m.d, dtm ? 0 : 1, i);
-        });
-        GF_SYNC();
-        mech_tail<R>(a, sm, cur, sig);
-        return;
-    }
-    for (int sweep = 0; sweep < 2; ++sweep) {
-        for_tiles(a, K_N, sm, cur, [&](const BatchMember &m, long long i) {
-            b_k_therm_sweep32(m.P, m.C, m.A, m.d, (const float *)m.A.t_coef, (float *)m.A.t_delta0, m.A.t_delta1,
-                              sweep, i);
-        });
-        GF_SYNC();
-    }
-    for_tiles(a, K_N, sm, cur, [&](const BatchMember &m, long long i) {
-        b_k_therm_apply32(m.P, m.A, m.d, m.A.t_delta1, i);
-    });
-    GF_SYNC();
-    if (sig & 1u) {
-        if (sig & 2u) { // change_phase
-            for_tiles(a, K_M, sm, cur, [&](const BatchMember &m, long long i) {
-                b_k_phase_markers32(m.P, m.A, m.d, m.nmarkers, i);
-            });
-            GF_SYNC();
-            for_tiles(a, K_E, sm, cur, [&](const BatchMember &m, long long i) {
-                b_k_phase_recount<R>(m.P, m.C, m.A, m.d, 0, i);
-            });
-            GF_SYNC();
-        }
-        const int upd = (sig & 4u) ? 1 : 0;
-        const int avg = (sig & (8u << 8)) ? 2 : ((sig & (4u << 8)) ? 1 : 0);
-        for_tiles(a, K_E, sm, cur, [&](const BatchMember &m, long long i) {
-            b_k_rheol<R>(m.P, m.C, m.A, m.d, upd, 0, i);
-        });
-        GF_SYNC();
-        if (avg > 0) {
-            for_tiles(a, K_E, sm, cur, [&](const BatchMember &m, long long i) {
-                b_k_rheol_avg<R>(m.C, m.A, m.d, avg == 2 ? 1 : 0, i);
-            });
-            GF_SYNC();
-            if (avg == 2) {
-                for_members(a, [&](const BatchMember &m) { b_k_rheol_clock(m.C, 1); });
-                GF_SYNC();
-            }
-        }
-        for_tiles(a, K_N, sm, cur, [&](const BatchMember &m, long long i) { b_k_node<R>(m.P, m.C, m.A, m.d, i); });
-        GF_SYNC();
-        const int dtm = (sig & 32u) ? 1 : 0;
-        for_tiles(a, K_N2, sm, cur, [&](const BatchMember &m, long long i) {
-            if (m.movegrid) b_k_move_cord(m.C, m.A, m.d, i);
-        });
-        GF_SYNC();
-        for_tiles(a, K_E, sm, cur, [&](const BatchMember &m, long long i) {
-            if (m.movegrid) b_k_move_elem<R>(m.C, m.A, m.d, dtm ? 0 : 1, i);
-        });
-        GF_SYNC();
-        mech_tail<R>(a, sm, cur, sig);
-    } else {
-        for_members(a, [&](const BatchMember &m) { m.C->time = m.C->time + m.C->dt; });
-    }
-#undef GF_SYNC
-}
+} };
+GF_PHASE(PhStepD, K_N) { // opt: time advances here (par.f90:86), unless dt_mass follows
+    if (part == 1) b_k_therm_apply32(m.P, m.A, m.d, m.A.t_delta1, i);
+    else if (m.movegrid) b_k_move_elem<float>(m.C, m.A, m.d, opt, i);
+    else if (opt && i == 0) m.C->time = m.C->time + m.C->dt;
+} };
+// the same parts one by one, for steps that need the new temperatures first
+GF_PHASE(PhPrep, K_E) { b_k_therm_prep32(m.P, m.A, m.d, (float *)m.A.t_coef, i); } };
+GF_PHASE(PhSweep, K_N) {
+    b_k_therm_sweep32(m.P, m.C, m.A, m.d, (const float *)m.A.t_coef, (float *)m.A.t_delta0, m.A.t_delta1, opt, i);
+} };
+GF_PHASE(PhApply, K_N) { b_k_therm_apply32(m.P, m.A, m.d, m.A.t_delta1, i); } };
+GF_PHASE(PhMarkers, K_M) { b_k_phase_markers32(m.P, m.A, m.d, m.nmarkers, i); } };
+GF_PHASE(PhRecount, K_E) { b_k_phase_recount<float>(m.P, m.C, m.A, m.d, 0, i); } };
+GF_PHASE(PhRheol, K_E) { b_k_rheol<float>(m.P, m.C, m.A, m.d, opt, 0, i); } };
+GF_PHASE(PhNode, K_N) { // and fl_rheol's averaging
+    if (part == 0) b_k_node<float>(m.P, m.C, m.A, m.d, i);
+    else b_k_rheol_avg<float>(m.C, m.A, m.d, opt == 2 ? 1 : 0, i);
+} };
+GF_PHASE(PhCord, K_N) {
+    if (opt == 2 && part == 0 && i == 0) b_k_rheol_clock(m.C, 1);
+    if (m.movegrid && i < m.d.N) b_k_move_cord(m.C, m.A, m.d, (GF_IDX)(part * m.d.N) + i);
+} };
+GF_PHASE(PhMove, K_E) {
+    if (m.movegrid) b_k_move_elem<float>(m.C, m.A, m.d, opt, i);
+    else if (opt && i == 0) m.C->time = m.C->time + m.C->dt;
+} };
+GF_PHASE(PhDens, K_E) { b_k_elem_dens<float>(m.P, m.C, m.A, m.d, i); } };
+GF_PHASE(PhRmass, K_N) { b_k_node_gather_tri<float>((const float *)m.A.e_tri, m.A.rmass, m.d, i); } };
+GF_PHASE(PhDt, K_EN) { b_k_dt_reduce<float>(m.P, m.C, m.A, m.d, i); } };
+GF_PHASE(PhAm3, K_E) { if (m.idt_scale != 0) b_k_elem_am3<float>(m.P, m.C, m.A, m.d, i); } };
+GF_PHASE(PhAmass, K_N) {
+    if (m.idt_scale != 0) b_k_node_gather_tri<float>((const float *)m.A.e_tri, m.A.amass, m.d, i);
+    else if (i < m.d.N) m.A.amass[i] = m.A.rmass[i];
+} };
+#undef GF_PHASE
+struct MemFrac { static __device__ void member(const BatchMember &m) { b_k_frac_fix<float>(m.P, m.C, m.A, m.d); } };
+struct MemDtReset { static __device__ void member(const BatchMember &m) { b_k_dt_reset(m.C); } };
+struct MemDtScalars { static __device__ void member(const BatchMember &m) { b_k_dt_scalars(m.P, m.C); } };
+struct MemTime { static __device__ void member(const BatchMember &m) { m.C->time = m.C->time + m.C->dt; } };
 
 // ---------------------------------------------------------------- surrogate I/O
 // Fields of every member resampled to an H x W grid (channels last, FP32):
@@ -627,24 +502,6 @@ __global__ void k_force_residual(const BatchMember *members, const int2 *tiles, 
     }
 }
 
-typedef void (*BatchKernel)(BatchArgs);
-
-// the kernel for a CTA width and residency: register-capped builds where
-// compiled, else the uncapped one
-BatchKernel kernel_for(int threads, int cps) {
-    switch (threads) {
-    case 128: return k_batch_step<128, 1>;
-    case 256:
-        if (cps == 2) return k_batch_step<256, 2>;
-        if (cps >= 3) return k_batch_step<256, 3>;
-        return k_batch_step<256, 1>;
-    case 512:
-        if (cps >= 2) return k_batch_step<512, 2>;
-        return k_batch_step<512, 1>;
-    default: return nullptr;
-    }
-}
-
 } // namespace
 
 struct gf_batch {
@@ -653,12 +510,12 @@ struct gf_batch {
     BatchMember *d_members = nullptr;
     int2 *d_tiles[K_KINDS] = {};
     int ntile[K_KINDS] = {};
-    BatchSync *d_sync = nullptr;
     cudaStream_t s = nullptr;
     gf_batch_config cfg{256, 2, 1, 10};
     double g = 10.0; // gravity of the members (one value; checked at creation)
-    int grid = 0;
-    int merge = 0;
+    int grid = 0;  // CTAs of an element phase
+    int ipt = 1;   // items per thread of the tile tables (the configuration's, or fewer for a small batch)
+    int merge = 0; // every member allows the joint launches
     long long elements = 0;
     struct Graph {
         std::vector<unsigned> sigs;
@@ -706,24 +563,25 @@ long long kind_count(const GfMemberView &v, int kind) {
     switch (kind) {
     case K_E: return v.d.E;
     case K_N: return v.d.N;
-    case K_N2: return 2 * v.d.N;
     case K_M: return v.nmarkers;
     default: return std::max(v.d.E, v.d.N);
     }
 }
 
-// tile tables and the co-resident grid for the current configuration
+// Tile tables for the current configuration.  A tile of several items per
+// thread saves stagings of the member record; a batch with fewer elements than
+// the SMs hold threads at that depth is cut finer, since its tiles would not
+// fill them once (a member's result does not depend on the tile depth).
 int build_tables(gf_batch *b) {
     const gf_batch_config &c = b->cfg;
-    BatchKernel k = kernel_for(c.threads, c.ctas_per_sm);
-    if (!k || c.items_per_thread < 1 || c.items_per_thread > 64 || c.ctas_per_sm < 1) return GF_ERR_ARG;
-    int dev = 0, sms = 0, occ = 0;
+    if (c.threads != 128 && c.threads != 256 && c.threads != 512) return GF_ERR_ARG;
+    if (c.items_per_thread < 1 || c.items_per_thread > 64 || c.ctas_per_sm < 1) return GF_ERR_ARG;
+    int dev = 0, sms = 0;
     GB_CK(cudaGetDevice(&dev));
     GB_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    GB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, c.threads, 0));
-    if (occ < 1) return GF_ERR_UNSUPPORTED;
-    const int full_grid = sms * std::min(occ, c.ctas_per_sm);
-    const long long tile = (long long)c.threads * c.items_per_thread;
+    b->ipt = c.items_per_thread;
+    while (b->ipt > 1 && b->elements < (long long)sms * 2048 * b->ipt) --b->ipt;
+    const long long tile = (long long)c.threads * b->ipt;
     for (int kind = 0; kind < K_KINDS; ++kind) {
         std::vector<int2> t;
         for (size_t m = 0; m < b->views.size(); ++m) {
@@ -741,11 +599,7 @@ int build_tables(gf_batch *b) {
             GB_CK(cudaMemcpy(b->d_tiles[kind], t.data(), t.size() * sizeof(int2), cudaMemcpyHostToDevice));
         }
     }
-    // a small batch (e.g. a few members rerun after screening) runs on no
-    // more CTAs than it has element or node tiles: its grid barriers then
-    // involve few CTAs
-    const int work = std::max(1, std::max(b->ntile[K_E], b->ntile[K_N]));
-    b->grid = std::min(full_grid, work);
+    b->grid = b->ntile[K_E];
     drop_graphs(b);
     return GF_OK;
 }
@@ -772,37 +626,93 @@ int upload_members(gf_batch *b) {
     return GF_OK;
 }
 
-BatchArgs args_of(const gf_batch *b, unsigned sig) {
+// Enqueue one FLAC step (flac.f90:5-91, mixed precision) of every member.
+struct StepLauncher {
+    gf_batch *b;
     BatchArgs a;
-    std::memset(&a, 0, sizeof a);
-    a.members = b->d_members;
-    a.nmembers = (int)b->members.size();
-    for (int k = 0; k < K_KINDS; ++k) {
-        a.tile[k] = b->d_tiles[k];
-        a.ntile[k] = b->ntile[k];
+    cudaError_t err = cudaSuccess;
+    explicit StepLauncher(gf_batch *batch) : b(batch) {
+        std::memset(&a, 0, sizeof a);
+        a.members = b->d_members;
+        a.nmembers = (int)b->members.size();
+        for (int k = 0; k < K_KINDS; ++k) {
+            a.tile[k] = b->d_tiles[k];
+            a.ntile[k] = b->ntile[k];
+        }
+        a.ipt = b->ipt;
     }
-    a.sync = b->d_sync;
-    a.sig = sig;
-    a.ipt = b->cfg.items_per_thread;
-    a.merge = b->merge;
-    return a;
-}
+    void launch(void (*kern)(BatchArgs), dim3 grid, int threads, int opt) {
+        if (grid.x == 0 || err != cudaSuccess) return;
+        a.opt = opt;
+        cudaLaunchConfig_t lc;
+        std::memset(&lc, 0, sizeof lc);
+        lc.gridDim = grid;
+        lc.blockDim = dim3((unsigned)threads);
+        lc.stream = b->s;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        lc.attrs = attr;
+        lc.numAttrs = 1;
+        err = cudaLaunchKernelEx(&lc, kern, a);
+    }
+    template <class Ph> void phase(unsigned parts = 1, int opt = 0) {
+        launch(k_phase<Ph>, dim3((unsigned)b->ntile[Ph::kind], parts), b->cfg.threads, opt);
+    }
+    template <class Ph> void scalars() {
+        launch(k_phase_members<Ph>, dim3((unsigned)((a.nmembers + 127) / 128)), 128, 0);
+    }
+    int step(unsigned sig) {
+        const int avg = (sig & (8u << 8)) ? 2 : ((sig & (4u << 8)) ? 1 : 0);
+        const int dtm = (sig & 32u) ? 1 : 0;
+        // Steps whose fl_rheol / fl_node read nothing the thermal update
+        // writes (no viscosity update, no change_phase; every member without
+        // thermal stress, Winkler foundation or flux bottom condition)
+        const bool joint = b->merge && (sig & 1u) && !(sig & 2u) && !(sig & 4u);
+        if (joint) {
+            phase<PhStepA>(2);
+            phase<PhStepB>(avg > 0 ? 3 : 2, avg);
+            phase<PhStepC>(3, avg);
+            phase<PhStepD>(2, !dtm);
+        } else {
+            phase<PhPrep>();
+            phase<PhSweep>(1, 0);
+            phase<PhSweep>(1, 1);
+            phase<PhApply>();
+            if (sig & 1u) {
+                if (sig & 2u) { // change_phase
+                    phase<PhMarkers>();
+                    phase<PhRecount>();
+                }
+                phase<PhRheol>(1, (sig & 4u) ? 1 : 0);
+                phase<PhNode>(avg > 0 ? 2 : 1, avg);
+                phase<PhCord>(2, avg);
+                phase<PhMove>(1, !dtm);
+            }
+        }
+        if (sig & 1u) {
+            if (sig & 16u) { // rmasses
+                phase<PhDens>();
+                scalars<MemFrac>();
+                phase<PhRmass>();
+            }
+            if (dtm) { // dt_mass, then the time advance with the new dt (par.f90:86)
+                scalars<MemDtReset>();
+                phase<PhDt>();
+                scalars<MemDtScalars>();
+                phase<PhAm3>();
+                phase<PhAmass>();
+                scalars<MemTime>();
+            }
+        } else {
+            scalars<MemTime>();
+        }
+        GB_CK(err);
+        return GF_OK;
+    }
+};
 
-int launch_step(gf_batch *b, unsigned sig) {
-    BatchArgs a = args_of(b, sig);
-    cudaLaunchConfig_t lc;
-    std::memset(&lc, 0, sizeof lc);
-    lc.gridDim = dim3((unsigned)b->grid);
-    lc.blockDim = dim3((unsigned)b->cfg.threads);
-    lc.stream = b->s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    lc.attrs = attr;
-    lc.numAttrs = 1;
-    GB_CK(cudaLaunchKernelEx(&lc, kernel_for(b->cfg.threads, b->cfg.ctas_per_sm), a));
-    return GF_OK;
-}
+int launch_step(gf_batch *b, unsigned sig) { return StepLauncher(b).step(sig); }
 
 // Signatures of the next n steps (all members share them).
 std::vector<unsigned> next_sigs(gf_batch *b, int n, std::vector<int> &nl, std::vector<int> &ns) {
@@ -846,9 +756,6 @@ int refresh_views(gf_batch *b) {
 
 int check_status(gf_batch *b) {
     GB_CK(cudaStreamSynchronize(b->s));
-    BatchSync hs;
-    GB_CK(cudaMemcpy(&hs, b->d_sync, sizeof hs, cudaMemcpyDeviceToHost));
-    if (hs.err) return GF_ERR_TIMEOUT;
     int first = GF_OK;
     for (gf_ctx *c : b->members) {
         int st = gf_ctx_take_status(c);
@@ -883,8 +790,6 @@ int gf_batch_create(gf_batch **out, gf_ctx **members, int n) {
     if (!rc) rc = batch_cuda(cudaStreamCreateWithFlags(&b->s, cudaStreamNonBlocking), "stream");
     if (!rc) rc = batch_cuda(cudaMalloc(&b->d_members, sizeof(BatchMember) * n), "members");
     if (!rc) rc = batch_cuda(cudaMalloc(&b->means, sizeof(float4) * 2 * (size_t)b->elements), "sampling scratch");
-    if (!rc) rc = batch_cuda(cudaMalloc(&b->d_sync, sizeof(BatchSync)), "sync");
-    if (!rc) rc = batch_cuda(cudaMemset(b->d_sync, 0, sizeof(BatchSync)), "sync");
     if (!rc) rc = upload_members(b);
     if (!rc) rc = build_tables(b);
     if (rc) {
@@ -902,7 +807,6 @@ void gf_batch_destroy(gf_batch *b) {
     for (int k = 0; k < K_KINDS; ++k)
         if (b->d_tiles[k]) cudaFree(b->d_tiles[k]);
     if (b->d_members) cudaFree(b->d_members);
-    if (b->d_sync) cudaFree(b->d_sync);
     if (b->backup) cudaFree(b->backup);
     if (b->means) cudaFree(b->means);
     if (b->s) cudaStreamDestroy(b->s);
@@ -976,8 +880,8 @@ int gf_batch_step(gf_batch *b, int nsteps) {
     return check_status(b);
 }
 
-// Autotuner: every CTA shape (threads), tile depth (items per thread) and
-// residency (CTAs per SM) that fits, each timed over `trial_steps` steps
+// Autotuner: every CTA shape (threads) and tile depth (items per thread), each
+// timed over `trial_steps` steps
 // with CUDA events after one untimed step; the fastest is kept.  The trial
 // steps advance the members like any other steps.
 int gf_batch_tune(gf_batch *b, int trial_steps, gf_batch_config *best, double *best_ms) {
@@ -991,29 +895,25 @@ int gf_batch_tune(gf_batch *b, int trial_steps, gf_batch_config *best, double *b
     const int ipts[4] = {1, 2, 4, 8};
     int rc = GF_OK;
     for (int t : threads) {
-        for (int ipt : ipts)
-            for (int cps = 1; cps <= 4; ++cps) {
-                int occ = 0;
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel_for(t, cps), t, 0);
-                if (occ < cps) continue;
-                gf_batch_config c{t, ipt, cps, 0}; // direct launches: no capture inside the timing
-                b->cfg = c;
-                if (build_tables(b)) continue;
-                rc = gf_batch_step(b, 1);
-                if (rc) break;
-                cudaEventRecord(e0, b->s);
-                rc = gf_batch_step(b, trial_steps);
-                if (rc) break;
-                cudaEventRecord(e1, b->s);
-                cudaEventSynchronize(e1);
-                float ms = 0.f;
-                cudaEventElapsedTime(&ms, e0, e1);
-                double per = ms / trial_steps;
-                if (per < win_ms) {
-                    win_ms = per;
-                    win = c;
-                }
+        for (int ipt : ipts) {
+            gf_batch_config c{t, ipt, 1, 0}; // direct launches: no capture inside the timing
+            b->cfg = c;
+            if (build_tables(b)) continue;
+            rc = gf_batch_step(b, 1);
+            if (rc) break;
+            cudaEventRecord(e0, b->s);
+            rc = gf_batch_step(b, trial_steps);
+            if (rc) break;
+            cudaEventRecord(e1, b->s);
+            cudaEventSynchronize(e1);
+            float ms = 0.f;
+            cudaEventElapsedTime(&ms, e0, e1);
+            double per = ms / trial_steps;
+            if (per < win_ms) {
+                win_ms = per;
+                win = c;
             }
+        }
         if (rc) break;
     }
     cudaEventDestroy(e0);
@@ -1032,7 +932,7 @@ int gf_batch_sample(gf_batch *b, float *grid, int H, int W, int phase_id) {
     GridArgs g{b->d_members, (int)b->members.size(), H, W, phase_id, grid, nullptr};
     if (b->ntile[K_E])
         k_sample_elems<<<b->ntile[K_E], b->cfg.threads, 0, b->s>>>(g, b->d_tiles[K_E], b->ntile[K_E],
-                                                                   b->cfg.items_per_thread, b->means);
+                                                                   b->ipt, b->means);
     const int ty = (H + 31) / 32, tx = (W + 31) / 32;
     k_sample<<<(unsigned)((long long)g.n * ty * tx), 256, 0, b->s>>>(g, b->means, ty, tx);
     GB_CK(cudaGetLastError());
@@ -1043,7 +943,7 @@ int gf_batch_inject(gf_batch *b, const float *grid, int H, int W) {
     if (!b || !grid || H < 2 || W < 2) return GF_ERR_ARG;
     for (gf_ctx *c : b->members) gf_ctx_invalidate_forces(c);
     GridArgs g{b->d_members, (int)b->members.size(), H, W, 1, nullptr, grid};
-    const int T = b->cfg.threads, ipt = b->cfg.items_per_thread;
+    const int T = b->cfg.threads, ipt = b->ipt;
     if (b->ntile[K_N]) k_inject_nodes<<<b->ntile[K_N], T, 0, b->s>>>(g, b->d_tiles[K_N], b->ntile[K_N], ipt);
     if (b->ntile[K_E])
         k_inject_elems<<<b->ntile[K_E], T, 0, b->s>>>(g, b->d_tiles[K_E], b->ntile[K_E], ipt, nullptr);
@@ -1099,7 +999,7 @@ int gf_batch_force_residual(gf_batch *b, double *residual) {
     const double g_acc = b->g;
     if (b->ntile[K_N])
         k_force_residual<<<b->ntile[K_N], b->cfg.threads, 0, b->s>>>(b->d_members, b->d_tiles[K_N], b->ntile[K_N],
-                                                                     b->cfg.items_per_thread, acc, g_acc);
+                                                                     b->ipt, acc, g_acc);
     std::vector<double> h(2 * n);
     cudaError_t e = cudaMemcpyAsync(h.data(), acc, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost, b->s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->s);
@@ -1107,35 +1007,6 @@ int gf_batch_force_residual(gf_batch *b, double *residual) {
     GB_CK(e);
     for (int m = 0; m < n; ++m) residual[m] = h[2 * m] / (h[2 * m + 1] > 0 ? h[2 * m + 1] : 1.0);
     return GF_OK;
-}
-
-int gf_grid_barrier_selftest(int absent_cta, long long limit, int *passed) {
-    if (!passed || absent_cta < -1 || absent_cta > 1 || limit < 1) return GF_ERR_ARG;
-    unsigned *bar = nullptr;
-    int *d_passed = nullptr;
-    GB_CK(cudaMalloc(&bar, 4 * sizeof(unsigned)));
-    cudaError_t e = cudaMalloc(&d_passed, 2 * sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(bar, 0, 4 * sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaMemset(d_passed, 0xff, 2 * sizeof(int));
-    unsigned err = 0;
-    if (e == cudaSuccess) {
-        cudaLaunchConfig_t lc = {};
-        lc.gridDim = dim3(2);
-        lc.blockDim = dim3(32);
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeCooperative;
-        attr[0].val.cooperative = 1;
-        lc.attrs = attr;
-        lc.numAttrs = 1;
-        e = cudaLaunchKernelEx(&lc, k_barrier_probe, bar, absent_cta, limit, d_passed);
-    }
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    if (e == cudaSuccess) e = cudaMemcpy(passed, d_passed, 2 * sizeof(int), cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess) e = cudaMemcpy(&err, bar + 2, sizeof(unsigned), cudaMemcpyDeviceToHost);
-    cudaFree(bar);
-    cudaFree(d_passed);
-    GB_CK(e);
-    return err ? GF_ERR_TIMEOUT : GF_OK;
 }
 
 } // extern "C"

@@ -741,39 +741,6 @@ __device__ __forceinline__ double therm_bc_value(const DevParams &P, const DevAr
     return src(gf_node(d, j, ii));
 }
 
-// Bounded grid barrier of a co-resident (cooperative) launch: generation
-// counter in bar[1], arrivals in bar[0], error flag in bar[2].  A CTA that
-// waits longer than `limit` polls sets the flag; every CTA returns false
-// once the flag is set.
-__device__ bool gf_grid_barrier(unsigned *bar, GF_IDX limit) {
-    __shared__ int bad;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned *vgen = bar + 1;
-        unsigned g0 = *vgen;
-        __threadfence();
-        unsigned arrived = atomicAdd(bar, 1u);
-        if (arrived == gridDim.x - 1) {
-            atomicExch(bar, 0u);
-            __threadfence();
-            atomicAdd(bar + 1, 1u);
-        } else {
-            GF_IDX it = 0;
-            while (*vgen == g0) {
-                if (++it > limit) {
-                    atomicExch(bar + 2, 1u);
-                    break;
-                }
-                __nanosleep(64);
-            }
-        }
-        __threadfence();
-        bad = *(volatile unsigned *)(bar + 2) != 0u;
-    }
-    __syncthreads();
-    return !bad;
-}
-
 // ---- mixed precision: FP32 coefficients, two sweeps.
 // The diffusion sum is taken over temperature differences to the updated
 // node (the rows of the triangle stiffness sum to zero), so FP32 keeps the

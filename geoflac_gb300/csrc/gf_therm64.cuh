@@ -65,16 +65,17 @@ __global__ void __launch_bounds__(GF_THREADS) k_therm_prep(const DevParams *__re
 // one of its values changed (high half) to the sweep's own counter and waits
 // until all have arrived, so that the barrier's word carries the convergence
 // test too.  1 / 0: some value changed / none did; -1: gave up.
-__device__ __forceinline__ int therm_sync(DevClock *C, int k, bool changed) {
+#define GF_TH_POLLS (1 << 22)
+__device__ __forceinline__ int therm_sync(unsigned *slot, bool changed, int polls = GF_TH_POLLS) {
     __shared__ int res;
     const int any = __syncthreads_or(changed);
     if (threadIdx.x == 0) {
-        unsigned *slot = reinterpret_cast<unsigned *>(C->therm_flags + k), v;
+        unsigned v;
         const unsigned add = any ? 0x10001u : 1u;
         asm volatile("atom.add.acq_rel.gpu.u32 %0, [%1], %2;" : "=r"(v) : "l"(slot), "r"(add) : "memory");
         v += add;
         int it = 0;
-        while ((v & 0xffffu) != gridDim.x && ++it < (1 << 22))
+        while ((v & 0xffffu) != gridDim.x && ++it < polls)
             asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(v) : "l"(slot) : "memory");
         res = (v & 0xffffu) != gridDim.x ? -1 : (v >> 16) != 0u;
     }
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(GF_TH_T, GF_TH_CTAS)
             if (redo) v = t;
         }
         if (act) ((k & 1) ? b1 : b0)[n] = v;
-        const int s = therm_sync(C, k, changed);
+        const int s = therm_sync(reinterpret_cast<unsigned *>(C->therm_flags + k), changed);
         if (s < 0) {
             if (nn == 0) set_status(C, GF_ERR_TIMEOUT, k);
             return;
@@ -343,7 +344,7 @@ __global__ void __launch_bounds__(GF_THREADS, 4)
                 if (w < words) now[w] = bits[threadIdx.x];
             }
         }
-        const int s = therm_sync(C, k, any);
+        const int s = therm_sync(reinterpret_cast<unsigned *>(C->therm_flags + k), any);
         if (s < 0) {
             if (blockIdx.x == 0 && threadIdx.x == 0) set_status(C, GF_ERR_TIMEOUT, k);
             return;

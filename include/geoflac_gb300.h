@@ -372,18 +372,17 @@ const char *gf_strerror(int code);
 int gf_min_angle_noalloc(const double *d_cord, int nx, int nz, void *stream, double *min_angle);
 
 /* ---- Ensembles (no reference counterpart) -----------------------------
- * A batch advances many independent models together: one persistent,
- * co-resident kernel per step walks every member's elements and nodes in
- * tiles of one member each, phase by phase (the reference runs one model
- * per process).  Members are GF_MODE_MIXED contexts that share the step
+ * A batch advances many independent models together: every phase of the
+ * step is one launch over tiles of all members' elements or nodes, each tile
+ * of one member (the reference runs one model per process).  Members are GF_MODE_MIXED contexts that share the step
  * schedule (nloop, nsrate, ifreq_*, itherm); they stay owned by the caller,
  * must outlive the batch, and must not be stepped by other calls while a
  * batch step runs.  Their states stay readable with gf_download. */
 typedef struct gf_batch gf_batch;
 typedef struct gf_batch_config {
     int threads;          /* threads per CTA: 128, 256 or 512 */
-    int items_per_thread; /* a tile is threads * items_per_thread items of one member */
-    int ctas_per_sm;      /* resident CTAs per SM (capped by occupancy) */
+    int items_per_thread; /* a tile is threads * items_per_thread items of one member (fewer in a small batch) */
+    int ctas_per_sm;      /* >= 1; the phases run at the residency that their registers allow */
     int graph_steps;      /* steps per captured CUDA graph; 0 = direct launches */
 } gf_batch_config;
 int gf_batch_create(gf_batch **out, gf_ctx **members, int n);
@@ -418,10 +417,9 @@ int gf_batch_backup(gf_batch *b);
 int gf_batch_restore(gf_batch *b, const int *members, int count);
 long long gf_batch_elements(gf_batch *b);
 int gf_batch_grid(gf_batch *b);
-/* Check of the bounded grid barrier that separates the phases of the
- * persistent kernels (the ensemble step, the FP64 thermal sweeps): a
+/* Check of the bounded grid barrier between the FP64 thermal sweeps: a
  * two-CTA co-resident launch in which CTA `absent_cta` (0 or 1) never
- * arrives, so the other gives up after `limit` polls (about 64 ns each) and
+ * arrives, so the other gives up after `limit` polls and
  * the call returns GF_ERR_TIMEOUT with the device still usable; absent_cta
  * = -1 lets both arrive (GF_OK).  passed[k] = 1 if CTA k left the barrier
  * normally, 0 if it gave up, -1 if it never reached it.  No reference
