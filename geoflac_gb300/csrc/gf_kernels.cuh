@@ -1112,18 +1112,31 @@ template <class R> __device__ __forceinline__ int plastic_branch(const DevParams
     }
     return 2;
 }
-template <class R>
-__device__ __forceinline__ int plastic_table_state(const DevParams &P, const DevArrays &A, const GfDims &d, GF_IDX e,
-                                                   int iph, R pls) {
-    if (P.itype_melting == 1) return -1;
-    for (int k = 0; k < P.nphase; ++k) {
-        const double r = A.phase_ratio[gf_pr(d, e, k)];
-        if (k == iph) {
-            if (__double_as_longlong(r) != 0x3ff0000000000000ll) return -1; // exactly 1
-        } else if (!gf_ratio_below_cut(r)) {
-            return -1;
+// Bit k: phase k's ratio in the element is exactly 1 (one) / below the cut
+// (low).  Four ratios at a time without an early exit, so that their loads
+// overlap, and early in the kernel: they need no other value.
+struct PhaseTests {
+    unsigned one, low;
+};
+__device__ __forceinline__ PhaseTests phase_tests(const DevParams &P, const DevArrays &A, const GfDims &d, GF_IDX e) {
+    PhaseTests t = {0u, 0u};
+    for (int k0 = 0; k0 < P.nphase; k0 += 4) {
+        double r[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) r[q] = k0 + q < P.nphase ? A.phase_ratio[gf_pr(d, e, k0 + q)] : 0.0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            t.one |= (unsigned)(__double_as_longlong(r[q]) == 0x3ff0000000000000ll) << (k0 + q);
+            t.low |= (unsigned)gf_ratio_below_cut(r[q]) << (k0 + q);
         }
     }
+    return t;
+}
+template <class R>
+__device__ __forceinline__ int plastic_table_state(const DevParams &P, int iph, R pls, PhaseTests t) {
+    if (P.itype_melting == 1) return -1;
+    const unsigned others = (~0u >> (32 - P.nphase)) & ~(1u << iph);
+    if (!((t.one >> iph) & 1u) || (t.low & others) != others) return -1;
     return plastic_branch(P, iph, pls);
 }
 

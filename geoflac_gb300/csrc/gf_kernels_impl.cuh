@@ -64,25 +64,51 @@ template <class R> __device__ __forceinline__ void b_k_rheol(const DevParams *__
     int j, i;
     elem_ji(d, e, j, i);
     const double dtd = C->dt;
-    if (e == 0) C->dtavg = C->dtavg + dtd; // fl_rheol.f90:43 (no thread reads dtavg here)
     const R dt = gf_to<R>(dtd);
     R *st = (R *)A.stress0;
     const R *area = (const R *)A.area;
 
     GF_IDX n1 = gf_node(d, j, i);
+    // Everything the element reads is loaded before its first store: the
+    // compiler keeps a load behind any store that might alias it, and with
+    // reads between the stores each field's latency came on top of the others'
+    R *se2sr = (R *)A.se2sr;
+    R *sshrheat = (R *)A.sshrheat;
+    R *strain = (R *)A.strain;
+    R *aps = (R *)A.aps;
+    R *visn = (R *)A.visn;
+    const R *dvol = (const R *)A.dvol;
     R vx[4], vy[4];
-    R ar[4];
+    R ar[4], dvl[4], se[3], sn3[3];
+    R s0v[4][4]; // start-of-step stresses [comp][tri]
     for (int k = 0; k < 4; ++k) ar[k] = area[gf_ek(d, e, k)];
     R dx[3][4], dz[3][4], sr[3][4];
-    {
-        // FP32 from the hi/lo splits: coordinates and velocities relative to
-        // the quad's node 1 (each triangle's shape derivatives sum to zero,
-        // so a common velocity offset drops out of the strain rates)
-        QuadF qf;
-        load_vel_rel(A, d, j, i, vx, vy);
-        load_quad_rel(A, d, j, i, qf);
-        shape_derivs_f(qf, ar, dx, dz);
+    // FP32 from the hi/lo splits: coordinates and velocities relative to
+    // the quad's node 1 (each triangle's shape derivatives sum to zero,
+    // so a common velocity offset drops out of the strain rates)
+    QuadF qf;
+    load_vel_rel(A, d, j, i, vx, vy);
+    load_quad_rel(A, d, j, i, qf);
+    int iph = A.iphase[e] - 1;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) s0v[c][k] = st[gf_s(d, e, c, k)];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        se[c] = se2sr[gf_ek(d, e, c)];
+        sn3[c] = strain[gf_ek(d, e, c)];
     }
+    R shr = sshrheat[e];
+    R aps_e = aps[e];
+    // mixed path: stored normal stresses are deviations from -pref
+    const R pref = A.pr_hi[e]; // == float(p_ref)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) dvl[k] = dvol[gf_ek(d, e, k)];
+    R dike = A.dike_released ? gf_to<R>(A.dike_released[e]) : R(0);
+    R vis = visn[e]; // (unless it is updated below)
+    const PhaseTests pt = phase_tests(P, A, d, e);
+    shape_derivs_f(qf, ar, dx, dz);
     // node triplets of triangles A,B,C,D: (1,2,3), (3,2,4), (1,2,4), (1,4,3)
     const int tn[4][3] = {{0, 1, 2}, {2, 1, 3}, {0, 1, 3}, {0, 3, 2}};
 #pragma unroll
@@ -106,45 +132,32 @@ template <class R> __device__ __forceinline__ void b_k_rheol(const DevParams *__
             sr[1][k + 1] = R(0.5) * (em - edb);
         }
     }
-    R *se2sr = (R *)A.se2sr;
-    R *sshrheat = (R *)A.sshrheat;
     R s11 = gf_scale<-2>(sr[0][0] + sr[0][1] + sr[0][2] + sr[0][3]);
     R s22 = gf_scale<-2>(sr[1][0] + sr[1][1] + sr[1][2] + sr[1][3]);
     R s12 = gf_scale<-2>(sr[2][0] + sr[2][1] + sr[2][2] + sr[2][3]);
     R srII = gf_scale<-1>(m_sqrt((s11 - s22) * (s11 - s22) + gf_scale<2>(s12) * s12));
     R srI = gf_scale<-1>(s11 + s22);
     R srs2 = (s11 - srI) * (s11 - srI) + (s22 - srI) * (s22 - srI) + gf_scale<1>(s12) * s12;
-    se2sr[gf_ek(d, e, 0)] = se2sr[gf_ek(d, e, 0)] + s11 * dt;
-    se2sr[gf_ek(d, e, 1)] = se2sr[gf_ek(d, e, 1)] + s22 * dt;
-    se2sr[gf_ek(d, e, 2)] = se2sr[gf_ek(d, e, 2)] + s12 * dt;
-    R s0v[4][4]; // start-of-step stresses [comp][tri]
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) s0v[c][k] = st[gf_s(d, e, c, k)];
+    se[0] = se[0] + s11 * dt;
+    se[1] = se[1] + s22 * dt;
+    se[2] = se[2] + s12 * dt;
     s11 = gf_scale<-2>(s0v[0][0] + s0v[0][1] + s0v[0][2] + s0v[0][3]);
     s22 = gf_scale<-2>(s0v[1][0] + s0v[1][1] + s0v[1][2] + s0v[1][3]);
     s12 = gf_scale<-2>(s0v[2][0] + s0v[2][1] + s0v[2][2] + s0v[2][3]);
     R stII = gf_scale<-1>(m_sqrt((s11 - s22) * (s11 - s22) + gf_scale<2>(s12) * s12));
-    R shr = sshrheat[e];
     if (srII != R(0.0)) shr = shr + gf_ddiv(stII, srII) * srs2 * dt;
 
-    int iph = A.iphase[e] - 1;
     int irh = P.irheol[iph];
     const R bulkm = P.f_bulkm[iph], rmu = P.f_rm[iph];
     R stherm = R(0.0);
     if (P.istress_therm > 0)
         stherm = R(-P.alfa[iph] * P.bulkm[iph] * (A.temp[n1] - A.temp0[n1]));
-    R *aps = (R *)A.aps;
-    R aps_e = aps[e];
-    // mixed path: stored normal stresses are deviations from -pref
-    const R pref = A.pr_hi[e]; // == float(p_ref)
     R hardn = 0;
     PlasticConsts<R> pc;
     if (irh == 6 || irh >= 11) {
         // single-phase elements outside the softening interval read the
         // per-phase table
-        const int pst = A.plast_tab ? plastic_table_state<R>(P, A, d, e, iph, aps_e) : -1;
+        const int pst = A.plast_tab ? plastic_table_state<R>(P, iph, aps_e, pt) : -1;
         if (pst >= 0) {
             const R *t = (const R *)A.plast_tab + (GF_IDX)(pst * GF_MAXPH + iph) * GF_PT_W;
             pc.anphi = t[0]; pc.anpsi = t[1]; pc.amc = t[2]; pc.e1 = t[3];
@@ -156,16 +169,13 @@ template <class R> __device__ __forceinline__ void b_k_rheol(const DevParams *__
             pc = plastic_consts<R>(bulkm, rmu, coh, phi, psi, P.f_ten_off);
         }
     }
-    R *visn = (R *)A.visn;
-    R vis;
     if ((irh == 3 || irh >= 11) && update_visc) {
         vis = R(visc_of<R>(P, A, d, j, i, e, st));
         visn[e] = vis;
-    } else {
-        vis = visn[e];
     }
-    R dike = A.dike_released ? gf_to<R>(A.dike_released[e]) : R(0);
-    const R *dvol = (const R *)A.dvol;
+    if (e == 0) C->dtavg = C->dtavg + dtd; // fl_rheol.f90:43 (no thread reads dtavg here)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) se2sr[gf_ek(d, e, c)] = se[c];
     R sp[4][4], sv[4][4], depl[4] = {0, 0, 0, 0};
     bool plas_mod = false;
     MaxwellConsts<R> mc;
@@ -177,7 +187,7 @@ template <class R> __device__ __forceinline__ void b_k_rheol(const DevParams *__
         R de11 = sr[0][k] * dt, de22 = sr[1][k] * dt, de12 = sr[2][k] * dt, de33 = R(0.0);
         // (dike and stherm are +0 without dikes and thermal stress:
         // gf_sub_z / gf_add_z take them on the integer pipes)
-        R dv = gf_sub_z(dvol[gf_ek(d, e, k)], dike);
+        R dv = gf_sub_z(dvl[k], dike);
         sp[0][k] = gf_add_z(s0v[0][k], stherm);
         sp[1][k] = gf_add_z(s0v[1][k], stherm);
         sp[2][k] = s0v[2][k];
@@ -253,10 +263,8 @@ template <class R> __device__ __forceinline__ void b_k_rheol(const DevParams *__
         // the node gather's corner forces of the new stresses (the mesh does
         // not move before fl_node); shape derivatives taken again rather than
         // kept live through the stress update
-        QuadF q2;
-        load_quad_rel(A, d, j, i, q2);
         float dx2[3][4], dz2[3][4];
-        shape_derivs_f(q2, ar, dx2, dz2);
+        shape_derivs_f(qf, ar, dx2, dz2);
         elem_corner_forces(dx2, dz2, ar, sn, A.e_frc, d.E, e);
     }
     if (irh == 6 || irh >= 11) {
@@ -268,12 +276,11 @@ template <class R> __device__ __forceinline__ void b_k_rheol(const DevParams *__
     }
     // accumulates the element-averaged start-of-step stress (s11/s22/s12 are
     // reassigned before this point in fl_rheol.f90:181-183)
-    R *strain = (R *)A.strain;
     s11 = s11 - pref; // total stress, not the stored deviation
     s22 = s22 - pref;
-    strain[gf_ek(d, e, 0)] = strain[gf_ek(d, e, 0)] + s11 * dt;
-    strain[gf_ek(d, e, 1)] = strain[gf_ek(d, e, 1)] + s22 * dt;
-    strain[gf_ek(d, e, 2)] = strain[gf_ek(d, e, 2)] + s12 * dt;
+    strain[gf_ek(d, e, 0)] = sn3[0] + s11 * dt;
+    strain[gf_ek(d, e, 1)] = sn3[1] + s22 * dt;
+    strain[gf_ek(d, e, 2)] = sn3[2] + s12 * dt;
     if (P.ishearh == 1) {
         R qsum = R(0.0);
         R lambda = bulkm - R(2.0 / 3.0) * rmu, mu = rmu;
@@ -301,9 +308,12 @@ template <class R> __device__ __forceinline__ void b_k_rheol(const DevParams *__
     sshrheat[e] = shr;
     (void)nloop;
 }
-// mixed path: 3 CTAs per SM (80 registers; its few spills cost less than the
-// occupancy they buy)
-template <class R> __global__ void __launch_bounds__(GF_THREADS, 3) k_rheol(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d, int update_visc, int nloop) {
+// mixed path: 2 CTAs per SM (128 registers).  Bound by the latency of its loads
+// (about half of the issue slots' wait), so they come first and together: a
+// step of 1000x300 elements 102.4 -> 93.5 us, of 60x20 32.6 -> 29.4 us with
+// k_move_elem's; 3 CTAs (80 registers, more spills) 97, 20 warps of 96
+// registers 93.
+template <class R> __global__ void __launch_bounds__(GF_THREADS, 2) k_rheol(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d, int update_visc, int nloop) {
     gf_pdl_entry();
     b_k_rheol<R>(Pp, C, A, d, update_visc, nloop, (GF_IDX)blockIdx.x * blockDim.x + threadIdx.x);
 }
@@ -647,7 +657,6 @@ template <class R> __device__ __forceinline__ void b_k_move_elem(DevClock *__res
     int j, i;
     elem_ji(d, e, j, i);
     const double dtd = C->dt;
-    if (advance_time && e == 0) C->time = C->time + dtd; // par.f90:86, after every reader of time
     QuadF qf;
     float rvx[4], rvy[4];
     load_quad_rel(A, d, j, i, qf);
@@ -656,6 +665,16 @@ template <class R> __device__ __forceinline__ void b_k_move_elem(DevClock *__res
     R *dvol = (R *)A.dvol;
     R *st = (R *)A.stress0;
     R *strain = (R *)A.strain;
+    // (all loads before the first store: see b_k_rheol)
+    R ar0[4], s0[3][4], e0[3];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        ar0[k] = area[gf_ek(d, e, k)];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) s0[c][k] = st[gf_s(d, e, c, k)];
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) e0[c] = strain[gf_ek(d, e, c)];
     const int nd1[4] = {0, 2, 0, 0}, nd2[4] = {1, 1, 1, 3}, nd3[4] = {2, 3, 3, 2};
     bool neg = false;
     // the surface nodes also moved by diff_topo's dtopo (zero without it)
@@ -667,7 +686,7 @@ template <class R> __device__ __forceinline__ void b_k_move_elem(DevClock *__res
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         int a = nd1[k], b = nd2[k], c = nd3[k];
-        R ar_old = area[gf_ek(d, e, k)];
+        R ar_old = ar0[k];
         R dw12, ar_new;
         {
             // FP32 from edge vectors of the relative coordinates: det = B x C
@@ -692,20 +711,21 @@ template <class R> __device__ __forceinline__ void b_k_move_elem(DevClock *__res
         }
         area[gf_ek(d, e, k)] = ar_new;
         neg |= !(ar_new > R(0));
-        R s11 = st[gf_s(d, e, 0, k)], s22 = st[gf_s(d, e, 1, k)], s12 = st[gf_s(d, e, 2, k)];
+        R s11 = s0[0][k], s22 = s0[1][k], s12 = s0[2][k];
         st[gf_s(d, e, 0, k)] = s11 + 2.0f * s12 * dw12;
         st[gf_s(d, e, 1, k)] = s22 - 2.0f * s12 * dw12;
         st[gf_s(d, e, 2, k)] = s12 + dw12 * (s22 - s11);
         if (k == 0) {
-            R e11 = strain[gf_ek(d, e, 0)], e22 = strain[gf_ek(d, e, 1)], e12 = strain[gf_ek(d, e, 2)];
+            R e11 = e0[0], e22 = e0[1], e12 = e0[2];
             strain[gf_ek(d, e, 0)] = e11 + 2.0f * e12 * dw12;
             strain[gf_ek(d, e, 1)] = e22 - 2.0f * e12 * dw12;
             strain[gf_ek(d, e, 2)] = e12 + dw12 * (e22 - e11);
         }
     }
+    if (advance_time && e == 0) C->time = C->time + dtd; // par.f90:86, after every reader of time
     if (neg) set_status(C, 40, (int)e);
 }
-template <class R> __global__ void __launch_bounds__(GF_THREADS) k_move_elem(DevClock *__restrict__ C, DevArrays A, GfDims d, int advance_time) {
+template <class R> __global__ void __launch_bounds__(GF_THREADS, 3) k_move_elem(DevClock *__restrict__ C, DevArrays A, GfDims d, int advance_time) {
     gf_pdl_entry();
     b_k_move_elem<R>(C, A, d, advance_time, (GF_IDX)blockIdx.x * blockDim.x + threadIdx.x);
 }
@@ -762,9 +782,10 @@ __device__ __forceinline__ void b_k_therm_prep32(const DevParams *__restrict__ P
     const float *area = (const float *)A.area;
     const GF_IDX E = d.E;
     const int tv[2][3] = {{0, 1, 2}, {2, 1, 3}};
+    const float at[2] = {area[gf_ek(d, e, 0)], area[gf_ek(d, e, 1)]}; // (before the first store)
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
-        float a = area[gf_ek(d, e, t)];
+        const float a = at[t];
         const int v1 = tv[t][0], v2 = tv[t][1], v3 = tv[t][2];
         float dd[3] = {(q.y[v2] - q.y[v3]) * a, (q.y[v3] - q.y[v1]) * a, (q.y[v1] - q.y[v2]) * a};
         float zz[3] = {(q.x[v3] - q.x[v2]) * a, (q.x[v1] - q.x[v3]) * a, (q.x[v2] - q.x[v1]) * a};
@@ -868,7 +889,9 @@ __global__ void __launch_bounds__(GF_THREADS) k_therm_apply32(const DevParams *_
 // each (grid y), the longer part first: in one thread after another the
 // parts' memory latencies add up (no load moves above the stores of the part
 // before), which costs more than the launches saved.
-__global__ void __launch_bounds__(GF_THREADS, 3) k_step_a(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d) {
+// (registers as for k_rheol; d: 80 registers for 3 CTAs, 95.4 against 97.5 us
+// a step of 1000x300 elements at the 106 it takes uncapped)
+__global__ void __launch_bounds__(GF_THREADS, 2) k_step_a(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d) {
     gf_pdl_entry();
     const GF_IDX e = (GF_IDX)blockIdx.x * blockDim.x + threadIdx.x;
     if (blockIdx.y == 0)
@@ -896,7 +919,7 @@ __global__ void __launch_bounds__(GF_THREADS) k_step_c(const DevParams *__restri
         b_k_move_cord(C, A, d, (GF_IDX)(blockIdx.y - 1) * d.N + n);
     }
 }
-__global__ void __launch_bounds__(GF_THREADS) k_step_d(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d, int advance_time) {
+__global__ void __launch_bounds__(GF_THREADS, 3) k_step_d(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d, int advance_time) {
     gf_pdl_entry();
     const GF_IDX n = (GF_IDX)blockIdx.x * blockDim.x + threadIdx.x;
     if (blockIdx.y == 0)
