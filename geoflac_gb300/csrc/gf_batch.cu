@@ -58,9 +58,12 @@ struct BatchArgs {
 // One phase: CTA (t, part) works on tile t of the phase's kind.  The parts of
 // a phase (grid y, the longest first) are independent of each other and share
 // its launch.  The member's record is constant while steps run, so it is
-// staged before the wait for the phase before.  128 registers at most at the
-// 512 threads a batch may be configured for.
-template <class Ph> __global__ void __launch_bounds__(512) k_phase(BatchArgs a) {
+// staged before the wait for the phase before.  Ph::regs caps the registers
+// (at most 128, for the 512 threads a batch may be configured for).  All phases
+// wait on memory: a large batch wants warps in flight, a small one many loads
+// of a thread together.  A step of 64 / of 8 members: 128 for all 534 / 34.7
+// us; these 511 / 34.5; b at 64, c at 48, d at 80 registers 503 / 38.6.
+template <class Ph> __global__ void __maxnreg__(Ph::regs) k_phase(BatchArgs a) {
     __shared__ BatchMember m;
     const int2 tl = a.tile[Ph::kind][blockIdx.x];
     const int *src = reinterpret_cast<const int *>(a.members + tl.x);
@@ -77,21 +80,21 @@ template <class Ph> __global__ void __launch_bounds__(128) k_phase_members(Batch
     if (k < a.nmembers) Ph::member(a.members[k]);
 }
 
-#define GF_PHASE(name, k) struct name { static constexpr int kind = k; \
+#define GF_PHASE(name, k, r) struct name { static constexpr int kind = k, regs = r; \
     static __device__ __forceinline__ void item(const BatchMember &m, int part, int opt, GF_IDX i)
 using namespace gfk;
 // the joint launches of an ordinary step (k_step_a to k_step_d)
-GF_PHASE(PhStepA, K_E) {
+GF_PHASE(PhStepA, K_E, 128) {
     if (part == 0) b_k_rheol<float>(m.P, m.C, m.A, m.d, 0, 0, i);
     else b_k_therm_prep32(m.P, m.A, m.d, (float *)m.A.t_coef, i);
 } };
-GF_PHASE(PhStepB, K_N) {
+GF_PHASE(PhStepB, K_N, 80) {
     if (part == 0) b_k_node<float>(m.P, m.C, m.A, m.d, i);
     else if (part == 1)
         b_k_therm_sweep32(m.P, m.C, m.A, m.d, (const float *)m.A.t_coef, (float *)m.A.t_delta0, m.A.t_delta1, 0, i);
     else b_k_rheol_avg<float>(m.C, m.A, m.d, opt == 2 ? 1 : 0, i);
 } };
-GF_PHASE(PhStepC, K_N) {
+GF_PHASE(PhStepC, K_N, 64) {
     if (part == 0) {
         b_k_therm_sweep32(m.P, m.C, m.A, m.d, (const float *)m.A.t_coef, (float *)m.A.t_delta0, m.A.t_delta1, 1, i);
         if (opt == 2 && i == 0) b_k_rheol_clock(m.C, 1);
@@ -99,37 +102,37 @@ GF_PHASE(PhStepC, K_N) {
         b_k_move_cord(m.C, m.A, m.d, (GF_IDX)((part - 1) * m.d.N) + i);
     }
 } };
-GF_PHASE(PhStepD, K_N) { // opt: time advances here (par.f90:86), unless dt_mass follows
+GF_PHASE(PhStepD, K_N, 128) { // opt: time advances here (par.f90:86), unless dt_mass follows
     if (part == 1) b_k_therm_apply32(m.P, m.A, m.d, m.A.t_delta1, i);
     else if (m.movegrid) b_k_move_elem<float>(m.C, m.A, m.d, opt, i);
     else if (opt && i == 0) m.C->time = m.C->time + m.C->dt;
 } };
 // the same parts one by one, for steps that need the new temperatures first
-GF_PHASE(PhPrep, K_E) { b_k_therm_prep32(m.P, m.A, m.d, (float *)m.A.t_coef, i); } };
-GF_PHASE(PhSweep, K_N) {
+GF_PHASE(PhPrep, K_E, 80) { b_k_therm_prep32(m.P, m.A, m.d, (float *)m.A.t_coef, i); } };
+GF_PHASE(PhSweep, K_N, 64) {
     b_k_therm_sweep32(m.P, m.C, m.A, m.d, (const float *)m.A.t_coef, (float *)m.A.t_delta0, m.A.t_delta1, opt, i);
 } };
-GF_PHASE(PhApply, K_N) { b_k_therm_apply32(m.P, m.A, m.d, m.A.t_delta1, i); } };
-GF_PHASE(PhMarkers, K_M) { b_k_phase_markers32(m.P, m.A, m.d, m.nmarkers, i); } };
-GF_PHASE(PhRecount, K_E) { b_k_phase_recount<float>(m.P, m.C, m.A, m.d, 0, i); } };
-GF_PHASE(PhRheol, K_E) { b_k_rheol<float>(m.P, m.C, m.A, m.d, opt, 0, i); } };
-GF_PHASE(PhNode, K_N) { // and fl_rheol's averaging
+GF_PHASE(PhApply, K_N, 80) { b_k_therm_apply32(m.P, m.A, m.d, m.A.t_delta1, i); } };
+GF_PHASE(PhMarkers, K_M, 80) { b_k_phase_markers32(m.P, m.A, m.d, m.nmarkers, i); } };
+GF_PHASE(PhRecount, K_E, 80) { b_k_phase_recount<float>(m.P, m.C, m.A, m.d, 0, i); } };
+GF_PHASE(PhRheol, K_E, 128) { b_k_rheol<float>(m.P, m.C, m.A, m.d, opt, 0, i); } };
+GF_PHASE(PhNode, K_N, 80) { // and fl_rheol's averaging
     if (part == 0) b_k_node<float>(m.P, m.C, m.A, m.d, i);
     else b_k_rheol_avg<float>(m.C, m.A, m.d, opt == 2 ? 1 : 0, i);
 } };
-GF_PHASE(PhCord, K_N) {
+GF_PHASE(PhCord, K_N, 80) {
     if (opt == 2 && part == 0 && i == 0) b_k_rheol_clock(m.C, 1);
     if (m.movegrid && i < m.d.N) b_k_move_cord(m.C, m.A, m.d, (GF_IDX)(part * m.d.N) + i);
 } };
-GF_PHASE(PhMove, K_E) {
+GF_PHASE(PhMove, K_E, 80) {
     if (m.movegrid) b_k_move_elem<float>(m.C, m.A, m.d, opt, i);
     else if (opt && i == 0) m.C->time = m.C->time + m.C->dt;
 } };
-GF_PHASE(PhDens, K_E) { b_k_elem_dens<float>(m.P, m.C, m.A, m.d, i); } };
-GF_PHASE(PhRmass, K_N) { b_k_node_gather_tri<float>((const float *)m.A.e_tri, m.A.rmass, m.d, i); } };
-GF_PHASE(PhDt, K_EN) { b_k_dt_reduce<float>(m.P, m.C, m.A, m.d, i); } };
-GF_PHASE(PhAm3, K_E) { if (m.idt_scale != 0) b_k_elem_am3<float>(m.P, m.C, m.A, m.d, i); } };
-GF_PHASE(PhAmass, K_N) {
+GF_PHASE(PhDens, K_E, 80) { b_k_elem_dens<float>(m.P, m.C, m.A, m.d, i); } };
+GF_PHASE(PhRmass, K_N, 80) { b_k_node_gather_tri<float>((const float *)m.A.e_tri, m.A.rmass, m.d, i); } };
+GF_PHASE(PhDt, K_EN, 80) { b_k_dt_reduce<float>(m.P, m.C, m.A, m.d, i); } };
+GF_PHASE(PhAm3, K_E, 80) { if (m.idt_scale != 0) b_k_elem_am3<float>(m.P, m.C, m.A, m.d, i); } };
+GF_PHASE(PhAmass, K_N, 80) {
     if (m.idt_scale != 0) b_k_node_gather_tri<float>((const float *)m.A.e_tri, m.A.amass, m.d, i);
     else if (i < m.d.N) m.A.amass[i] = m.A.rmass[i];
 } };
