@@ -20,11 +20,16 @@
 // here; the FP32 spectral term stays in TMEM; an activation is read once and
 // written once per layer.  Sums, their order and every BF16 rounding are those
 // of the GEMM path, so the results are the same bits.  A row CTA is then bound
-// by the GELU's erff (about 50 instructions per value), for which twelve
-// epilogue warps share the SM with one TMA and one MMA warp.
-// Measured at 64 samples of 128 x 384 points (ncu): k_row 150 us for the lift
-// and about 300 us per layer, k_proj 453 us, k_fwd_h 17, k_modes 27 and k_inv_h
-// 30 us; the forecast of 64 members 11.9 -> 2.44 ms, a training step 44 -> 33.
+// by the GELU's erff (about 30 instructions per value, half of them on the
+// half-rate ALU pipe), for which 24 epilogue warps, half of the channels each,
+// share the SM with one TMA and one MMA warp.
+// The new activations have a tile of their own, so that the next row's load
+// starts when the products have read v, not when the row is stored.
+// Measured at 64 samples of 128 x 384 points (ncu): k_row 160 us for the lift
+// and 286 us per layer (12 warps writing in place: 302), k_proj 422 us (12
+// warps that wait for the row's second product: 453), k_fwd_h 17, k_modes 27
+// and k_inv_h 30 us; the forecast of 64 members 2.27 -> 2.17 ms (by GEMMs layer
+// by layer 11.9).
 //
 // Every mbarrier wait is bounded; a wait that gives up raises the error flag
 // that gf_gemm_error() reads.
@@ -43,44 +48,46 @@ struct RowArgs {
 };
 // shared memory of k_row: the DFT matrix of the forward transform first (its
 // MMA reads 128 rows from every 64-column block and ignores all but K2, so
-// 16 KB past the last block must stay inside), then IW, Wl, Z and v
+// 16 KB past the last block must stay inside), then IW, Wl, Z, v and the new v
 template <int NT> struct RowSmem {
     __host__ __device__ static uint32_t iw(int K2) { return (uint32_t)(2 * NT * K2 * 128); }
     __host__ __device__ static uint32_t wl(int K2) { return iw(K2) + NT * 16384; }
     __host__ __device__ static uint32_t zz(int K2) { return wl(K2) + 8192; }
-    __host__ __device__ static uint32_t vv(int K2) { return zz(K2) + 2 * 8192; }
-    __host__ __device__ static uint32_t bars(int K2) { return vv(K2) + 2 * NT * 16384; }
+    __host__ __device__ static uint32_t vv(int K2) { return zz(K2) + 8192; }
+    __host__ __device__ static uint32_t oo(int K2) { return vv(K2) + NT * 16384; }
+    __host__ __device__ static uint32_t bars(int K2) { return oo(K2) + NT * 16384; }
     __host__ __device__ static uint32_t total(int K2) { return bars(K2) + 512 + 1024; }
 };
 
-// warps 0 .. 4 NT - 1: epilogue of point tile warp / 4; then two warps for the
-// DFT's accumulator, the TMA warp and the MMA warp
+// warps 0 .. 8 NT - 1: epilogue of point tile (warp / 4) % NT, half of the
+// channels each; then two warps for the DFT's accumulator, the TMA warp and the
+// MMA warp
 template <int NT>
-__global__ void __launch_bounds__(NT * 128 + 128, 1)
+__global__ void __launch_bounds__(NT * 256 + 128, 1)
     k_row(const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmZ,
           const __grid_constant__ CUtensorMap tmIW, const __grid_constant__ CUtensorMap tmW,
           const __grid_constant__ CUtensorMap tmFW, const __grid_constant__ CUtensorMap tmO, RowArgs a) {
     extern __shared__ uint8_t dsmem[];
     typedef RowSmem<NT> L;
-    constexpr int W = NT * 128, EW = NT * 4;
+    constexpr int W = NT * 128, EW = NT * 8;
     constexpr uint32_t TCOLS = NT == 1 ? 256 : 512;
     uint8_t *base = align1k(dsmem);
     uint8_t *sFW = base, *sIW = base + L::iw(a.K2), *sW = base + L::wl(a.K2), *sZ = base + L::zz(a.K2),
-            *sV = base + L::vv(a.K2);
+            *sV = base + L::vv(a.K2), *sO = base + L::oo(a.K2);
     uint64_t *full = reinterpret_cast<uint64_t *>(base + L::bars(a.K2));
-    uint64_t *wfull = full + 2, *dready = full + 3, *dfree = full + 4, *vready = full + 5, *fready = full + 6,
-             *ffree = full + 7;
+    uint64_t *ofree = full + 1, *wfull = full + 2, *dready = full + 3, *dfree = full + 4, *vready = full + 5,
+             *fready = full + 6, *ffree = full + 7;
     uint32_t *slot = reinterpret_cast<uint32_t *>(full + 8);
     float *sbias = reinterpret_cast<float *>(full + 10);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool has_fw = a.Xw != nullptr;
     if (threadIdx.x == 0) {
-        mbar_init(&full[0], 1);
-        mbar_init(&full[1], 1);
+        mbar_init(full, 1);
+        mbar_init(ofree, 1);
         mbar_init(wfull, 1);
         mbar_init(dready, 1);
         mbar_init(dfree, EW);
-        mbar_init(vready, EW + 2); // and the TMA and the MMA thread: neither may be two phases behind
+        mbar_init(vready, EW);
         mbar_init(fready, 1);
         mbar_init(ffree, 2);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -93,12 +100,12 @@ __global__ void __launch_bounds__(NT * 128 + 128, 1)
     if (warp == EW + 2) {
         if (lane == 0) { // TMA
             const uint32_t bytes = NT * 16384 + (a.has_spec ? a.K2 * 128 : 0);
-            auto load = [&](int it) {
-                const int s = it & 1, r = r0 + it * (int)gridDim.x;
-                mbar_expect_tx(&full[s], bytes);
-                for (int t = 0; t < NT; ++t)
-                    tma_load_2d(sV + (s * NT + t) * 16384, &tmV, 0, r * W + t * 128, &full[s]);
-                if (a.has_spec) tma_load_2d(sZ + s * 8192, &tmZ, 0, r * a.K2, &full[s]);
+            int loaded = 0;
+            auto load = [&]() {
+                const int r = r0 + loaded++ * (int)gridDim.x;
+                mbar_expect_tx(full, bytes);
+                for (int t = 0; t < NT; ++t) tma_load_2d(sV + t * 16384, &tmV, 0, r * W + t * 128, full);
+                if (a.has_spec) tma_load_2d(sZ, &tmZ, 0, r * a.K2, full);
             };
             mbar_expect_tx(wfull, 8192 + (a.has_spec ? NT * 16384 : 0) + (has_fw ? 2 * NT * a.K2 * 128 : 0));
             tma_load_2d(sW, &tmW, 0, 0, wfull);
@@ -106,29 +113,32 @@ __global__ void __launch_bounds__(NT * 128 + 128, 1)
                 for (int t = 0; t < NT; ++t) tma_load_2d(sIW + t * 16384, &tmIW, 0, t * 128, wfull);
             if (has_fw)
                 for (int k = 0; k < 2 * NT; ++k) tma_load_2d(sFW + k * a.K2 * 128, &tmFW, k * 64, 0, wfull);
-            int loaded = 0;
-            for (; loaded < 2 && loaded < n; ++loaded) load(loaded);
-            mbar_arrive(vready);
+            if (n > 0) load();
+            if (n > 1) {
+                ok = mbar_wait(dready, 0); // row 0's products have read v and Z
+                if (ok) load();
+            }
             for (int it = 0; ok && it < n; ++it) {
                 ok = mbar_wait(vready, it & 1);
                 if (!ok) break;
                 if (a.store_v) {
                     for (int t = 0; t < NT; ++t)
-                        tma_store_2d(&tmO, 0, (r0 + it * (int)gridDim.x) * W + t * 128,
-                                     sV + ((it & 1) * NT + t) * 16384);
+                        tma_store_2d(&tmO, 0, (r0 + it * (int)gridDim.x) * W + t * 128, sO + t * 16384);
                     bulk_commit();
                 }
-                if (it + 2 < n) {
-                    if (has_fw) ok = mbar_wait(fready, it & 1);
-                    bulk_wait_read();
-                    if (ok) load(loaded++);
+                if (it + 2 < n) { // before the store's and the DFT's reads are waited for
+                    ok = mbar_wait(dready, (it + 1) & 1);
+                    if (!ok) break;
+                    load();
                 }
-                mbar_arrive(vready);
+                if (has_fw) ok = mbar_wait(fready, it & 1);
+                bulk_wait_read();
+                mbar_arrive(ofree);
             }
             bulk_wait();
             // no copy of this CTA is in flight when it ends, on any path
             mbar_wait(wfull, 0);
-            for (int q = loaded > 2 ? loaded - 2 : 0; q < loaded; ++q) mbar_wait(&full[q & 1], (q >> 1) & 1);
+            if (loaded > 0) mbar_wait(full, (loaded - 1) & 1);
         }
         __syncwarp();
     } else if (warp == EW + 3) {
@@ -136,13 +146,12 @@ __global__ void __launch_bounds__(NT * 128 + 128, 1)
             const uint32_t id = idesc_of(64, 0, 0), ids = idesc_of(64, 0, 1);
             ok = mbar_wait(wfull, 0);
             auto mix = [&](int it) {
-                const int s = it & 1;
-                ok = ok && mbar_wait(&full[s], (it >> 1) & 1);
+                ok = ok && mbar_wait(full, it & 1);
                 if (!ok) return;
                 fence_after();
-                const uint64_t dw = sdesc(smem_u32(sW)), dz = sdesc_mn(smem_u32(sZ + s * 8192), 1024);
+                const uint64_t dw = sdesc(smem_u32(sW)), dz = sdesc_mn(smem_u32(sZ), 1024);
                 for (int t = 0; t < NT; ++t) {
-                    const uint64_t dv = sdesc(smem_u32(sV + (s * NT + t) * 16384));
+                    const uint64_t dv = sdesc(smem_u32(sV + t * 16384));
                     for (int k = 0; k < a.kin / 16; ++k)
                         mma(tmem + t * 64, dv + K_STEP * k, dw + K_STEP * k, id, k > 0);
                     if (a.has_spec) {
@@ -154,21 +163,18 @@ __global__ void __launch_bounds__(NT * 128 + 128, 1)
                 mma_commit(dready);
             };
             if (n > 0) mix(0);
-            mbar_arrive(vready);
             for (int it = 0; ok && it < n; ++it) {
                 if (it + 1 < n) {
                     ok = mbar_wait(dfree, it & 1);
                     if (ok) mix(it + 1);
                 }
-                ok = ok && mbar_wait(vready, it & 1);
-                mbar_arrive(vready);
                 if (has_fw && ok) {
-                    ok = it == 0 || mbar_wait(ffree, (it - 1) & 1);
+                    ok = mbar_wait(vready, it & 1) && (it == 0 || mbar_wait(ffree, (it - 1) & 1));
                     if (!ok) break;
                     fence_after();
                     for (int kb = 0; kb < 2 * NT; ++kb) {
                         const uint64_t df = sdesc(smem_u32(sFW + kb * a.K2 * 128)),
-                                       dv = sdesc_mn(smem_u32(sV + (it & 1) * NT * 16384 + kb * 8192), 1024);
+                                       dv = sdesc_mn(smem_u32(sO + kb * 8192), 1024);
                         for (int k = 0; k < 4; ++k)
                             mma(tmem + 2 * NT * 64, df + K_STEP * k, dv + MN_STEP * k, ids, (kb | k) > 0);
                     }
@@ -200,43 +206,47 @@ __global__ void __launch_bounds__(NT * 128 + 128, 1)
             }
         }
     } else {
-        const int t = warp >> 2, q = warp & 3, w = t * 128 + q * 32 + lane;
+        const int t = (warp >> 2) % NT, q = warp & 3, w = t * 128 + q * 32 + lane, ch = warp / (4 * NT) * 32;
         const uint32_t td = tmem + t * 64 + ((uint32_t)(q * 32) << 16);
         for (int it = 0; it < n; ++it) {
             ok = mbar_wait(dready, it & 1);
             if (!ok) break;
             fence_after();
-            uint8_t *tile = sV + (it & 1) * NT * 16384;
             float *zrow = a.z ? a.z + ((long long)(r0 + it * (int)gridDim.x) * W + w) * CH : nullptr;
-#pragma unroll
-            for (int c0 = 0; c0 < CH; c0 += 32) {
-                float v[32];
-                tmem_ld<32>(td + c0, v);
+#pragma unroll 1
+            for (int c0 = ch; c0 < ch + 32; c0 += 16) { // (one copy of the GELU's code)
+                float v[16];
+                tmem_ld<16>(td + c0, v);
                 if (a.has_spec) {
-                    float s[32];
-                    tmem_ld<32>(td + NT * 64 + c0, s);
+                    float s[16];
+                    tmem_ld<16>(td + NT * 64 + c0, s);
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) v[i] = (v[i] + sbias[c0 + i]) + s[i];
+                    for (int i = 0; i < 16; ++i) v[i] = (v[i] + sbias[c0 + i]) + s[i];
                 } else {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) v[i] = v[i] + sbias[c0 + i];
+                    for (int i = 0; i < 16; ++i) v[i] = v[i] + sbias[c0 + i];
                 }
-                if (c0 == 32) { // both accumulators of this row are in registers
+                if (c0 == ch + 16) { // this warp's part of both accumulators is in registers
                     fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(dfree);
                 }
                 if (zrow) {
 #pragma unroll
-                    for (int i = 0; i < 32; i += 8) st_global8(zrow + c0 + i, v + i);
+                    for (int i = 0; i < 16; i += 8) st_global8(zrow + c0 + i, v + i);
                 }
                 if (a.act) {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) v[i] = act_gelu(v[i]);
+                    for (int i = 0; i < 16; ++i) v[i] = act_gelu(v[i]);
+                }
+                if (c0 == ch && it > 0) { // row it - 1's new activations are stored and transformed
+                    ok = mbar_wait(ofree, (it - 1) & 1);
+                    if (!ok) break;
                 }
 #pragma unroll
-                for (int j = 0; j < 4; ++j) *swz(tile, w, c0 / 8 + j) = pack8(v + 8 * j);
+                for (int j = 0; j < 2; ++j) *swz(sO, w, c0 / 8 + j) = pack8(v + 8 * j);
             }
+            if (!ok) break;
             fence_async();
             __syncwarp();
             if (lane == 0) mbar_arrive(vready);
@@ -255,11 +265,11 @@ struct ProjArgs {
     float *out;  // [M][16]
 };
 template <int NT>
-__global__ void __launch_bounds__(NT * 128 + 64, 1)
+__global__ void __launch_bounds__(NT * 256 + 64, 1)
     k_proj(const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmP1,
            const __grid_constant__ CUtensorMap tmP2, const __grid_constant__ CUtensorMap tmH, ProjArgs a) {
     extern __shared__ uint8_t dsmem[];
-    constexpr int W = NT * 128, EW = NT * 4, P = 128, CO = 16;
+    constexpr int W = NT * 128, EW = NT * 8, P = 128, CO = 16;
     constexpr uint32_t TCOLS = NT == 1 ? 256 : 512;
     uint8_t *base = align1k(dsmem);
     uint8_t *sV = base, *sH = sV + 2 * NT * 16384, *sP1 = sH + NT * 32768, *sP2 = sP1 + 16384;
@@ -355,49 +365,62 @@ __global__ void __launch_bounds__(NT * 128 + 64, 1)
         }
         __syncwarp();
     } else {
-        const int t = warp >> 2, q = warp & 3, rt = q * 32 + lane, w = t * 128 + rt;
+        const int t = (warp >> 2) % NT, q = warp & 3, rt = q * 32 + lane, w = t * 128 + rt, half = warp / (4 * NT);
         const uint32_t lanes = (uint32_t)(q * 32) << 16;
         const uint32_t td = tmem + t * P + lanes, to = tmem + NT * P + t * CO + lanes;
-        uint8_t *tile = sH + t * 32768;
-        for (int it = 0; it < n; ++it) {
-            ok = mbar_wait(dready, it & 1) && (it == 0 || mbar_wait(hfree, (it - 1) & 1));
-            if (!ok) break;
-            fence_after();
-            const long long m = (long long)(r0 + it * (int)gridDim.x) * W + w;
-#pragma unroll
-            for (int c0 = 0; c0 < P; c0 += 32) {
-                float v[32];
-                tmem_ld<32>(td + c0, v);
-                if (c0 == P - 32) {
-                    fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(dfree);
-                }
-#pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = v[i] + sb1[c0 + i];
-                if (a.zp) {
-#pragma unroll
-                    for (int i = 0; i < 32; i += 8) st_global8(a.zp + m * P + c0 + i, v + i);
-                }
-#pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = act_gelu(v[i]);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) *swz(tile + (c0 / 64) * 16384, rt, (c0 % 64) / 8 + j) = pack8(v + 8 * j);
-            }
-            fence_async();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(hready);
-            ok = mbar_wait(oready, it & 1);
-            if (!ok) break;
+        uint8_t *tile = sH + t * 32768 + half * 16384;
+        // the second product of row it - 1 is read and stored after the first
+        // chunk of row it is computed, which hides it
+        auto finish = [&](int it) {
+            if (!mbar_wait(oready, it & 1)) return false;
+            if (half) return true;
             fence_after();
             float o[16];
             tmem_ld<16>(to, o);
             fence_before();
 #pragma unroll
             for (int i = 0; i < 16; ++i) o[i] = o[i] + sb2[i];
-            st_global8(a.out + m * CO, o);
-            st_global8(a.out + m * CO + 8, o + 8);
+            float *out = a.out + ((long long)(r0 + it * (int)gridDim.x) * W + w) * CO;
+            st_global8(out, o);
+            st_global8(out + 8, o + 8);
+            return true;
+        };
+        for (int it = 0; ok && it < n; ++it) {
+            ok = mbar_wait(dready, it & 1);
+            if (!ok) break;
+            fence_after();
+            const long long m = (long long)(r0 + it * (int)gridDim.x) * W + w;
+#pragma unroll 1
+            for (int c = 0; c < 64; c += 16) { // (one copy of the GELU's code, as in k_row)
+                const int c0 = half * 64 + c;
+                float v[16];
+                tmem_ld<16>(td + c0, v);
+                if (c == 48) {
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(dfree);
+                }
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] = v[i] + sb1[c0 + i];
+                if (a.zp) {
+#pragma unroll
+                    for (int i = 0; i < 16; i += 8) st_global8(a.zp + m * P + c0 + i, v + i);
+                }
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] = act_gelu(v[i]);
+                if (c == 0 && it > 0) { // row it - 1: its product has read the tile, its copy out too
+                    ok = finish(it - 1) && mbar_wait(hfree, (it - 1) & 1);
+                    if (!ok) break;
+                }
+#pragma unroll
+                for (int j = 0; j < 2; ++j) *swz(tile, rt, c / 8 + j) = pack8(v + 8 * j);
+            }
+            if (!ok) break;
+            fence_async();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(hready);
         }
+        if (ok && n > 0) ok = finish(n - 1);
     }
     if (!ok) atomicExch(&g_tc_err, 1);
     tmem_free(tmem, TCOLS, warp);
@@ -633,13 +656,13 @@ template <int NT> int run_row(const CUtensorMap *m, const RowArgs &a, cudaStream
     const uint32_t smem = RowSmem<NT>::total(a.K2);
     if (!allow_smem(k_row<NT>, smem)) return GF_FNO_ERR_CUDA;
     const int sms = sm_count(), grid = a.rows < sms ? a.rows : sms;
-    k_row<NT><<<grid, NT * 128 + 128, smem, s>>>(m[0], m[1], m[2], m[3], m[4], m[5], a);
+    k_row<NT><<<grid, NT * 256 + 128, smem, s>>>(m[0], m[1], m[2], m[3], m[4], m[5], a);
     return launched();
 }
 template <int NT> int run_proj(const CUtensorMap *m, const ProjArgs &a, cudaStream_t s) {
     if (!allow_smem(k_proj<NT>, proj_smem<NT>())) return GF_FNO_ERR_CUDA;
     const int sms = sm_count(), grid = a.rows < sms ? a.rows : sms;
-    k_proj<NT><<<grid, NT * 128 + 64, proj_smem<NT>(), s>>>(m[0], m[1], m[2], m[3], a);
+    k_proj<NT><<<grid, NT * 256 + 64, proj_smem<NT>(), s>>>(m[0], m[1], m[2], m[3], a);
     return launched();
 }
 
