@@ -22,15 +22,25 @@
 // fifth, but one FP32 ulp of a bias moves the next step's BF16 activations,
 // and its gradients by 4e-4).  Bound: memory (the FP32 pre-activations and
 // gradients) and GELU' (erff and expf), about equally.
-// Measured at 64 samples of 128 x 384 points (ncu, before the FP32 gradients):
-// k_proj_bwd 1046 us, k_row_bwd 349, k_wgrad 110 (64 x 64) and 153 (128 wide),
-// k_modes_bwd 39, k_fwd_h_bwd 36, k_inv_h_bwd 21; the training step 33 -> 8.6 ms.
+// 24 epilogue warps take half of the channels each, with one copy of GELU' in
+// the instruction cache.
+// Measured at 64 samples of 128 x 384 points (ncu): k_proj_bwd 1133 us (12 warps,
+// unrolled code, gradients stored by rows: 1309), k_row_bwd 390 (452), k_wgrad
+// 110 (64 x 64) and 153 (128 wide), k_modes_bwd 40, k_fwd_h_bwd 36, k_inv_h_bwd
+// 22; the training step 8.6 -> 7.7 ms with k_sum_batches_staged (by GEMMs layer
+// by layer 44).
 
 #include "fno_tc.cuh"
 
 namespace {
 
 // ---------------------------------------------------------------- rows
+// The FP32 gradients are written in blocks of 32 points x 8 channels (a warp
+// stores one block, 1 KB, at a time; by rows its 32-byte pieces lay in 32
+// different lines); gf_fno_colsum_blocked reads them.
+__device__ __forceinline__ long long blocked(long long m, int c, int C) {
+    return ((m >> 5) * (C / 8) + (c >> 3)) * 256 + (m & 31) * 8 + (c & 7);
+}
 struct RowBwdArgs {
     int rows, K2;
     const float *z;     // pre-activations of the layer before (FP32), or null: no GELU
@@ -49,13 +59,13 @@ template <int NT> struct BwdSmem {
 
 // warps as in k_row; the phases of its barriers too (see there)
 template <int NT>
-__global__ void __launch_bounds__(NT * 128 + 128, 1)
+__global__ void __launch_bounds__(NT * 256 + 128, 1)
     k_row_bwd(const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmX,
               const __grid_constant__ CUtensorMap tmFW, const __grid_constant__ CUtensorMap tmW,
               const __grid_constant__ CUtensorMap tmIWT, const __grid_constant__ CUtensorMap tmO, RowBwdArgs a) {
     extern __shared__ uint8_t dsmem[];
     typedef BwdSmem<NT> L;
-    constexpr int W = NT * 128, EW = NT * 4;
+    constexpr int W = NT * 128, EW = NT * 8;
     constexpr uint32_t TCOLS = NT == 1 ? 256 : 512;
     uint8_t *base = align1k(dsmem);
     uint8_t *sI = base, *sF = base + L::fw(a.K2), *sW = base + L::wl(a.K2), *sX = base + L::xx(a.K2),
@@ -183,26 +193,27 @@ __global__ void __launch_bounds__(NT * 128 + 128, 1)
             }
         }
     } else {
-        const int t = warp >> 2, q = warp & 3, w = t * 128 + q * 32 + lane;
+        const int t = (warp >> 2) % NT, q = warp & 3, w = t * 128 + q * 32 + lane, ch = warp / (4 * NT) * 32;
         const uint32_t td = tmem + t * 64 + ((uint32_t)(q * 32) << 16);
         for (int it = 0; it < n; ++it) {
-            float *frow = a.df + ((long long)(r0 + it * step) * W + w) * CH;
-            const float *zrow = a.z ? a.z + ((long long)(r0 + it * step) * W + w) * CH : nullptr;
+            const long long m = (long long)(r0 + it * step) * W + w;
+            float *frow = a.df + blocked(m, ch, CH);
+            const float *zrow = a.z ? a.z + m * CH : nullptr;
             float zn[16]; // the next 16 pre-activations, in flight while this chunk is worked on
             if (zrow) {
-                ld_global8(zrow, zn);
-                ld_global8(zrow + 8, zn + 8);
+                ld_global8(zrow + ch, zn);
+                ld_global8(zrow + ch + 8, zn + 8);
             }
             ok = mbar_wait(dready, it & 1);
             if (!ok) break;
             fence_after();
             uint8_t *tile = sV + (it & 1) * NT * 16384;
-#pragma unroll
-            for (int c0 = 0; c0 < CH; c0 += 16) {
+#pragma unroll 1
+            for (int c0 = ch; c0 < ch + 32; c0 += 16, frow += 512) { // (one copy of GELU' in the instruction cache)
                 float v[16], s[16];
                 tmem_ld<16>(td + c0, v);
                 tmem_ld<16>(td + NT * 64 + c0, s);
-                if (c0 == CH - 16) {
+                if (c0 == ch + 16) {
                     fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(dfree);
@@ -213,15 +224,15 @@ __global__ void __launch_bounds__(NT * 128 + 128, 1)
                     float z[16];
 #pragma unroll
                     for (int i = 0; i < 16; ++i) z[i] = zn[i];
-                    if (c0 < CH - 16) {
+                    if (c0 == ch) {
                         ld_global8(zrow + c0 + 16, zn);
                         ld_global8(zrow + c0 + 24, zn + 8);
                     }
 #pragma unroll
                     for (int i = 0; i < 16; ++i) v[i] = v[i] * gelu_d(z[i]);
                 }
-                st_global8(frow + c0, v);
-                st_global8(frow + c0 + 8, v + 8);
+                st_global8(frow, v);
+                st_global8(frow + 256, v + 8);
                 *swz(tile, w, c0 / 8) = pack8(v);
                 *swz(tile, w, c0 / 8 + 1) = pack8(v + 8);
             }
@@ -253,13 +264,13 @@ template <int NT> struct ProjBwdSmem {
 // Row by row: dh = dout P2 -> times GELU'(zp) -> dzp (BF16 to shared memory and
 // memory) -> dv = dzp P1 (in dh's TMEM columns) -> BF16 -> transform along W.
 template <int NT>
-__global__ void __launch_bounds__(NT * 128 + 128, 1)
+__global__ void __launch_bounds__(NT * 256 + 128, 1)
     k_proj_bwd(const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmP1,
                const __grid_constant__ CUtensorMap tmP2, const __grid_constant__ CUtensorMap tmIWT,
                const __grid_constant__ CUtensorMap tmH, const __grid_constant__ CUtensorMap tmO, ProjBwdArgs a) {
     extern __shared__ uint8_t dsmem[];
     typedef ProjBwdSmem<NT> L;
-    constexpr int W = NT * 128, EW = NT * 4, P = 128;
+    constexpr int W = NT * 128, EW = NT * 8, P = 128;
     constexpr uint32_t TCOLS = NT == 1 ? 256 : 512;
     uint8_t *base = align1k(dsmem);
     uint8_t *sI = base, *sH = base + L::hh(a.K2), *sV = base + L::vv(a.K2), *sP1 = base + L::p1(a.K2),
@@ -379,34 +390,35 @@ __global__ void __launch_bounds__(NT * 128 + 128, 1)
             }
         }
     } else {
-        const int t = warp >> 2, q = warp & 3, rt = q * 32 + lane, w = t * 128 + rt;
+        const int t = (warp >> 2) % NT, q = warp & 3, rt = q * 32 + lane, w = t * 128 + rt, half = warp / (4 * NT);
         const uint32_t td = tmem + t * P + ((uint32_t)(q * 32) << 16);
-        uint8_t *th = sH + t * 32768, *tv = sV + t * 16384;
+        uint8_t *th = sH + t * 32768 + half * 16384, *tv = sV + t * 16384;
         for (int it = 0; it < n; ++it) {
             const long long m = (long long)(r0 + it * step) * W + w;
-            const float *zrow = a.zp + m * P;
+            const float *zrow = a.zp + m * P + half * 64;
+            float *frow = a.df1 + blocked(m, half * 64, P);
             float zn[16];
             ld_global8(zrow, zn);
             ld_global8(zrow + 8, zn + 8);
             ok = mbar_wait(dready, it & 1) && (it == 0 || mbar_wait(bfree, (it - 1) & 1));
             if (!ok) break;
             fence_after();
-#pragma unroll
-            for (int c0 = 0; c0 < P; c0 += 16) {
+#pragma unroll 1
+            for (int c = 0; c < 64; c += 16, frow += 512) { // (one copy of GELU', as in k_row_bwd)
                 float v[16], z[16];
-                tmem_ld<16>(td + c0, v);
+                tmem_ld<16>(td + half * 64 + c, v);
 #pragma unroll
                 for (int i = 0; i < 16; ++i) z[i] = zn[i];
-                if (c0 < P - 16) {
-                    ld_global8(zrow + c0 + 16, zn);
-                    ld_global8(zrow + c0 + 24, zn + 8);
+                if (c < 48) {
+                    ld_global8(zrow + c + 16, zn);
+                    ld_global8(zrow + c + 24, zn + 8);
                 }
 #pragma unroll
                 for (int i = 0; i < 16; ++i) v[i] = v[i] * gelu_d(z[i]);
-                st_global8(a.df1 + m * P + c0, v);
-                st_global8(a.df1 + m * P + c0 + 8, v + 8);
-                *swz(th + (c0 / 64) * 16384, rt, (c0 % 64) / 8) = pack8(v);
-                *swz(th + (c0 / 64) * 16384, rt, (c0 % 64) / 8 + 1) = pack8(v + 8);
+                st_global8(frow, v);
+                st_global8(frow + 256, v + 8);
+                *swz(th, rt, c / 8) = pack8(v);
+                *swz(th, rt, c / 8 + 1) = pack8(v + 8);
             }
             fence_before();
             fence_async();
@@ -415,19 +427,20 @@ __global__ void __launch_bounds__(NT * 128 + 128, 1)
             ok = mbar_wait(oready, it & 1);
             if (!ok) break;
             fence_after();
+            frow = a.df + blocked(m, half * 32, CH);
 #pragma unroll
-            for (int c0 = 0; c0 < CH; c0 += 16) {
+            for (int c0 = 0; c0 < 32; c0 += 16, frow += 512) {
                 float v[16];
-                tmem_ld<16>(td + c0, v);
-                if (c0 == CH - 16) {
+                tmem_ld<16>(td + half * 32 + c0, v);
+                if (c0 == 16) {
                     fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(ofree);
                 }
-                st_global8(a.df + m * CH + c0, v);
-                st_global8(a.df + m * CH + c0 + 8, v + 8);
-                *swz(tv, rt, c0 / 8) = pack8(v);
-                *swz(tv, rt, c0 / 8 + 1) = pack8(v + 8);
+                st_global8(frow, v);
+                st_global8(frow + 256, v + 8);
+                *swz(tv, rt, half * 4 + c0 / 8) = pack8(v);
+                *swz(tv, rt, half * 4 + c0 / 8 + 1) = pack8(v + 8);
             }
             fence_async();
             __syncwarp();
@@ -782,13 +795,13 @@ __global__ void __launch_bounds__(256) k_wgrad(const __grid_constant__ CUtensorM
 template <int NT> int run_row_bwd(const CUtensorMap *m, const RowBwdArgs &a, int grid, cudaStream_t s) {
     const uint32_t smem = BwdSmem<NT>::total(a.K2);
     if (!allow_smem(k_row_bwd<NT>, smem)) return GF_FNO_ERR_CUDA;
-    k_row_bwd<NT><<<grid, NT * 128 + 128, smem, s>>>(m[0], m[1], m[2], m[3], m[4], m[5], a);
+    k_row_bwd<NT><<<grid, NT * 256 + 128, smem, s>>>(m[0], m[1], m[2], m[3], m[4], m[5], a);
     return launched();
 }
 template <int NT> int run_proj_bwd(const CUtensorMap *m, const ProjBwdArgs &a, int grid, cudaStream_t s) {
     const uint32_t smem = ProjBwdSmem<NT>::total(a.K2);
     if (!allow_smem(k_proj_bwd<NT>, smem)) return GF_FNO_ERR_CUDA;
-    k_proj_bwd<NT><<<grid, NT * 128 + 128, smem, s>>>(m[0], m[1], m[2], m[3], m[4], m[5], a);
+    k_proj_bwd<NT><<<grid, NT * 256 + 128, smem, s>>>(m[0], m[1], m[2], m[3], m[4], m[5], a);
     return launched();
 }
 template <int NA, int ST> int run_wgrad(const CUtensorMap &ma, const CUtensorMap &mb, const WgradArgs &a,

@@ -180,14 +180,18 @@ template <class T> __global__ void k_colsum(const T *__restrict__ X, float *__re
 // column sums, stage 1: block b sums rows [b*rpb, (b+1)*rpb) of a row-major
 // matrix whose column count divides the block size (coalesced reads; each
 // thread stays on one column), partial[b][c]
-template <class T> __global__ void k_colsum_part(const T *__restrict__ X, float *__restrict__ part, long long rows, int cols,
-                              long long rpb) {
+// BLK: the matrix lies in blocks of 32 rows x 8 columns (as the backward row
+// kernels write their FP32 gradients); the sums and their order are the same.
+template <class T, bool BLK>
+__global__ void k_colsum_part(const T *__restrict__ X, float *__restrict__ part, long long rows, int cols, long long rpb) {
     __shared__ float red[TB];
     const long long r0 = (long long)blockIdx.x * rpb, r1 = min(rows, r0 + rpb);
     const int per = TB / cols; // rows per pass
     const int c = threadIdx.x % cols, rr = threadIdx.x / cols;
     float s = 0.0f;
-    for (long long r = r0 + rr; r < r1; r += per) s += (float)X[r * cols + c];
+#pragma unroll 8 // (eight loads in flight)
+    for (long long r = r0 + rr; r < r1; r += per)
+        s += (float)X[BLK ? (r >> 5) * (32 * cols) + (c >> 3) * 256 + (r & 31) * 8 + (c & 7) : r * cols + c];
     red[threadIdx.x] = s;
     __syncthreads();
     if (threadIdx.x < cols) {
@@ -197,6 +201,8 @@ template <class T> __global__ void k_colsum_part(const T *__restrict__ X, float 
     }
 }
 
+// dst[i] = sum over b of src[b][i] in the order b = 0, 1, ...
+// Many columns: one per thread, sixteen loads in flight.
 __global__ void k_sum_batches(const float *__restrict__ src, float *__restrict__ dst, int nb, long long n, int accum) {
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -204,6 +210,47 @@ __global__ void k_sum_batches(const float *__restrict__ src, float *__restrict__
 #pragma unroll 16 // sixteen loads in flight; the sum's order is b = 0, 1, ...
     for (int b = 0; b < nb; ++b) s += src[(long long)b * n + i];
     dst[i] = (accum ? dst[i] : 0.0f) + s;
+}
+// Few columns: that leaves a handful of warps waiting for one group of loads
+// after another (1024 partial sums of 64 columns 65 us).  Here a CTA stages 256
+// rows of 32 columns at a time through shared memory, all loads in flight and
+// the next tile's while one warp adds up this one's, in the same order.
+// Now 9 us; 256 x 8192 partial sums of a weight 42 -> 12.
+constexpr int SB_R = 256, SB_C = 32, SB_Q = SB_R * SB_C / TB;
+__global__ void __launch_bounds__(TB) k_sum_batches_staged(const float *__restrict__ src, float *__restrict__ dst, int nb,
+                                                           long long n, int accum) {
+    __shared__ float tile[SB_R][SB_C];
+    const int c = threadIdx.x % SB_C, r = threadIdx.x / SB_C;
+    const long long i = (long long)blockIdx.x * SB_C + c;
+    float v[SB_Q], s = 0.0f;
+    auto load = [&](int b0) {
+#pragma unroll
+        for (int q = 0; q < SB_Q; ++q) {
+            const int b = b0 + q * (TB / SB_C) + r;
+            v[q] = b < nb && i < n ? src[(long long)b * n + i] : 0.0f;
+        }
+    };
+    load(0);
+    for (int b0 = 0; b0 < nb; b0 += SB_R) {
+#pragma unroll
+        for (int q = 0; q < SB_Q; ++q) tile[q * (TB / SB_C) + r][c] = v[q];
+        __syncthreads();
+        if (b0 + SB_R < nb) load(b0 + SB_R);
+        if (threadIdx.x < SB_C) {
+            const int m = min(SB_R, nb - b0);
+#pragma unroll 16
+            for (int b = 0; b < m; ++b) s += tile[b][threadIdx.x];
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x < SB_C && i < n) dst[i] = (accum ? dst[i] : 0.0f) + s;
+}
+void sum_batches(const float *src, float *dst, int nb, long long n, int accum, cudaStream_t st) {
+    // (the line: where a column per thread fills the SMs with two CTAs each)
+    if (n <= 2LL * 152 * TB)
+        k_sum_batches_staged<<<(unsigned)((n + SB_C - 1) / SB_C), TB, 0, st>>>(src, dst, nb, n, accum);
+    else
+        k_sum_batches<<<nblk(n), TB, 0, st>>>(src, dst, nb, n, accum);
 }
 
 __global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m, float *__restrict__ v,
@@ -367,9 +414,10 @@ __global__ void k_gather_rows(const uint32_t *__restrict__ src, uint32_t *__rest
 
 #define FNO_RET(s) return cudaGetLastError() == cudaSuccess ? GF_FNO_OK : GF_FNO_ERR_CUDA
 
-template <class T>
+template <class T, bool BLK = false>
 int run_colsum(const T *X, float *out, long long rows, int cols, int accum, void *stream) {
     if (!X || !out || rows < 1 || cols < 1) return GF_FNO_ERR_ARG;
+    if (BLK && (rows % 32 || rows < 4096 || cols % 8 || cols > TB || TB % cols)) return GF_FNO_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     if (cols <= TB && TB % cols == 0 && rows >= 4096) {
         // two stages through a fixed scratch of 1024 partial rows
@@ -383,8 +431,8 @@ int run_colsum(const T *X, float *out, long long rows, int cols, int accum, void
             part_cols = TB;
         }
         long long rpb = (rows + nb - 1) / nb;
-        k_colsum_part<<<nb, TB, 0, st>>>(X, part, rows, cols, rpb);
-        k_sum_batches<<<nblk(cols), TB, 0, st>>>(part, out, nb, cols, accum);
+        k_colsum_part<T, BLK><<<nb, TB, 0, st>>>(X, part, rows, cols, rpb);
+        sum_batches(part, out, nb, cols, accum, st);
     } else {
         k_colsum<<<(unsigned)cols, TB, 0, st>>>(X, out, rows, cols, accum);
     }
@@ -489,13 +537,16 @@ int gf_fno_modes_grad(const float *dRm, float *dR, int modes, int C, void *strea
 int gf_fno_colsum(const float *X, float *out, long long rows, int cols, int accum, void *stream) {
     return run_colsum(X, out, rows, cols, accum, stream);
 }
+int gf_fno_colsum_blocked(const float *X, float *out, long long rows, int cols, int accum, void *stream) {
+    return run_colsum<float, true>(X, out, rows, cols, accum, stream);
+}
 int gf_fno_colsum_bf16(const void *X, float *out, long long rows, int cols, int accum, void *stream) {
     return run_colsum((const __nv_bfloat16 *)X, out, rows, cols, accum, stream);
 }
 
 int gf_fno_sum_batches(const float *src, float *dst, int nb, long long n, int accum, void *stream) {
     if (!src || !dst || nb < 1 || n < 1) return GF_FNO_ERR_ARG;
-    k_sum_batches<<<nblk(n), TB, 0, (cudaStream_t)stream>>>(src, dst, nb, n, accum);
+    sum_batches(src, dst, nb, n, accum, (cudaStream_t)stream);
     FNO_RET(stream);
 }
 

@@ -63,6 +63,7 @@ def _lib():
         "gf_fno_inv_h": [vp, vp, vp, i, i, i, i, vp],
         "gf_fno_proj": [vp, vp, vp, vp, vp, vp, vp, vp, i, i, vp],
         "gf_fno_colsum_bf16": [vp, vp, ll, i, i, vp],
+        "gf_fno_colsum_blocked": [vp, vp, ll, i, i, vp],
         "gf_fno_proj_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, vp],
         "gf_fno_row_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, vp],
         "gf_fno_inv_h_bwd": [vp, vp, vp, i, i, i, i, vp],
@@ -230,6 +231,9 @@ class Fno:
     def gelu_bwd(self, z, da, dz, dz_b=None):
         _ck(self.lib.gf_fno_gelu_bwd(_p(z), _p(da), int(da.dtype == self.torch.bfloat16), _p(dz), _p(dz_b),
                                      z.numel(), self.s), "gelu_bwd")
+
+    def colsum_blocked(self, X, out, rows, cols):
+        _ck(self.lib.gf_fno_colsum_blocked(_p(X), _p(out), rows, cols, 0, self.s), "colsum")
 
     def colsum(self, X, out, rows, cols):
         _ck(self.lib.gf_fno_colsum(_p(X), _p(out), rows, cols, 0, self.s), "colsum")
@@ -446,11 +450,11 @@ class Fno:
         _ck(lib.gf_fno_colsum_bf16(_p(d2), _p(self.g["p2_b"]), M, cfg.cout, 0, s), "colsum")
         _ck(lib.gf_fno_proj_bwd(_p(d2), _p(sv["zp"]), _p(wb["p1_w"]), _p(wb["p2_w"]), _p(IWT), _p(dzp), _p(df1),
                                 _p(dz), _p(df), _p(dZ), rows, W, K2, s), "proj_bwd")
-        self.colsum(df1, self.g["p1_b"], M, cfg.P)
+        self.colsum_blocked(df1, self.g["p1_b"], M, cfg.P)
         self.wgrad_fused(dzp, cfg.P, sv["vL"], Cc, M, self.g["p1_w"])
         for l in reversed(range(cfg.layers)):
             # dz: gradient of layer l's pre-activations, dZ: its transform along W
-            self.colsum(df, self.g[f"b{l}"], M, Cc)
+            self.colsum_blocked(df, self.g[f"b{l}"], M, Cc)
             self.wgrad_fused(dz, Cc, sv["v"][l], Cc, M, self.g[f"w{l}"])
             _ck(lib.gf_fno_inv_h_bwd(_p(dZ), _p(self.mat["IHT"]), _p(dV), B, H, m2, Q, s), "inv_h_bwd")
             _ck(lib.gf_fno_modes_bwd(_p(dV), _p(sv["spec"][l][0]), _p(self.p[f"R{l}"]), _p(dU), _p(self.g[f"R{l}"]),
@@ -460,7 +464,7 @@ class Fno:
             _ck(lib.gf_fno_row_bwd(_p(dz), _p(dXw), _p(self.mat["FW"]), _p(wb[f"w{l}"]), _p(z), _p(IWT), _p(dn), _p(df),
                                    _p(dZ) if l else None, rows, W, K2, s), "row_bwd")
             dz, dn = dn, dz
-        self.colsum(df, self.g["lift_b"], M, Cc)
+        self.colsum_blocked(df, self.g["lift_b"], M, Cc)
         self.wgrad_fused(dz, Cc, sv["x"].reshape(M, cfg.cin), cfg.cin, M, self.g["lift_w"])
         self.saved = None
         return self.g

@@ -61,6 +61,9 @@ int gf_fno_modes_grad(const float *dRm, float *dR, int modes, int C, void *strea
 /* out[c] (+)= sum_r X[r][c]; dst[i] (+)= sum_b src[b][i]. */
 int gf_fno_colsum(const float *X, float *out, long long rows, int cols, int accum, void *stream);
 int gf_fno_colsum_bf16(const void *X, float *out, long long rows, int cols, int accum, void *stream);
+/* X in blocks of 32 rows x 8 columns, [rows / 32][cols / 8][32][8] (rows >= 4096,
+ * a multiple of 32; cols a multiple of 8 that divides 256): gf_fno_colsum's sums. */
+int gf_fno_colsum_blocked(const float *X, float *out, long long rows, int cols, int accum, void *stream);
 int gf_fno_sum_batches(const float *src, float *dst, int nb, long long n, int accum, void *stream);
 /* Adam (bias-corrected, decoupled from the loss scale), step counts from 1. */
 int gf_fno_adam(float *p, const float *g, float *m, float *v, long long n, float lr, float b1, float b2, float eps,
@@ -116,7 +119,8 @@ int gf_fno_proj(const void *v, const void *P1, const float *b1, const void *P2, 
                 float *out, int rows, int W, void *stream);
 
 /* ---- the backward pass in fused kernels, under the same shapes ----
- * Gradients BF16, and (df1, df) FP32 for the bias gradients (gf_fno_colsum).
+ * Gradients BF16, and (df1, df) FP32 for the bias gradients, in gf_fno_colsum_blocked's
+ * layout.
  * gf_fno_proj_bwd: dzp [rows W][128] = (dout P2) GELU'(zp), dzo [rows W][64] =
  * dzp P1, dZ [rows][K2][64] = IWT dzo.
  * gf_fno_row_bwd: dzo = (dz Wl + FW^T dXw) GELU'(z) (z NULL: no factor), dZ =
