@@ -1142,3 +1142,19 @@ __device__ __forceinline__ int plastic_table_state(const DevParams &P, int iph, 
 
 } // namespace gfk
 } // namespace
+
+// Launch with programmatic stream serialization (the kernel starts with
+// gf_pdl_entry).
+template <class... KArgs, class... Args>
+inline void gf_launch_pdl(void (*kern)(KArgs...), dim3 grid, unsigned threads, cudaStream_t s, Args... args) {
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = grid;
+    lc.blockDim = dim3(threads);
+    lc.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    cudaLaunchKernelEx(&lc, kern, (KArgs)args...);
+}

@@ -1640,21 +1640,6 @@ template <class R> __global__ void k_convert_back(const R *__restrict__ src, dou
 #endif
 
 // ---------------------------------------------------------------- launchers
-// Launch with programmatic stream serialization (the kernel starts with
-// gf_pdl_entry); `n` items, GF_THREADS per CTA.
-template <class... KArgs, class... Args>
-inline void gf_launch_pdl(void (*kern)(KArgs...), dim3 grid, unsigned threads, cudaStream_t s, Args... args) {
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = grid;
-    lc.blockDim = dim3(threads);
-    lc.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    lc.attrs = at;
-    lc.numAttrs = 1;
-    cudaLaunchKernelEx(&lc, kern, (KArgs)args...);
-}
 // Threads per CTA for n items.  FP64 kernels: fewer than `most`, down to 64,
 // while that leaves SMs without a CTA, since warps that share an SM queue for
 // its FP64 pipe (ten steps of 60x20 elements 1.055 -> 1.020 ms, 241x61 1.265

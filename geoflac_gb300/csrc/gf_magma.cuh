@@ -55,6 +55,10 @@ __device__ __forceinline__ void mg_nji(const GfDims &d, long long n, int &j, int
 }
 __device__ __forceinline__ double mg_min(double a, double b) { return b < a ? b : a; }
 __device__ __forceinline__ double mg_max(double a, double b) { return b > a ? b : a; }
+// whether 0.5 / x is an ordinary positive number (x within 2^-900 .. 2^900)
+__device__ __forceinline__ bool mg_ordinary(double x) {
+    return (unsigned)(__double2hiint(x) >> 20) - 123u < 1800u;
+}
 // ceiling() of a ratio that may be huge, held to +-2^29 (beyond every loop
 // bound it feeds)
 __device__ __forceinline__ int mg_ceil(double x) {
@@ -130,12 +134,14 @@ __device__ __forceinline__ bool mg_pred(int mode, const DevArrays &A, const GfDi
     // migration sources: MOR melt with a valid melting zone (MOR), melting
     // below the column's Moho (dikes and the mantle cone: ARC)
     if (mode == MG_PRED_MOR) return A.fmelt2[e] > 0 && A.mg_s[MS_VALID] != 0.0;
+    if (!(A.fmelt[e] > 0)) return false;
     int j, i;
     mg_eji(d, e, j, i);
-    return j + 1 > A.jmoho[i] && A.fmelt[e] > 0;
+    return j + 1 > A.jmoho[i];
 }
 // block b counts its MG_CB elements
 __global__ void __launch_bounds__(MG_CB) k_mg_count(DevArrays A, GfDims d, int mode) {
+    gf_pdl_entry();
     const long long e = (long long)blockIdx.x * MG_CB + threadIdx.x;
     const int v = (e < d.E && mg_pred(mode, A, d, e)) ? 1 : 0;
     const int c = __syncthreads_count(v);
@@ -146,6 +152,7 @@ __global__ void __launch_bounds__(MG_CB) k_mg_count(DevArrays A, GfDims d, int m
 __global__ void __launch_bounds__(MG_CB) k_mg_write(DevArrays A, GfDims d, int mode, int *list, int *count) {
     __shared__ int red[32];
     __shared__ int wsum[32];
+    gf_pdl_entry();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int part = 0;
     for (int b = threadIdx.x; b < (int)blockIdx.x; b += MG_CB) part += A.mg_blk[b];
@@ -175,6 +182,7 @@ __global__ void __launch_bounds__(MG_CB) k_mg_write(DevArrays A, GfDims d, int m
 // melting depth (flux melting starts there; -1: none), or fl_therm's
 // topmost non-sediment row (1-based) for the dikes
 __global__ void k_mg_cols(DevArrays A, GfDims d, int mode) {
+    gf_pdl_entry();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= d.nx - 1) return;
     if (mode == 0) {
@@ -202,6 +210,7 @@ __global__ void k_mg_cols(DevArrays A, GfDims d, int mode) {
 // zero the melt fractions; mark the elements above a solidus at the start
 // (bit 0 mantle, 1 sediments, 2 basalt, 3 flux melting)
 __global__ void __launch_bounds__(GF_THREADS) k_melt_flags(const DevParams *__restrict__ Pp, DevArrays A, GfDims d) {
+    gf_pdl_entry();
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= d.E) return;
     const DevParams &P = *Pp;
@@ -223,6 +232,7 @@ __global__ void __launch_bounds__(GF_THREADS) k_melt_flags(const DevParams *__re
 // the static part of each listed candidate: corner nodes, and per loop the
 // phase sum and the solidus (depth and phases do not change while melting)
 __global__ void __launch_bounds__(GF_THREADS) k_melt_prep(const DevParams *__restrict__ Pp, DevArrays A, GfDims d) {
+    gf_pdl_entry();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= A.mg_i[MI_COUNT]) return;
     const DevParams &P = *Pp;
@@ -252,6 +262,7 @@ __global__ void __launch_bounds__(GF_THREADS) k_melt_prep(const DevParams *__res
 // then column by column, each column's run reversed (upwards).  Slot
 // loop * E of mg_order, the flux order at 4 E; counts in mg_i[MI_P0 + loop].
 __global__ void __launch_bounds__(MG_CB) k_melt_order(DevArrays A, GfDims d) {
+    gf_pdl_entry();
     __shared__ int wsum[32];
     __shared__ int carry;
     const int n = A.mg_i[MI_COUNT];
@@ -399,6 +410,7 @@ __device__ __forceinline__ void melt_one(const DevParams &P, double *__restrict_
 // list, one thread walks the list instead.
 constexpr int MG_LEVELS = 4096;
 __global__ void __launch_bounds__(MG_CB) k_melt_serial(const DevParams *__restrict__ Pp, DevArrays A, GfDims d) {
+    gf_pdl_entry();
     __shared__ int start[MG_LEVELS + 1];
     __shared__ int fill[MG_LEVELS];
     __shared__ int psum[MG_CB];
@@ -467,6 +479,7 @@ __global__ void __launch_bounds__(MG_CB) k_melt_serial(const DevParams *__restri
 // element's four corners kept for the node pass
 __global__ void __launch_bounds__(GF_THREADS) k_mg_freeze(const DevParams *__restrict__ Pp, DevClock *C, DevArrays A,
                                                           GfDims d) {
+    gf_pdl_entry();
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= d.E) return;
     const DevParams &P = *Pp;
@@ -477,8 +490,14 @@ __global__ void __launch_bounds__(GF_THREADS) k_mg_freeze(const DevParams *__res
     const double cp_eff = P.cp[A.iphase[e] - 1];
     const double tmpr = 0.25 * (T0[gf_node(d, j, i)] + T0[gf_node(d, j + 1, i)] + T0[gf_node(d, j, i + 1)] +
                                 T0[gf_node(d, j + 1, i + 1)]);
-    const double fr_lambda = P.lambda_freeze * gfm::exp(-P.lambda_freeze_tdep * (tmpr - P.t_top));
     const double f1 = A.fmagma[e], f2 = A.fmagma2[e];
+    const double ex = -P.lambda_freeze_tdep * (tmpr - P.t_top);
+    if (__double_as_longlong(f1) == 0 && __double_as_longlong(f2) == 0 && fabs(ex) < 700.0 && fabs(P.lambda_freeze) < 1e300 &&
+        P.latent_heat_magma >= 0.0 && P.latent_heat_magma < 1e300 && cp_eff > 1e-300) {
+        A.mg_e[e] = 0.0; // no magma: nothing freezes, no exponential and no quotients
+        return;
+    }
+    const double fr_lambda = P.lambda_freeze * gfm::exp(ex);
     const double d1 = mg_min(f1, f1 * dt * fr_lambda), d2 = mg_min(f2, f2 * dt * fr_lambda);
     A.fmagma[e] = f1 - d1;
     A.fmagma2[e] = f2 - d2;
@@ -488,6 +507,7 @@ __global__ void __launch_bounds__(GF_THREADS) k_mg_freeze(const DevParams *__res
 // temp = min(temp, t_bot)
 __global__ void __launch_bounds__(GF_THREADS) k_mg_freeze_nodes(const DevParams *__restrict__ Pp, DevArrays A,
                                                                 GfDims d) {
+    gf_pdl_entry();
     const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= d.N) return;
     int J, I;
@@ -514,6 +534,7 @@ __device__ __forceinline__ double mg_cz(const double *c, const GfDims &d, int j,
 // parallel into shared memory, sums by one thread in serial order); also
 // the mantle cone's tan and width
 __global__ void __launch_bounds__(MG_CB) k_mg_zone1(const DevParams *__restrict__ Pp, DevArrays A, GfDims d) {
+    gf_pdl_entry();
     __shared__ double sx[MG_CB], sz[MG_CB], sw[MG_CB];
     const DevParams &P = *Pp;
     const int n = A.mg_i[MI_COUNT];
@@ -561,6 +582,7 @@ __global__ void __launch_bounds__(MG_CB) k_mg_zone1(const DevParams *__restrict_
 }
 // the first element (serial order) holding the centre
 __global__ void __launch_bounds__(GF_THREADS) k_mg_find(DevArrays A, GfDims d) {
+    gf_pdl_entry();
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= d.E || !(A.mg_s[MS_WSUM] > 0.0)) return;
     int j, i;
@@ -572,6 +594,7 @@ __global__ void __launch_bounds__(GF_THREADS) k_mg_find(DevArrays A, GfDims d) {
 }
 // widths on either side of the centre and the zone's cone (one CTA as above)
 __global__ void __launch_bounds__(MG_CB) k_mg_zone2(const DevParams *__restrict__ Pp, DevArrays A, GfDims d) {
+    gf_pdl_entry();
     __shared__ double sx[MG_CB], sw[MG_CB], sl[MG_CB], sr[MG_CB];
     const int found = A.mg_i[MI_FOUND];
     if (found == 0x7fffffff) return;
@@ -642,6 +665,7 @@ __global__ void __launch_bounds__(MG_CB) k_mg_zone2(const DevParams *__restrict_
 // the terms each listed migration source adds
 __global__ void __launch_bounds__(GF_THREADS) k_mg_src(const DevParams *__restrict__ Pp, DevClock *C, DevArrays A,
                                                        GfDims d, const int *list, const int *count, double *out) {
+    gf_pdl_entry();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= *count) return;
     const DevParams &P = *Pp;
@@ -712,6 +736,7 @@ __device__ __forceinline__ int mg_lower(const int *list, int n, long long e) {
 // whose FP64 pipes run side by side) carry fmagma, fmagma2, dike_added and
 // the MOR marker volume.
 __global__ void __launch_bounds__(GF_THREADS) k_mg_migrate(const DevParams *__restrict__ Pp, DevArrays A, GfDims d) {
+    gf_pdl_entry();
     const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int part = (int)((gid >> 5) & 3);
     const long long t = ((gid >> 7) << 5) + (gid & 31);
@@ -821,16 +846,25 @@ __global__ void __launch_bounds__(GF_THREADS) k_mg_migrate(const DevParams *__re
 
 // rate-capped dike release; mark the elements that receive new markers
 __global__ void __launch_bounds__(GF_THREADS) k_mg_release(const DevParams *__restrict__ Pp, DevArrays A, GfDims d) {
+    gf_pdl_entry();
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= d.E) return;
     const DevParams &P = *Pp;
     const double *area = (const double *)A.area;
-    const double elem_area = 0.5 / area[gf_ek(d, e, 0)] + 0.5 / area[gf_ek(d, e, 1)];
-    const double pending = A.dike_added[e] * elem_area + A.dike_backlog[e];
+    const double a0 = area[gf_ek(d, e, 0)], a1 = area[gf_ek(d, e, 1)];
+    const double added = A.dike_added[e], backlog = A.dike_backlog[e], volume = A.dike_marker_vol[e];
+    if ((__double_as_longlong(added) | __double_as_longlong(backlog) | __double_as_longlong(volume) |
+         __double_as_longlong(A.mor_marker_vol[e])) == 0 && mg_ordinary(a0) && mg_ordinary(a1) && P.Amin > 0.0) {
+        A.dike_released[e] = 0.0; // nothing pending, no volume: no quotients
+        A.mg_mask[e] = 0;
+        return;
+    }
+    const double elem_area = 0.5 / a0 + 0.5 / a1;
+    const double pending = added * elem_area + backlog;
     const double released = mg_min(pending, 1.0e-4 * P.Amin);
     A.dike_backlog[e] = pending - released;
     A.dike_released[e] = released / elem_area;
-    const double dmv = A.dike_marker_vol[e] + released;
+    const double dmv = volume + released;
     A.dike_marker_vol[e] = dmv;
     const int kinc = A.nmark_elem[e];
     bool add = false;
@@ -845,6 +879,7 @@ __global__ void __launch_bounds__(GF_THREADS) k_mg_release(const DevParams *__re
 // new arc (karc1) and oceanic-crust (kocean1) markers at the centres of the
 // listed elements, numbered in serial order
 __global__ void k_mg_markers(const DevParams *__restrict__ Pp, DevClock *C, DevArrays A, GfDims d, int max_markers) {
+    gf_pdl_entry();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const DevParams &P = *Pp;
     const int n = A.mg_i[MI_COUNT];
@@ -878,26 +913,35 @@ __global__ void k_mg_markers(const DevParams *__restrict__ Pp, DevClock *C, DevA
 
 // ---------------------------------------------------------------- diff_topo's magma blocks
 // the area-weighted column sum of f (rows in order): one warp, each lane
-// one row of every 32, every lane adding the same terms in row order
+// one row of every 32, every lane adding the same terms in row order.  A zero
+// field on an ordinary area adds nothing: such rows, most of them, skip the
+// divisions and the chain of additions on the FP64 pipe (the sums of 300
+// columns of 75 rows 16.5 -> 6.5 us).
 __device__ __forceinline__ double mg_col_sum(const DevArrays &A, const GfDims &d, int i, const double *f, int lane) {
     const double *area = (const double *)A.area;
     double tot = 0;
     for (int j0 = 0; j0 < d.nz - 1; j0 += 32) {
         const int j = j0 + lane;
         double term = 0;
+        bool adds = false;
         if (j < d.nz - 1) {
             const long long e = gf_elem(d, j, i);
-            const double quad_area = 0.5 / area[gf_ek(d, e, 0)] + 0.5 / area[gf_ek(d, e, 1)];
-            term = quad_area * f[e];
+            const double a0 = area[gf_ek(d, e, 0)], a1 = area[gf_ek(d, e, 1)], fe = f[e];
+            if ((__double_as_longlong(fe) << 1) != 0 || !mg_ordinary(a0) || !mg_ordinary(a1)) {
+                const double quad_area = 0.5 / a0 + 0.5 / a1;
+                term = quad_area * fe;
+                adds = true;
+            }
         }
-        const int m = d.nz - 1 - j0 < 32 ? d.nz - 1 - j0 : 32;
-        for (int k = 0; k < m; ++k) tot = tot + __shfl_sync(0xffffffffu, term, k);
+        for (unsigned bal = __ballot_sync(0xffffffffu, adds); bal; bal &= bal - 1)
+            tot = tot + __shfl_sync(0xffffffffu, term, __ffs(bal) - 1);
     }
     return tot;
 }
 // arc extrusion of each inner column (fl_move.f90:213-237), one warp per column
 __global__ void __launch_bounds__(GF_THREADS) k_arc_cols(const DevParams *__restrict__ Pp, DevClock *C, DevArrays A,
                                                          GfDims d, double rate) {
+    gf_pdl_entry();
     const int i = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) + 1, lane = threadIdx.x & 31;
     if (i >= d.nx - 2) return;
     const DevParams &P = *Pp;
@@ -914,6 +958,7 @@ __global__ void __launch_bounds__(GF_THREADS) k_arc_cols(const DevParams *__rest
 // each surface node takes the extrusion of the column on its left, then of
 // the one on its right (serial column order)
 __global__ void k_arc_nodes(DevArrays A, GfDims d) {
+    gf_pdl_entry();
     const int I = blockIdx.x * blockDim.x + threadIdx.x;
     if (I >= d.nx) return;
     const long long nz_ = d.N + gf_node(d, 0, I);
@@ -934,6 +979,7 @@ __global__ void k_arc_nodes(DevArrays A, GfDims d) {
 // one warp per column
 __global__ void __launch_bounds__(GF_THREADS) k_mor_cols(const DevParams *__restrict__ Pp, DevClock *C, DevArrays A,
                                                          GfDims d) {
+    gf_pdl_entry();
     const int i = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) + 1, lane = threadIdx.x & 31;
     if (i >= d.nx - 2) return;
     const DevParams &P = *Pp;
@@ -960,39 +1006,65 @@ __device__ void mg_newphase(DevArrays &A, const GfDims &d, int j1, int j2, int i
             if (off < total) A.phase_ratio[off] = 1.0;
         }
 }
-// the columns with MOR magma in serial order: one warp loads 32 columns'
-// erupted heights and surface / second-row heights, its first lane walks the
-// active ones, converting rows to oceanic crust (newphase2marker) when the
-// erupted height reaches an element's, and adding the remainder to the
-// column's two surface nodes; the left node of the next column is the one
-// this column just raised
-__global__ void k_mor_chain(DevArrays A, GfDims d) {
-    __shared__ double s_eh[32], s_z0[32], s_z0n[32], s_z1[32], s_z1n[32], s_ea[32];
-    if (blockIdx.x != 0 || threadIdx.x >= 32) return;
-    const int lane = threadIdx.x, nx = d.nx, nz = d.nz;
+// the columns with MOR magma in serial order: when the erupted height reaches
+// an element's, rows become oceanic crust (newphase2marker), and the remainder
+// is added to the column's two surface nodes; the left node of the next column
+// is the one this column just raised.
+// A column whose erupted height lies below its element's keeps all of it as
+// the remainder, whatever the columns before it raised (the quotient is below
+// 1), so 256 columns are done at once under that assumption, checked for each
+// with the heights it implies; only if one fails does a thread walk the 256 in
+// order.  (One thread's divisions and fmod on the FP64 pipe, column after
+// column: 300 columns 49 us, now 6.)
+constexpr int MC_T = 256;
+__global__ void __launch_bounds__(MC_T) k_mor_chain(DevArrays A, GfDims d) {
+    __shared__ double s_eh[MC_T], s_z0[MC_T], s_z0n[MC_T], s_z1[MC_T], s_z1n[MC_T], s_ea[MC_T];
+    __shared__ int s_last;       // the last column processed, if it lies before this chunk
+    __shared__ double s_last_z;  // its right surface node's new height
+    gf_pdl_entry();
+    const int t = threadIdx.x, nx = d.nx, nz = d.nz;
     double *c = A.cord;
     const long long N = d.N;
-    int last = -1;       // the last column processed
-    double last_z = 0.0; // its right surface node's new height
-    for (int base = 1; base < nx - 2; base += 32) {
-        const int ii = base + lane;
+    if (t == 0) s_last = -1;
+    for (int base = 1; base < nx - 2; base += MC_T) {
+        const int ii = base + t;
         const bool in = ii < nx - 2;
-        const double eh = in ? A.mg_c[ii] : 0.0;
+        s_eh[t] = in ? A.mg_c[ii] : 0.0;
         if (in) {
-            s_eh[lane] = eh;
-            s_z0[lane] = CY(c, d, 0, ii);
-            s_z0n[lane] = CY(c, d, 0, ii + 1);
-            s_z1[lane] = CY(c, d, 1, ii);
-            s_z1n[lane] = CY(c, d, 1, ii + 1);
-            s_ea[lane] = A.extr_acc[ii];
+            s_z0[t] = CY(c, d, 0, ii);
+            s_z0n[t] = CY(c, d, 0, ii + 1);
+            s_z1[t] = CY(c, d, 1, ii);
+            s_z1n[t] = CY(c, d, 1, ii + 1);
+            s_ea[t] = A.extr_acc[ii];
         }
-        unsigned bal = __ballot_sync(0xffffffffu, in && eh != 0.0);
-        __syncwarp();
-        if (lane == 0)
-            while (bal) {
-                const int l = __ffs(bal) - 1, i = base + l;
-                bal &= bal - 1;
+        __syncthreads();
+        const double h = s_eh[t];
+        const bool act = h != 0.0;
+        double z0 = 0.0;
+        bool fast = true;
+        if (act) {
+            if (t == 0) z0 = s_last == ii - 1 ? s_last_z : s_z0[0];
+            else z0 = s_eh[t - 1] != 0.0 ? s_z0n[t - 1] + s_eh[t - 1] / 2 : s_z0[t];
+            const double ele_height = fabs(0.5 * (s_z1n[t] + s_z1[t]) - 0.5 * (s_z0n[t] + z0));
+            fast = h >= 0.0 && h < ele_height;
+        }
+        if (__syncthreads_and(fast)) {
+            if (act) {
+                A.extr_acc[ii] = s_ea[t] + h / 2;
+                c[N + gf_node(d, 0, ii)] = z0 + h / 2;
+                if (t == MC_T - 1 || s_eh[t + 1] == 0.0) c[N + gf_node(d, 0, ii + 1)] = s_z0n[t] + h / 2;
+            }
+            if (t == MC_T - 1) {
+                s_last = act ? ii : -1;
+                s_last_z = s_z0n[t] + h / 2;
+            }
+        } else if (t == 0) {
+            int last = s_last;
+            double last_z = s_last_z;
+            for (int l = 0; l < MC_T; ++l) {
                 const double h = s_eh[l];
+                if (h == 0.0) continue;
+                const int i = base + l;
                 const double z0 = (last == i - 1) ? last_z : s_z0[l], z0n = s_z0n[l];
                 double ele_height = fabs(0.5 * (s_z1n[l] + s_z1[l]) - 0.5 * (z0n + z0));
                 double quotient = h / ele_height, remainder = fmod(h, ele_height);
@@ -1022,6 +1094,9 @@ __global__ void k_mor_chain(DevArrays A, GfDims d) {
                 c[N + gf_node(d, 0, i + 1)] = last_z;
                 last = i;
             }
-        __syncwarp();
+            s_last = last;
+            s_last_z = last_z;
+        }
+        __syncthreads();
     }
 }

@@ -12,6 +12,7 @@ namespace {
 namespace gfr {
 
 using gfk::gf_ddiv_by;
+using gfk::gf_pdl_entry;
 using gfk::gf_int_recip;
 using gfk::gf_mul;
 using gfk::GfIntRecip;
@@ -668,6 +669,7 @@ __global__ void k_jmoho(DevArrays A, GfDims d) {
 // hi/lo split in the mixed path).  The magma blocks add zero without melt.
 __global__ void __launch_bounds__(1024) k_diff_topo(const DevParams *__restrict__ Pp, DevClock *C, DevArrays A,
                                                     GfDims d) {
+    gf_pdl_entry();
     const DevParams &P = *Pp;
     const int nx = d.nx;
     const double dt = C->dt;
@@ -1109,6 +1111,16 @@ __global__ void __launch_bounds__(1024) k_surface_acc_remesh(DevArrays A, GfDims
         }                                                                                                              \
     } while (0)
 
+// The kernels of the magma sub-model and diff_topo start with gf_pdl_entry:
+// they run some twenty short launches a step, one after another.
+#define GF_MLAUNCH(kern, grid, threads, ...)                                                                           \
+    do {                                                                                                               \
+        if ((grid) > 0) {                                                                                              \
+            gf_launch_pdl(kern, dim3((unsigned)(grid)), threads, g.s, __VA_ARGS__);                                    \
+            ++*g.launches;                                                                                             \
+        }                                                                                                              \
+    } while (0)
+
 namespace {
 // e_offset = exclusive scan of e_count (m_slot, which the scan's readers
 // fill or no longer need, holds the CTAs' sums)
@@ -1214,17 +1226,15 @@ template <class R> void GfRemesh<R>::flexure(const GfLaunch &g, double Te, doubl
 
 template <class R> void GfRemesh<R>::diff_topo(const GfLaunch &g, int resurface, int nloop, int max_markers) {
     using namespace gfr;
-    k_diff_topo<<<1, 1024, 0, g.s>>>(g.P, g.C, g.A, g.d);
-    ++*g.launches;
+    GF_MLAUNCH(k_diff_topo, 1, 1024, g.P, g.C, g.A, g.d);
     if (g.A.dike_backlog && g.d.nx > 3) { // magma sub-model: arc extrusion and MOR crust
-        const long long ncol = g.d.nx - 3;
+        const int cols = (g.d.nx - 3 + 1) / 2; // one warp per column, two to a CTA (each with an FP64 pipe of its own)
         if (g.arc_rate > 0) {
-            GF_RLAUNCH(k_arc_cols, 32 * ncol, g.P, g.C, g.A, g.d, g.arc_rate); // one warp per column
-            GF_RLAUNCH(k_arc_nodes, (long long)g.d.nx, g.A, g.d);
+            GF_MLAUNCH(k_arc_cols, cols, 64, g.P, g.C, g.A, g.d, g.arc_rate);
+            GF_MLAUNCH(k_arc_nodes, blocks_for(g.d.nx), GF_THREADS, g.A, g.d);
         }
-        GF_RLAUNCH(k_mor_cols, 32 * ncol, g.P, g.C, g.A, g.d);
-        k_mor_chain<<<1, 32, 0, g.s>>>(g.A, g.d);
-        ++*g.launches;
+        GF_MLAUNCH(k_mor_cols, cols, 64, g.P, g.C, g.A, g.d);
+        GF_MLAUNCH(k_mor_chain, 1, MC_T, g.A, g.d);
     }
     if (resurface) {
         GF_RLAUNCH(k_resurface_erode, (long long)(g.d.nx - 1), g.P, g.C, g.A, g.d);
@@ -1240,45 +1250,44 @@ template struct GfRemesh<float>;
 namespace {
 // the elements of `mode` in serial order into list, their number into *count
 void mg_compact(const GfLaunch &g, int mode, int *list, int *count) {
-    const unsigned nb = (unsigned)((g.d.E + gfr::MG_CB - 1) / gfr::MG_CB);
-    gfr::k_mg_count<<<nb, gfr::MG_CB, 0, g.s>>>(g.A, g.d, mode);
-    gfr::k_mg_write<<<nb, gfr::MG_CB, 0, g.s>>>(g.A, g.d, mode, list, count);
-    *g.launches += 2;
+    using namespace gfr;
+    const unsigned nb = (unsigned)((g.d.E + MG_CB - 1) / MG_CB);
+    GF_MLAUNCH(k_mg_count, nb, MG_CB, g.A, g.d, mode);
+    GF_MLAUNCH(k_mg_write, nb, MG_CB, g.A, g.d, mode, list, count);
 }
 } // namespace
 
 void GfMagma::melting(const GfLaunch &g) {
     using namespace gfr;
     const DevArrays &A = g.A;
-    GF_RLAUNCH(k_mg_cols, (long long)(g.d.nx - 1), A, g.d, 0);
-    GF_RLAUNCH(k_melt_flags, g.d.E, g.P, A, g.d);
+    const unsigned be = blocks_for(g.d.E);
+    GF_MLAUNCH(k_mg_cols, blocks_for(g.d.nx - 1), GF_THREADS, A, g.d, 0);
+    GF_MLAUNCH(k_melt_flags, be, GF_THREADS, g.P, A, g.d);
     mg_compact(g, MG_PRED_MASK, A.mg_list, A.mg_i + MI_COUNT);
-    GF_RLAUNCH(k_melt_prep, g.d.E, g.P, A, g.d);
-    k_melt_order<<<1, MG_CB, 0, g.s>>>(A, g.d);
-    k_melt_serial<<<1, MG_CB, 0, g.s>>>(g.P, A, g.d);
-    *g.launches += 2;
+    GF_MLAUNCH(k_melt_prep, be, GF_THREADS, g.P, A, g.d);
+    GF_MLAUNCH(k_melt_order, 1, MG_CB, A, g.d);
+    GF_MLAUNCH(k_melt_serial, 1, MG_CB, g.P, A, g.d);
 }
 
 void GfMagma::therm(const GfLaunch &g, int max_markers) {
     using namespace gfr;
     const GfDims &d = g.d;
     const DevArrays &A = g.A;
-    GF_RLAUNCH(k_mg_freeze, d.E, g.P, g.C, A, d);
-    GF_RLAUNCH(k_mg_freeze_nodes, d.N, g.P, A, d);
+    const unsigned be = blocks_for(d.E);
+    GF_MLAUNCH(k_mg_freeze, be, GF_THREADS, g.P, g.C, A, d);
+    GF_MLAUNCH(k_mg_freeze_nodes, blocks_for(d.N), GF_THREADS, g.P, A, d);
     mg_compact(g, MG_PRED_W, A.mg_list, A.mg_i + MI_COUNT);
-    k_mg_zone1<<<1, MG_CB, 0, g.s>>>(g.P, A, d);
-    GF_RLAUNCH(k_mg_find, d.E, A, d);
-    k_mg_zone2<<<1, MG_CB, 0, g.s>>>(g.P, A, d);
-    *g.launches += 2;
-    GF_RLAUNCH(k_mg_cols, (long long)(d.nx - 1), A, d, 1);
+    GF_MLAUNCH(k_mg_zone1, 1, MG_CB, g.P, A, d);
+    GF_MLAUNCH(k_mg_find, be, GF_THREADS, A, d);
+    GF_MLAUNCH(k_mg_zone2, 1, MG_CB, g.P, A, d);
+    GF_MLAUNCH(k_mg_cols, blocks_for(d.nx - 1), GF_THREADS, A, d, 1);
     // the MOR sources and the dike / mantle-cone sources, each in serial order
     mg_compact(g, MG_PRED_MOR, A.mg_list, A.mg_i + MI_COUNT);
-    GF_RLAUNCH(k_mg_src, d.E, g.P, g.C, A, d, (const int *)A.mg_list, (const int *)(A.mg_i + MI_COUNT), A.mg_src);
+    GF_MLAUNCH(k_mg_src, be, GF_THREADS, g.P, g.C, A, d, (const int *)A.mg_list, (const int *)(A.mg_i + MI_COUNT), A.mg_src);
     mg_compact(g, MG_PRED_ARC, A.mg_list2, A.mg_i + MI_COUNT2);
-    GF_RLAUNCH(k_mg_src, d.E, g.P, g.C, A, d, (const int *)A.mg_list2, (const int *)(A.mg_i + MI_COUNT2), A.mg_src2);
-    GF_RLAUNCH(k_mg_migrate, 4 * ((d.E + 31) / 32) * 32, g.P, A, d); // four threads per element
-    GF_RLAUNCH(k_mg_release, d.E, g.P, A, d);
+    GF_MLAUNCH(k_mg_src, be, GF_THREADS, g.P, g.C, A, d, (const int *)A.mg_list2, (const int *)(A.mg_i + MI_COUNT2), A.mg_src2);
+    GF_MLAUNCH(k_mg_migrate, blocks_for(4 * ((d.E + 31) / 32) * 32), GF_THREADS, g.P, A, d); // four threads per element
+    GF_MLAUNCH(k_mg_release, be, GF_THREADS, g.P, A, d);
     mg_compact(g, MG_PRED_MASK, A.mg_list, A.mg_i + MI_COUNT);
-    k_mg_markers<<<1, 1, 0, g.s>>>(g.P, g.C, A, d, max_markers);
-    ++*g.launches;
+    GF_MLAUNCH(k_mg_markers, 1, 1, g.P, g.C, A, d, max_markers);
 }
