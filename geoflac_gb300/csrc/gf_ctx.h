@@ -91,7 +91,7 @@ struct DevArrays {
     int *mark_ntriag, *mark_id_elem, *nmark_elem;
     // scratch
     double *t_delta0, *t_delta1; // thermal sweep iterates (node)
-    double *t_coef;              // thermal per-element coefficients (18 per element)
+    double *t_coef;              // thermal coefficients (FP64: 18 per element; mixed: 7 floats per node)
     uint8_t *t_chg;              // FP64 thermal sweeps: one bit per node, changed in sweep k (by parity)
     double *t_pred;              // FP64 thermal sweeps: each node's last increment (the next start)
     double *p_ref; // mixed: per-element reference pressure; stored normal stresses are total + p_ref

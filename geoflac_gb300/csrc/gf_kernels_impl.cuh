@@ -733,7 +733,6 @@ template <class R> __global__ void __launch_bounds__(GF_THREADS, 3) k_move_elem(
 // ======================================================================
 // fl_therm (fl_therm.f90:393-598): the FP64 path in gf_therm64.cuh, the mixed
 // path's two sweeps below.
-#define GF_TC 18 // coefficients per element: KA[6], KB[6], raA, raB, preA, preB, srA, srB
 // K index of (a,b), a,b in 0..2 (symmetric)
 __device__ __forceinline__ int kidx(int a, int b) {
     int lo = a < b ? a : b, hi = a < b ? b : a;
@@ -767,38 +766,86 @@ __device__ __forceinline__ double therm_bc_value(const DevParams &P, const DevAr
 // accuracy that a sum of ~1000 C values would lose.  Sweep 0 is the all-old
 // (Jacobi) update, sweep 1 reuses the upstream increments of sweep 0, which
 // leaves an error of order (kappa dt/h^2)^2 relative to the increment.
-__device__ __forceinline__ void b_k_therm_prep32(const DevParams *__restrict__ Pp, DevArrays A, GfDims d, float *__restrict__ tc, GF_IDX e) {
-    if (e >= d.E) return;
+//
+// The coefficients are kept per node: the weights of its six neighbours
+// (sums over the node's six triangles) and the heat term, each over the node's
+// area sum.  A sweep then reads 7 values a node instead of some 30 of four
+// elements' 18; the prep, which does each triangle's products for its three
+// nodes, runs beside fl_rheol or at full occupancy.  A step of 60x20 elements
+// 29.4 -> 27.6 us, of 64 ensemble members 511 -> 468 us; 1000x300 elements
+// unchanged (what the sweeps save the prep takes); the increments' error
+// against FP64 is no larger (3.1e-7 to 6.5e-7 of them).
+#define GF_TN 7
+// offsets of the neighbours (j-1,i), (j,i-1), (j+1,i-1), (j-1,i+1), (j,i+1), (j+1,i): upstream ones first
+__device__ __forceinline__ void therm_neighbours(const GfDims &d, int j, int i, GF_IDX n, GF_IDX m[6]) {
+    const bool up = j != 0, dn = j != d.nz - 1, lf = i != 0, rt = i != d.nx - 1;
+    m[0] = up ? n - 1 : n;
+    m[1] = lf ? n - d.nz : n;
+    m[2] = lf && dn ? n - d.nz + 1 : n;
+    m[3] = up && rt ? n + d.nz - 1 : n;
+    m[4] = rt ? n + d.nz : n;
+    m[5] = dn ? n + 1 : n;
+}
+__device__ __forceinline__ void b_k_therm_prep32(const DevParams *__restrict__ Pp, DevArrays A, GfDims d, float *__restrict__ tc, GF_IDX n) {
+    if (n >= d.N) return;
     const DevParams &P = *Pp;
     int j, i;
-    elem_ji(d, e, j, i);
-    int iph = A.iphase[e] - 1;
-    float cp_eff = P.f_cp[iph], cond_eff = P.f_cond[iph], den = P.f_den[iph];
-    float dissip = (P.ishearh == 1 && P.itherm != 2) ? ((const float *)A.shrheat)[e] : 0.0f;
-    float diff = cond_eff / den / cp_eff;
-    float src = (gf_d2f(A.source[e]) + dissip / den) / cp_eff;
-    QuadF q;
-    load_quad_rel(A, d, j, i, q);
-    const float *area = (const float *)A.area;
-    const GF_IDX E = d.E;
-    const int tv[2][3] = {{0, 1, 2}, {2, 1, 3}};
-    const float at[2] = {area[gf_ek(d, e, 0)], area[gf_ek(d, e, 1)]}; // (before the first store)
+    node_ji(d, n, j, i);
+    GF_IDX m[6];
+    therm_neighbours(d, j, i, n, m);
+    const float *xh = A.cord_hi, *xl = A.cord_lo, *yh = A.cord_hi + d.N, *yl = A.cord_lo + d.N;
+    float x[6], y[6], w[6] = {0, 0, 0, 0, 0, 0};
 #pragma unroll
-    for (int t = 0; t < 2; ++t) {
-        const float a = at[t];
-        const int v1 = tv[t][0], v2 = tv[t][1], v3 = tv[t][2];
-        float dd[3] = {(q.y[v2] - q.y[v3]) * a, (q.y[v3] - q.y[v1]) * a, (q.y[v1] - q.y[v2]) * a};
-        float zz[3] = {(q.x[v3] - q.x[v2]) * a, (q.x[v1] - q.x[v3]) * a, (q.x[v2] - q.x[v1]) * a};
-#pragma unroll
-        for (int m = 0; m < 3; ++m)
-#pragma unroll
-            for (int n = m; n < 3; ++n) tc[(t * 6 + kidx(m, n)) * E + e] = dd[m] * dd[n] + zz[m] * zz[n];
-        float inv_area = 1.0f / a;
-        float ra = inv_area / 6.0f;
-        tc[(12 + t) * E + e] = ra;
-        tc[(14 + t) * E + e] = 0.5f * diff * inv_area;
-        tc[(16 + t) * E + e] = src * ra;
+    for (int q = 0; q < 6; ++q) {
+        x[q] = hl_diff(xh, xl, m[q], n);
+        y[q] = hl_diff(yh, yl, m[q], n);
     }
+    const float *area = (const float *)A.area, *shrheat = (const float *)A.shrheat;
+    float s = 0.0f, area_n = 0.0f;
+    // the triangle (self, p, q) of neighbours p and q in the element's
+    // orientation, area factor a, from the element's diffusivity and source
+    auto tri = [&](float a, float diff, float src, int p, int q) {
+        const float ds = (y[p] - y[q]) * a, dp = y[q] * a, dq = -y[p] * a;
+        const float zs = (x[q] - x[p]) * a, zp = -x[q] * a, zq = x[p] * a;
+        const float inv_area = 1.0f / a, ra = inv_area / 6.0f, pre = 0.5f * diff * inv_area;
+        area_n += ra;
+        s += src * ra;
+        w[p] -= pre * (dp * ds + zp * zs);
+        w[q] -= pre * (dq * ds + zq * zs);
+    };
+    auto elem = [&](int je, int ie, float &diff, float &src) {
+        const GF_IDX e = gf_elem(d, je, ie);
+        const int iph = A.iphase[e] - 1;
+        const float cp = P.f_cp[iph], den = P.f_den[iph];
+        const float dissip = (P.ishearh == 1 && P.itherm != 2) ? shrheat[e] : 0.0f;
+        diff = P.f_cond[iph] / den / cp;
+        src = (gf_d2f(A.source[e]) + dissip / den) / cp;
+        return e;
+    };
+    // triangles A = (1,2,3) and B = (3,2,4) of the quad's nodes (j,i), (j+1,i), (j,i+1), (j+1,i+1)
+    float diff, src;
+    if (j != 0 && i != 0) { // self is node 4: B, (self, 3, 2)
+        const GF_IDX e = elem(j - 1, i - 1, diff, src);
+        tri(area[gf_ek(d, e, 1)], diff, src, 0, 1);
+    }
+    if (j != 0 && i != d.nx - 1) { // self is node 2: A, (self, 3, 1), and B, (self, 4, 3)
+        const GF_IDX e = elem(j - 1, i, diff, src);
+        tri(area[gf_ek(d, e, 0)], diff, src, 3, 0);
+        tri(area[gf_ek(d, e, 1)], diff, src, 4, 3);
+    }
+    if (j != d.nz - 1 && i != 0) { // self is node 3: A, (self, 1, 2), and B, (self, 2, 4)
+        const GF_IDX e = elem(j, i - 1, diff, src);
+        tri(area[gf_ek(d, e, 0)], diff, src, 1, 2);
+        tri(area[gf_ek(d, e, 1)], diff, src, 2, 5);
+    }
+    if (j != d.nz - 1 && i != d.nx - 1) { // self is node 1: A, (self, 2, 3)
+        const GF_IDX e = elem(j, i, diff, src);
+        tri(area[gf_ek(d, e, 0)], diff, src, 5, 4);
+    }
+    const float r = 1.0f / area_n;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) tc[q * d.N + n] = w[q] * r;
+    tc[6 * d.N + n] = s * r;
 }
 __global__ void __launch_bounds__(GF_THREADS) k_therm_prep32(const DevParams *__restrict__ Pp, DevArrays A, GfDims d, float *__restrict__ tc) {
     gf_pdl_entry();
@@ -812,40 +859,19 @@ __device__ __forceinline__ void b_k_therm_sweep32(const DevParams *__restrict__ 
     if (n >= d.N) return;
     int j, i;
     node_ji(d, n, j, i);
-    const int nx = d.nx, nz = d.nz;
-    const GF_IDX E = d.E;
+    GF_IDX m[6];
+    therm_neighbours(d, j, i, n, m);
     const float *th = A.temp_hi, *tl = A.temp_lo;
-    float rhs = 0.0f, area_n = 0.0f;
-    auto Nd = [&](int jj, int ii) { return gf_node(d, jj, ii); };
-    // temperature difference to the updated node; upstream nodes carry the
-    // increment of sweep 0 in the final sweep
-    auto dT = [&](GF_IDX m, bool up) {
-        float v = hl_diff(th, tl, m, n);
-        if (up && final_sweep) v += d0[m];
-        return v;
-    };
-    auto tri = [&](GF_IDX e, int t, int vs, int v0, float D0, int v1, float D1, int v2, float D2) {
-        float ra = tc[(12 + t) * E + e];
-        area_n += ra;
-        const float *K = tc + (GF_IDX)t * 6 * E + e;
-        rhs += tc[(16 + t) * E + e] - tc[(14 + t) * E + e] * (D0 * K[kidx(v0, vs) * E] + D1 * K[kidx(v1, vs) * E] +
-                                                           D2 * K[kidx(v2, vs) * E]);
-    };
-    if (j != 0 && i != 0)
-        tri(gf_elem(d, j - 1, i - 1), 1, 2, 0, dT(Nd(j - 1, i), true), 1, dT(Nd(j, i - 1), true), 2, 0.0f);
-    if (j != 0 && i != nx - 1) {
-        GF_IDX e = gf_elem(d, j - 1, i);
-        tri(e, 0, 1, 0, dT(Nd(j - 1, i), true), 1, 0.0f, 2, dT(Nd(j - 1, i + 1), false));
-        tri(e, 1, 1, 0, dT(Nd(j - 1, i + 1), false), 1, 0.0f, 2, dT(Nd(j, i + 1), false));
+    float w[6], t[6], inc = tc[6 * d.N + n];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+        w[q] = tc[q * d.N + n];
+        t[q] = hl_diff(th, tl, m[q], n);
+        if (q < 3 && final_sweep) t[q] += d0[m[q]]; // upstream nodes carry sweep 0's increment
     }
-    if (j != nz - 1 && i != 0) {
-        GF_IDX e = gf_elem(d, j, i - 1);
-        tri(e, 0, 2, 0, dT(Nd(j, i - 1), true), 1, dT(Nd(j + 1, i - 1), true), 2, 0.0f);
-        tri(e, 1, 0, 0, 0.0f, 1, dT(Nd(j + 1, i - 1), true), 2, dT(Nd(j + 1, i), false));
-    }
-    if (j != nz - 1 && i != nx - 1)
-        tri(gf_elem(d, j, i), 0, 0, 0, 0.0f, 1, dT(Nd(j + 1, i), false), 2, dT(Nd(j, i + 1), false));
-    float inc = rhs * gf_d2f(C->dt) / area_n;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) inc += w[q] * t[q];
+    inc *= gf_d2f(C->dt);
     if (!final_sweep)
         d0[n] = inc;
     else
@@ -1640,6 +1666,15 @@ template <class R> __global__ void k_convert_back(const R *__restrict__ src, dou
 #endif
 
 // ---------------------------------------------------------------- launchers
+inline int gf_sm_count() {
+    static const int sms = [] {
+        int dev = 0, v = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+        return v;
+    }();
+    return sms;
+}
 // Threads per CTA for n items.  FP64 kernels: fewer than `most`, down to 64,
 // while that leaves SMs without a CTA, since warps that share an SM queue for
 // its FP64 pipe (ten steps of 60x20 elements 1.055 -> 1.020 ms, 241x61 1.265
@@ -1648,13 +1683,7 @@ template <class R> __global__ void k_convert_back(const R *__restrict__ src, dou
 // that warps of one SM fetch once for all.
 inline unsigned gf_threads_for(long long n, unsigned most) {
 #ifdef GF_FP64_UNIT
-    static const int sms = [] {
-        int dev = 0, v = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-        return v;
-    }();
-    while (most > 64 && n <= (long long)(most / 2) * sms) most /= 2;
+    while (most > 64 && n <= (long long)(most / 2) * gf_sm_count()) most /= 2;
 #else
     (void)n;
 #endif
@@ -1716,7 +1745,12 @@ template <class R> void GfKernels<R>::step_forces(const GfLaunch &g, int avg_mod
         gf_launch_pdl(kern, dim3(grid_for(g.d.N), parts), GF_THREADS, g.s, args...);
         ++*g.launches;
     };
-    launch(k_step_a, 2u, g.P, g.C, g.A, g.d);
+    // beside fl_rheol's CTAs (two an SM, by their registers) while both fit the
+    // SMs at once; on larger meshes the prep, which wants warps in flight, is a
+    // launch of its own (a step of 1000x300 elements 93.2 against 98.5 us)
+    const bool beside = grid_for(g.d.N) <= (unsigned)gf_sm_count();
+    if (!beside) GF_LAUNCH(k_therm_prep32, g.d.N, g.P, g.A, g.d, (float *)g.A.t_coef);
+    launch(k_step_a, beside ? 2u : 1u, g.P, g.C, g.A, g.d);
     launch(k_step_b, avg_mode > 0 ? 3u : 2u, g.P, g.C, g.A, g.d, avg_mode);
     launch(k_step_c, move ? 3u : 1u, g.P, g.C, g.A, g.d, avg_mode);
     if (move)
@@ -1730,7 +1764,7 @@ template <class R> void GfKernels<R>::therm(const GfLaunch &g, int sweeps, int k
     if (sizeof(R) == sizeof(float)) {
         const float *tc = (const float *)g.A.t_coef;
         float *d0 = (float *)g.A.t_delta0;
-        GF_LAUNCH(k_therm_prep32, g.d.E, g.P, g.A, g.d, (float *)g.A.t_coef);
+        GF_LAUNCH(k_therm_prep32, g.d.N, g.P, g.A, g.d, (float *)g.A.t_coef);
         GF_LAUNCH(k_therm_sweep32, g.d.N, g.P, g.C, g.A, g.d, tc, d0, g.A.t_delta1, 0);
         GF_LAUNCH(k_therm_sweep32, g.d.N, g.P, g.C, g.A, g.d, tc, d0, g.A.t_delta1, 1);
         GF_LAUNCH(k_therm_apply32, g.d.N, g.P, g.A, g.d, g.A.t_delta1);
