@@ -333,6 +333,23 @@ int take_status(gf_ctx *c) {
     return st;
 }
 
+// itest_mesh's scalars beside the smallest angle: out[0] = 180 (the angle's
+// start), the surface's end points along x, two heights of the first column,
+// dhacc and extr_acc
+__global__ void k_itest_gather(DevArrays A, GfDims d, double *out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= d.nx) return;
+    if (i == 0) {
+        out[0] = 180.0;
+        out[1] = A.cord[gf_node(d, 0, 0)];
+        out[2] = A.cord[gf_node(d, 0, d.nx - 1)];
+        out[3] = A.cord[d.N + gf_node(d, 0, 0)];
+        out[4] = A.cord[d.N + gf_node(d, 1, 0)];
+    }
+    out[5 + i] = A.dhacc[i];
+    out[5 + d.nx + i] = A.extr_acc[i];
+}
+
 __global__ void k_clock_advance(DevClock *C) { C->time = C->time + C->dt; }
 
 // ---- dispatch on precision
@@ -708,7 +725,7 @@ int gf_create(gf_ctx **out, const gf_params *p, const gf_layout *L, int mode) {
     A_(dalloc(c, &A.e_rho, E));
     A_(dalloc(c, &A.e_flag, E));
     A_(dalloc(c, &A.nmarkers, 1));
-    A_(dalloc(c, &c->d_angle, 1));
+    A_(dalloc(c, &c->d_angle, 5 + 2 * (size_t)p->nx));
     A_(dalloc(c, &A.cord_old, 2 * N));
     A_(dalloc(c, &A.orig, 2 * N));
     if (p->itype_melting == 1) {
@@ -1114,36 +1131,30 @@ int gf_step(gf_ctx *c, int nsteps) {
 
 int gf_itest_mesh(gf_ctx *c, double *min_angle) {
     if (!c) return GF_ERR_ARG;
-    double init = 180.0;
-    GF_CK(cudaMemcpyAsync(c->d_angle, &init, sizeof init, cudaMemcpyHostToDevice, c->s));
+    const gf_params &p = c->p;
+    const int nx = p.nx;
+    // everything the test reads comes back in one copy (seven small ones cost
+    // some 8 us each, a third of a step of 60x20 elements)
+    k_itest_gather<<<(nx + 255) / 256, 256, 0, c->s>>>(c->A, c->d, c->d_angle);
+    ++c->launches;
     GfLaunch g = launch_of(c);
     GfKernels<double>::min_angle(g, c->d_angle);
-    double a = 0.0;
-    GF_CK(cudaMemcpyAsync(&a, c->d_angle, sizeof a, cudaMemcpyDeviceToHost, c->s));
+    std::vector<double> h(5 + 2 * (size_t)nx);
+    GF_CK(cudaMemcpyAsync(h.data(), c->d_angle, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c->s));
     GF_CK(cudaStreamSynchronize(c->s));
+    const double a = h[0], x0 = h[1], xn = h[2], z00 = h[3], z10 = h[4];
+    const double *dh = h.data() + 5, *ex = dh + nx;
     if (min_angle) *min_angle = a;
     // rem_test.f90:23-66: shortening (code 2), surface topography change
     // (code 3), before the angle (code 1)
-    const gf_params &p = c->p;
-    const int nx = p.nx;
-    const long long N = c->d.N;
     int need = 0;
     if (p.mode_rem == 11 || p.mode_rem == 3) {
-        double x0 = 0.0, xn = 0.0;
-        GF_CK(cudaMemcpy(&x0, c->A.cord + gf_node(c->d, 0, 0), sizeof(double), cudaMemcpyDeviceToHost));
-        GF_CK(cudaMemcpy(&xn, c->A.cord + gf_node(c->d, 0, nx - 1), sizeof(double), cudaMemcpyDeviceToHost));
         double testcr = p.dx_rem * p.rxbo / (nx - 1);
         double shortening = std::fabs(xn - x0 - p.rxbo);
         if (shortening > testcr) need = 2;
     }
     const double arc_extrusion_rate = 1.0 - p.ratio_mantle_mzone;
     if (need == 0 && (p.topo_kappa > 0 || arc_extrusion_rate > 0)) {
-        std::vector<double> dh(nx), ex(nx);
-        double z00 = 0.0, z10 = 0.0;
-        GF_CK(cudaMemcpy(dh.data(), c->A.dhacc, sizeof(double) * nx, cudaMemcpyDeviceToHost));
-        GF_CK(cudaMemcpy(ex.data(), c->A.extr_acc, sizeof(double) * nx, cudaMemcpyDeviceToHost));
-        GF_CK(cudaMemcpy(&z00, c->A.cord + N + gf_node(c->d, 0, 0), sizeof(double), cudaMemcpyDeviceToHost));
-        GF_CK(cudaMemcpy(&z10, c->A.cord + N + gf_node(c->d, 1, 0), sizeof(double), cudaMemcpyDeviceToHost));
         for (int i = 0; i < nx - 1; ++i) {
             double testcr = (z00 - z10) * 0.3333;
             double topochanges = std::fabs(dh[i]) + ex[i];
