@@ -140,6 +140,12 @@ GF_PHASE(PhAmass, K_N, 80) {
 struct MemFrac { static __device__ void member(const BatchMember &m) { b_k_frac_fix<float>(m.P, m.C, m.A, m.d); } };
 struct MemDtReset { static __device__ void member(const BatchMember &m) { b_k_dt_reset(m.C); } };
 struct MemDtScalars { static __device__ void member(const BatchMember &m) { b_k_dt_scalars(m.P, m.C); } };
+// every member's status side by side (fetched one by one they cost some 7 us
+// each: 0.4 ms of ten steps of 64 members)
+__global__ void k_batch_status(const BatchMember *members, int n, int *out) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n) out[k] = members[k].C->status;
+}
 struct MemTime { static __device__ void member(const BatchMember &m) { m.C->time = m.C->time + m.C->dt; } };
 
 // ---------------------------------------------------------------- surrogate I/O
@@ -529,6 +535,7 @@ struct gf_batch {
     // device copy of the fields gf_batch_inject overwrites (restore point)
     void *backup = nullptr;
     std::vector<size_t> backup_off;
+    int *status = nullptr, *h_status = nullptr; // the members' status words, device and pinned host
     float4 *means = nullptr; // gf_batch_sample's element pairs (two per element)
 };
 
@@ -763,10 +770,14 @@ int refresh_views(gf_batch *b) {
 }
 
 int check_status(gf_batch *b) {
+    const int n = (int)b->members.size();
+    k_batch_status<<<(n + 127) / 128, 128, 0, b->s>>>(b->d_members, n, b->status);
+    GB_CK(cudaMemcpyAsync(b->h_status, b->status, sizeof(int) * n, cudaMemcpyDeviceToHost, b->s));
     GB_CK(cudaStreamSynchronize(b->s));
     int first = GF_OK;
-    for (gf_ctx *c : b->members) {
-        int st = gf_ctx_take_status(c);
+    for (int k = 0; k < n; ++k) {
+        if (!b->h_status[k]) continue;
+        const int st = gf_ctx_take_status(b->members[k]); // and clears it
         if (st && !first) first = st;
     }
     return first;
@@ -798,6 +809,8 @@ int gf_batch_create(gf_batch **out, gf_ctx **members, int n) {
     if (!rc) rc = batch_cuda(cudaStreamCreateWithFlags(&b->s, cudaStreamNonBlocking), "stream");
     if (!rc) rc = batch_cuda(cudaMalloc(&b->d_members, sizeof(BatchMember) * n), "members");
     if (!rc) rc = batch_cuda(cudaMalloc(&b->means, sizeof(float4) * 2 * (size_t)b->elements), "sampling scratch");
+    if (!rc) rc = batch_cuda(cudaMalloc(&b->status, sizeof(int) * n), "status");
+    if (!rc) rc = batch_cuda(cudaMallocHost(&b->h_status, sizeof(int) * n), "status");
     if (!rc) rc = upload_members(b);
     if (!rc) rc = build_tables(b);
     if (rc) {
@@ -817,6 +830,8 @@ void gf_batch_destroy(gf_batch *b) {
     if (b->d_members) cudaFree(b->d_members);
     if (b->backup) cudaFree(b->backup);
     if (b->means) cudaFree(b->means);
+    if (b->status) cudaFree(b->status);
+    if (b->h_status) cudaFreeHost(b->h_status);
     if (b->s) cudaStreamDestroy(b->s);
     delete b;
 }

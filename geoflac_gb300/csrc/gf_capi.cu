@@ -40,6 +40,7 @@ struct gf_ctx {
     DevArrays A{};
     double *staging = nullptr; // FP64 staging for mixed-mode conversions
     double *d_angle = nullptr;
+    void *pinned = nullptr; // host side of the small copies back: a DevClock, or the mesh test's values
     GfRemeshBufs rb{};         // remesh scratch
     double ar_x = 0, ar_z = 0; // mesh1 zone-pattern totals
     // host mirrors of the host-controlled scalars
@@ -321,11 +322,11 @@ int call_status(gf_ctx *c) {
 }
 
 int take_status(gf_ctx *c) {
-    int st = 0;
-    cudaError_t e = cudaStreamSynchronize(c->s);
+    // (through pinned memory behind the work it reports on: one wait)
+    cudaError_t e = cudaMemcpyAsync(c->pinned, &c->dC->status, sizeof(int), cudaMemcpyDeviceToHost, c->s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->s);
     if (e != cudaSuccess) return cuda_err(e, "step");
-    e = cudaMemcpy(&st, &c->dC->status, sizeof(int), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return cuda_err(e, "status");
+    const int st = *(const int *)c->pinned;
     if (st) {
         int zero = 0;
         cudaMemcpy(&c->dC->status, &zero, sizeof(int), cudaMemcpyHostToDevice);
@@ -726,6 +727,8 @@ int gf_create(gf_ctx **out, const gf_params *p, const gf_layout *L, int mode) {
     A_(dalloc(c, &A.e_flag, E));
     A_(dalloc(c, &A.nmarkers, 1));
     A_(dalloc(c, &c->d_angle, 5 + 2 * (size_t)p->nx));
+    A_(cuda_err(cudaMallocHost(&c->pinned, std::max(sizeof(DevClock), sizeof(double) * (5 + 2 * (size_t)p->nx))),
+                "cudaMallocHost"));
     A_(dalloc(c, &A.cord_old, 2 * N));
     A_(dalloc(c, &A.orig, 2 * N));
     if (p->itype_melting == 1) {
@@ -811,6 +814,7 @@ void gf_destroy(gf_ctx *c) {
     if (c->s) cudaStreamSynchronize(c->s);
     for (auto &g : c->graphs) cudaGraphExecDestroy(g.exec);
     for (void *p : c->allocs) cudaFree(p);
+    if (c->pinned) cudaFreeHost(c->pinned);
     if (c->s) cudaStreamDestroy(c->s);
     delete c;
 }
@@ -852,13 +856,14 @@ int gf_get_params(gf_ctx *c, gf_params *p) {
 
 int gf_set_clock(gf_ctx *c, const gf_clock *k) {
     if (!c || !k) return GF_ERR_ARG;
+    GF_CK(cudaMemcpyAsync(c->pinned, c->dC, sizeof(DevClock), cudaMemcpyDeviceToHost, c->s));
     GF_CK(cudaStreamSynchronize(c->s));
-    DevClock C;
-    GF_CK(cudaMemcpy(&C, c->dC, sizeof C, cudaMemcpyDeviceToHost));
+    DevClock &C = *(DevClock *)c->pinned;
     C.dt = k->dt; C.time = k->time; C.dtavg = k->dtavg; C.dt_elastic = k->dt_elastic;
     C.dt_maxwell = k->dt_maxwell; C.dtmax_therm = k->dtmax_therm; C.frac = k->frac;
     C.vel_max = k->vel_max; C.dlmin = k->dlmin;
-    GF_CK(cudaMemcpy(c->dC, &C, sizeof C, cudaMemcpyHostToDevice));
+    // (the buffer is next written in this stream's order, or by the host after a wait for it)
+    GF_CK(cudaMemcpyAsync(c->dC, c->pinned, sizeof(DevClock), cudaMemcpyHostToDevice, c->s));
     c->nloop = k->nloop;
     c->nsrate = k->nsrate;
     c->nmarkers = k->nmarkers;
@@ -868,9 +873,9 @@ int gf_set_clock(gf_ctx *c, const gf_clock *k) {
 
 int gf_get_clock(gf_ctx *c, gf_clock *k) {
     if (!c || !k) return GF_ERR_ARG;
+    GF_CK(cudaMemcpyAsync(c->pinned, c->dC, sizeof(DevClock), cudaMemcpyDeviceToHost, c->s));
     GF_CK(cudaStreamSynchronize(c->s));
-    DevClock C;
-    GF_CK(cudaMemcpy(&C, c->dC, sizeof C, cudaMemcpyDeviceToHost));
+    const DevClock &C = *(const DevClock *)c->pinned;
     k->dt = C.dt; k->time = C.time; k->dtavg = C.dtavg; k->dt_elastic = C.dt_elastic;
     k->dt_maxwell = C.dt_maxwell; k->dtmax_therm = C.dtmax_therm; k->frac = C.frac;
     k->vel_max = C.vel_max; k->dlmin = C.dlmin;
@@ -1139,11 +1144,11 @@ int gf_itest_mesh(gf_ctx *c, double *min_angle) {
     ++c->launches;
     GfLaunch g = launch_of(c);
     GfKernels<double>::min_angle(g, c->d_angle);
-    std::vector<double> h(5 + 2 * (size_t)nx);
-    GF_CK(cudaMemcpyAsync(h.data(), c->d_angle, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c->s));
+    GF_CK(cudaMemcpyAsync(c->pinned, c->d_angle, sizeof(double) * (5 + 2 * (size_t)nx), cudaMemcpyDeviceToHost, c->s));
     GF_CK(cudaStreamSynchronize(c->s));
+    const double *h = (const double *)c->pinned;
     const double a = h[0], x0 = h[1], xn = h[2], z00 = h[3], z10 = h[4];
-    const double *dh = h.data() + 5, *ex = dh + nx;
+    const double *dh = h + 5, *ex = dh + nx;
     if (min_angle) *min_angle = a;
     // rem_test.f90:23-66: shortening (code 2), surface topography change
     // (code 3), before the angle (code 1)
