@@ -85,12 +85,13 @@ __device__ __forceinline__ int therm_sync(unsigned *slot, bool changed, int poll
 
 // The boundary conditions (fl_therm.f90:577-598) and temp0 = temp from the
 // last sweep's values, and the increment that the next step's start uses
-__device__ __forceinline__ void therm_finish(const DevParams *Pp, const DevArrays &A, const GfDims &d,
-                                             const double *src, int keep_temp0, GF_IDX n) {
+template <class Src>
+__device__ __forceinline__ void therm_finish(const DevParams *Pp, const DevArrays &A, const GfDims &d, Src src,
+                                             int keep_temp0, GF_IDX n) {
     int j, i;
     i = (int)((unsigned)n / (unsigned)d.nz);
     j = (int)n - i * d.nz;
-    const double t = therm_bc_value(*Pp, A, d, [src](GF_IDX m) { return __ldcg(src + m); }, j, i);
+    const double t = therm_bc_value(*Pp, A, d, src, j, i);
     const double told = A.temp[n];
     if (!keep_temp0) A.temp0[n] = told;
     A.temp[n] = t;
@@ -110,12 +111,39 @@ __device__ __forceinline__ void therm_count(DevClock *C, int kc, int kmax) {
 // it the barrier: fl_therm 76 -> 39 us on 60x20 and 241x61 elements, 91 -> 53
 // on 400x120, 112 -> 62 on 600x150 (events) against the general kernel's
 // predecessor, where a sweep took 9 to 15 us.
+//
+// CL: a mesh of up to GF_TH_CL x 256 nodes runs as one cluster.  The iterates
+// and the sweep's changed flags then live in the CTAs' shared memory, read
+// across the cluster, and the hardware's cluster barrier ends a sweep: no trip
+// to L2 and back for the values nor for the barrier (fl_therm of 60x20
+// elements 40 -> 32 us).  Every CTA has as many nodes as it has threads, four
+// warps (one on each FP64 pipe) up to 2048 nodes.
 #define GF_TH_T 128
 #define GF_TH_CTAS 5 // per SM: 102 registers
-__global__ void __launch_bounds__(GF_TH_T, GF_TH_CTAS)
+#define GF_TH_CL 16
+#define GF_TH_CLT 256
+__device__ __forceinline__ unsigned cl_map(const void *p, unsigned rank) { // p in CTA rank's shared memory
+    unsigned a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ double cl_load(unsigned a) {
+    double v;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cl_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+template <bool CL>
+__global__ void __launch_bounds__(CL ? GF_TH_CLT : GF_TH_T, CL ? 1 : GF_TH_CTAS)
     k_therm_sweeps_reg(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d,
                        const double *__restrict__ tc, double *b0, double *b1, int kmax, int keep_temp0) {
-    const GF_IDX nn = (GF_IDX)blockIdx.x * GF_TH_T + threadIdx.x;
+    __shared__ double iter[2][CL ? GF_TH_CLT : 1];
+    __shared__ unsigned moved[2][CL ? GF_TH_CL : 1]; // by the sweep's parity and the CTA that reports
+    if (CL) gf_pdl_entry();
+    const unsigned T_ = blockDim.x;
+    const GF_IDX nn = (GF_IDX)blockIdx.x * T_ + threadIdx.x;
     const bool act = nn < d.N;
     const GF_IDX n = act ? nn : d.N - 1; // idle threads follow along and store nothing
     const int nz = d.nz, i = (int)((unsigned)n / (unsigned)nz), j = (int)n - i * nz;
@@ -187,13 +215,19 @@ __global__ void __launch_bounds__(GF_TH_T, GF_TH_CTAS)
     // many nodes the sweeps recompute before they reach it
     double a = T[na] + A.t_pred[na], b = T[nb] + A.t_pred[nb], c = T[nc] + A.t_pred[nc];
     double v = Ts + A.t_pred[n];
+    auto where = [&](GF_IDX m) { return cl_map(&iter[0][(unsigned)m % T_], (unsigned)m / T_); };
+    const unsigned wa = CL ? where(na) : 0u, wb = CL ? where(nb) : 0u, wc = CL ? where(nc) : 0u;
+    const unsigned report = CL ? cl_map(&moved[0][blockIdx.x], threadIdx.x % gridDim.x) : 0u;
+    if (CL) cl_sync(); // every CTA of the cluster runs
     int kc = kmax; // the first sweep that changed nothing
     for (int k = 0; k < kmax; ++k) {
         bool changed = false;
         bool redo = true;
         if (k > 0) {
             const double *src = (k - 1) & 1 ? b1 : b0;
-            const double a1 = __ldcg(src + na), c1n = __ldcg(src + nc), b1n = __ldcg(src + nb);
+            const unsigned off = ((k - 1) & 1) * (GF_TH_CLT * 8u);
+            const double a1 = CL ? cl_load(wa + off) : __ldcg(src + na), c1n = CL ? cl_load(wc + off) : __ldcg(src + nc),
+                         b1n = CL ? cl_load(wb + off) : __ldcg(src + nb);
             redo = (up && !gf_deq(a1, a)) || (lf && !gf_deq(b1n, b)) || (lf && dn && !gf_deq(c1n, c));
             a = a1;
             b = b1n;
@@ -204,11 +238,22 @@ __global__ void __launch_bounds__(GF_TH_T, GF_TH_CTAS)
             changed = act && redo && !gf_deq(t, v);
             if (redo) v = t;
         }
-        if (act) ((k & 1) ? b1 : b0)[n] = v;
-        const int s = therm_sync(reinterpret_cast<unsigned *>(C->therm_flags + k), changed);
-        if (s < 0) {
-            if (nn == 0) set_status(C, GF_ERR_TIMEOUT, k);
-            return;
+        int s;
+        if constexpr (CL) {
+            iter[k & 1][threadIdx.x] = v;
+            const unsigned any = __syncthreads_or(changed);
+            if (threadIdx.x < gridDim.x)
+                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(report + (k & 1) * (GF_TH_CL * 4u)), "r"(any) : "memory");
+            cl_sync();
+            const unsigned lane = threadIdx.x & 31u;
+            s = __any_sync(0xffffffffu, lane < gridDim.x && moved[k & 1][lane % GF_TH_CL] != 0u);
+        } else {
+            if (act) ((k & 1) ? b1 : b0)[n] = v;
+            s = therm_sync(reinterpret_cast<unsigned *>(C->therm_flags + k), changed);
+            if (s < 0) {
+                if (nn == 0) set_status(C, GF_ERR_TIMEOUT, k);
+                return;
+            }
         }
         if (s == 0) {
             kc = k;
@@ -216,7 +261,15 @@ __global__ void __launch_bounds__(GF_TH_T, GF_TH_CTAS)
         }
     }
     if (nn == 0) therm_count(C, kc, kmax);
-    if (act) therm_finish(Pp, A, d, ((kc < kmax ? kc : kmax - 1) & 1) ? b1 : b0, keep_temp0, n);
+    const int last = (kc < kmax ? kc : kmax - 1) & 1;
+    if constexpr (CL) {
+        if (act)
+            therm_finish(Pp, A, d, [&](GF_IDX m) { return cl_load(where(m) + last * (GF_TH_CLT * 8u)); }, keep_temp0, n);
+        cl_sync(); // no CTA leaves while another reads its values
+    } else {
+        const double *src = last ? b1 : b0;
+        if (act) therm_finish(Pp, A, d, [src](GF_IDX m) { return __ldcg(src + m); }, keep_temp0, n);
+    }
 }
 
 // One node of a sweep from its coefficients in memory.  Tup holds the current
@@ -357,12 +410,34 @@ __global__ void __launch_bounds__(GF_THREADS, 4)
     if (blockIdx.x == 0 && threadIdx.x == 0) therm_count(C, kc, kmax);
     const double *src = ((kc < kmax ? kc : kmax - 1) & 1) ? b1 : b0;
     for (GF_IDX n = (GF_IDX)blockIdx.x * GF_THREADS + threadIdx.x; n < d.N; n += (GF_IDX)gridDim.x * GF_THREADS)
-        therm_finish(Pp, A, d, src, keep_temp0, n);
+        therm_finish(Pp, A, d, [src](GF_IDX m) { return __ldcg(src + m); }, keep_temp0, n);
 }
 
 } // namespace gfk
 } // namespace
 
+// CTAs of the widest cluster of k_therm_sweeps_reg<true> that the device
+// takes (16 needs an opt-in), 0: none
+inline int cluster_ctas() {
+    using namespace gfk;
+    if (cudaFuncSetAttribute(k_therm_sweeps_reg<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+        (void)cudaGetLastError();
+    for (int c = GF_TH_CL; c >= 8; c /= 2) {
+        cudaLaunchConfig_t lc = {};
+        lc.gridDim = dim3((unsigned)c);
+        lc.blockDim = dim3(GF_TH_CLT);
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)c;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        lc.attrs = attr;
+        lc.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, k_therm_sweeps_reg<true>, &lc) == cudaSuccess && n > 0) return c;
+        (void)cudaGetLastError();
+    }
+    return 0;
+}
 // fl_therm after an optional temp0 = temp of the caller (keep_temp0)
 inline void therm_launch(const GfLaunch &g, int kmax, int keep_temp0) {
     using namespace gfk;
@@ -370,17 +445,37 @@ inline void therm_launch(const GfLaunch &g, int kmax, int keep_temp0) {
     gf_launch_pdl(k_therm_prep, grid_for(2 * g.d.E, t), t, g.s, g.P, g.C, g.A, g.d, g.A.t_coef);
     ++*g.launches;
     // resident CTAs of the two kernels, once per device
-    static int cap_reg[64] = {0}, cap_gen[64] = {0};
+    static int cap_reg[64] = {0}, cap_gen[64] = {0}, cap_cl[64] = {0}; // (cap_cl: CTAs of a cluster, 0: none fits)
     int dev = 0;
     cudaGetDevice(&dev);
     dev = dev & 63;
     if (cap_gen[dev] == 0) {
         int a = 0, b = 0, sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_therm_sweeps_reg, GF_TH_T, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_therm_sweeps_reg<false>, GF_TH_T, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_therm_sweeps, GF_THREADS, 0);
+        cap_cl[dev] = cluster_ctas();
         cap_reg[dev] = a * sms;
         cap_gen[dev] = (b > 0 ? b : 1) * sms;
+    }
+    if (g.d.N <= (GF_IDX)cap_cl[dev] * GF_TH_CLT) { // one cluster holds the mesh
+        const unsigned thr = (unsigned)((g.d.N + cap_cl[dev] - 1) / cap_cl[dev] + 31) & ~31u;
+        cudaLaunchConfig_t lc = {};
+        lc.gridDim = dim3((unsigned)cap_cl[dev]);
+        lc.blockDim = dim3(thr);
+        lc.stream = g.s;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)cap_cl[dev];
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        lc.attrs = attr;
+        lc.numAttrs = 2;
+        cudaLaunchKernelEx(&lc, k_therm_sweeps_reg<true>, g.P, g.C, g.A, g.d, (const double *)g.A.t_coef, g.A.t_delta0,
+                           g.A.t_delta1, kmax, keep_temp0);
+        ++*g.launches;
+        return;
     }
     const bool reg = g.d.N <= (GF_IDX)cap_reg[dev] * GF_TH_T; // one node per thread fits
     const int threads = reg ? GF_TH_T : GF_THREADS;
@@ -394,7 +489,7 @@ inline void therm_launch(const GfLaunch &g, int kmax, int keep_temp0) {
     attr[0].val.cooperative = 1;
     lc.attrs = attr;
     lc.numAttrs = 1;
-    cudaLaunchKernelEx(&lc, reg ? k_therm_sweeps_reg : k_therm_sweeps, g.P, g.C, g.A, g.d, (const double *)g.A.t_coef,
+    cudaLaunchKernelEx(&lc, reg ? k_therm_sweeps_reg<false> : k_therm_sweeps, g.P, g.C, g.A, g.d, (const double *)g.A.t_coef,
                        g.A.t_delta0, g.A.t_delta1, kmax, keep_temp0);
     ++*g.launches;
 }
