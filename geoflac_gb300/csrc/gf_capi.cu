@@ -342,6 +342,7 @@ __global__ void k_itest_gather(DevArrays A, GfDims d, double *out) {
     if (i >= d.nx) return;
     if (i == 0) {
         out[0] = 180.0;
+        out[5 + 2 * (long long)d.nx] = 0.0; // the FP32 pass's largest cosine
         out[1] = A.cord[gf_node(d, 0, 0)];
         out[2] = A.cord[gf_node(d, 0, d.nx - 1)];
         out[3] = A.cord[d.N + gf_node(d, 0, 0)];
@@ -726,7 +727,7 @@ int gf_create(gf_ctx **out, const gf_params *p, const gf_layout *L, int mode) {
     A_(dalloc(c, &A.e_rho, E));
     A_(dalloc(c, &A.e_flag, E));
     A_(dalloc(c, &A.nmarkers, 1));
-    A_(dalloc(c, &c->d_angle, 5 + 2 * (size_t)p->nx));
+    A_(dalloc(c, &c->d_angle, 6 + 2 * (size_t)p->nx));
     A_(cuda_err(cudaMallocHost(&c->pinned, std::max(sizeof(DevClock), sizeof(double) * (5 + 2 * (size_t)p->nx))),
                 "cudaMallocHost"));
     A_(dalloc(c, &A.cord_old, 2 * N));
