@@ -315,6 +315,13 @@ __device__ __forceinline__ double gf_mulq(double a, double b) {
 }
 __device__ __forceinline__ float gf_mulq(float a, float b) { return a * b; }
 
+// Products and quotients of the kernels that run now and then (densities, time
+// step, mass scaling): on the integer pipes (I) where the FP64 pipe is the
+// bound, as FP64 instructions on small meshes, where a kernel is one chain of
+// latencies and theirs are the shorter ones.  Same bits.
+template <bool I> __device__ __forceinline__ double gf_mulc(double a, double b) { return I ? gf_mul(a, b) : a * b; }
+template <bool I> __device__ __forceinline__ double gf_divc(double a, double b) { return I ? gf_ddiv(a, b) : a / b; }
+
 // x * 2^K (K = -2 .. 2, the constant factors 0.25 .. 4 of the step): the
 // exponent field moves by K while x and the result are normal doubles, a
 // zero keeps its bits, and anything else takes the FP64 multiply out of line.
@@ -599,7 +606,7 @@ __device__ __forceinline__ double visc_of(const DevParams &P, const DevArrays &A
 
 // Eff_dens (matprops.f90:3-83), FP64.  *wrote_frac/*frac_val report the
 // write of the global frac the reference performs (matprops.f90:37,48).
-template <class R>
+template <class R, bool I = false>
 __device__ double eff_dens(const DevParams &P, const DevArrays &A, const GfDims &d, int j, int i, GF_IDX e,
                            int *wrote_frac, double *frac_val) {
     const double adi_grad = 3e-1, den_ramp_dist = 30e3, amp410 = 0.05, amp660 = 0.085;
@@ -609,24 +616,24 @@ __device__ double eff_dens(const DevParams &P, const DevArrays &A, const GfDims 
     double zcord = 0.25 * (cord[d.N + n1] + cord[d.N + n1 + 1] + cord[d.N + n3] + cord[d.N + n3 + 1]);
     double tmpr0 = 0.25 * (temp[n1] + temp[n1 + 1] + temp[n3] + temp[n3 + 1]);
     double zsurf = 0.50 * (cord[d.N + gf_node(d, 0, i)] + cord[d.N + gf_node(d, 0, i + 1)]);
-    double tmpr = (zsurf - zcord) * 1e-3 * adi_grad + tmpr0;
+    double tmpr = gf_mulc<I>(gf_mulc<I>(zsurf - zcord, 1e-3), adi_grad) + tmpr0;
     int iph = A.iphase[e];
-    double deptmpr410 = -101.58 * (tmpr + 273.0) - 216828.0;
+    double deptmpr410 = gf_mulc<I>(-101.58, tmpr + 273.0) - 216828.0;
     double deptmpr420 = deptmpr410 - den_ramp_dist;
     double den_amp = 1.0;
     *wrote_frac = 0;
     if (deptmpr410 > zcord) {
-        double f = (deptmpr410 - zcord) / (deptmpr410 - deptmpr420);
+        double f = gf_divc<I>(deptmpr410 - zcord, deptmpr410 - deptmpr420);
         if (f < 0.0) f = 0.0;
         if (f > 1.0) f = 1.0;
         *wrote_frac = 1;
         *frac_val = f;
         den_amp = 1.0 + amp410 * f;
     }
-    double deptmpr660 = 66.55 * (tmpr + 273.0) - 788494.0;
+    double deptmpr660 = gf_mulc<I>(66.55, tmpr + 273.0) - 788494.0;
     double deptmpr670 = deptmpr660 - den_ramp_dist;
     if (deptmpr660 > zcord) {
-        double f = (deptmpr660 - zcord) / (deptmpr660 - deptmpr670);
+        double f = gf_divc<I>(deptmpr660 - zcord, deptmpr660 - deptmpr670);
         if (f < 0.0) f = 0.0;
         if (f > 1.0) f = 1.0;
         *wrote_frac = 1;
@@ -636,18 +643,19 @@ __device__ double eff_dens(const DevParams &P, const DevArrays &A, const GfDims 
     double press = 0;
     for (int k = 0; k < 4; ++k)
         press = press - ((double)st[gf_s(d, e, 0, k)] + (double)st[gf_s(d, e, 1, k)] + (double)st[gf_s(d, e, 3, k)]);
-    press = press / 12;
+    press = gf_divc<I>(press, 12.0);
     if (sizeof(R) == sizeof(float)) press = press + A.p_ref[e]; // mixed: stored stresses exclude -p_ref
     double ed = 0.0;
     for (int k = 0; k < P.nphase; ++k) {
         double ratio = A.phase_ratio[gf_pr(d, e, k)];
         if (ratio < 0.01) continue;
-        double dens = P.den[k] * (1 - P.alfa[k] * tmpr + P.beta[k] * press);
-        press = dens * P.g * zcord;
-        dens = P.den[k] * (1 - P.alfa[k] * tmpr + P.beta[k] * press);
-        ed = ed + ratio * dens;
+        const double expand = 1 - gf_mulc<I>(P.alfa[k], tmpr);
+        double dens = gf_mulc<I>(P.den[k], expand + gf_mulc<I>(P.beta[k], press));
+        press = gf_mulc<I>(gf_mulc<I>(dens, P.g), zcord);
+        dens = gf_mulc<I>(P.den[k], expand + gf_mulc<I>(P.beta[k], press));
+        ed = ed + gf_mulc<I>(ratio, dens);
     }
-    if (iph == 4 || iph == 8 || iph == 9 || iph == 16 || iph == 18) ed = ed * den_amp;
+    if (iph == 4 || iph == 8 || iph == 9 || iph == 16 || iph == 18) ed = gf_mulc<I>(ed, den_amp);
     double fma = fmin(A.fmagma[e] + A.fmagma2[e], P.fmagma_max);
     ed = ed - fma * (ed - P.rho_magma);
     return ed;

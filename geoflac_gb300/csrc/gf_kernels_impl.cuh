@@ -957,7 +957,7 @@ __global__ void __launch_bounds__(GF_THREADS, 3) k_step_d(const DevParams *__res
 // ======================================================================
 // rmasses (rmasses.f90:4-63): per-element density, then a node gather in
 // the reference's colour order with each element's triangles in order.
-template <class R> __device__ __forceinline__ void b_k_elem_dens(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d, GF_IDX e) {
+template <class R, bool I = false> __device__ __forceinline__ void b_k_elem_dens(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d, GF_IDX e) {
     if (e >= d.E) return;
     int j, i;
     elem_ji(d, e, j, i);
@@ -973,14 +973,14 @@ template <class R> __device__ __forceinline__ void b_k_elem_dens(const DevParams
         for (int k = 0; k < 4; ++k) tri[k * d.E + e] = (1.0f / 12.0f) / area[gf_ek(d, e, k)] * dens;
     } else {
         double fval = 0.0;
-        double dens = eff_dens<R>(*Pp, A, d, j, i, e, &wrote, &fval);
+        double dens = eff_dens<R, I>(*Pp, A, d, j, i, e, &wrote, &fval);
         A.e_dens[e] = dens;
         // each triangle's share c1d12/area*dens (rmasses.f90:35-57),
         // computed once here with the reference's operations and gathered
         // per node
         const double c1d12 = 1.0 / 12.0;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) A.e_tri[k * d.E + e] = c1d12 / (double)area[gf_ek(d, e, k)] * dens;
+        for (int k = 0; k < 4; ++k) A.e_tri[k * d.E + e] = gf_mulc<I>(gf_divc<I>(c1d12, (double)area[gf_ek(d, e, k)]), dens);
     }
     if (wrote) {
         // serial position of this element in the coloured sweep
@@ -997,9 +997,9 @@ template <class R> __device__ __forceinline__ void b_k_elem_dens(const DevParams
         atomicMax((unsigned long long *)&C->frac_writer, (unsigned long long)(pos + 1));
     }
 }
-template <class R> __global__ void __launch_bounds__(GF_THREADS) k_elem_dens(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d) {
+template <class R, bool I = false> __global__ void __launch_bounds__(GF_THREADS) k_elem_dens(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d) {
     gf_pdl_entry();
-    b_k_elem_dens<R>(Pp, C, A, d, (GF_IDX)blockIdx.x * blockDim.x + threadIdx.x);
+    b_k_elem_dens<R, I>(Pp, C, A, d, (GF_IDX)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 template <class R> __device__ __forceinline__ void b_k_frac_fix(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d) {
@@ -1110,7 +1110,7 @@ __device__ __forceinline__ void dt_block_commit(DevClock *__restrict__ C, double
     __syncthreads(); // the shared slots are free for the CTA's next item
 }
 
-template <class R> __device__ __forceinline__ void b_k_dt_reduce(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d, GF_IDX t) {
+template <class R, bool I = false> __device__ __forceinline__ void b_k_dt_reduce(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d, GF_IDX t) {
     const DevParams &P = *Pp;
     double dl = 1e300, vmax = 0.0, dmax = 0.0;
     unsigned pm = 0;
@@ -1156,26 +1156,35 @@ template <class R> __device__ __forceinline__ void b_k_dt_reduce(const DevParams
             const R *area = (const R *)A.area;
             Quad q;
             load_quad(A.cord, d, j, i, q);
+            // (squares, products, comparisons and quotients on the integer
+            // pipes; the six roots and their sums stay on the FP64 pipe)
             auto len = [&](int a, int b) {
                 double ddx = q.x[a] - q.x[b], ddy = q.y[a] - q.y[b];
-                return sqrt(ddx * ddx + ddy * ddy);
+                return sqrt(gf_mulc<I>(ddx, ddx) + gf_mulc<I>(ddy, ddy));
             };
             double a0 = (double)area[gf_ek(d, e, 0)], a1 = (double)area[gf_ek(d, e, 1)],
                    a2 = (double)area[gf_ek(d, e, 2)], a3 = (double)area[gf_ek(d, e, 3)];
             // the smallest of the twelve quotients 1/(area*length) of
             // dlmin_prop (dt_mass.f90:174-231) is the quotient of the largest
             // product: correctly rounded division is monotone, so
-            // min fl(1/x_k) = fl(1/max x_k) exactly, for one division
-            double l, xm = 0.0;
-            l = len(1, 0); xm = fmax(xm, a0 * l); xm = fmax(xm, a2 * l);
-            l = len(3, 1); xm = fmax(xm, a1 * l); xm = fmax(xm, a2 * l);
-            l = len(3, 2); xm = fmax(xm, a1 * l); xm = fmax(xm, a3 * l);
-            l = len(2, 0); xm = fmax(xm, a0 * l); xm = fmax(xm, a3 * l);
-            l = len(3, 0); xm = fmax(xm, a2 * l); xm = fmax(xm, a3 * l);
-            l = len(1, 2); xm = fmax(xm, a0 * l); xm = fmax(xm, a1 * l);
-            dl = fmin(dl, 1.0 / xm);
+            // min fl(1/x_k) = fl(1/max x_k) exactly, for one division.  The
+            // largest of 0 and the products, by their bits: negative numbers
+            // and NaNs, whose bits lie above infinity's, count for nothing
+            unsigned long long xm = 0ull;
+            auto top = [&](double ar, double l) {
+                const unsigned long long u = (unsigned long long)__double_as_longlong(gf_mulc<I>(ar, l));
+                if (u <= 0x7ff0000000000000ull && u > xm) xm = u;
+            };
+            double l;
+            l = len(1, 0); top(a0, l); top(a2, l);
+            l = len(3, 1); top(a1, l); top(a2, l);
+            l = len(3, 2); top(a1, l); top(a3, l);
+            l = len(2, 0); top(a0, l); top(a3, l);
+            l = len(3, 0); top(a2, l); top(a3, l);
+            l = len(1, 2); top(a0, l); top(a1, l);
+            dl = fmin(dl, gf_divc<I>(1.0, __longlong_as_double((long long)xm)));
             int iph = A.iphase[e] - 1;
-            dmax = P.conduct[iph] / P.den[iph] / P.cp[iph];
+            dmax = gf_divc<I>(gf_divc<I>(P.conduct[iph], P.den[iph]), P.cp[iph]);
             pm = 1u << iph;
         }
         if (t < d.N) vmax = fmax(fabs(A.vel[t]), fabs(A.vel[d.N + t]));
@@ -1186,9 +1195,9 @@ template <class R> __device__ __forceinline__ void b_k_dt_reduce(const DevParams
         dt_block_commit(C, dl, vmax, dmax, pm, nullptr, 0);
     }
 }
-template <class R> __global__ void __launch_bounds__(GF_THREADS) k_dt_reduce(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d) {
+template <class R, bool I = false> __global__ void __launch_bounds__(GF_THREADS) k_dt_reduce(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d) {
     gf_pdl_entry();
-    b_k_dt_reduce<R>(Pp, C, A, d, (GF_IDX)blockIdx.x * blockDim.x + threadIdx.x);
+    b_k_dt_reduce<R, I>(Pp, C, A, d, (GF_IDX)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 __device__ __forceinline__ void b_k_dt_scalars(const DevParams *__restrict__ Pp, DevClock *__restrict__ C) {
@@ -1240,7 +1249,7 @@ __global__ void k_dt_scalars(const DevParams *__restrict__ Pp, DevClock *__restr
 
 // inertial mass share of each triangle c1d12*rho_inert/area
 // (dt_mass.f90:83-120), one element per thread
-template <class R> __device__ __forceinline__ void b_k_elem_am3(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d, GF_IDX e) {
+template <class R, bool I = false> __device__ __forceinline__ void b_k_elem_am3(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d, GF_IDX e) {
     if (e >= d.E) return;
     const DevParams &P = *Pp;
     const R *area = (const R *)A.area;
@@ -1266,18 +1275,18 @@ template <class R> __device__ __forceinline__ void b_k_elem_am3(const DevParams 
     double dlmin = C->dlmin, frac = C->frac, dt_elastic = C->dt_elastic, vel_max = C->vel_max;
     int iph = A.iphase[e] - 1;
     double pwave = P.rl[iph] + 0.6666 * P.rm[iph];
-    double vel_sound = dlmin * frac / dt_elastic;
-    double rho_inert = pwave / (vel_sound * vel_sound);
+    double vel_sound = gf_divc<I>(gf_mulc<I>(dlmin, frac), dt_elastic);
+    double rho_inert = gf_divc<I>(pwave, gf_mulc<I>(vel_sound, vel_sound));
     if (P.i_rey == 1 && vel_max > 0.0) {
         double rho_inert2 = (P.xReyn * P.v_min) / (vel_max * fabs(P.rzbo));
         if (rho_inert > rho_inert2) rho_inert = rho_inert2;
     }
 #pragma unroll
-    for (int k = 0; k < 4; ++k) A.e_tri[k * d.E + e] = c1d12 * rho_inert / (double)area[gf_ek(d, e, k)];
+    for (int k = 0; k < 4; ++k) A.e_tri[k * d.E + e] = gf_divc<I>(gf_mulc<I>(c1d12, rho_inert), (double)area[gf_ek(d, e, k)]);
 }
-template <class R> __global__ void __launch_bounds__(GF_THREADS) k_elem_am3(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d) {
+template <class R, bool I = false> __global__ void __launch_bounds__(GF_THREADS) k_elem_am3(const DevParams *__restrict__ Pp, DevClock *__restrict__ C, DevArrays A, GfDims d) {
     gf_pdl_entry();
-    b_k_elem_am3<R>(Pp, C, A, d, (GF_IDX)blockIdx.x * blockDim.x + threadIdx.x);
+    b_k_elem_am3<R, I>(Pp, C, A, d, (GF_IDX)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 __device__ __forceinline__ void b_k_dt_reset(DevClock *C) {
@@ -1913,9 +1922,16 @@ template <class R> void GfKernels<R>::move(const GfLaunch &g) {
     move_elem(g);
 }
 
+// elements from which the FP64 pipe, not a thread's chain, bounds such kernels
+constexpr long long GF_INT_PIPE_E = 8192;
 template <class R> void GfKernels<R>::rmasses(const GfLaunch &g) {
     using namespace gfk;
-    GF_LAUNCH(k_elem_dens<R>, g.d.E, g.P, g.C, g.A, g.d);
+    // (gf_mulc: 60x20 elements lose 1 % of ten steps on the integer pipes, 241x61
+    // gain 3 %, and fl's rmasses + dt_mass of 1000x300 take 161 instead of 262 us)
+    if (sizeof(R) == sizeof(double) && g.d.E >= GF_INT_PIPE_E)
+        GF_LAUNCH((k_elem_dens<R, true>), g.d.E, g.P, g.C, g.A, g.d);
+    else
+        GF_LAUNCH(k_elem_dens<R>, g.d.E, g.P, g.C, g.A, g.d);
     k_frac_fix<R><<<1, 1, 0, g.s>>>(g.P, g.C, g.A, g.d);
     ++*g.launches;
     GF_LAUNCH(k_node_gather_tri<R>, g.d.N, (const R *)g.A.e_tri, g.A.rmass, g.d);
@@ -1926,13 +1942,20 @@ template <class R> void GfKernels<R>::dt_mass(const GfLaunch &g) {
     k_dt_reset<<<1, 1, 0, g.s>>>(g.C);
     ++*g.launches;
     GF_IDX n = g.d.E > g.d.N ? g.d.E : g.d.N;
-    GF_LAUNCH(k_dt_reduce<R>, n, g.P, g.C, g.A, g.d);
+    const bool ip = sizeof(R) == sizeof(double) && g.d.E >= GF_INT_PIPE_E;
+    if (ip)
+        GF_LAUNCH((k_dt_reduce<R, true>), n, g.P, g.C, g.A, g.d);
+    else
+        GF_LAUNCH(k_dt_reduce<R>, n, g.P, g.C, g.A, g.d);
     k_dt_scalars<<<1, 1, 0, g.s>>>(g.P, g.C);
     ++*g.launches;
     if (g.idt_scale == 0) {
         cudaMemcpyAsync(g.A.amass, g.A.rmass, sizeof(double) * g.d.N, cudaMemcpyDeviceToDevice, g.s);
     } else {
-        GF_LAUNCH(k_elem_am3<R>, g.d.E, g.P, g.C, g.A, g.d);
+        if (ip)
+            GF_LAUNCH((k_elem_am3<R, true>), g.d.E, g.P, g.C, g.A, g.d);
+        else
+            GF_LAUNCH(k_elem_am3<R>, g.d.E, g.P, g.C, g.A, g.d);
         GF_LAUNCH(k_node_gather_tri<R>, g.d.N, (const R *)g.A.e_tri, g.A.amass, g.d);
     }
 }
