@@ -351,7 +351,7 @@ def run_ours(args):
     gp.close()
     value = ws * E * args.steps / fp["t"]
     mixed_value = ws * E * args.steps / res["mixed"]["t"]
-    # dominant kernel: fl_rheol (k_rheol), timed alone
+    # dominant kernel: fl_rheol (k_rheol_tri), timed alone
     g = fp["g"]
     t_rheol = _time_kernel(g, "fl_rheol", 10, flush)
     peak, peak_kind = _peaks()
@@ -373,7 +373,7 @@ def run_ours(args):
     e2e = {"value": e2e_value, "unit": "element-steps/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
            "steps": e2e_steps,
            "path": "per-subroutine C-ABI calls, clock scalars in/out, cord+vel to host every step"}
-    roofline = {"bound": "hbm", "kernel": "k_rheol (fl_rheol, FP64)", "achieved": achieved, "peak": peak,
+    roofline = {"bound": "hbm", "kernel": "k_rheol_tri (fl_rheol, FP64)", "achieved": achieved, "peak": peak,
                 "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind, "traffic": traffic,
                 "avg_launch_s": t_rheol, "algorithmic_bytes_per_launch": alg, "compute": _ncu_pipe("k_rheol_fp64")}
     for r in res.values():
