@@ -513,6 +513,7 @@ __global__ void k_force_residual(const BatchMember *members, const int2 *tiles, 
 
 } // namespace
 
+constexpr int GF_BATCH_CAPTURE = 8;
 struct gf_batch {
     std::vector<gf_ctx *> members;
     std::vector<GfMemberView> views;
@@ -529,7 +530,8 @@ struct gf_batch {
     long long elements = 0;
     struct Graph {
         std::vector<unsigned> sigs;
-        cudaGraphExec_t exec;
+        cudaGraphExec_t exec; // null: not captured yet
+        int uses;             // before it is captured
     };
     std::vector<Graph> graphs;
     // device copy of the fields gf_batch_inject overwrites (restore point)
@@ -566,7 +568,8 @@ int batch_cuda(cudaError_t e, const char *what) {
     } while (0)
 
 void drop_graphs(gf_batch *b) {
-    for (auto &g : b->graphs) cudaGraphExecDestroy(g.exec);
+    for (auto &g : b->graphs)
+        if (g.exec) cudaGraphExecDestroy(g.exec);
     b->graphs.clear();
 }
 
@@ -872,11 +875,20 @@ int gf_batch_step(gf_batch *b, int nsteps) {
         int chunk = G > 0 ? std::min(G, nsteps - done) : 1;
         std::vector<int> nl, ns;
         std::vector<unsigned> sigs = next_sigs(b, chunk, nl, ns);
+        // (a chunk that has not come up GF_BATCH_CAPTURE times yet is launched
+        // directly: capturing ten steps costs some 0.3 ms)
+        gf_batch::Graph *g = nullptr;
         if (G > 0) {
-            cudaGraphExec_t exec = nullptr;
-            for (auto &g : b->graphs)
-                if (g.sigs == sigs) exec = g.exec;
-            if (!exec) {
+            for (auto &x : b->graphs)
+                if (x.sigs == sigs) g = &x;
+            if (!g) {
+                b->graphs.push_back(gf_batch::Graph{sigs, nullptr, 0});
+                g = &b->graphs.back();
+            }
+            if (!g->exec && ++g->uses < GF_BATCH_CAPTURE) g = nullptr;
+        }
+        if (g) {
+            if (!g->exec) {
                 cudaGraph_t graph;
                 GB_CK(cudaStreamBeginCapture(b->s, cudaStreamCaptureModeThreadLocal));
                 int lrc = GF_OK;
@@ -885,14 +897,15 @@ int gf_batch_step(gf_batch *b, int nsteps) {
                 cudaError_t e = cudaStreamEndCapture(b->s, &graph);
                 if (lrc) return lrc;
                 GB_CK(e);
-                GB_CK(cudaGraphInstantiate(&exec, graph, 0));
+                e = cudaGraphInstantiate(&g->exec, graph, 0);
                 cudaGraphDestroy(graph);
-                b->graphs.push_back(gf_batch::Graph{sigs, exec});
+                if (e != cudaSuccess) g->exec = nullptr;
+                GB_CK(e);
             }
-            GB_CK(cudaGraphLaunch(exec, b->s));
+            GB_CK(cudaGraphLaunch(g->exec, b->s));
         } else {
-            rc = launch_step(b, sigs[0]);
-            if (rc) return rc;
+            for (unsigned sig : sigs)
+                if ((rc = launch_step(b, sig))) return rc;
         }
         for (unsigned sig : sigs)
             for (gf_ctx *c : b->members) gf_ctx_advance(c, sig);

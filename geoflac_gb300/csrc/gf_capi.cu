@@ -22,9 +22,10 @@ namespace {
 
 struct GraphEntry {
     unsigned sig;
-    cudaGraphExec_t exec;
+    cudaGraphExec_t exec; // null: not captured yet
     long long nlaunch;
     int nmarkers; // that change_phase's launch covers (steps with it)
+    int uses;     // before it is captured
 };
 
 } // namespace
@@ -505,7 +506,8 @@ int sidewall_temps(gf_ctx *c) {
 }
 
 void drop_graphs(gf_ctx *c) {
-    for (auto &g : c->graphs) cudaGraphExecDestroy(g.exec);
+    for (auto &g : c->graphs)
+        if (g.exec) cudaGraphExecDestroy(g.exec);
     c->graphs.clear();
 }
 
@@ -600,35 +602,51 @@ void advance_host(gf_ctx *c, unsigned sig) {
     c->nloop = c->nloop + 1;
 }
 
-int run_graph(gf_ctx *c, unsigned sig) {
-    for (size_t k = 0; k < c->graphs.size(); ++k) {
-        GraphEntry &g = c->graphs[k];
-        if (g.sig != sig) continue;
-        // of a captured step only change_phase's launch depends on anything
-        // that changes: it covers the markers there were
-        if ((sig & 2u) && g.nmarkers != c->nmarkers) {
-            cudaGraphExecDestroy(g.exec);
-            c->graphs.erase(c->graphs.begin() + k);
-            break;
-        }
-        GF_CK(cudaGraphLaunch(g.exec, c->s));
-        c->launches += g.nlaunch;
+// One step: launched directly the first GF_CAPTURE_AFTER - 1 times that its
+// signature comes up, then captured and replayed.  Capturing and instantiating
+// a step costs 50 to 90 us, what a replay saves over its launches is 0 to 6 us
+// (a step of 60x20 elements none, of 241x61 6), so a short run is better off
+// without (a new 60x20 mixed state's first ten steps and sample 451 -> 352 us,
+// 1000x300 1265 -> 1090).
+constexpr int GF_CAPTURE_AFTER = 16;
+int run_step(gf_ctx *c, unsigned sig) {
+    GraphEntry *g = nullptr;
+    for (GraphEntry &x : c->graphs)
+        if (x.sig == sig) g = &x;
+    if (!g) {
+        c->graphs.push_back(GraphEntry{sig, nullptr, 0, 0, 0});
+        g = &c->graphs.back();
+    }
+    // of a captured step only change_phase's launch depends on anything
+    // that changes: it covers the markers there were
+    if (g->exec && (sig & 2u) && g->nmarkers != c->nmarkers) {
+        cudaGraphExecDestroy(g->exec);
+        g->exec = nullptr;
+        g->uses = 0;
+    }
+    if (!g->exec && ++g->uses < GF_CAPTURE_AFTER) {
+        enqueue_step(c, sig);
         return GF_OK;
     }
-    cudaGraph_t graph;
-    long long before = c->launches;
-    GF_CK(cudaStreamBeginCapture(c->s, cudaStreamCaptureModeThreadLocal));
-    enqueue_step(c, sig);
-    GF_CK(cudaStreamEndCapture(c->s, &graph));
-    cudaGraphExec_t exec;
-    cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
-    cudaGraphDestroy(graph);
-    if (e != cudaSuccess) return cuda_err(e, "cudaGraphInstantiate");
-    long long n = c->launches - before;
-    c->launches = before;
-    c->graphs.push_back(GraphEntry{sig, exec, n, c->nmarkers});
-    GF_CK(cudaGraphLaunch(exec, c->s));
-    c->launches += n;
+    if (!g->exec) {
+        cudaGraph_t graph;
+        const long long before = c->launches;
+        GF_CK(cudaStreamBeginCapture(c->s, cudaStreamCaptureModeThreadLocal));
+        enqueue_step(c, sig);
+        GF_CK(cudaStreamEndCapture(c->s, &graph));
+        cudaError_t e = cudaGraphInstantiate(&g->exec, graph, 0);
+        cudaGraphDestroy(graph);
+        g->nlaunch = c->launches - before;
+        c->launches = before;
+        if (e != cudaSuccess) {
+            g->exec = nullptr;
+            return cuda_err(e, "cudaGraphInstantiate");
+        }
+        g->nmarkers = c->nmarkers;
+    }
+    GF_CK(cudaGraphLaunch(g->exec, c->s));
+    c->launches += g->nlaunch;
+    c->frc_valid = 0; // (a replay runs none of enqueue_step's bookkeeping)
     return GF_OK;
 }
 
@@ -813,7 +831,8 @@ int gf_create(gf_ctx **out, const gf_params *p, const gf_layout *L, int mode) {
 void gf_destroy(gf_ctx *c) {
     if (!c) return;
     if (c->s) cudaStreamSynchronize(c->s);
-    for (auto &g : c->graphs) cudaGraphExecDestroy(g.exec);
+    for (auto &g : c->graphs)
+        if (g.exec) cudaGraphExecDestroy(g.exec);
     for (void *p : c->allocs) cudaFree(p);
     if (c->pinned) cudaFreeHost(c->pinned);
     if (c->s) cudaStreamDestroy(c->s);
@@ -844,7 +863,8 @@ int gf_set_params(gf_ctx *c, const gf_params *p) {
     else
         GfKernels<float>::plastic_table(launch_of(c));
     GF_CK(cudaGetLastError());
-    for (auto &g : c->graphs) cudaGraphExecDestroy(g.exec);
+    for (auto &g : c->graphs)
+        if (g.exec) cudaGraphExecDestroy(g.exec);
     c->graphs.clear();
     return GF_OK;
 }
@@ -1098,7 +1118,7 @@ static int sync_markers_after_resurface(gf_ctx *c) {
     int nm = c->nmarkers;
     GF_CK(cudaMemcpyAsync(&nm, c->A.nmarkers, sizeof(int), cudaMemcpyDeviceToHost, c->s));
     GF_CK(cudaStreamSynchronize(c->s));
-    c->nmarkers = nm; // (run_graph captures change_phase anew)
+    c->nmarkers = nm; // (run_step takes change_phase's launch anew)
     return GF_OK;
 }
 
@@ -1123,7 +1143,7 @@ int gf_step(gf_ctx *c, int nsteps) {
             int rc = sync_markers_after_resurface(c);
             if (rc) return rc;
         } else {
-            int rc = run_graph(c, sig);
+            int rc = run_step(c, sig);
             if (rc) return rc;
         }
         advance_host(c, sig);

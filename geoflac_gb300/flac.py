@@ -151,7 +151,7 @@ class Flac:
         return events
 
     def step(self, n: int):
-        """n steps, each replayed from a captured CUDA graph."""
+        """n steps, replayed from captured CUDA graphs once they recur."""
         check(self.lib.gf_step(self.ctx, int(n)), "gf_step")
 
     def itest_mesh(self) -> float:

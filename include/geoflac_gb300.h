@@ -291,8 +291,8 @@ int gf_marker2elem(gf_ctx *ctx);
 /* One call of `flac` (src/flac.f90:5-91) with its frequency tests, followed
  * by the bookkeeping of src/par.f90:84-87 (nloop += 1, time += dt). */
 int gf_flac(gf_ctx *ctx);
-/* nsteps calls of gf_flac; the step sequence is captured once into a CUDA
- * graph per frequency phase and replayed. */
+/* nsteps calls of gf_flac; each kind of step (frequency phase) is captured into
+ * a CUDA graph once it has come up 16 times, and replayed from then on. */
 int gf_step(gf_ctx *ctx, int nsteps);
 
 /* itest_mesh (src/rem_test.f90:9-139): minimum triangle angle; sets
@@ -383,7 +383,7 @@ typedef struct gf_batch_config {
     int threads;          /* threads per CTA: 128, 256 or 512 */
     int items_per_thread; /* a tile is threads * items_per_thread items of one member (fewer in a small batch) */
     int ctas_per_sm;      /* >= 1; the phases run at the residency that their registers allow */
-    int graph_steps;      /* steps per captured CUDA graph; 0 = direct launches */
+    int graph_steps;      /* steps per CUDA graph (captured when it has come up 8 times); 0 = direct launches */
 } gf_batch_config;
 int gf_batch_create(gf_batch **out, gf_ctx **members, int n);
 void gf_batch_destroy(gf_batch *b);
