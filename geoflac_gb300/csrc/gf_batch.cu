@@ -455,8 +455,7 @@ __global__ void k_inject_elems(GridArgs g, const int2 *tiles, int ntile, int ipt
 
 // Force imbalance at the free nodes (fl_node.f90 without damping): per member
 // sum |F| and sum (|gravity| + sum over triangles |stress-divergence term|).
-__global__ void k_force_residual(const BatchMember *members, const int2 *tiles, int ntile, int ipt, double *acc,
-                                 double g_acc) {
+__global__ void k_force_residual(const BatchMember *members, const int2 *tiles, int ntile, int ipt, double *acc) {
     for (int t = blockIdx.x; t < ntile; t += gridDim.x) {
         const int2 tl = tiles[t];
         const BatchMember &m = members[tl.x];
@@ -495,7 +494,7 @@ __global__ void k_force_residual(const BatchMember *members, const int2 *tiles, 
                     mag += sqrt(tx * tx + ty * ty);
                 }
             }
-            const double grav = m.A.rmass[n] * g_acc;
+            const double grav = m.A.rmass[n] * m.P->g;
             fy -= grav;
             if (c0 == 1) fx = 0.0; // fixed velocity components carry reactions
             if (c1 == 1) fy = 0.0;
@@ -518,11 +517,11 @@ struct gf_batch {
     std::vector<gf_ctx *> members;
     std::vector<GfMemberView> views;
     BatchMember *d_members = nullptr;
+    std::vector<BatchMember> records; // what d_members holds
     int2 *d_tiles[K_KINDS] = {};
     int ntile[K_KINDS] = {};
     cudaStream_t s = nullptr;
     gf_batch_config cfg{256, 2, 1, 10};
-    double g = 10.0; // gravity of the members (one value; checked at creation)
     int grid = 0;  // CTAs of an element phase
     int sms = 1;   // multiprocessors
     int ipt = 1;   // items per thread of the tile tables (the configuration's, or fewer for a small batch)
@@ -618,7 +617,8 @@ int build_tables(gf_batch *b) {
     return GF_OK;
 }
 
-int upload_members(gf_batch *b) {
+// The members' records as they are now.
+std::vector<BatchMember> member_records(const gf_batch *b) {
     std::vector<BatchMember> h(b->views.size());
     long long e0 = 0;
     for (size_t m = 0; m < h.size(); ++m) {
@@ -636,7 +636,11 @@ int upload_members(gf_batch *b) {
         h[m].e0 = e0;
         e0 += v.d.E;
     }
-    GB_CK(cudaMemcpy(b->d_members, h.data(), h.size() * sizeof(BatchMember), cudaMemcpyHostToDevice));
+    return h;
+}
+int upload_members(gf_batch *b) {
+    b->records = member_records(b);
+    GB_CK(cudaMemcpy(b->d_members, b->records.data(), b->records.size() * sizeof(BatchMember), cudaMemcpyHostToDevice));
     return GF_OK;
 }
 
@@ -758,18 +762,40 @@ std::vector<unsigned> next_sigs(gf_batch *b, int n, std::vector<int> &nl, std::v
     return sigs;
 }
 
-int refresh_views(gf_batch *b) {
-    b->merge = 1;
+// The members as they are now: their calls between two batch calls may have
+// changed their parameters (gf_set_params) or their marker counts (gf_remesh,
+// gf_marker2elem, gf_set_clock).
+int read_views(gf_batch *b) {
     for (size_t m = 0; m < b->members.size(); ++m) {
         int rc = gf_ctx_view(b->members[m], &b->views[m]);
         if (rc) return rc;
-        const gf_params &p = *b->views[m].hp;
-        if (p.istress_therm != 0 || p.nyhydro != 0 || p.itemp_bc == 2) b->merge = 0;
-        // surface processes (diff_topo / resurface) are not part of the
-        // ensemble step
+    }
+    return GF_OK;
+}
+// Whether the members allow the joint launches; surface processes (diff_topo /
+// resurface) are not part of the ensemble step
+int members_merge(const gf_batch *b, int *merge) {
+    *merge = 1;
+    for (const GfMemberView &v : b->views) {
+        const gf_params &p = *v.hp;
+        if (p.istress_therm != 0 || p.nyhydro != 0 || p.itemp_bc == 2) *merge = 0;
         if (p.topo_kappa > 0.0) return GF_ERR_UNSUPPORTED;
     }
     return GF_OK;
+}
+// Device records, tile tables and captured steps follow the members: a member
+// whose markers were added to or whose parameters changed has the records and
+// the marker tiles rebuilt, and a change of the schedule drops what was captured.
+int follow_members(gf_batch *b) {
+    int rc = read_views(b);
+    if (rc) return rc;
+    const std::vector<BatchMember> now = member_records(b);
+    if (std::memcmp(now.data(), b->records.data(), now.size() * sizeof(BatchMember)) == 0) return GF_OK;
+    bool markers = false;
+    for (size_t m = 0; m < now.size(); ++m) markers = markers || now[m].nmarkers != b->records[m].nmarkers;
+    GB_CK(cudaStreamSynchronize(b->s)); // the old records' last readers
+    rc = upload_members(b);
+    return rc || !markers ? rc : build_tables(b);
 }
 
 int check_status(gf_batch *b) {
@@ -797,7 +823,8 @@ int gf_batch_create(gf_batch **out, gf_ctx **members, int n) {
     if (!b) return GF_ERR_NOMEM;
     b->members.assign(members, members + n);
     b->views.resize(n);
-    int rc = refresh_views(b);
+    int rc = read_views(b);
+    if (!rc) rc = members_merge(b, &b->merge);
     for (int m = 0; m < n && !rc; ++m) {
         const GfMemberView &v = b->views[m], &v0 = b->views[0];
         if (v.mode != GF_MODE_MIXED) rc = GF_ERR_UNSUPPORTED;
@@ -808,7 +835,6 @@ int gf_batch_create(gf_batch **out, gf_ctx **members, int n) {
         b->elements += v.d.E;
         if (v.g != b->views[0].g) rc = GF_ERR_ARG;
     }
-    if (!rc) b->g = b->views[0].g;
     if (!rc) rc = batch_cuda(cudaStreamCreateWithFlags(&b->s, cudaStreamNonBlocking), "stream");
     if (!rc) rc = batch_cuda(cudaMalloc(&b->d_members, sizeof(BatchMember) * n), "members");
     if (!rc) rc = batch_cuda(cudaMalloc(&b->means, sizeof(float4) * 2 * (size_t)b->elements), "sampling scratch");
@@ -867,8 +893,11 @@ int gf_batch_step(gf_batch *b, int nsteps) {
     if (!b || nsteps < 0) return GF_ERR_ARG;
     // members must be idle: their own streams may still hold work
     for (const GfMemberView &v : b->views) GB_CK(cudaStreamSynchronize(v.s));
-    int rc = refresh_views(b);
+    int rc = follow_members(b), merge = 0;
+    if (!rc) rc = members_merge(b, &merge);
     if (rc) return rc;
+    if (merge != b->merge) drop_graphs(b); // (captured with the other launches)
+    b->merge = merge;
     int done = 0;
     const int G = b->cfg.graph_steps;
     while (done < nsteps) {
@@ -909,7 +938,7 @@ int gf_batch_step(gf_batch *b, int nsteps) {
         }
         for (unsigned sig : sigs)
             for (gf_ctx *c : b->members) gf_ctx_advance(c, sig);
-        rc = refresh_views(b);
+        rc = read_views(b); // (the steps' counters)
         if (rc) return rc;
         done += chunk;
     }
@@ -965,6 +994,8 @@ int gf_batch_tune(gf_batch *b, int trial_steps, gf_batch_config *best, double *b
 
 int gf_batch_sample(gf_batch *b, float *grid, int H, int W, int phase_id) {
     if (!b || !grid || H < 1 || W < 1 || phase_id < 1) return GF_ERR_ARG;
+    const int rc = follow_members(b);
+    if (rc) return rc;
     GridArgs g{b->d_members, (int)b->members.size(), H, W, phase_id, grid, nullptr};
     if (b->ntile[K_E])
         k_sample_elems<<<b->ntile[K_E], b->cfg.threads, 0, b->s>>>(g, b->d_tiles[K_E], b->ntile[K_E],
@@ -977,6 +1008,8 @@ int gf_batch_sample(gf_batch *b, float *grid, int H, int W, int phase_id) {
 
 int gf_batch_inject(gf_batch *b, const float *grid, int H, int W) {
     if (!b || !grid || H < 2 || W < 2) return GF_ERR_ARG;
+    const int rc = follow_members(b);
+    if (rc) return rc;
     for (gf_ctx *c : b->members) gf_ctx_invalidate_forces(c);
     GridArgs g{b->d_members, (int)b->members.size(), H, W, 1, nullptr, grid};
     const int T = b->cfg.threads, ipt = b->ipt;
@@ -1028,14 +1061,15 @@ int gf_batch_restore(gf_batch *b, const int *members, int count) {
 
 int gf_batch_force_residual(gf_batch *b, double *residual) {
     if (!b || !residual) return GF_ERR_ARG;
+    const int rc = follow_members(b);
+    if (rc) return rc;
     const int n = (int)b->members.size();
     double *acc = nullptr;
     GB_CK(cudaMalloc(&acc, sizeof(double) * 2 * n));
     cudaMemsetAsync(acc, 0, sizeof(double) * 2 * n, b->s);
-    const double g_acc = b->g;
     if (b->ntile[K_N])
         k_force_residual<<<b->ntile[K_N], b->cfg.threads, 0, b->s>>>(b->d_members, b->d_tiles[K_N], b->ntile[K_N],
-                                                                     b->ipt, acc, g_acc);
+                                                                     b->ipt, acc);
     std::vector<double> h(2 * n);
     cudaError_t e = cudaMemcpyAsync(h.data(), acc, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost, b->s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->s);
