@@ -299,10 +299,10 @@ class Fno:
         _ck(self.lib.gf_fno_row(_p(v), kin, _p(Z), _p(self.mat["IW"]), _p(w), _p(bias), act, _p(self.mat["FW"]),
                                 _p(z), _p(vout), _p(Xw), rows, self.cfg.W, 2 * self.cfg.m2, self.s), "row")
 
-    def forward_fused(self, x, wb, train: bool):
+    def forward_fused(self, x, B, wb, train: bool):
         """forward() by the fused kernels"""
         torch, cfg = self.torch, self.cfg
-        B, H, Cc, m2, Q = x.shape[0], cfg.H, cfg.C, cfg.m2, cfg.Q
+        H, Cc, m2, Q = cfg.H, cfg.C, cfg.m2, cfg.Q
         M, rows, bf = B * H * cfg.W, B * H, torch.bfloat16
 
         def new(*shape, dtype=bf):
@@ -352,15 +352,18 @@ class Fno:
         B = x.shape[0]
         M = B * cfg.H * cfg.W
         bf = torch.bfloat16
+        # the kernels read M rows of cin values from x's address on: view()
+        # refuses other sizes and strides, a view of wider rows is copied
+        x = x.view(M, cfg.cin).contiguous()
         wb = {k: self.bf16(self.p[k]) for k in self.p if not k.startswith("R") and not k.endswith("_b")
               and not (k.startswith("b") and k[1:].isdigit())}
         if self.fused:
-            return self.forward_fused(x, wb, train)
+            return self.forward_fused(x, B, wb, train)
         # inference keeps only the BF16 activations (no FP32 copies of the
         # pre-activations, which only the backward pass reads)
         z = torch.empty((M, cfg.C), dtype=torch.float32, device="cuda") if train else None
         v = torch.empty((M, cfg.C), dtype=bf, device="cuda")
-        self.mm(x.view(M, cfg.cin), wb["lift_w"], z, M, cfg.C, cfg.cin, bias=self.p["lift_b"], aux=v, keep_c=train)
+        self.mm(x, wb["lift_w"], z, M, cfg.C, cfg.cin, bias=self.p["lift_b"], aux=v, keep_c=train)
         saved = {"x": x, "v": [], "z": [], "spec": [], "wb": wb}
         for l in range(cfg.layers):
             s_cl, sp = self.spectral(v.view(B, cfg.H, cfg.W, cfg.C), l, B, train)
@@ -465,7 +468,7 @@ class Fno:
                                    _p(dZ) if l else None, rows, W, K2, s), "row_bwd")
             dz, dn = dn, dz
         self.colsum_blocked(df, self.g["lift_b"], M, Cc)
-        self.wgrad_fused(dz, Cc, sv["x"].reshape(M, cfg.cin), cfg.cin, M, self.g["lift_w"])
+        self.wgrad_fused(dz, Cc, sv["x"], cfg.cin, M, self.g["lift_w"])
         self.saved = None
         return self.g
 
@@ -515,7 +518,7 @@ class Fno:
             self.mm(dz_b, wT, dv_spec.view(M, cfg.C), M, cfg.C, cfg.C, beta=1.0)
             dv = dv_spec.view(M, cfg.C)
         dz0_b = self.bf16(dv)
-        self.wgrad(dz0_b, sv["x"].reshape(M, cfg.cin), M, cfg.C, cfg.cin, self.g["lift_w"])
+        self.wgrad(dz0_b, sv["x"], M, cfg.C, cfg.cin, self.g["lift_w"])
         self.colsum(dv, self.g["lift_b"], M, cfg.C)
         self.saved = None
         return self.g
