@@ -414,25 +414,25 @@ __global__ void k_gather_rows(const uint32_t *__restrict__ src, uint32_t *__rest
 
 #define FNO_RET(s) return cudaGetLastError() == cudaSuccess ? GF_FNO_OK : GF_FNO_ERR_CUDA
 
+// Column sums in two stages through COLSUM_NB partial rows: the caller's `part`,
+// or, without one, scratch allocated in the stream's order for this call, so that
+// calls on several streams, threads or devices share nothing.
+constexpr int COLSUM_NB = 1024;
 template <class T, bool BLK = false>
-int run_colsum(const T *X, float *out, long long rows, int cols, int accum, void *stream) {
+int run_colsum(const T *X, float *part, float *out, long long rows, int cols, int accum, void *stream) {
     if (!X || !out || rows < 1 || cols < 1) return GF_FNO_ERR_ARG;
     if (BLK && (rows % 32 || rows < 4096 || cols % 8 || cols > TB || TB % cols)) return GF_FNO_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     if (cols <= TB && TB % cols == 0 && rows >= 4096) {
-        // two stages through a fixed scratch of 1024 partial rows
-        static float *part = nullptr;
-        static int part_cols = 0;
-        const int nb = 1024;
-        if (!part || part_cols < cols) {
-            if (part) cudaFree(part);
-            part = nullptr;
-            if (cudaMalloc(&part, sizeof(float) * nb * TB) != cudaSuccess) return GF_FNO_ERR_CUDA;
-            part_cols = TB;
+        float *own = nullptr;
+        if (!part) {
+            if (cudaMallocAsync(&own, sizeof(float) * COLSUM_NB * cols, st) != cudaSuccess) return GF_FNO_ERR_CUDA;
+            part = own;
         }
-        long long rpb = (rows + nb - 1) / nb;
-        k_colsum_part<T, BLK><<<nb, TB, 0, st>>>(X, part, rows, cols, rpb);
-        sum_batches(part, out, nb, cols, accum, st);
+        const long long rpb = (rows + COLSUM_NB - 1) / COLSUM_NB;
+        k_colsum_part<T, BLK><<<COLSUM_NB, TB, 0, st>>>(X, part, rows, cols, rpb);
+        sum_batches(part, out, COLSUM_NB, cols, accum, st);
+        if (own && cudaFreeAsync(own, st) != cudaSuccess) return GF_FNO_ERR_CUDA;
     } else {
         k_colsum<<<(unsigned)cols, TB, 0, st>>>(X, out, rows, cols, accum);
     }
@@ -535,13 +535,23 @@ int gf_fno_modes_grad(const float *dRm, float *dR, int modes, int C, void *strea
 }
 
 int gf_fno_colsum(const float *X, float *out, long long rows, int cols, int accum, void *stream) {
-    return run_colsum(X, out, rows, cols, accum, stream);
+    return run_colsum(X, nullptr, out, rows, cols, accum, stream);
 }
 int gf_fno_colsum_blocked(const float *X, float *out, long long rows, int cols, int accum, void *stream) {
-    return run_colsum<float, true>(X, out, rows, cols, accum, stream);
+    return run_colsum<float, true>(X, nullptr, out, rows, cols, accum, stream);
 }
 int gf_fno_colsum_bf16(const void *X, float *out, long long rows, int cols, int accum, void *stream) {
-    return run_colsum((const __nv_bfloat16 *)X, out, rows, cols, accum, stream);
+    return run_colsum((const __nv_bfloat16 *)X, nullptr, out, rows, cols, accum, stream);
+}
+int gf_fno_colsum_with(const void *X, int layout, float *part, float *out, long long rows, int cols, int accum,
+                       void *stream) {
+    if (!part) return GF_FNO_ERR_ARG;
+    switch (layout) {
+    case 0: return run_colsum((const float *)X, part, out, rows, cols, accum, stream);
+    case 1: return run_colsum((const __nv_bfloat16 *)X, part, out, rows, cols, accum, stream);
+    case 2: return run_colsum<float, true>((const float *)X, part, out, rows, cols, accum, stream);
+    default: return GF_FNO_ERR_ARG;
+    }
 }
 
 int gf_fno_sum_batches(const float *src, float *dst, int nb, long long n, int accum, void *stream) {

@@ -46,7 +46,7 @@ def _lib():
         "gf_fno_spec_combine_bwd": [vp, vp, i, i, i, i, vp],
         "gf_fno_expand_modes": [vp, vp, vp, i, i, vp],
         "gf_fno_modes_grad": [vp, vp, i, i, vp],
-        "gf_fno_colsum": [vp, vp, ll, i, i, vp],
+        "gf_fno_colsum_with": [vp, i, vp, vp, ll, i, i, vp],
         "gf_fno_sum_batches": [vp, vp, i, ll, i, vp],
         "gf_fno_adam": [vp, vp, vp, vp, ll, f, f, f, f, i, f, vp],
         "gf_fno_mse": [vp, vp, vp, i, vp, ll, f, vp],
@@ -62,8 +62,6 @@ def _lib():
         "gf_fno_modes": [vp, vp, vp, i, i, vp],
         "gf_fno_inv_h": [vp, vp, vp, i, i, i, i, vp],
         "gf_fno_proj": [vp, vp, vp, vp, vp, vp, vp, vp, i, i, vp],
-        "gf_fno_colsum_bf16": [vp, vp, ll, i, i, vp],
-        "gf_fno_colsum_blocked": [vp, vp, ll, i, i, vp],
         "gf_fno_proj_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, vp],
         "gf_fno_row_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, vp],
         "gf_fno_inv_h_bwd": [vp, vp, vp, i, i, i, i, vp],
@@ -232,11 +230,11 @@ class Fno:
         _ck(self.lib.gf_fno_gelu_bwd(_p(z), _p(da), int(da.dtype == self.torch.bfloat16), _p(dz), _p(dz_b),
                                      z.numel(), self.s), "gelu_bwd")
 
-    def colsum_blocked(self, X, out, rows, cols):
-        _ck(self.lib.gf_fno_colsum_blocked(_p(X), _p(out), rows, cols, 0, self.s), "colsum")
-
-    def colsum(self, X, out, rows, cols):
-        _ck(self.lib.gf_fno_colsum(_p(X), _p(out), rows, cols, 0, self.s), "colsum")
+    def colsum(self, X, out, rows, cols, blocked=False):
+        """out = column sums of X (FP32 or BF16 rows, or FP32 in blocks)"""
+        layout = 2 if blocked else int(X.dtype == self.torch.bfloat16)
+        part = self.torch.empty(1024 * cols, dtype=self.torch.float32, device="cuda")
+        _ck(self.lib.gf_fno_colsum_with(_p(X), layout, _p(part), _p(out), rows, cols, 0, self.s), "colsum")
 
     @staticmethod
     def wgrad_chunks(M):
@@ -450,14 +448,14 @@ class Fno:
         dV, dU = new(cfg.modes, B, 2 * Cc), new(cfg.modes, B, 2 * Cc)
         d2 = dout.reshape(M, cfg.cout)
         self.wgrad_fused(sv["h"], cfg.P, d2, cfg.cout, M, self.g["p2_w"], 1)
-        _ck(lib.gf_fno_colsum_bf16(_p(d2), _p(self.g["p2_b"]), M, cfg.cout, 0, s), "colsum")
+        self.colsum(d2, self.g["p2_b"], M, cfg.cout)
         _ck(lib.gf_fno_proj_bwd(_p(d2), _p(sv["zp"]), _p(wb["p1_w"]), _p(wb["p2_w"]), _p(IWT), _p(dzp), _p(df1),
                                 _p(dz), _p(df), _p(dZ), rows, W, K2, s), "proj_bwd")
-        self.colsum_blocked(df1, self.g["p1_b"], M, cfg.P)
+        self.colsum(df1, self.g["p1_b"], M, cfg.P, blocked=True)
         self.wgrad_fused(dzp, cfg.P, sv["vL"], Cc, M, self.g["p1_w"])
         for l in reversed(range(cfg.layers)):
             # dz: gradient of layer l's pre-activations, dZ: its transform along W
-            self.colsum_blocked(df, self.g[f"b{l}"], M, Cc)
+            self.colsum(df, self.g[f"b{l}"], M, Cc, blocked=True)
             self.wgrad_fused(dz, Cc, sv["v"][l], Cc, M, self.g[f"w{l}"])
             _ck(lib.gf_fno_inv_h_bwd(_p(dZ), _p(self.mat["IHT"]), _p(dV), B, H, m2, Q, s), "inv_h_bwd")
             _ck(lib.gf_fno_modes_bwd(_p(dV), _p(sv["spec"][l][0]), _p(self.p[f"R{l}"]), _p(dU), _p(self.g[f"R{l}"]),
@@ -467,7 +465,7 @@ class Fno:
             _ck(lib.gf_fno_row_bwd(_p(dz), _p(dXw), _p(self.mat["FW"]), _p(wb[f"w{l}"]), _p(z), _p(IWT), _p(dn), _p(df),
                                    _p(dZ) if l else None, rows, W, K2, s), "row_bwd")
             dz, dn = dn, dz
-        self.colsum_blocked(df, self.g["lift_b"], M, Cc)
+        self.colsum(df, self.g["lift_b"], M, Cc, blocked=True)
         self.wgrad_fused(dz, Cc, sv["x"], cfg.cin, M, self.g["lift_w"])
         self.saved = None
         return self.g

@@ -64,6 +64,11 @@ int gf_fno_colsum_bf16(const void *X, float *out, long long rows, int cols, int 
 /* X in blocks of 32 rows x 8 columns, [rows / 32][cols / 8][32][8] (rows >= 4096,
  * a multiple of 32; cols a multiple of 8 that divides 256): gf_fno_colsum's sums. */
 int gf_fno_colsum_blocked(const float *X, float *out, long long rows, int cols, int accum, void *stream);
+/* The same sums with the caller's scratch of 1024 x cols floats (the others
+ * allocate theirs in the stream's order): layout 0 gf_fno_colsum, 1
+ * gf_fno_colsum_bf16, 2 gf_fno_colsum_blocked. */
+int gf_fno_colsum_with(const void *X, int layout, float *part, float *out, long long rows, int cols, int accum,
+                       void *stream);
 int gf_fno_sum_batches(const float *src, float *dst, int nb, long long n, int accum, void *stream);
 /* Adam (bias-corrected, decoupled from the loss scale), step counts from 1. */
 int gf_fno_adam(float *p, const float *g, float *m, float *v, long long n, float lr, float b1, float b2, float eps,
