@@ -347,7 +347,9 @@ __global__ void k_add(const float *__restrict__ x, const float *__restrict__ y, 
 // TB points of one member (`nb` CTAs each): their 36-byte records are staged in
 // shared memory, the member's parameters are normalised once, and a point's
 // 32 bytes leave in two stores (one thread a point with 2-byte stores and 13
-// divisions: 246 us for 64 members, now 43 us).
+// divisions: 246 us for 64 members, now 43 us), or, VEC = false, value by value
+// to an `out` that is not 16-byte aligned.
+template <bool VEC>
 __global__ void __launch_bounds__(TB) k_pack_input(const float *__restrict__ raw, const float *__restrict__ prm,
                                                    const float *__restrict__ stats, __nv_bfloat16 *__restrict__ out,
                                                    int H, int W, unsigned nb) {
@@ -373,9 +375,15 @@ __global__ void __launch_bounds__(TB) k_pack_input(const float *__restrict__ raw
     __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(o);
 #pragma unroll
     for (int c = 0; c < 8; ++c) h[c] = __floats2bfloat162_rn(v[2 * c], v[2 * c + 1]);
-    uint4 *dst = reinterpret_cast<uint4 *>(out + (base + t) * 16);
-    dst[0] = o[0];
-    dst[1] = o[1];
+    if constexpr (VEC) {
+        uint4 *dst = reinterpret_cast<uint4 *>(out + (base + t) * 16);
+        dst[0] = o[0];
+        dst[1] = o[1];
+    } else {
+        const __nv_bfloat16 *src = reinterpret_cast<const __nv_bfloat16 *>(o);
+#pragma unroll
+        for (int c = 0; c < 16; ++c) out[(base + t) * 16 + c] = src[c];
+    }
 }
 
 // training target: normalised increments (y - x - mean_d) / std_d in 9 of 16 channels
@@ -448,7 +456,8 @@ int gf_fno_pack_input(const float *raw, const float *params, const float *stats,
                       void *stream) {
     if (!raw || !params || !stats || !out || n < 1 || H < 1 || W < 1) return GF_FNO_ERR_ARG;
     const unsigned nb = nblk((long long)H * W);
-    k_pack_input<<<nb * (unsigned)n, TB, 0, (cudaStream_t)stream>>>(raw, params, stats, (__nv_bfloat16 *)out, H, W, nb);
+    auto kern = ((uintptr_t)out & 15) == 0 ? k_pack_input<true> : k_pack_input<false>;
+    kern<<<nb * (unsigned)n, TB, 0, (cudaStream_t)stream>>>(raw, params, stats, (__nv_bfloat16 *)out, H, W, nb);
     FNO_RET(stream);
 }
 
