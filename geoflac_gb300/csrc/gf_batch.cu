@@ -176,24 +176,28 @@ __device__ __forceinline__ void lerp_index(float f, int n, int &i0, float &w) {
     w = f - (float)i0;
 }
 
-__device__ double elem_value(const BatchMember &m, long long e, int ch, int phase_id) {
+// a float as a double by integer operations; only subnormals, infinities and
+// NaNs take the conversion instruction (a slot of the FP64 pipe)
+__device__ __forceinline__ double sample_f2d(float f) {
+    const unsigned u = __float_as_uint(f), e = (u >> 23) & 0xffu;
+    if (e - 1u >= 254u && (u << 1) != 0u) return (double)f;
+    return gfk::gf_f2d(f);
+}
+// an element's mean of stress component c over its triangles, as stored (normal
+// components exclude -p_ref)
+__device__ __forceinline__ double mean_stress(const BatchMember &m, long long e, int c) {
     const float *st = (const float *)m.A.stress0;
-    const GfDims &d = m.d;
-    const double pr = m.A.p_ref[e];
+    double s = gfk::gf_plus_pzero(sample_f2d(st[gf_s(m.d, e, c, 0)]));
+#pragma unroll
+    for (int k = 1; k < 4; ++k) s = s + sample_f2d(st[gf_s(m.d, e, c, k)]);
+    return gfk::gf_scale<-2>(s);
+}
+__device__ double elem_value(const BatchMember &m, long long e, int ch, int phase_id) {
     switch (ch) {
-    case 2: case 3: {
-        int c = ch - 2;
-        double s = 0.0;
-        for (int k = 0; k < 4; ++k) s += (double)st[gf_s(d, e, c, k)];
-        return 0.25 * s - pr;
-    }
-    case 4: {
-        double s = 0.0;
-        for (int k = 0; k < 4; ++k) s += (double)st[gf_s(d, e, 2, k)];
-        return 0.25 * s;
-    }
+    case 2: case 3: return mean_stress(m, e, ch - 2) - m.A.p_ref[e];
+    case 4: return mean_stress(m, e, 2);
     case 5: return (double)((const float *)m.A.aps)[e];
-    default: return m.A.phase_ratio[gf_pr(d, e, phase_id - 1)];
+    default: return m.A.phase_ratio[gf_pr(m.d, e, phase_id - 1)];
     }
 }
 
@@ -207,12 +211,15 @@ __device__ double node_value(const BatchMember &m, long long n, int j, int ch) {
     }
 }
 
-// Sampling runs on FP32 pairs (hi + lo, about 2^-46 relative): the values are
-// FP32 fields, hi/lo splits or FP64 numbers split by integer operations, and
-// the bilinear sums in pairs leave only the rounding of the FP32 result.  In
-// FP64 (200 operations a point, the elements' means anew at each of a point's
-// corners) the FP64 pipe took 1.23 ms for 64 members on a 128 x 384 grid; now
-// about 0.5 ms, ten steps and a sample of 64 members 7.92 -> 7.27 ms.
+// A sampled value is the FP64 bilinear sum rounded to FP32 (sample_plain).  Nearly
+// all of them are decided without the FP64 pipe: the sum is formed in FP32 pairs
+// (hi + lo) with an error below 2^-42 of the largest corner, and where adding and
+// subtracting that much rounds to the same float, that float is the result.  Only
+// the others (a sum next to a rounding boundary, cancelling corners, values too
+// small for pairs, infinities and NaNs) are evaluated in FP64.  All values in FP64
+// (200 operations a point, the elements' means anew at each of a point's corners)
+// took 1.23 ms for 64 members on a 128 x 384 grid, with the means formed once and
+// half of the products on the integer pipes 0.38 ms, this 0.19 ms.
 struct ff {
     float h, l;
 };
@@ -220,66 +227,65 @@ __device__ __forceinline__ ff ff_two(float a, float b) { // a + b exactly
     const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
     return ff{s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t))};
 }
-__device__ __forceinline__ ff ff_plus(ff a, ff b) {
-    const ff s = ff_two(a.h, b.h);
-    return ff{s.h, s.l + (a.l + b.l)};
+// v a + w b for weights v, w in [0, 1] of sum 1 (to a rounding)
+__device__ __forceinline__ ff ff_mix(float v, ff a, float w, ff b) {
+    const float p = __fmul_rn(v, a.h), q = __fmul_rn(w, b.h);
+    const float ep = fmaf(v, a.l, fmaf(v, a.h, -p)), eq = fmaf(w, b.l, fmaf(w, b.h, -q));
+    const ff s = ff_two(p, q);
+    return ff{s.h, __fadd_rn(s.l, __fadd_rn(ep, eq))};
 }
-__device__ __forceinline__ ff ff_minus(ff a, ff b) { return ff_plus(a, ff{-b.h, -b.l}); }
-// a + w d
-__device__ __forceinline__ ff ff_madd(float w, ff d, ff a) {
-    const float p = __fmul_rn(w, d.h);
-    const float e = fmaf(w, d.l, fmaf(w, d.h, -p));
-    return ff_plus(a, ff{p, e});
+// The bilinear sum rounded to FP32; false where the rounding is not certain.
+// With corners up to M whose lo parts are below 2^-23 M and err by 2^-47 M, the
+// roundings of the lo parts add up to 14 x 2^-47 M: 6 in a sum along x (the
+// corners' 1, products' ends 1.5, additions 1.5 and 2; lo parts then up to twice as
+// large), 8 in the one along z (2.5, 2.5, 3).  The bound taken, 32, leaves room for
+// those of the test itself and of the FP64 sum.  `floor`: what the corners' splits
+// may have lost to underflow.
+__device__ __forceinline__ bool ff_bilinear(ff a, ff b, ff c, ff d, float wx, float wy, float floor, float &out) {
+    const float vx = 1 - wx, vy = 1 - wy;
+    const ff r = ff_mix(vy, ff_mix(vx, a, wx, b), wy, ff_mix(vx, c, wx, d));
+    const ff n = ff_two(r.h, r.l);
+    const float m = fmaxf(fmaxf(fabsf(a.h), fabsf(b.h)), fmaxf(fabsf(c.h), fabsf(d.h)));
+    const float eps = fmaf(m, 0x1p-42f, floor);
+    out = __fadd_rn(n.h, __fadd_rn(n.l, eps));
+    return out == __fadd_rn(n.h, __fsub_rn(n.l, eps)); // (false for NaN)
 }
-__device__ __forceinline__ float ff_bilinear(ff a, ff b, ff c, ff d, float wx, float wy) {
-    const ff t = ff_madd(wx, ff_minus(b, a), a), u = ff_madd(wx, ff_minus(d, c), c);
-    const ff r = ff_madd(wy, ff_minus(u, t), t);
-    return r.h + r.l;
-}
-// the 48 leading bits of a double, truncated, without the FP64 pipe (values
-// outside the float range give a pair whose sum is not finite or zero)
+// the 48 leading bits of a double, truncated, without the FP64 pipe; NaN where a
+// pair cannot hold them (below 2^-78 but for zero, from 2^128 on)
 __device__ __forceinline__ ff ff_of(double x) {
     unsigned lo, hi;
     gfk::gf_dsplit(x, lo, hi);
-    const int e = (int)((hi >> 20) & 0x7ffu) - 1023 + 127;
-    if (e >= 255) return ff{__uint_as_float(0x7fc00000u), 0.0f};
-    if (e <= 0) return ff{0.0f, 0.0f};
+    const unsigned e = ((hi >> 20) & 0x7ffu) - 1023u + 127u;
+    if (e - 49u >= 206u) return ff{__uint_as_float(((hi << 1) | lo) == 0u ? 0u : 0x7fc00000u), 0.0f};
     const unsigned sg = hi & 0x80000000u;
-    const float h = __uint_as_float(sg | ((unsigned)e << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
+    const float h = __uint_as_float(sg | (e << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
     const float l = __uint2float_rz((lo >> 5) & 0xffffffu); // the next 24 bits, scaled by 2^(e - 127 - 47)
-    return ff{h, e > 48 ? l * __uint_as_float(sg | ((unsigned)(e - 47) << 23)) : 0.0f};
+    return ff{h, l * __uint_as_float(sg | ((e - 47u) << 23))};
 }
 
+// the same for a float
+__device__ __forceinline__ ff ff_of(float x) { return ff{fabsf(x) >= 0x1p-78f || x == 0.0f ? x : __uint_as_float(0x7fc00000u), 0.0f}; }
+
 // The elements' share of a sample: total stresses (mean of the four
-// triangles) and the phase fraction as pairs, once per element.
+// triangles, as elem_value forms them) and the phase fraction as pairs, once
+// per element.
 __global__ void k_sample_elems(GridArgs g, const int2 *tiles, int ntile, int ipt, float4 *means) {
     for (int t = blockIdx.x; t < ntile; t += gridDim.x) {
         const int2 tl = tiles[t];
         const BatchMember &m = g.members[tl.x];
-        const GfDims &d = m.d;
-        const float *st = (const float *)m.A.stress0;
         for (int r = 0; r < ipt; ++r) {
             const int e = tl.y + r * (int)blockDim.x + (int)threadIdx.x;
-            if (e >= d.E) continue;
-            ff s[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                ff v = ff_two(st[gf_s(d, e, c, 0)], st[gf_s(d, e, c, 1)]);
-                v = ff_plus(v, ff_two(st[gf_s(d, e, c, 2)], st[gf_s(d, e, c, 3)]));
-                s[c] = ff{0.25f * v.h, 0.25f * v.l};
-            }
-            const ff p = ff_of(m.A.p_ref[e]);
-            s[0] = ff_minus(s[0], p);
-            s[1] = ff_minus(s[1], p);
-            const ff f = ff_of(m.A.phase_ratio[gf_pr(d, e, g.phase_id - 1)]);
+            if (e >= m.d.E) continue;
+            const ff xx = ff_of(elem_value(m, e, 2, 0)), zz = ff_of(elem_value(m, e, 3, 0)),
+                     xz = ff_of(elem_value(m, e, 4, 0)), f = ff_of(elem_value(m, e, 7, g.phase_id));
             float4 *o = means + 2 * (m.e0 + e);
-            o[0] = make_float4(s[0].h, s[0].l, s[1].h, s[1].l);
-            o[1] = make_float4(s[2].h, s[2].l, f.h, f.l);
+            o[0] = make_float4(xx.h, xx.l, zz.h, zz.l);
+            o[1] = make_float4(xz.h, xz.l, f.h, f.l);
         }
     }
 }
 
-// A value that is not finite in pairs, by the plain FP64 sum
+// The value itself: FP64 corners, weights and sums
 __device__ __noinline__ float sample_plain(const BatchMember &m, int ch, int phase_id, int j0, int j1, int i0, int i1,
                                            float wx, float wy) {
     double v[4];
@@ -325,16 +331,21 @@ __global__ void __launch_bounds__(256) k_sample(GridArgs g, const float4 *means,
             float wx;
             lerp_index(at(gx, nx, g.W), nx, i0, wx);
             const int a = gf_node(d, jn, i0), c = a + 1, bb = a + nz, dd = bb + 1; // (j,i), (j+1,i), (j,i+1), (j+1,i+1)
-            auto pairs = [&](const float *h, const float *l, int off) {
-                return ff_bilinear(ff{h[off + a], l[off + a]}, ff{h[off + bb], l[off + bb]}, ff{h[off + c], l[off + c]},
-                                   ff{h[off + dd], l[off + dd]}, wx, wyn);
-            };
             float v[SAMPLE_CH];
-            v[0] = pairs(A.vel_hi, A.vel_lo, 0);
-            v[1] = pairs(A.vel_hi, A.vel_lo, N);
-            v[6] = pairs(A.temp_hi, A.temp_lo, 0);
+            unsigned sure = 0u; // channels decided in pairs
+            auto put = [&](int ch, ff p, ff r, ff q, ff w, float fx, float fy, float floor) {
+                if (ff_bilinear(p, r, q, w, fx, fy, floor, v[ch])) sure |= 1u << ch;
+            };
+            // (a hi/lo split loses what lies below 2^-126)
+            auto nodes = [&](int ch, const float *h, const float *l, int off) {
+                put(ch, ff{h[off + a], l[off + a]}, ff{h[off + bb], l[off + bb]}, ff{h[off + c], l[off + c]},
+                    ff{h[off + dd], l[off + dd]}, wx, wyn, 0x1p-112f);
+            };
+            nodes(0, A.vel_hi, A.vel_lo, 0);
+            nodes(1, A.vel_hi, A.vel_lo, N);
+            nodes(6, A.temp_hi, A.temp_lo, 0);
             const double *z = A.cord + N;
-            v[8] = ff_bilinear(ff_of(z[a] - r0), ff_of(z[bb] - r0), ff_of(z[c] - r1), ff_of(z[dd] - r1), wx, wyn);
+            put(8, ff_of(z[a] - r0), ff_of(z[bb] - r0), ff_of(z[c] - r1), ff_of(z[dd] - r1), wx, wyn, 0.0f);
             int ie;
             float wxe;
             lerp_index(at(gx, nx, g.W) - 0.5f, nx - 1, ie, wxe);
@@ -342,23 +353,23 @@ __global__ void __launch_bounds__(256) k_sample(GridArgs g, const float4 *means,
             const int ea = gf_elem(d, je, ie), eb = gf_elem(d, je, ie1), ec = gf_elem(d, je1, ie), ed = gf_elem(d, je1, ie1);
             {
                 const float4 p = mean[2 * ea], r = mean[2 * eb], s = mean[2 * ec], t = mean[2 * ed];
-                v[2] = ff_bilinear(ff{p.x, p.y}, ff{r.x, r.y}, ff{s.x, s.y}, ff{t.x, t.y}, wxe, wye);
-                v[3] = ff_bilinear(ff{p.z, p.w}, ff{r.z, r.w}, ff{s.z, s.w}, ff{t.z, t.w}, wxe, wye);
+                put(2, ff{p.x, p.y}, ff{r.x, r.y}, ff{s.x, s.y}, ff{t.x, t.y}, wxe, wye, 0.0f);
+                put(3, ff{p.z, p.w}, ff{r.z, r.w}, ff{s.z, s.w}, ff{t.z, t.w}, wxe, wye, 0.0f);
             }
             {
                 const float4 p = mean[2 * ea + 1], r = mean[2 * eb + 1], s = mean[2 * ec + 1], t = mean[2 * ed + 1];
-                v[4] = ff_bilinear(ff{p.x, p.y}, ff{r.x, r.y}, ff{s.x, s.y}, ff{t.x, t.y}, wxe, wye);
-                v[7] = ff_bilinear(ff{p.z, p.w}, ff{r.z, r.w}, ff{s.z, s.w}, ff{t.z, t.w}, wxe, wye);
+                put(4, ff{p.x, p.y}, ff{r.x, r.y}, ff{s.x, s.y}, ff{t.x, t.y}, wxe, wye, 0.0f);
+                put(7, ff{p.z, p.w}, ff{r.z, r.w}, ff{s.z, s.w}, ff{t.z, t.w}, wxe, wye, 0.0f);
             }
             const float *aps = (const float *)A.aps;
-            v[5] = ff_bilinear(ff{aps[ea], 0.0f}, ff{aps[eb], 0.0f}, ff{aps[ec], 0.0f}, ff{aps[ed], 0.0f}, wxe, wye);
+            put(5, ff_of(aps[ea]), ff_of(aps[eb]), ff_of(aps[ec]), ff_of(aps[ed]), wxe, wye, 0.0f);
 #pragma unroll
-            for (int ch = 0; ch < SAMPLE_CH; ++ch) {
+            for (int ch = 0; ch < SAMPLE_CH; ++ch) o[ch] = v[ch];
+            for (unsigned rest = 0x1ffu & ~sure; rest; rest &= rest - 1u) {
+                const int ch = __ffs(rest) - 1;
                 const bool node = ch == 0 || ch == 1 || ch == 6 || ch == 8;
-                if (!isfinite(v[ch]))
-                    v[ch] = node ? sample_plain(m, ch, g.phase_id, jn, jn + 1, i0, i0 + 1, wx, wyn)
-                                 : sample_plain(m, ch, g.phase_id, je, je1, ie, ie1, wxe, wye);
-                o[ch] = v[ch];
+                o[ch] = node ? sample_plain(m, ch, g.phase_id, jn, jn + 1, i0, i0 + 1, wx, wyn)
+                             : sample_plain(m, ch, g.phase_id, je, je1, ie, ie1, wxe, wye);
             }
         }
     }
