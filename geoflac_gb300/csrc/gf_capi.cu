@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -877,14 +878,18 @@ int gf_get_params(gf_ctx *c, gf_params *p) {
 
 int gf_set_clock(gf_ctx *c, const gf_clock *k) {
     if (!c || !k) return GF_ERR_ARG;
-    GF_CK(cudaMemcpyAsync(c->pinned, c->dC, sizeof(DevClock), cudaMemcpyDeviceToHost, c->s));
     GF_CK(cudaStreamSynchronize(c->s));
+    // The caller's scalars alone, which lead the structure: this copy may still
+    // be on its way when a batch, on a stream of its own, sets the status word.
+    // (The buffer is next written in this stream's order, or by the host after
+    // a wait for it.)
+    constexpr size_t bytes = offsetof(DevClock, r_dlmin);
+    static_assert(bytes == 9 * sizeof(double), "the scalars of gf_clock");
     DevClock &C = *(DevClock *)c->pinned;
     C.dt = k->dt; C.time = k->time; C.dtavg = k->dtavg; C.dt_elastic = k->dt_elastic;
     C.dt_maxwell = k->dt_maxwell; C.dtmax_therm = k->dtmax_therm; C.frac = k->frac;
     C.vel_max = k->vel_max; C.dlmin = k->dlmin;
-    // (the buffer is next written in this stream's order, or by the host after a wait for it)
-    GF_CK(cudaMemcpyAsync(c->dC, c->pinned, sizeof(DevClock), cudaMemcpyHostToDevice, c->s));
+    GF_CK(cudaMemcpyAsync(c->dC, c->pinned, bytes, cudaMemcpyHostToDevice, c->s));
     c->nloop = k->nloop;
     c->nsrate = k->nsrate;
     c->nmarkers = k->nmarkers;
