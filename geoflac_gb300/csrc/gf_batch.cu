@@ -532,6 +532,7 @@ struct gf_batch {
     int2 *d_tiles[K_KINDS] = {};
     int ntile[K_KINDS] = {};
     cudaStream_t s = nullptr;
+    std::shared_ptr<GfEvent> done = std::make_shared<GfEvent>(); // behind a call that returns before its kernels end
     gf_batch_config cfg{256, 2, 1, 10};
     int grid = 0;  // CTAs of an element phase
     int sms = 1;   // multiprocessors
@@ -794,11 +795,31 @@ int members_merge(const gf_batch *b, int *merge) {
     }
     return GF_OK;
 }
+// Order between the batch's stream and the members'.  A call first waits for
+// what the members' own calls enqueued (calls with gf_set_sync(0), gf_set_clock);
+// behind a call that returns before its kernels end, the members' next changes of
+// their state wait for these.
+int settle(const gf_batch *b) {
+    for (gf_ctx *c : b->members) {
+        const int rc = gf_ctx_settle(c, b->s, b->done.get());
+        if (rc) return rc;
+    }
+    return GF_OK;
+}
+int release(gf_batch *b) {
+    GB_CK(cudaEventRecord(b->done->e, b->s));
+    for (gf_ctx *c : b->members) {
+        const int rc = gf_ctx_read_until(c, b->done);
+        if (rc) return rc;
+    }
+    return GF_OK;
+}
 // Device records, tile tables and captured steps follow the members: a member
 // whose markers were added to or whose parameters changed has the records and
 // the marker tiles rebuilt, and a change of the schedule drops what was captured.
 int follow_members(gf_batch *b) {
-    int rc = read_views(b);
+    int rc = settle(b);
+    if (!rc) rc = read_views(b);
     if (rc) return rc;
     const std::vector<BatchMember> now = member_records(b);
     if (std::memcmp(now.data(), b->records.data(), now.size() * sizeof(BatchMember)) == 0) return GF_OK;
@@ -847,6 +868,7 @@ int gf_batch_create(gf_batch **out, gf_ctx **members, int n) {
         if (v.g != b->views[0].g) rc = GF_ERR_ARG;
     }
     if (!rc) rc = batch_cuda(cudaStreamCreateWithFlags(&b->s, cudaStreamNonBlocking), "stream");
+    if (!rc) rc = batch_cuda(cudaEventCreateWithFlags(&b->done->e, cudaEventDisableTiming), "event");
     if (!rc) rc = batch_cuda(cudaMalloc(&b->d_members, sizeof(BatchMember) * n), "members");
     if (!rc) rc = batch_cuda(cudaMalloc(&b->means, sizeof(float4) * 2 * (size_t)b->elements), "sampling scratch");
     if (!rc) rc = batch_cuda(cudaMalloc(&b->status, sizeof(int) * n), "status");
@@ -1014,7 +1036,7 @@ int gf_batch_sample(gf_batch *b, float *grid, int H, int W, int phase_id) {
     const int ty = (H + 31) / 32, tx = (W + 31) / 32;
     k_sample<<<(unsigned)((long long)g.n * ty * tx), 256, 0, b->s>>>(g, b->means, ty, tx);
     GB_CK(cudaGetLastError());
-    return GF_OK;
+    return release(b);
 }
 
 int gf_batch_inject(gf_batch *b, const float *grid, int H, int W) {
@@ -1034,6 +1056,8 @@ int gf_batch_inject(gf_batch *b, const float *grid, int H, int W) {
 int gf_batch_backup(gf_batch *b) {
     if (!b) return GF_ERR_ARG;
     for (const GfMemberView &v : b->views) GB_CK(cudaStreamSynchronize(v.s));
+    const int rc = settle(b);
+    if (rc) return rc;
     if (!b->backup) {
         size_t total = 0;
         b->backup_off.clear();
@@ -1050,12 +1074,14 @@ int gf_batch_backup(gf_batch *b) {
             off += (f.second + 255) & ~(size_t)255;
         }
     }
-    return GF_OK;
+    return release(b);
 }
 
 int gf_batch_restore(gf_batch *b, const int *members, int count) {
     if (!b || (count > 0 && !members)) return GF_ERR_ARG;
     if (!b->backup) return GF_ERR_ARG;
+    const int rc = settle(b);
+    if (rc) return rc;
     for (int k = 0; k < count; ++k) {
         int m = members[k];
         if (m < 0 || m >= (int)b->views.size()) return GF_ERR_ARG;

@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <vector>
 
@@ -52,6 +53,8 @@ struct gf_ctx {
     std::vector<void *> allocs;
     int sweeps = 0; // cap on the thermal sweeps (0: library cap)
     int sync = 1;
+    int pending = 0;                 // the last calls enqueued work that no call has waited for
+    std::shared_ptr<GfEvent> reader; // another stream reads the state until then
     int frc_valid = 0; // e_frc (mixed) / n_frc (FP64) hold the node-force terms of the current stresses and mesh
 };
 
@@ -314,6 +317,21 @@ int move_fields(gf_ctx *c, unsigned m, int dir) {
 // Read and clear the device status word.
 int take_status(gf_ctx *c);
 
+// Start of a call that changes the state.
+int enter(gf_ctx *c) {
+    if (!c) return GF_ERR_ARG;
+    c->pending = 1;
+    if (c->reader) {
+        GF_CK(cudaStreamWaitEvent(c->s, c->reader->e, 0));
+        c->reader.reset();
+    }
+    return GF_OK;
+}
+#define GF_ENTER(c)                                                                                                    \
+    do {                                                                                                               \
+        if (int _rc = enter(c)) return _rc;                                                                            \
+    } while (0)
+
 // Status after a per-subroutine call: waits only in sync mode.
 int call_status(gf_ctx *c) {
     if (!c->sync) {
@@ -328,6 +346,7 @@ int take_status(gf_ctx *c) {
     cudaError_t e = cudaMemcpyAsync(c->pinned, &c->dC->status, sizeof(int), cudaMemcpyDeviceToHost, c->s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->s);
     if (e != cudaSuccess) return cuda_err(e, "step");
+    c->pending = 0;
     const int st = *(const int *)c->pinned;
     if (st) {
         int zero = 0;
@@ -841,7 +860,7 @@ void gf_destroy(gf_ctx *c) {
 }
 
 int gf_upload(gf_ctx *c, unsigned mask) {
-    if (!c) return GF_ERR_ARG;
+    GF_ENTER(c);
     return move_fields(c, mask, 1);
 }
 
@@ -853,6 +872,7 @@ int gf_download(gf_ctx *c, unsigned mask) {
 int gf_set_params(gf_ctx *c, const gf_params *p) {
     if (!c || !p) return GF_ERR_ARG;
     if (p->nx != c->p.nx || p->nz != c->p.nz || p->nphase != c->p.nphase) return GF_ERR_ARG;
+    GF_ENTER(c);
     c->p = *p;
     c->sweeps = p->therm_sweeps;
     DevParams P;
@@ -883,6 +903,7 @@ int gf_set_clock(gf_ctx *c, const gf_clock *k) {
     // be on its way when a batch, on a stream of its own, sets the status word.
     // (The buffer is next written in this stream's order, or by the host after
     // a wait for it.)
+    c->pending = 1;
     constexpr size_t bytes = offsetof(DevClock, r_dlmin);
     static_assert(bytes == 9 * sizeof(double), "the scalars of gf_clock");
     DevClock &C = *(DevClock *)c->pinned;
@@ -919,7 +940,7 @@ int gf_get_clock(gf_ctx *c, gf_clock *k) {
 static int sync_markers_after_resurface(gf_ctx *c);
 
 int gf_fl_therm(gf_ctx *c) {
-    if (!c) return GF_ERR_ARG;
+    GF_ENTER(c);
     const bool magma = c->mode == GF_MODE_FP64 && c->p.itype_melting == 1; // may add markers
     if (magma) GF_CK(cudaMemcpyAsync(c->A.nmarkers, &c->nmarkers, sizeof(int), cudaMemcpyHostToDevice, c->s));
     k_therm(c);
@@ -931,13 +952,13 @@ int gf_fl_therm(gf_ctx *c) {
 }
 
 int gf_change_phase(gf_ctx *c) {
-    if (!c) return GF_ERR_ARG;
+    GF_ENTER(c);
     k_change_phase(c);
     return call_status(c);
 }
 
 int gf_fl_rheol(gf_ctx *c) {
-    if (!c) return GF_ERR_ARG;
+    GF_ENTER(c);
     const gf_params &p = c->p;
     int avg = (c->nsrate == p.ifreq_avgsr) ? 2 : (c->nsrate == -1 ? 1 : 0);
     k_rheol(c, c->nloop % p.ifreq_visc == 0, avg);
@@ -947,13 +968,13 @@ int gf_fl_rheol(gf_ctx *c) {
 }
 
 int gf_fl_node(gf_ctx *c) {
-    if (!c) return GF_ERR_ARG;
+    GF_ENTER(c);
     k_node(c);
     return call_status(c);
 }
 
 int gf_fl_move(gf_ctx *c) {
-    if (!c) return GF_ERR_ARG;
+    GF_ENTER(c);
     if (c->p.movegrid == 0) return GF_OK;
     const bool resurf = c->p.topo_kappa > 0.0 && c->nloop % c->p.ifreq_avgsr == 0;
     if (resurf) GF_CK(cudaMemcpyAsync(c->A.nmarkers, &c->nmarkers, sizeof(int), cudaMemcpyHostToDevice, c->s));
@@ -966,25 +987,25 @@ int gf_fl_move(gf_ctx *c) {
 }
 
 int gf_rmasses(gf_ctx *c) {
-    if (!c) return GF_ERR_ARG;
+    GF_ENTER(c);
     k_rmasses(c);
     return call_status(c);
 }
 
 int gf_dt_mass(gf_ctx *c) {
-    if (!c) return GF_ERR_ARG;
+    GF_ENTER(c);
     k_dt_mass(c);
     return call_status(c);
 }
 
 int gf_init_visc(gf_ctx *c) {
-    if (!c) return GF_ERR_ARG;
+    GF_ENTER(c);
     k_init_visc(c);
     return call_status(c);
 }
 
 int gf_marker2elem(gf_ctx *c) {
-    if (!c) return GF_ERR_ARG;
+    GF_ENTER(c);
     GF_CK(cudaMemcpyAsync(c->A.nmarkers, &c->nmarkers, sizeof(int), cudaMemcpyHostToDevice, c->s));
     GfLaunch g = launch_of(c);
     GfRemeshArgs a = remesh_args(c);
@@ -998,7 +1019,7 @@ int gf_marker2elem(gf_ctx *c) {
 }
 
 int gf_finish_setflac(gf_ctx *c) {
-    if (!c) return GF_ERR_ARG;
+    GF_ENTER(c);
     // xoriginal = cord(:,:,1), zoriginal = cord(:,:,2) (setflac.f90:54-55)
     // (when the host layout does not provide the start-up positions)
     if (!c->L.xoriginal || !c->L.zoriginal)
@@ -1017,7 +1038,7 @@ int gf_finish_setflac(gf_ctx *c) {
 }
 
 int gf_flac(gf_ctx *c) {
-    if (!c) return GF_ERR_ARG;
+    GF_ENTER(c);
     unsigned sig = step_signature(c);
     // the magma sub-model's fl_therm may add markers: the host count is
     // re-read after every call, so that it is current for the next one
@@ -1079,7 +1100,7 @@ template <class R> void restart_fields(gf_ctx *c) {
 extern "C" {
 
 int gf_ctx_restart_finish(gf_ctx *c) {
-    if (!c) return GF_ERR_ARG;
+    GF_ENTER(c);
     int rc;
     GfLaunch g = launch_of(c);
     if (c->mode == GF_MODE_MIXED) {
@@ -1114,6 +1135,19 @@ void gf_ctx_advance(gf_ctx *c, unsigned sig) {
 
 int gf_ctx_take_status(gf_ctx *c) { return take_status(c); }
 
+int gf_ctx_settle(gf_ctx *c, cudaStream_t s, const GfEvent *own) {
+    if (c->pending) GF_CK(cudaStreamSynchronize(c->s));
+    c->pending = 0;
+    if (c->reader && c->reader.get() != own) GF_CK(cudaStreamWaitEvent(s, c->reader->e, 0));
+    return GF_OK;
+}
+
+int gf_ctx_read_until(gf_ctx *c, const std::shared_ptr<GfEvent> &until) {
+    if (c->reader && c->reader != until) GF_CK(cudaStreamWaitEvent(c->s, c->reader->e, 0)); // (two batches)
+    c->reader = until;
+    return GF_OK;
+}
+
 void gf_ctx_invalidate_forces(gf_ctx *c) { c->frc_valid = 0; }
 
 // After a step with resurface or the magma sub-model: the device marker
@@ -1129,6 +1163,7 @@ static int sync_markers_after_resurface(gf_ctx *c) {
 
 int gf_step(gf_ctx *c, int nsteps) {
     if (!c || nsteps < 0) return GF_ERR_ARG;
+    GF_ENTER(c);
     // The magma sub-model's fl_therm may add markers on any step (device
     // count).  Its steps are graph-replayed too; the host copy of the count
     // is brought up to date before a step that uses it (change_phase's
@@ -1198,7 +1233,7 @@ int gf_itest_mesh(gf_ctx *c, double *min_angle) {
 }
 
 int gf_remesh(gf_ctx *c) {
-    if (!c) return GF_ERR_ARG;
+    GF_ENTER(c);
     const int mr = c->p.mode_rem;
     if (!(mr == 1 || mr == 3 || mr == 4 || mr == 11)) return GF_ERR_UNSUPPORTED;
     if (c->p.nx < 4 || c->p.nz < 3) return GF_ERR_UNSUPPORTED; // element-centre grid needs 2 x 3 cells

@@ -377,7 +377,9 @@ int gf_min_angle_noalloc(const double *d_cord, int nx, int nz, void *stream, dou
  * of one member (the reference runs one model per process).  Members are GF_MODE_MIXED contexts that share the step
  * schedule (nloop, nsrate, ifreq_*, itherm); they stay owned by the caller,
  * must outlive the batch, and must not be stepped by other calls while a
- * batch step runs.  Their states stay readable with gf_download. */
+ * batch step runs.  Their states stay readable with gf_download.  Batch calls
+ * wait for what the members' own calls enqueued before, and what those enqueue
+ * after gf_batch_sample or gf_batch_backup waits on the device for these. */
 typedef struct gf_batch gf_batch;
 typedef struct gf_batch_config {
     int threads;          /* threads per CTA: 128, 256 or 512 */
