@@ -320,6 +320,7 @@ int take_status(gf_ctx *c);
 // Start of a call that changes the state.
 int enter(gf_ctx *c) {
     if (!c) return GF_ERR_ARG;
+    (void)cudaGetLastError(); // what others left behind is not this call's
     c->pending = 1;
     if (c->reader) {
         GF_CK(cudaStreamWaitEvent(c->s, c->reader->e, 0));
@@ -332,14 +333,18 @@ int enter(gf_ctx *c) {
         if (int _rc = enter(c)) return _rc;                                                                            \
     } while (0)
 
-// Status after a per-subroutine call: waits only in sync mode.
-int call_status(gf_ctx *c) {
-    if (!c->sync) {
-        cudaError_t e = cudaGetLastError();
-        return e == cudaSuccess ? GF_OK : cuda_err(e, "launch");
-    }
-    return take_status(c);
+// Whether the driver refused a launch since the call's start, or since the last
+// test (the launchers do not look at what each launch returns).
+int refused(const char *what = "launch") {
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? GF_OK : cuda_err(e, what);
 }
+int end_status(gf_ctx *c) {
+    const int rc = refused();
+    return rc ? rc : take_status(c);
+}
+// Status after a per-subroutine call: waits only in sync mode.
+int call_status(gf_ctx *c) { return c->sync ? end_status(c) : refused(); }
 
 int take_status(gf_ctx *c) {
     // (through pinned memory behind the work it reports on: one wait)
@@ -646,18 +651,20 @@ int run_step(gf_ctx *c, unsigned sig) {
     }
     if (!g->exec && ++g->uses < GF_CAPTURE_AFTER) {
         enqueue_step(c, sig);
-        return GF_OK;
+        return refused("step's launch");
     }
     if (!g->exec) {
         cudaGraph_t graph;
         const long long before = c->launches;
         GF_CK(cudaStreamBeginCapture(c->s, cudaStreamCaptureModeThreadLocal));
         enqueue_step(c, sig);
+        const int rc = refused("step's capture");
         GF_CK(cudaStreamEndCapture(c->s, &graph));
-        cudaError_t e = cudaGraphInstantiate(&g->exec, graph, 0);
+        cudaError_t e = rc ? cudaSuccess : cudaGraphInstantiate(&g->exec, graph, 0);
         cudaGraphDestroy(graph);
         g->nlaunch = c->launches - before;
         c->launches = before;
+        if (rc) return rc;
         if (e != cudaSuccess) {
             g->exec = nullptr;
             return cuda_err(e, "cudaGraphInstantiate");
@@ -1015,7 +1022,7 @@ int gf_marker2elem(gf_ctx *c) {
         enqueue_marker2elem<double>(c, g, a);
     GF_CK(cudaMemcpyAsync(&c->nmarkers, c->A.nmarkers, sizeof(int), cudaMemcpyDeviceToHost, c->s));
     GF_CK(cudaStreamSynchronize(c->s));
-    return take_status(c);
+    return end_status(c);
 }
 
 int gf_finish_setflac(gf_ctx *c) {
@@ -1027,7 +1034,7 @@ int gf_finish_setflac(gf_ctx *c) {
     k_rmasses(c);
     if (c->p.ivis_present == 1) k_init_visc(c);
     k_dt_mass(c);
-    int st = take_status(c);
+    int st = end_status(c);
     if (st) return st;
     gf_clock k;
     int rc = gf_get_clock(c, &k);
@@ -1045,10 +1052,9 @@ int gf_flac(gf_ctx *c) {
     const bool resync = (sig & 64u) || (c->mode == GF_MODE_FP64 && c->p.itype_melting == 1);
     if (resync) GF_CK(cudaMemcpyAsync(c->A.nmarkers, &c->nmarkers, sizeof(int), cudaMemcpyHostToDevice, c->s));
     enqueue_step(c, sig);
-    if (resync) {
-        int rc = sync_markers_after_resurface(c);
-        if (rc) return rc;
-    }
+    int rc = refused("step's launch");
+    if (!rc && resync) rc = sync_markers_after_resurface(c);
+    if (rc) return rc;
     advance_host(c, sig);
     return call_status(c);
 }
@@ -1110,12 +1116,12 @@ int gf_ctx_restart_finish(gf_ctx *c) {
         GfRemesh<double>::init_areas(g);
         restart_fields<double>(c);
     }
-    rc = take_status(c);
+    rc = end_status(c);
     if (rc) return rc;
     k_rmasses(c);
     if (c->p.ivis_present == 1) k_init_visc(c);
     k_dt_mass(c);
-    rc = take_status(c);
+    rc = end_status(c);
     if (rc) return rc;
     DevClock C;
     GF_CK(cudaMemcpy(&C, c->dC, sizeof C, cudaMemcpyDeviceToHost));
@@ -1180,7 +1186,8 @@ int gf_step(gf_ctx *c, int nsteps) {
         if (sig & 64u) { // resurface: uncaptured (its seeds use nloop)
             GF_CK(cudaMemcpyAsync(c->A.nmarkers, &c->nmarkers, sizeof(int), cudaMemcpyHostToDevice, c->s));
             enqueue_step(c, sig);
-            int rc = sync_markers_after_resurface(c);
+            int rc = refused("step's launch");
+            if (!rc) rc = sync_markers_after_resurface(c);
             if (rc) return rc;
         } else {
             int rc = run_step(c, sig);
@@ -1192,7 +1199,7 @@ int gf_step(gf_ctx *c, int nsteps) {
         int rc = sync_markers_after_resurface(c);
         if (rc) return rc;
     }
-    return take_status(c);
+    return end_status(c);
 }
 
 int gf_itest_mesh(gf_ctx *c, double *min_angle) {
@@ -1244,7 +1251,7 @@ int gf_remesh(gf_ctx *c) {
     GF_CK(cudaMemcpyAsync(&c->nmarkers, c->A.nmarkers, sizeof(int), cudaMemcpyDeviceToHost, c->s));
     GF_CK(cudaStreamSynchronize(c->s));
     c->need_remeshing = 0;
-    return take_status(c);
+    return end_status(c);
 }
 
 int gf_set_sync(gf_ctx *c, int sync) {
