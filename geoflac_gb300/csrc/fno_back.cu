@@ -594,10 +594,13 @@ __global__ void __launch_bounds__(128) k_fwd_h_bwd(const __grid_constant__ CUten
 // dU[mode][b][(part, i)] = dV[mode][b] times the transposed real block, and
 // the weights' gradient dR[mode][i][o][re, im] from the block gradient
 // M = dV^T U (over all samples): re = M[2o][2i] + M[2o+1][2i+1],
-// im = M[2o+1][2i] - M[2o][2i+1]
+// im = M[2o+1][2i] - M[2o][2i+1].  C2: R's complex values, FP32 or as k_modes kept them.
+__device__ __forceinline__ __nv_bfloat162 bf2(float2 c) { return __floats2bfloat162_rn(c.x, c.y); }
+__device__ __forceinline__ __nv_bfloat162 bf2(__nv_bfloat162 c) { return c; }
+template <class C2>
 __global__ void __launch_bounds__(128) k_modes_bwd(const __grid_constant__ CUtensorMap tmV,
                                                    const __grid_constant__ CUtensorMap tmU,
-                                                   const float *__restrict__ R, __nv_bfloat16 *__restrict__ dU,
+                                                   const C2 *__restrict__ R, __nv_bfloat16 *__restrict__ dU,
                                                    float *__restrict__ dR, int B) {
     extern __shared__ uint8_t dsmem[];
     uint8_t *base = align1k(dsmem);
@@ -622,15 +625,15 @@ __global__ void __launch_bounds__(128) k_modes_bwd(const __grid_constant__ CUten
     };
     if (threadIdx.x == 0) load(0);
     // rows (part, i), columns (o, part')
-    const float2 *w = reinterpret_cast<const float2 *>(R) + (long long)mode * CH * CH;
+    const C2 *w = R + (long long)mode * CH * CH;
 #pragma unroll 4
     for (int k = threadIdx.x; k < CH * CH; k += 128) {
         const int o = k % CH, i = k / CH;
-        const float2 c = w[k];
+        const __nv_bfloat162 c = bf2(w[k]);
         const int col = (2 * o) % 64, off = (((col >> 3) ^ (i & 7)) << 4) + (col & 7) * 2;
         uint8_t *r0 = sR + (o / 32) * 16384 + i * 128 + off;
-        *reinterpret_cast<__nv_bfloat162 *>(r0) = __floats2bfloat162_rn(c.x, c.y);
-        *reinterpret_cast<__nv_bfloat162 *>(r0 + CH * 128) = __floats2bfloat162_rn(-c.y, c.x);
+        *reinterpret_cast<__nv_bfloat162 *>(r0) = c;
+        *reinterpret_cast<__nv_bfloat162 *>(r0 + CH * 128) = __halves2bfloat162(__hneg(c.y), c.x);
     }
     fence_async();
     __syncthreads();
@@ -812,6 +815,19 @@ template <int NA, int ST> int run_wgrad(const CUtensorMap &ma, const CUtensorMap
     k_wgrad<NA, ST><<<a.chunks < cap ? a.chunks : cap, 256, smem, s>>>(ma, mb, a);
     return launched();
 }
+template <class C2>
+int run_modes_bwd(const void *dV, const void *U, const C2 *R, void *dU, float *dR, int B, int modes, void *stream) {
+    if (!dV || !U || !R || !dU || !dR || B < 1 || modes < 1) return GF_FNO_ERR_ARG;
+    if (unaligned(dV) || unaligned(U) || unaligned(R, sizeof(C2)) || unaligned(dU)) return GF_FNO_ERR_ALIGN;
+    CUtensorMap mv, mu;
+    const long long d[3] = {128, B, modes}, st[2] = {128, 128LL * B};
+    const int box[3] = {64, 128, 1};
+    if (!map_of(&mv, dV, 3, d, st, box) || !map_of(&mu, U, 3, d, st, box)) return GF_FNO_ERR_CUDA;
+    const uint32_t smem = 98304 + 64 + 1024;
+    if (!allow_smem(k_modes_bwd<C2>, smem)) return GF_FNO_ERR_CUDA;
+    k_modes_bwd<C2><<<modes, 128, smem, (cudaStream_t)stream>>>(mv, mu, R, (__nv_bfloat16 *)dU, dR, B);
+    return launched();
+}
 bool bad_w(int W) { return W != 128 && W != 256 && W != 384; }
 bool bad_modes(int B, int H, int m2, int Q) {
     return B < 1 || (H != 64 && H != 128) || m2 < 1 || m2 > 32 || Q % 16 || Q < 16 || Q > 64;
@@ -895,16 +911,11 @@ int gf_fno_fwd_h_bwd(const void *dU, const void *FHT, void *dXw, int B, int H, i
 
 int gf_fno_modes_bwd(const void *dV, const void *U, const float *R, void *dU, float *dR, int B, int modes,
                      void *stream) {
-    if (!dV || !U || !R || !dU || !dR || B < 1 || modes < 1) return GF_FNO_ERR_ARG;
-    if (unaligned(dV) || unaligned(U) || unaligned(R, 8) || unaligned(dU)) return GF_FNO_ERR_ALIGN;
-    CUtensorMap mv, mu;
-    const long long d[3] = {128, B, modes}, st[2] = {128, 128LL * B};
-    const int box[3] = {64, 128, 1};
-    if (!map_of(&mv, dV, 3, d, st, box) || !map_of(&mu, U, 3, d, st, box)) return GF_FNO_ERR_CUDA;
-    const uint32_t smem = 98304 + 64 + 1024;
-    if (!allow_smem(k_modes_bwd, smem)) return GF_FNO_ERR_CUDA;
-    k_modes_bwd<<<modes, 128, smem, (cudaStream_t)stream>>>(mv, mu, R, (__nv_bfloat16 *)dU, dR, B);
-    return launched();
+    return run_modes_bwd(dV, U, (const float2 *)R, dU, dR, B, modes, stream);
+}
+int gf_fno_modes_bwd_kept(const void *dV, const void *U, const void *Rb, void *dU, float *dR, int B, int modes,
+                          void *stream) {
+    return run_modes_bwd(dV, U, (const __nv_bfloat162 *)Rb, dU, dR, B, modes, stream);
 }
 
 int gf_fno_wgrad(const void *A, int na, const void *B, int nb, int transposed, float *part, long long M, int chunks,

@@ -578,8 +578,9 @@ __global__ void __launch_bounds__(128) k_inv_h(const __grid_constant__ CUtensorM
 // V[mode][b][(part, o)] = sum over (i, part') of U[mode][b][(i, part')] times
 // the mode's real block, built from R[mode][i][o][re, im]:
 //   out_re = sum_i u_re re - u_im im ; out_im = sum_i u_re im + u_im re
+// Rb: R as it was multiplied by, in BF16, for the backward pass (null: not kept).
 __global__ void __launch_bounds__(128) k_modes(const __grid_constant__ CUtensorMap tmU, const float *__restrict__ R,
-                                               __nv_bfloat16 *__restrict__ V, int B) {
+                                               __nv_bfloat16 *__restrict__ V, __nv_bfloat162 *__restrict__ Rb, int B) {
     extern __shared__ uint8_t dsmem[];
     uint8_t *base = align1k(dsmem);
     uint8_t *sU = base, *sR = base + 32768;
@@ -609,6 +610,7 @@ __global__ void __launch_bounds__(128) k_modes(const __grid_constant__ CUtensorM
         uint8_t *r0 = sR + (i / 32) * 16384 + o * 128 + off; // (CH + o) & 7 == o & 7
         *reinterpret_cast<__nv_bfloat162 *>(r0) = __floats2bfloat162_rn(c.x, -c.y);
         *reinterpret_cast<__nv_bfloat162 *>(r0 + CH * 128) = __floats2bfloat162_rn(c.y, c.x);
+        if (Rb) Rb[(long long)mode * CH * CH + k] = __floats2bfloat162_rn(c.x, c.y);
     }
     fence_async();
     __syncthreads();
@@ -715,17 +717,20 @@ int gf_fno_fwd_h(const void *Xw, const void *FH, void *U, int B, int H, int m2, 
     return launched();
 }
 
-int gf_fno_modes(const void *U, const float *R, void *V, int B, int modes, void *stream) {
+int gf_fno_modes_keep(const void *U, const float *R, void *V, void *Rb, int B, int modes, void *stream) {
     if (!U || !R || !V || B < 1 || modes < 1) return GF_FNO_ERR_ARG;
-    if (unaligned(U) || unaligned(R, 8) || unaligned(V)) return GF_FNO_ERR_ALIGN;
+    if (unaligned(U) || unaligned(R, 8) || unaligned(V) || unaligned(Rb, 4)) return GF_FNO_ERR_ALIGN;
     CUtensorMap mu;
     const long long d[3] = {128, B, modes}, st[2] = {128, 128LL * B};
     const int box[3] = {64, 128, 1};
     if (!map_of(&mu, U, 3, d, st, box)) return GF_FNO_ERR_CUDA;
     const uint32_t smem = 65536 + 64 + 1024;
     if (!allow_smem(k_modes, smem)) return GF_FNO_ERR_CUDA;
-    k_modes<<<modes, 128, smem, (cudaStream_t)stream>>>(mu, R, (__nv_bfloat16 *)V, B);
+    k_modes<<<modes, 128, smem, (cudaStream_t)stream>>>(mu, R, (__nv_bfloat16 *)V, (__nv_bfloat162 *)Rb, B);
     return launched();
+}
+int gf_fno_modes(const void *U, const float *R, void *V, int B, int modes, void *stream) {
+    return gf_fno_modes_keep(U, R, V, nullptr, B, modes, stream);
 }
 
 int gf_fno_inv_h(const void *V, const void *IH, void *Z, int B, int H, int m2, int Q, void *stream) {

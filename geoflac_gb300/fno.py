@@ -59,13 +59,13 @@ def _lib():
         "gf_fno_layer_ok": [i, i, i, i, i, i, i, i],
         "gf_fno_row": [vp, i, vp, vp, vp, vp, i, vp, vp, vp, vp, i, i, i, vp],
         "gf_fno_fwd_h": [vp, vp, vp, i, i, i, i, vp],
-        "gf_fno_modes": [vp, vp, vp, i, i, vp],
+        "gf_fno_modes_keep": [vp, vp, vp, vp, i, i, vp],
         "gf_fno_inv_h": [vp, vp, vp, i, i, i, i, vp],
         "gf_fno_proj": [vp, vp, vp, vp, vp, vp, vp, vp, i, i, vp],
         "gf_fno_proj_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, vp],
         "gf_fno_row_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, vp],
         "gf_fno_inv_h_bwd": [vp, vp, vp, i, i, i, i, vp],
-        "gf_fno_modes_bwd": [vp, vp, vp, vp, vp, i, i, vp],
+        "gf_fno_modes_bwd_kept": [vp, vp, vp, vp, vp, i, i, vp],
         "gf_fno_fwd_h_bwd": [vp, vp, vp, i, i, i, i, vp],
         "gf_fno_wgrad": [vp, i, vp, i, i, vp, ll, i, vp],
     }
@@ -308,20 +308,24 @@ class Fno:
 
         v, Xw = new(M, Cc), new(rows, 2 * m2, Cc)
         self.row(x, cfg.cin, None, wb["lift_w"], self.p["lift_b"], 0, None, v, Xw, rows)
-        saved = {"x": x, "v": [], "z": [], "spec": [], "wb": wb}
+        # the backward pass multiplies by the weights of this pass, whatever becomes
+        # of them in between: BF16 copies (wb, R)
+        saved = {"x": x, "v": [], "z": [], "spec": [], "wb": wb, "R": []}
         vn, V, Z = new(M, Cc), new(cfg.modes, B, 2 * Cc), new(rows, 2 * m2, Cc)
         U = new(cfg.modes, B, 2 * Cc)
         for l in range(cfg.layers):
             last = l == cfg.layers - 1
             zl = new(M, Cc, dtype=torch.float32) if train else None
             _ck(self.lib.gf_fno_fwd_h(_p(Xw), _p(self.mat["FH"]), _p(U), B, H, m2, Q, self.s), "fwd_h")
-            _ck(self.lib.gf_fno_modes(_p(U), _p(self.p[f"R{l}"]), _p(V), B, cfg.modes, self.s), "modes")
+            Rb = new(cfg.modes, Cc, Cc, 2) if train else None
+            _ck(self.lib.gf_fno_modes_keep(_p(U), _p(self.p[f"R{l}"]), _p(V), _p(Rb), B, cfg.modes, self.s), "modes")
             _ck(self.lib.gf_fno_inv_h(_p(V), _p(self.mat["IH"]), _p(Z), B, H, m2, Q, self.s), "inv_h")
             self.row(v, Cc, Z, wb[f"w{l}"], self.p[f"b{l}"], 0 if last else 1, zl, vn, None if last else Xw, rows)
             if train:
                 saved["v"].append(v)
                 saved["z"].append(zl)
                 saved["spec"].append((U, None))
+                saved["R"].append(Rb)
                 v, vn, U = vn, new(M, Cc), new(cfg.modes, B, 2 * Cc)
             else:
                 v, vn = vn, v
@@ -335,12 +339,12 @@ class Fno:
             self.saved = saved
         return out.view(B, H, cfg.W, cfg.cout)
 
-    def modes_t(self, l):
-        """the transposed real blocks of layer l's mode weights (BF16)"""
+    def modes_t(self, R):
+        """the transposed real blocks of a layer's mode weights R (BF16)"""
         n2 = 2 * self.cfg.C
         Rm = self.torch.empty((self.cfg.modes, n2, n2), dtype=self.torch.bfloat16, device="cuda")
         RmT = self.torch.empty_like(Rm)
-        _ck(self.lib.gf_fno_expand_modes(_p(self.p[f"R{l}"]), _p(Rm), _p(RmT), self.cfg.modes, self.cfg.C, self.s),
+        _ck(self.lib.gf_fno_expand_modes(_p(R), _p(Rm), _p(RmT), self.cfg.modes, self.cfg.C, self.s),
             "expand")
         return RmT
 
@@ -392,7 +396,7 @@ class Fno:
         H, W, Cc, m2, Q = cfg.H, cfg.W, cfg.C, cfg.m2, cfg.Q
         bf = torch.bfloat16
         U, RmT = sp
-        RmT = self.modes_t(l) if RmT is None else RmT
+        RmT = self.modes_t(self.saved["R"][l].float()) if RmT is None else RmT
         ds = torch.empty((B, H, Cc, W), dtype=bf, device="cuda")
         self.tr(ds_cl, ds, B * H, W, Cc)
         dZt = torch.empty((B, H, Cc, 2 * m2), dtype=bf, device="cuda")
@@ -458,8 +462,8 @@ class Fno:
             self.colsum(df, self.g[f"b{l}"], M, Cc, blocked=True)
             self.wgrad_fused(dz, Cc, sv["v"][l], Cc, M, self.g[f"w{l}"])
             _ck(lib.gf_fno_inv_h_bwd(_p(dZ), _p(self.mat["IHT"]), _p(dV), B, H, m2, Q, s), "inv_h_bwd")
-            _ck(lib.gf_fno_modes_bwd(_p(dV), _p(sv["spec"][l][0]), _p(self.p[f"R{l}"]), _p(dU), _p(self.g[f"R{l}"]),
-                                     B, cfg.modes, s), "modes_bwd")
+            _ck(lib.gf_fno_modes_bwd_kept(_p(dV), _p(sv["spec"][l][0]), _p(sv["R"][l]), _p(dU), _p(self.g[f"R{l}"]),
+                                          B, cfg.modes, s), "modes_bwd")
             _ck(lib.gf_fno_fwd_h_bwd(_p(dU), _p(self.mat["FHT"]), _p(dXw), B, H, m2, Q, s), "fwd_h_bwd")
             z = sv["z"][l - 1] if l else None
             _ck(lib.gf_fno_row_bwd(_p(dz), _p(dXw), _p(self.mat["FW"]), _p(wb[f"w{l}"]), _p(z), _p(IWT), _p(dn), _p(df),
@@ -478,7 +482,7 @@ class Fno:
         M = B * cfg.H * cfg.W
         bf = torch.bfloat16
         # batches of eight and whole 128-row tiles per chunk of the weight gradients
-        if self.fused and B % 8 == 0 and (M // self.wgrad_chunks(M)) % 128 == 0:
+        if "R" in sv and B % 8 == 0 and (M // self.wgrad_chunks(M)) % 128 == 0:
             return self.backward_fused(dout)
         wb = sv["wb"]
         d2 = dout.reshape(M, cfg.cout)

@@ -119,6 +119,8 @@ int gf_fno_row(const void *v, int kin, const void *Z, const void *IW, const void
                const void *FW, float *z, void *vout, void *Xw, int rows, int W, int K2, void *stream);
 int gf_fno_fwd_h(const void *Xw, const void *FH, void *U, int B, int H, int m2, int Q, void *stream);
 int gf_fno_modes(const void *U, const float *R, void *V, int B, int modes, void *stream);
+/* and keeps R in BF16, Rb[mode][i][o][re, im], as the products took it */
+int gf_fno_modes_keep(const void *U, const float *R, void *V, void *Rb, int B, int modes, void *stream);
 int gf_fno_inv_h(const void *V, const void *IH, void *Z, int B, int H, int m2, int Q, void *stream);
 int gf_fno_proj(const void *v, const void *P1, const float *b1, const void *P2, const float *b2, float *zp, void *h,
                 float *out, int rows, int W, void *stream);
@@ -143,6 +145,9 @@ int gf_fno_row_bwd(const void *dz, const void *dXw, const void *FW, const void *
 int gf_fno_inv_h_bwd(const void *dZ, const void *IHT, void *dV, int B, int H, int m2, int Q, void *stream);
 int gf_fno_modes_bwd(const void *dV, const void *U, const float *R, void *dU, float *dR, int B, int modes,
                      void *stream);
+/* the same from gf_fno_modes_keep's Rb */
+int gf_fno_modes_bwd_kept(const void *dV, const void *U, const void *Rb, void *dU, float *dR, int B, int modes,
+                          void *stream);
 int gf_fno_fwd_h_bwd(const void *dU, const void *FHT, void *dXw, int B, int H, int m2, int Q, void *stream);
 int gf_fno_wgrad(const void *A, int na, const void *B, int nb, int transposed, float *part, long long M, int chunks,
                  void *stream);
