@@ -7,6 +7,7 @@
 // FP64 expression rounds as in the serial Fortran.
 
 #include "gf_kernels.cuh"
+#include "gf_tribox.h"
 
 namespace {
 namespace gfr {
@@ -185,14 +186,9 @@ struct PtGrid {
     __device__ double Y(int j, int i) const { return xy[P + (long long)i * nzt + j]; }
 };
 
-// rem_trpars (remesh.f90:267-320): 6 coefficients per old triangle, and the
-// FP32 box outside which no point has all three barycentric coordinates in
-// (-1e-4, 1 + 1e-4), for the search of k_barcord.  The box is the triangle's,
-// widened by 2 % of its extent L and the rounding of the FP32 copies.  The
-// coordinates that the search evaluates err by less than 1e-3 for triangles
-// with |det| >= 1e-3 L^2 and coordinates up to 1e4 L (their numerators round
-// at 4 2^-53 of the coordinates' squares); any other triangle gets no box.
-__global__ void __launch_bounds__(GF_THREADS) k_trpars(PtGrid g, double *pt, float4 *box) {
+// rem_trpars (remesh.f90:267-320): 6 coefficients per old triangle, and its box
+// for the search of k_barcord.
+__global__ void __launch_bounds__(GF_THREADS) k_trpars(PtGrid g, double *pt, GfTriBox *box) {
     long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long ntri = 2LL * (g.nzt - 1) * (g.nxt - 1);
     if (n >= ntri) return;
@@ -217,16 +213,7 @@ __global__ void __launch_bounds__(GF_THREADS) k_trpars(PtGrid g, double *pt, flo
     q[3] = gf_ddiv_by(gf_mul(x3, y1) - gf_mul(y3, x1), r);
     q[4] = gf_ddiv_by(y3 - y1, r);
     q[5] = gf_ddiv_by(x1 - x3, r);
-    const float f1 = (float)x1, f2 = (float)x2, f3 = (float)x3, h1 = (float)y1, h2 = (float)y2, h3 = (float)y3;
-    float4 b = make_float4(fminf(f1, fminf(f2, f3)), fmaxf(f1, fmaxf(f2, f3)), fminf(h1, fminf(h2, h3)),
-                           fmaxf(h1, fmaxf(h2, h3)));
-    const float X = fmaxf(fmaxf(fabsf(b.x), fabsf(b.y)), fmaxf(fabsf(b.z), fabsf(b.w)));
-    const float L = fmaxf(b.y - b.x, b.w - b.z), m = 0.02f * L + 1e-6f * X;
-    if (fabsf((float)det) >= 1e-3f * L * L && X <= 1e4f * L && L > 1e-15f && X < 1e15f)
-        b = make_float4(b.x - m, b.y + m, b.z - m, b.w + m);
-    else
-        b = make_float4(-INFINITY, INFINITY, -INFINITY, INFINITY);
-    box[n] = b;
+    box[n] = gf_tri_box(x1, x2, x3, y1, y2, y3, det);
 }
 
 __device__ __forceinline__ void weights2(double da, double db, double &wa, double &wb) {
@@ -244,7 +231,7 @@ __device__ __forceinline__ void weights2(double da, double db, double &wa, doubl
 // squares.  Bound before by the FP64 evaluation of some 80 triangles a point
 // (238 us for 48,000 points, 33 to 60 us now).
 __global__ void __launch_bounds__(GF_THREADS) k_barcord(PtGrid old, const double *cnew, const double *pt,
-                                                        const float4 *box, int *numtr, double *bc) {
+                                                        const GfTriBox *box, int *numtr, double *bc) {
     long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int nzt = old.nzt, nxt = old.nxt;
     if (p >= old.P) return;
@@ -254,12 +241,12 @@ __global__ void __launch_bounds__(GF_THREADS) k_barcord(PtGrid old, const double
     const int mm = 4;
     int io0 = max(0, i - mm), io1 = min(nxt - 2, i + mm), jo0 = max(0, j - mm), jo1 = min(nzt - 2, j + mm);
     const float xf = (float)xx, yf = (float)yy;
+    const bool boxed = gf_box_applies(xf, yf);
     for (int io = io0; io <= io1; ++io)
         for (int jo = jo0; jo <= jo1; ++jo)
             for (int k = 1; k <= 2; ++k) {
                 const int n1 = 2 * ((nzt - 1) * io + jo) + k;
-                const float4 b = box[n1 - 1];
-                if (!(xf >= b.x && xf <= b.y && yf >= b.z && yf <= b.w)) continue;
+                if (boxed && !gf_box_holds(box[n1 - 1], xf, yf)) continue;
                 const double *q = pt + (long long)(n1 - 1) * 6;
                 double a1 = q[0] + xx * q[1] + yy * q[2];
                 double a2 = q[3] + xx * q[4] + yy * q[5];
@@ -1158,9 +1145,9 @@ template <class R> void GfRemesh<R>::regrid(const GfLaunch &g, const GfRemeshArg
     int nzt = d.nz - 1, nxt = d.nx - 1;
     GF_RLAUNCH(k_centres, d.E, A, d, b.cold, b.cnew);
     PtGrid ge{b.cold, nzt, nxt, d.E};
-    float4 *box = (float4 *)event_scratch(A); // two triangles of 16 bytes per element
+    GfTriBox *box = (GfTriBox *)event_scratch(A); // two triangles of 16 bytes per element
     GF_RLAUNCH(k_trpars, 2LL * (nzt - 1) * (nxt - 1), ge, b.pt, box);
-    GF_RLAUNCH(k_barcord, d.E, ge, (const double *)b.cnew, (const double *)b.pt, (const float4 *)box, b.numtr, b.bc);
+    GF_RLAUNCH(k_barcord, d.E, ge, (const double *)b.cnew, (const double *)b.pt, (const GfTriBox *)box, b.numtr, b.bc);
     interp_planes<R>(g, b, (R *)A.stress0, 16, nzt, d.E, 0);
     if (sizeof(R) == sizeof(float)) interp_planes<double>(g, b, A.p_ref, 1, nzt, d.E, 0);
     interp_planes<R>(g, b, (R *)A.strain, 3, nzt, d.E, 0);
@@ -1177,7 +1164,7 @@ template <class R> void GfRemesh<R>::regrid(const GfLaunch &g, const GfRemeshArg
     cudaMemcpyAsync(A.temp0, A.temp, sizeof(double) * d.N, cudaMemcpyDeviceToDevice, g.s);
     PtGrid gn{A.cord_old, d.nz, d.nx, d.N};
     GF_RLAUNCH(k_trpars, 2LL * (d.nz - 1) * (d.nx - 1), gn, b.pt, box);
-    GF_RLAUNCH(k_barcord, d.N, gn, (const double *)A.cord, (const double *)b.pt, (const float4 *)box, b.numtr, b.bc);
+    GF_RLAUNCH(k_barcord, d.N, gn, (const double *)A.cord, (const double *)b.pt, (const GfTriBox *)box, b.numtr, b.bc);
     interp_planes<double>(g, b, A.vel, 2, d.nz, d.N, 0);
     interp_planes<double>(g, b, A.temp, 1, d.nz, d.N, 0);
     // xoriginal, zoriginal (remesh.f90:242-243)
