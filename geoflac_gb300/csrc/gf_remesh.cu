@@ -246,7 +246,8 @@ __global__ void __launch_bounds__(GF_THREADS) k_barcord(PtGrid old, const double
         for (int jo = jo0; jo <= jo1; ++jo)
             for (int k = 1; k <= 2; ++k) {
                 const int n1 = 2 * ((nzt - 1) * io + jo) + k;
-                if (boxed && !gf_box_holds(box[n1 - 1], xf, yf)) continue;
+                const float4 b = reinterpret_cast<const float4 *>(box)[n1 - 1]; // (one load)
+                if (boxed && !gf_box_holds(GfTriBox{b.x, b.y, b.z, b.w}, xf, yf)) continue;
                 const double *q = pt + (long long)(n1 - 1) * 6;
                 double a1 = q[0] + xx * q[1] + yy * q[2];
                 double a2 = q[3] + xx * q[4] + yy * q[5];
