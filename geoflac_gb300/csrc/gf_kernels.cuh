@@ -244,7 +244,9 @@ __device__ __forceinline__ double gf_neg(double x) {
 // twice the exact residual Ma 2^k - Mb q (below 2^55, so its low 64 bits
 // are exact) against +-Mb decides (no ties: a quotient of two 53-bit
 // significands is never halfway between two 53-bit values).  Restated on words and checked
-// against IEEE division by tests/test_int_reciprocal.py.
+// against IEEE division, as the device evaluates it too, by tests/test_int_quotient.py.
+// (tests/test_int_reciprocal.py restates a quotient with a truncated estimate and
+// two steps each way; tests/test_division.py one from an FP64 reciprocal.)
 __device__ __noinline__ double gf_ddiv_rare(double a, double b) { return a / b; }
 // The denominator's part of gf_ddiv, for quotients that share it: its
 // significand, t = RN(2^105 / Mb) and whether b lies inside gf_dmid.
@@ -293,7 +295,8 @@ __device__ __forceinline__ float gf_ddiv(float a, float b) { return a / b; }
 
 // gf_mul for kernels with many products (the rheology): a zero operand takes
 // the FP64 multiply out of line as well, which leaves one range test for
-// both operands and no select on the result (38 -> 30 instructions)
+// both operands and no select on the result (38 -> 30 instructions).  Checked by
+// tests/test_int_quotient.py.
 __device__ __forceinline__ double gf_mulq(double a, double b) {
     unsigned la, ha, lb, hb;
     gf_dsplit(a, la, ha);

@@ -15,7 +15,7 @@
 // the four triangles) and added there, one component per lane.
 // Measured against one thread per element (CUDA events): fl_rheol 546 ->
 // 463 us on 1000x300 elements (152 FP64 warp instructions and 5,950 in all
-// per eight elements; the FP64 pipe 64 % busy), 225 -> 184 us on 600x150,
+// per eight elements; the FP64 pipe 66 % busy), 225 -> 184 us on 600x150,
 // 106 -> 51 us on 241x61, 91 -> 43 us on 60x20; fl_move 84 -> 78, 40 -> 31,
 // 25 -> 14 and 21 -> 12 us.  Every size gains, so there is no other variant.
 #pragma once
