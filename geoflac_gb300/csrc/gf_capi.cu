@@ -1204,6 +1204,7 @@ int gf_step(gf_ctx *c, int nsteps) {
 
 int gf_itest_mesh(gf_ctx *c, double *min_angle) {
     if (!c) return GF_ERR_ARG;
+    (void)cudaGetLastError(); // (as in enter)
     const gf_params &p = c->p;
     const int nx = p.nx;
     // everything the test reads comes back in one copy (seven small ones cost
@@ -1212,6 +1213,7 @@ int gf_itest_mesh(gf_ctx *c, double *min_angle) {
     ++c->launches;
     GfLaunch g = launch_of(c);
     GfKernels<double>::min_angle(g, c->d_angle);
+    if (int rc = refused("mesh test's launch")) return rc; // (what is there would be the last call's answer)
     GF_CK(cudaMemcpyAsync(c->pinned, c->d_angle, sizeof(double) * (5 + 2 * (size_t)nx), cudaMemcpyDeviceToHost, c->s));
     GF_CK(cudaStreamSynchronize(c->s));
     const double *h = (const double *)c->pinned;
