@@ -607,8 +607,9 @@ int build_tables(gf_batch *b) {
     b->ipt = c.items_per_thread;
     while (b->ipt > 1 && b->elements < (long long)b->sms * 2048 * b->ipt) --b->ipt;
     const long long tile = (long long)c.threads * b->ipt;
+    std::vector<int2> tiles[K_KINDS]; // until their copies end
     for (int kind = 0; kind < K_KINDS; ++kind) {
-        std::vector<int2> t;
+        std::vector<int2> &t = tiles[kind];
         for (size_t m = 0; m < b->views.size(); ++m) {
             long long n = kind_count(b->views[m], kind);
             for (long long s = 0; s < n; s += tile) {
@@ -621,9 +622,12 @@ int build_tables(gf_batch *b) {
         b->ntile[kind] = (int)t.size();
         if (!t.empty()) {
             GB_CK(cudaMalloc(&b->d_tiles[kind], t.size() * sizeof(int2)));
-            GB_CK(cudaMemcpy(b->d_tiles[kind], t.data(), t.size() * sizeof(int2), cudaMemcpyHostToDevice));
+            GB_CK(cudaMemcpyAsync(b->d_tiles[kind], t.data(), t.size() * sizeof(int2), cudaMemcpyHostToDevice, b->s));
         }
     }
+    // (a plain copy from pageable memory may return before it has landed, and is not
+    // in the order of a non-blocking stream)
+    GB_CK(cudaStreamSynchronize(b->s));
     b->grid = b->ntile[K_E];
     drop_graphs(b);
     return GF_OK;
@@ -652,7 +656,9 @@ std::vector<BatchMember> member_records(const gf_batch *b) {
 }
 int upload_members(gf_batch *b) {
     b->records = member_records(b);
-    GB_CK(cudaMemcpy(b->d_members, b->records.data(), b->records.size() * sizeof(BatchMember), cudaMemcpyHostToDevice));
+    GB_CK(cudaMemcpyAsync(b->d_members, b->records.data(), b->records.size() * sizeof(BatchMember),
+                          cudaMemcpyHostToDevice, b->s));
+    GB_CK(cudaStreamSynchronize(b->s)); // (as in build_tables)
     return GF_OK;
 }
 

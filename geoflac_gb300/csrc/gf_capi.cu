@@ -884,8 +884,10 @@ int gf_set_params(gf_ctx *c, const gf_params *p) {
     c->sweeps = p->therm_sweeps;
     DevParams P;
     fill_params(P, *p);
+    // (in the stream's order: a plain copy from pageable memory may return before it
+    // has landed, and no wait for this stream, a batch's neither, would cover it)
+    GF_CK(cudaMemcpyAsync(c->dP, &P, sizeof P, cudaMemcpyHostToDevice, c->s));
     GF_CK(cudaStreamSynchronize(c->s));
-    GF_CK(cudaMemcpy(c->dP, &P, sizeof P, cudaMemcpyHostToDevice));
     if (c->mode == GF_MODE_FP64)
         GfKernels<double>::plastic_table(launch_of(c));
     else
